@@ -44,19 +44,28 @@
 //     rows are zero-filled and their weight is exactly 0 (NaN-safe, decode_v2_kernel.cuh:262-278).
 //
 // Warp roles (768 threads per CTA):
-//   warps 0-7    softmax + epilogue + Q quantisation (thread = one head x 32 tokens of a tile; the four
-//                warps that share 32 heads exchange row maxima through shared memory).
-//   warps 8-15   gather: warp g reads rows [8 g, +8) of the CTA's 64 from a raw stage (the rows as they
-//                lie in the cache) into registers, takes the largest of their scales as the scale of its
-//                group, every lane shifts its pieces and stores them in the layout the MMAs read.  The
-//                gather warps never wait for each other.
-//   warp 16      lane 0 issues the score MMAs, warp 17 lane 0 the P.V MMAs -- in the even CTA only, which
+//   warps 0-7    softmax + epilogue + Q quantisation (thread = one head x 32 tokens of a tile).  The four warps that
+//                share 32 heads meet at one barrier per tile that also ORs "some row has outgrown its running
+//                maximum": only then, rarely after a request's first tiles, they exchange the partial row maxima.
+//                A score costs a comparison, half a packed FMA, an exponential and half a packed addition.
+//   warps 8-15   gather: warp g reads group g of eight rows of every tile of the CTA from a raw slot (the rows as
+//                they lie in the cache) into registers, takes the largest of their scales as the scale of the
+//                group, every lane shifts its pieces and stores them in the layout the MMAs read.  The gather
+//                warps never wait for each other.
+//   warp 16      issues the score MMAs, warp 17 the P.V MMAs (one elected lane) -- in the even CTA only, which
 //                is also where the barriers that collect arrivals from both CTAs live.  Completion of
 //                MMAs reaches both CTAs through one tcgen05.commit per CTA.
-//   warp 19      lane 0 issues the bulk copies K stage -> V slots (own and partner's), sends the half
-//                tile's scale records to the partner, waits for the V slots of its CTA to fill and passes
-//                that on (V full to the even CTA, K stage free to both).
-//   warps 20-23  copy issuers: one bulk copy global -> raw stage per row, two tiles ahead.
+//   warp 18      sends the half tile's scale records to the partner as soon as they are complete.
+//   warp 19      issues the bulk copies K stage -> V slots (own and partner's), waits for the V slots of its CTA
+//                to fill and passes that on (V full to the even CTA, K stage free to both).
+//   warps 20-23  copy issuers: one bulk copy global -> raw slot per row, refilled as soon as the slot has been read.
+// What bounds it (4096 query tokens, top-k 2048, per 128-token tile of about 4400 cycles): issue slots 48 % busy, the
+// integer pipe 46 % (exponent shifts), tensor pipe 25 %, shared memory about half; the chains gather -> scores -> softmax ->
+// P.V are latency-bound.  Two V stages (paid for by raw slots of one tile instead of two) let the K -> V copies of a
+// tile run under the P.V of the one before, the records no longer wait behind those copies, and MMAs issued under an
+// elected lane take 500 cycles per tile instead of 1800: 64 requests 52.7 -> 49.3 us.  Measured and not kept: rows
+// loaded straight into gather registers (8, 12 or 16 warps: 54 / 59 / 70 us), 16-byte asynchronous copies from the copy
+// warps instead of bulk copies (49.8 us, prefill 7 % slower), eight copy warps (51.3 us).
 // Every wait is bounded; a wait that gives up records a code in status[] and the CTA drains and
 // exits.  Warps that meet at a named barrier leave the loop together (a warp whose wait gave up
 // still goes to the next named barrier, where all of them see the flag).
@@ -71,24 +80,25 @@ using namespace ptx;
 using namespace attn;
 
 constexpr int N_SM_WARPS = 8, N_G_WARPS = 8;
-constexpr int RPW = 64 / N_G_WARPS;     // rows of a tile per gather warp
+constexpr int RPW = 8, N_GROUPS = 64 / RPW;     // rows of a group; groups of a CTA's half tile
 constexpr int MMA_WARP = N_SM_WARPS + N_G_WARPS;
-constexpr int FWD_WARP = MMA_WARP + 3;
-constexpr int PROD_WARP0 = MMA_WARP + 4, N_P_WARPS = 4;      // copy issuers: warp p looks after the rows of gather warps 2 p and 2 p + 1
+constexpr int INFO_WARP = MMA_WARP + 2, FWD_WARP = MMA_WARP + 3;
+constexpr int PROD_WARP0 = MMA_WARP + 4, N_P_WARPS = 4;      // copy issuers
 constexpr int PAIR_THREADS = (PROD_WARP0 + N_P_WARPS) * 32;
 // Register budgets after the warpgroups trade registers.  setmaxnreg.inc can only draw on what the CTA
 // was launched with (PAIR_THREADS x REGS_LAUNCH), so the budgets must fit it or the increase would block
 // for ever; the launcher checks the compiled register count against REGS_LAUNCH before it launches.
 // A gather thread keeps 8 + 2 sixteen-byte pieces in flight; the MMA-issuing and copy threads need few
 // registers, so their warpgroup gives up more than half of its allocation.
-constexpr int REGS_LAUNCH = 80, REGS_SOFTMAX = 120, REGS_GATHER = 80, REGS_MMA = 40, REGS_PROD = 40;
+constexpr int REGS_LAUNCH = 80, REGS_SOFTMAX = 128, REGS_GATHER = 72, REGS_MMA = 40, REGS_PROD = 40;
 static_assert(N_SM_WARPS * 32 * REGS_SOFTMAX + N_G_WARPS * 32 * REGS_GATHER + 128 * REGS_MMA + N_P_WARPS * 32 * REGS_PROD
                   <= PAIR_THREADS * REGS_LAUNCH, "register budgets exceed what the CTA owns");
 static_assert(65536 / PAIR_THREADS / 8 * 8 == REGS_LAUNCH, "launch-time registers per thread");
 
 constexpr int TILE_N = 128;            // tokens per tile: two scheduler blocks, 64 rows gathered by each CTA
 constexpr int OWN_N = 64;
-constexpr int NK = 2, NV = 1, NR = 2;  // K stages (own rows, MMA layout), V stages (V slots), raw stages (own rows as they lie in the cache)
+constexpr int NK = 2, NV = 2, NR = N_G_WARPS; // K stages (own rows, MMA layout), V stages (V slots), raw slots (groups of eight rows as they lie in the cache)
+static_assert(NR % N_G_WARPS == 0, "a raw slot is always read by the same gather warp: parity waits must not run a phase ahead");
 constexpr int P_SHIFT = 5;             // P' is stored as e4m3(P' * 2^P_SHIFT)
 constexpr float RESCALE_TAU = 3.0f;    // lazy-rescale threshold (log2 units); P' <= 2^TAU
 
@@ -102,10 +112,10 @@ constexpr uint32_t KS_BYTES = KS_ROPE + CHUNK;       // 40960
 constexpr uint32_t VS_OFF = KS_OFF + NK * KS_BYTES;  // V stages
 constexpr uint32_t VSLOT = 32 * 128;                 //   slot (kb, nb): 32 tokens x 128 dims, at (4 nb + kb) * VSLOT
 constexpr uint32_t VS_BYTES = 8 * VSLOT;             // 32768
-constexpr uint32_t RAW_OFF = VS_OFF + NV * VS_BYTES; // raw stages: [64 rows x 656 B] as they lie in the cache
-constexpr uint32_t RAW_BYTES = OWN_N * ROW_BYTES;    // 41984
+constexpr uint32_t RAW_OFF = VS_OFF + NV * VS_BYTES; // raw slots: [8 rows x 656 B] as they lie in the cache
+constexpr uint32_t RAW_BYTES = RPW * ROW_BYTES;      // 5248
 constexpr int INFO_RING = 8;                         // half-tile records outlive their K stage: the softmax reads them after the scores
-constexpr uint32_t INFO_HALF = N_G_WARPS * 16;       // a half tile's record: per gather warp (s, log2 s, 1/s, validity bits) of its RPW rows
+constexpr uint32_t INFO_HALF = N_GROUPS * 16;        // a half tile's record: per group (s, log2 s, 1/s, validity bits) of its RPW rows
 constexpr uint32_t INFO_OFF = RAW_OFF + NR * RAW_BYTES;  // [INFO_RING][2 halves] x INFO_HALF
 constexpr uint32_t XCH_OFF = INFO_OFF + INFO_RING * 2 * INFO_HALF; // row-maximum exchange [2][4][64] fp32, then Q scales [64] fp32
 constexpr uint32_t XCH_BYTES = 2 * 4 * 64 * 4 + 64 * 4;
@@ -115,7 +125,7 @@ constexpr int BAR_KSTORED = 0, BAR_KFULLP = BAR_KSTORED + NK, BAR_KEMPTY = BAR_K
               BAR_VFULL = BAR_KEMPTY + NK, BAR_VFULLP = BAR_VFULL + NV, BAR_VEMPTY = BAR_VFULLP + NV,
               BAR_INFO = BAR_VEMPTY + NV, BAR_SREADY = BAR_INFO + INFO_RING, BAR_SFREEP = BAR_SREADY + 2,
               BAR_PREADYP = BAR_SFREEP + 2, BAR_PVDONE = BAR_PREADYP + 2, BAR_QREADYP = BAR_PVDONE + 2,
-              BAR_RAWFULL = BAR_QREADYP + 1, BAR_RAWEMPTY = BAR_RAWFULL + NR * N_P_WARPS, BAR_QSTAGE = BAR_RAWEMPTY + NR * N_P_WARPS,
+              BAR_RAWFULL = BAR_QREADYP + 1, BAR_RAWEMPTY = BAR_RAWFULL + NR, BAR_QSTAGE = BAR_RAWEMPTY + NR,
               BAR_QFREE = BAR_QSTAGE + 1, NBAR = BAR_QFREE + 1;
 constexpr uint32_t MISC_OFF = BAR_OFF + NBAR * 8;    // tmem base (4 B), abort flag (4 B)
 constexpr uint32_t SMEM_BYTES = MISC_OFF + 16;
@@ -123,7 +133,7 @@ constexpr uint32_t SMEM_ALLOC = SMEM_BYTES + 1024;   // slack for the 1024-byte 
 static_assert(SMEM_ALLOC <= 227 * 1024, "shared memory budget");
 static_assert(KS_BYTES % 1024 == 0 && VS_BYTES % 1024 == 0 && KS_OFF % 1024 == 0, "swizzled tiles need 1024-byte alignment");
 constexpr uint32_t QSTAGE_OFF = KS_OFF + KS_BYTES;   // the staged Q rows of the first request: K stage 1 and the V stage behind it
-static_assert(NK == 2 && (NK - 1) * KS_BYTES + NV * VS_BYTES >= OWN_N * D_QK * 2, "K stage 1 + V stage hold the staged Q rows of a CTA");
+static_assert(NK == 2 && KS_BYTES + VS_BYTES >= OWN_N * D_QK * 2, "K stage 1 + the first V stage hold the staged Q rows of a CTA");
 static_assert(RPW == 8, "a softmax thread reads the records of four groups of eight tokens");
 static_assert(BAR_OFF % 8 == 0 && INFO_OFF % 16 == 0 && RAW_OFF % 16 == 0 && RAW_BYTES % 16 == 0, "alignment of barriers and bulk-copied records");
 
@@ -143,14 +153,17 @@ enum { W_QSTAGE = 33, W_QFREE = 34, W_RAWEMPTY = 35, W_RAWFULL = 36, W_KEMPTY = 
 // Timeline of one CTA (instrumented builds only): lane 0 of every warp appends (tag, tile, clock) records.
 __device__ long long* g_trace_buf = nullptr;   // [warps][cap][2]
 __device__ int g_trace_cap = 0;
-struct TraceCursor { int n = 0; };
 __device__ int g_trace_block = 0;
+struct TraceCursor { long long* at = nullptr; };     // looked up once: a trace point is a clock read and a store
+__device__ __forceinline__ void trace_open(TraceCursor& c) {
+    if (g_trace_buf != nullptr && (int)blockIdx.x == g_trace_block && (threadIdx.x & 31) == 0)
+        c.at = g_trace_buf + (size_t)(threadIdx.x >> 5) * g_trace_cap * 2;
+}
 __device__ __forceinline__ void trace(TraceCursor& c, int tag, int tile) {
-    if (g_trace_buf != nullptr && (int)blockIdx.x == g_trace_block && (threadIdx.x & 31) == 0 && c.n < g_trace_cap) {
-        long long* slot = g_trace_buf + ((size_t)(threadIdx.x >> 5) * g_trace_cap + c.n) * 2;
-        slot[0] = ((long long)tag << 32) | (unsigned)tile;
-        slot[1] = clock64();
-        ++c.n;
+    if (c.at != nullptr) {
+        c.at[0] = ((long long)tag << 32) | (unsigned)tile;
+        c.at[1] = clock64();
+        c.at += 2;
     }
 }
 #ifdef SMLA_TRACE_FROM             // only the trace points with tags in [SMLA_TRACE_FROM, SMLA_TRACE_TO): the other roles keep their registers
@@ -219,6 +232,33 @@ __device__ __forceinline__ int tile_entry(const AttnParams& p, const Work& w, in
     return (j < nst && pos < lim) ? __ldg(p.indices + (size_t)w.req * p.topk + pos) : -1;
 }
 
+// A partition's rows as one sequence of groups of eight (eight groups per tile of a CTA, the tiles of all its requests
+// one after the other), walked in increasing order by a warp that takes every n-th of them.
+struct Entry { int idx; bool have, extra; };    // index of a row (-1: no entry), whether the group exists, whether it is the second cache's
+template <bool EXTRA>
+struct ItemWalk {
+    Work w;
+    int req, nst;          // the request that the walk has reached and its number of tiles
+    uint32_t base;         // number of its first tile
+    __device__ __forceinline__ explicit ItemWalk(int begin_req) : req(begin_req - 1), nst(0), base(0u) {}
+    __device__ __forceinline__ Entry entry(const AttnParams& p, const SchedMeta& meta, int last_req, uint32_t item, int rank, int r) {
+        const uint32_t t = item / N_GROUPS;
+        Entry e;
+        e.idx = -1; e.have = false; e.extra = false;
+        while (t >= base + (uint32_t)nst) {
+            base += (uint32_t)nst;
+            nst = 0;
+            do { if (++req > last_req) { req = last_req; return e; } } while (!get_work(p, meta, req, w));
+            nst = (w.nblk + 1) >> 1;
+        }
+        const int j = (int)(t - base);
+        e.have = true;
+        e.idx = tile_entry<EXTRA>(p, w, j, rank, (int)(item % N_GROUPS) * RPW + r, nst, min(w.len, (w.blk0 + w.nblk) * BLOCK_N));
+        if (EXTRA) e.extra = w.blk0 + 2 * j + rank >= w.main_blocks;
+        return e;
+    }
+};
+
 // STAGE_Q: the Q rows of a partition's first request come in by one bulk copy into shared memory (see below) instead
 // of being read from global memory by the softmax warps (after an L2 prefetch that the copy warps issue as soon as the
 // partition is known).  The copy wins where the kernel follows the scheduler and partitions are short (one request
@@ -240,6 +280,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) att
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 #ifdef SMLA_TRACE
     TraceCursor tcur;
+    trace_open(tcur);
 #endif
 #ifdef SMLA_PROF
     unsigned prof_acc = 0;
@@ -256,9 +297,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) att
         mbar_init(bar(BAR_QSTAGE), 1);
         mbar_init(bar(BAR_QFREE), 2 * N_SM_WARPS);   // both CTAs' softmax warps: the partner's copies land in this CTA's V stage too
         for (int s = 0; s < NK; ++s) {
-            mbar_init(bar(BAR_KSTORED + s), N_G_WARPS);          // this CTA's rows of the stage are in shared memory
-            mbar_init(bar(BAR_KFULLP + s), 2 * N_G_WARPS);       // both CTAs' rows are
-            mbar_init(bar(BAR_KEMPTY + s), 3);                   // the score MMAs have read the stage; both CTAs' V slots hold its copies
+            mbar_init(bar(BAR_KSTORED + s), N_GROUPS);          // this CTA's rows of the stage are in shared memory
+            mbar_init(bar(BAR_KFULLP + s), 2 * N_GROUPS);       // both CTAs' rows are
+            mbar_init(bar(BAR_KEMPTY + s), 4);                   // the score MMAs have read the stage; both CTAs' V slots hold its copies; its records are on their way
         }
         for (int s = 0; s < NV; ++s) {
             mbar_init(bar(BAR_VFULL + s), 1);                    // + the bytes of the four quarter tiles copied into this CTA's slots
@@ -266,9 +307,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) att
             mbar_init(bar(BAR_VEMPTY + s), 1);
         }
         for (int s = 0; s < INFO_RING; ++s) mbar_init(bar(BAR_INFO + s), 1);   // + the bytes of the partner's record
-        for (int s = 0; s < NR * N_P_WARPS; ++s) {
-            mbar_init(bar(BAR_RAWFULL + s), 1);        // + the bytes of a copy warp's 16 rows of a raw stage
-            mbar_init(bar(BAR_RAWEMPTY + s), 16 / RPW); // the gather warps that read these 16 rows have them in registers
+        for (int s = 0; s < NR; ++s) {
+            mbar_init(bar(BAR_RAWFULL + s), 1);        // + the bytes of the slot's rows
+            mbar_init(bar(BAR_RAWEMPTY + s), 1);       // the gather warp has them in registers
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(bar(BAR_SREADY + b), 1);
@@ -342,6 +383,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) att
         float* sqv = xch + 2 * 4 * 64;                         // [64]
         const bool wide_out = (reinterpret_cast<size_t>(p.out) & 31) == 0;        // rows are 1024 bytes apart
         const bool wide_acc = (reinterpret_cast<size_t>(p.o_accum) & 31) == 0;
+        // The sign of the softmax scale goes into Q, so that scores are always multiplied by a positive number.
+        const uint32_t scale_sign = __float_as_uint(p.sm_scale) & 0x80000000u;
         uint32_t it = 0;                                  // running tile counter of this CTA
         bool dead = false;                                // a wait of this warp gave up: no more work, only barriers
         bool stop = false;
@@ -425,8 +468,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) att
                     am_a = fmaxf(am_a, xch[(1 - ch) * 64 + r_a]);
                     am_b = fmaxf(am_b, xch[(1 - ch) * 64 + r_b]);
                     const float sq_a = pow2_ceil(fmaxf(am_a, 1e-4f) * (1.f / 448.f)), sq_b = pow2_ceil(fmaxf(am_b, 1e-4f) * (1.f / 448.f));
-                    const float ia = __uint_as_float(0x7f000000u - __float_as_uint(sq_a));   // 1/sq, sq a power of two
-                    const float ib = __uint_as_float(0x7f000000u - __float_as_uint(sq_b));
+                    const float ia = __uint_as_float((0x7f000000u - __float_as_uint(sq_a)) | scale_sign);   // 1/sq, sq a power of two
+                    const float ib = __uint_as_float((0x7f000000u - __float_as_uint(sq_b)) | scale_sign);
                     if (c4 == 0) { sqv[r_a] = sq_a; sqv[r_b] = sq_b; }
                     if (!dead) {
 #pragma unroll
@@ -455,7 +498,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) att
                         uint4 c = make_uint4(0, 0, 0, 0);
                         if (hr < heads_cta && head0 + hr < p.num_heads)
                             c = *reinterpret_cast<const uint4*>(qrows + (size_t)(head0 + hr) * L::QD + L::NOPE + (lane & 7) * 8);
-                        const __nv_bfloat162 f = __float2bfloat162_rn(__uint_as_float(0x7f000000u - __float_as_uint(sqv[hr])));   // 1/sq
+                        const __nv_bfloat162 f = __float2bfloat162_rn(__uint_as_float((0x7f000000u - __float_as_uint(sqv[hr])) | scale_sign));   // 1/sq
                         c.x = mul_bf16x2(c.x, f); c.y = mul_bf16x2(c.y, f); c.z = mul_bf16x2(c.z, f); c.w = mul_bf16x2(c.w, f);
                         *reinterpret_cast<uint4*>(sm + QR_OFF + swz((uint32_t)hr, (uint32_t)lane & 7u)) = c;
                     }
@@ -483,7 +526,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) att
                 for (int i = tid; i < lines; i += N_SM_WARPS * 32)
                     asm volatile("prefetch.global.L2 [%0];" ::"l"(qn + (size_t)i * 128));
             }
-            my_sqc = live ? sqv[hrow] * p.sm_scale * LOG2E : 0.f;
+            my_sqc = live ? sqv[hrow] * fabsf(p.sm_scale) * LOG2E : 1.f;
             __syncwarp();
             if (lane == 0) mbar_arrive_remote(barp(BAR_QREADYP));
 
@@ -606,9 +649,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) att
             float x_max = -INFINITY;   // this thread's share of the maximum of the scaled logits (max_logits output)
             for (int j = 0; j < nst; ++j, ++it) {
                 const uint32_t b = it & 1u;
-                float z[32];
+                uint32_t sv[32];                           // raw scores; -inf where there is no entry
                 float mx_loc = -INFINITY;
-                float inv_g[4] = {0.f, 0.f, 0.f, 0.f};     // 1/s of the four groups of eight tokens that this thread holds
+                float c_g[4], off_g[4], inv_g[4];          // of the four groups of eight tokens that this thread holds: z = s * c + off, 1/s
                 // the records of this thread's 32 tokens: half tile thalf, gather warps [4 ch, 4 ch + 4)
                 const uint8_t* info = sm + INFO_OFF + (it & (INFO_RING - 1)) * (2 * INFO_HALF) + thalf * INFO_HALF + ch * 64;
                 PROF(0);
@@ -619,43 +662,49 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) att
                 PROF(2);
                 if (!dead) {
                     tc_fence_after();
-                    uint32_t sv[32];
                     tmem_ld32(lane_addr + TM_S + 64 * b + 32 * ch, sv);
-                    tmem_wait_ld();
-                    PROF(3);
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive_remote(barp(BAR_SFREEP + b));   // the score buffer may be overwritten
                     uint32_t valid = 0u;
-                    float mx0 = -INFINITY, mx1 = -INFINITY;
 #pragma unroll
                     for (int g = 0; g < 4; ++g) {
                         const float4 ti = *reinterpret_cast<const float4*>(info + 16 * g);    // (s, log2 s, 1/s, validity bits) of the group
-                        const float c_g = ti.x * my_sqc, off = ti.y;
+                        const uint32_t vb = __float_as_uint(ti.w) & 0xffu;
+                        c_g[g] = vb != 0u ? ti.x * my_sqc : 1.f;       // positive: the largest score of a group is its largest logit
+                        off_g[g] = ti.y;
                         inv_g[g] = ti.z;
-                        valid |= (__float_as_uint(ti.w) & 0xffu) << (8 * g);
-                        float gm = -INFINITY;
-#pragma unroll
-                        for (int t = 8 * g; t < 8 * g + 8; ++t) {
-                            z[t] = fmaf(__uint_as_float(sv[t]), c_g, off);
-                            if (!((__float_as_uint(ti.w) >> (t - 8 * g)) & 1u)) z[t] = -INFINITY;   // no entry: weight exactly 0
-                            gm = fmaxf(gm, z[t]);
-                        }
-                        // z - log2(s) is the scaled logit itself
-                        if (p.out_max_logits != nullptr && gm > -INFINITY) x_max = fmaxf(x_max, gm - off);
-                        if (g & 1) mx1 = fmaxf(mx1, gm); else mx0 = fmaxf(mx0, gm);
+                        valid |= vb << (8 * g);
                     }
-                    (void)valid;
-                    mx_loc = fmaxf(mx0, mx1);
-                    xch[(b * 4 + xpart) * 64 + hrow] = mx_loc;
+                    tmem_wait_ld();
+                    PROF(3);
+                    TRACE(11, it);
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive_remote(barp(BAR_SFREEP + b));   // the score buffer may be overwritten
+                    if (valid != 0xffffffffu) {                                // the same in all lanes
+#pragma unroll
+                        for (int t = 0; t < 32; ++t)
+                            if (!((valid >> t) & 1u)) sv[t] = 0xff800000u;     // no entry: weight exactly 0
+                    }
+                    mx_loc = -INFINITY;
+#pragma unroll
+                    for (int g = 0; g < 4; ++g) {
+                        const uint32_t* v = sv + 8 * g;
+                        auto f = [](uint32_t x) { return __uint_as_float(x); };
+                        const float gm = fmaxf(fmaxf(fmaxf(f(v[0]), f(v[1])), fmaxf(f(v[2]), f(v[3]))),
+                                               fmaxf(fmaxf(f(v[4]), f(v[5])), fmaxf(f(v[6]), f(v[7]))));
+                        mx_loc = fmaxf(mx_loc, fmaf(gm, c_g[g], off_g[g]));
+                        if (p.out_max_logits != nullptr) x_max = fmaxf(x_max, gm * c_g[g]);   // without log2(s): the scaled logit itself
+                    }
                     PROF(4);
+                    TRACE(16, it);
                 }
-                if (named_bar_or(1 + grp, 128, dead || *abort_flag != 0)) { stop = true; break; }   // the four partial row maxima are in place
-                const float* xr = xch + b * 256 + hrow;
-                const float mx = fmaxf(fmaxf(xr[0], xr[64]), fmaxf(xr[128], xr[192]));
-                PROF(5);
-                const bool grow = mx > m_run + RESCALE_TAU;   // false while the row has seen no valid entry
-                if (__any_sync(0xffffffffu, grow)) {
+                // Some row of the group of 128 threads has outgrown its running maximum (or a wait gave up): rare after the
+                // first tiles of a request, so only then the four partial row maxima are exchanged.
+                if (named_bar_or(1 + grp, 128, mx_loc > m_run + RESCALE_TAU || dead || *abort_flag != 0)) {
+                    xch[(b * 4 + xpart) * 64 + hrow] = mx_loc;
+                    if (named_bar_or(1 + grp, 128, dead || *abort_flag != 0)) { stop = true; break; }
+                    const float* xr = xch + b * 256 + hrow;
+                    const float mx = fmaxf(fmaxf(xr[0], xr[64]), fmaxf(xr[128], xr[192]));
+                    const bool grow = mx > m_run + RESCALE_TAU;   // false while the row has seen no valid entry
                     if (j > 0) {   // the accumulator holds earlier tiles: wait for the last P.V, then scale it
                         dead = !mbar_wait_hot(bar(BAR_PVDONE + ((it - 1) & 1u)), ((it - 1) >> 1) & 1u, abort_flag, W_PVDONE);
                         if (dead) continue;
@@ -682,27 +731,39 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) att
                     if (dead) continue;
                 }
                 PROF(7);
+                TRACE(13, it);
                 const float m_off = ((m_run == -INFINITY) ? 0.f : m_run) - (float)P_SHIFT;
                 uint32_t pw[8];
 #pragma unroll
                 for (int g = 0; g < 4; ++g) {
-                    float l0 = 0.f, l1 = 0.f;
+                    // two scores per FMA and per addition (packed fp32, each half rounded as the scalar operation)
+                    const uint64_t c2 = pack_f32x2(c_g[g], c_g[g]), e2 = pack_f32x2(off_g[g] - m_off, off_g[g] - m_off);
+                    uint64_t l2 = 0ull;
 #pragma unroll
                     for (int t = 8 * g; t < 8 * g + 8; t += 4) {
-                        const float p0 = ex2(z[t + 0] - m_off), p1 = ex2(z[t + 1] - m_off);
-                        const float p2 = ex2(z[t + 2] - m_off), p3 = ex2(z[t + 3] - m_off);
-                        l0 += p0 + p2; l1 += p1 + p3;
+                        uint64_t a01 = e2, a23 = e2;
+                        fma_f32x2(a01, pack_f32x2(__uint_as_float(sv[t + 0]), __uint_as_float(sv[t + 1])), c2);
+                        fma_f32x2(a23, pack_f32x2(__uint_as_float(sv[t + 2]), __uint_as_float(sv[t + 3])), c2);
+                        float p0, p1, p2, p3;
+                        unpack_f32x2(a01, p0, p1); unpack_f32x2(a23, p2, p3);
+                        p0 = ex2(p0); p1 = ex2(p1); p2 = ex2(p2); p3 = ex2(p3);
+                        add_f32x2(l2, pack_f32x2(p0, p1));
+                        add_f32x2(l2, pack_f32x2(p2, p3));
                         pw[t >> 2] = pack_e4m3x4(p0, p1, p2, p3);
                     }
+                    float l0, l1;
+                    unpack_f32x2(l2, l0, l1);
                     l_run = fmaf(l0 + l1, inv_g[g], l_run);
                 }
                 PROF(8);
+                TRACE(15, it);
                 // P' of tokens [64*thalf + 32*ch, +32) of head hrow: two 16-byte pieces of the row
                 uint8_t* pb = sm + PB_OFF + b * CHUNK;
                 *reinterpret_cast<uint4*>(pb + swz(hrow, 4 * thalf + 2 * ch)) = make_uint4(pw[0], pw[1], pw[2], pw[3]);
                 *reinterpret_cast<uint4*>(pb + swz(hrow, 4 * thalf + 2 * ch + 1)) = make_uint4(pw[4], pw[5], pw[6], pw[7]);
                 fence_proxy_async();
                 PROF(9);
+                TRACE(17, it);
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive_remote(barp(BAR_PREADYP + b));
@@ -716,163 +777,142 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) att
         }
     } else if (warp < MMA_WARP) {
         // =================================================================== gather
-        // Warp gw reads rows [8 gw, +8) of this CTA's 64 rows of every tile from the raw stage into registers: per
-        // row one 16-byte piece of the 512 no-PE bytes per lane, plus (spread over the lanes) the rows' RoPE bytes
-        // and scale words.  The largest of the rows' scales is the scale of the warp's group; every lane shifts its
-        // pieces onto it and stores them in the layout the MMAs read.
+        // The groups of eight rows of all tiles (eight groups per tile and CTA) go round the gather warps: warp g takes
+        // groups g, g + N_G_WARPS, ... of the CTA's sequence (tile 0: groups 0-7, tile 1: groups 0-7, ...), whatever
+        // request they belong to.  It reads the group from its raw slot into registers: per row one 16-byte piece of the
+        // 512 no-PE bytes per lane, plus (spread over the lanes) the rows' RoPE bytes and scale words.  The largest of
+        // the rows' scales is the scale of the group; every lane shifts its pieces onto it and stores them in the layout
+        // the MMAs read.
         // MODEL1: 28 lanes hold the 448 no-PE bytes of a row; the rows' scale bytes do not travel with the rows (they
-        // lie in the page footer), so the warp reads them from global memory itself, a tile ahead of their use.
-        const int gw = warp - N_SM_WARPS;
+        // lie in the page footer), so the warp reads them from global memory itself, a group ahead of their use.
         const int blk = lane >> 3;                                   // 128-value chunk of this lane's piece
         const CacheGeom main_c = cache_geom(p.kv, p.block_stride, p.page_block_size);
         const CacheGeom extra_c = cache_geom(p.extra_kv, p.extra_block_stride, p.extra_topk > 0 ? p.extra_page_block_size : 1);
-        uint32_t it = 0;
-        bool ok = true, stop = false;
-        for (int req = meta.begin_req; req <= last_req && !stop; ++req) {
-            Work w;
-            if (!get_work(p, meta, req, w)) continue;
-            const int nst = (w.nblk + 1) >> 1;
-            // tile j of this CTA is block blk0 + 2 j + rank of the request; this lane looks after row RPW gw + lane % RPW
-            const int lim = min(w.len, (w.blk0 + w.nblk) * BLOCK_N);
-            auto fetch_idx = [&](int j) -> int { return tile_entry<EXTRA>(p, w, j, (int)rank, gw * RPW + (lane & (RPW - 1)), nst, lim); };
-            auto fetch_scales = [&](int j, int idx) -> uint2 {       // MODEL1: the row's 7 UE8M0 bytes (+ 1 pad)
-                if (!L::M1 || idx < 0) return make_uint2(0u, 0u);
-                const CacheGeom& c = (!EXTRA || w.blk0 + 2 * j + (int)rank < w.main_blocks) ? main_c : extra_c;
-                unsigned in;
-                const uint8_t* pg = cache_page(c, idx, in);
-                return __ldg(reinterpret_cast<const uint2*>(pg + (int64_t)c.pbs * L::DATA + (int64_t)in * 8));
-            };
-            // Which of the warp's rows have an entry (the rows themselves are brought in by the copy warps).
-            int idx_cur = fetch_idx(0), idx_nxt = fetch_idx(1);
-            uint2 sc8_nxt = fetch_scales(0, idx_cur);
+        auto fetch_scales = [&](const Entry& a) -> uint2 {           // MODEL1: the row's 7 UE8M0 bytes (+ 1 pad)
+            if (!L::M1 || a.idx < 0) return make_uint2(0u, 0u);
+            const CacheGeom& c = EXTRA && a.extra ? extra_c : main_c;
+            unsigned in;
+            const uint8_t* pg = cache_page(c, a.idx, in);
+            return __ldg(reinterpret_cast<const uint2*>(pg + (int64_t)c.pbs * L::DATA + (int64_t)in * 8));
+        };
+        // Which of the group's rows have an entry is read ahead (the rows themselves are brought in by the copy warps).
+        ItemWalk<EXTRA> walk(meta.begin_req);
+        uint32_t item = (uint32_t)(warp - N_SM_WARPS);
+        auto fetch = [&](uint32_t i) { return walk.entry(p, meta, last_req, i, (int)rank, lane & (RPW - 1)); };
+        Entry cur = fetch(item), nxt = fetch(item + N_G_WARPS);
+        uint2 sc8_nxt = fetch_scales(cur);
+        bool ok = true;
 #pragma unroll 1
-            for (int k = 0; k < nst; ++k) {
-                const uint32_t t_it = it + k, ks = t_it % NK, rs = t_it % NR;
-                PROF(0);
-                TRACE(60, t_it);
-                if (ok) ok = mbar_wait_hot(bar(BAR_RAWFULL + rs * N_P_WARPS + gw * RPW / 16), (t_it / NR) & 1u, abort_flag, W_RAWFULL);
-                PROF(1);
-                TRACE(61, t_it);
-                const uint32_t vbits = __ballot_sync(0xffffffffu, idx_cur >= 0) & ((1u << RPW) - 1u);
-                const uint2 sc8 = sc8_nxt;
-                sc8_nxt = fetch_scales(k + 1, idx_nxt);
-                idx_cur = idx_nxt;
-                idx_nxt = fetch_idx(k + 2);
-                const uint8_t* raw_rows = sm + RAW_OFF + rs * RAW_BYTES + (gw * RPW) * ROW_BYTES;
-                uint4 nope[RPW], rp[RPW / 4];
-                float sc = 0.f;
-                if (ok) {
+        while (cur.have) {
+            const uint32_t t_it = item / N_GROUPS, gw = item % N_GROUPS, ks = t_it % NK, slot = item % NR;
+            TRACE(60, t_it);
+            ok = mbar_wait_hot(bar(BAR_RAWFULL + slot), (item / NR) & 1u, abort_flag, W_RAWFULL);
+            TRACE(61, t_it);
+            if (!ok) break;
+            const uint32_t vbits = __ballot_sync(0xffffffffu, cur.idx >= 0) & ((1u << RPW) - 1u);
+            const uint2 sc8 = sc8_nxt;
+            const uint8_t* raw_rows = sm + RAW_OFF + slot * RAW_BYTES;
+            uint4 nope[RPW], rp[RPW / 4];
+            float sc = 0.f;
 #pragma unroll
-                    for (int i = 0; i < RPW; ++i)
-                        nope[i] = ((vbits >> i) & 1u) ? *reinterpret_cast<const uint4*>(raw_rows + i * ROW_BYTES + lane * 16) : make_uint4(0, 0, 0, 0);
+            for (int i = 0; i < RPW; ++i)
+                nope[i] = ((vbits >> i) & 1u) ? *reinterpret_cast<const uint4*>(raw_rows + i * ROW_BYTES + lane * 16) : make_uint4(0, 0, 0, 0);
 #pragma unroll
-                    for (int u = 0; u < RPW / 4; ++u) {                      // RoPE piece lane % 8 of row lane / 8 (+ 4 u)
-                        const int r = (lane >> 3) + 4 * u;
-                        rp[u] = ((vbits >> r) & 1u) ? *reinterpret_cast<const uint4*>(raw_rows + r * ROW_BYTES + L::ROPE_AT + (lane & 7) * 16)
-                                                    : make_uint4(0, 0, 0, 0);
-                    }
-                    if (!L::M1 && lane < 4 * RPW && ((vbits >> (lane >> 2)) & 1u))     // scale lane % 4 of row lane / 4
-                        sc = *reinterpret_cast<const float*>(raw_rows + (lane >> 2) * ROW_BYTES + SCALE_OFF + (lane & 3) * 4);
-                } else {
+            for (int u = 0; u < RPW / 4; ++u) {                      // RoPE piece lane % 8 of row lane / 8 (+ 4 u)
+                const int r = (lane >> 3) + 4 * u;
+                rp[u] = ((vbits >> r) & 1u) ? *reinterpret_cast<const uint4*>(raw_rows + r * ROW_BYTES + L::ROPE_AT + (lane & 7) * 16)
+                                            : make_uint4(0, 0, 0, 0);
+            }
+            if (!L::M1 && ((vbits >> (lane >> 2)) & 1u))             // scale lane % 4 of row lane / 4
+                sc = *reinterpret_cast<const float*>(raw_rows + (lane >> 2) * ROW_BYTES + SCALE_OFF + (lane & 3) * 4);
+            sc8_nxt = fetch_scales(nxt);
+            cur = nxt;
+            nxt = fetch(item + 2 * N_G_WARPS);
+            float wm = sc;
+            if (L::M1) {
+                // The group's scale as a biased exponent: the largest of the rows' 7 scale bytes (0 for a row without
+                // an entry) and of what the rows' RoPE needs to fit e4m3 (2^ceil(log2(amax / 448))).
+                uint32_t e = __vmaxu4(sc8.x, sc8.y & 0x00ffffffu);
+                e = max(max(e & 0xffu, (e >> 8) & 0xffu), max((e >> 16) & 0xffu, e >> 24));
+                auto absmax8 = [](const uint4& a) {
+                    return fmaxf(fmaxf(fmaxf(fabsf(bf16lo(a.x)), fabsf(bf16hi(a.x))), fmaxf(fabsf(bf16lo(a.y)), fabsf(bf16hi(a.y)))),
+                                 fmaxf(fmaxf(fabsf(bf16lo(a.z)), fabsf(bf16hi(a.z))), fmaxf(fabsf(bf16lo(a.w)), fabsf(bf16hi(a.w)))));
+                };
+                float am = 0.f;
 #pragma unroll
-                    for (int i = 0; i < RPW; ++i) nope[i] = make_uint4(0, 0, 0, 0);
+                for (int u = 0; u < RPW / 4; ++u) am = fmaxf(am, absmax8(rp[u]));
+                const uint32_t ab = __float_as_uint(am * (1.f / 448.f));
+                e = max(e, (ab >> 23) + ((ab & 0x007fffffu) ? 1u : 0u));
+                if (vbits != 0u) e = max(e, 1u);
+                wm = __uint_as_float(min(e, 254u) << 23);
+            }
+            // scales are not negative, so their bits order as integers do: one reduction instead of five exchanges
+            const float s_half = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(wm)));
+            // the maximum needed the last shared-memory load of every lane (they return in order): the rows have left the slot
+            if (lane == 0) mbar_arrive(bar(BAR_RAWEMPTY + slot));
+            TRACE(62, t_it);
+            const float inv_half = (s_half > 0.f) ? __uint_as_float(0x7f000000u - __float_as_uint(s_half)) : 0.f;
+            const __nv_bfloat162 rope_f = __float2bfloat162_rn(inv_half);
+            // V32: exponent shift of the block whose scale this lane loaded (row lane / 4, block lane % 4): 0 for a block at the scale.
+            // MODEL1: lanes 0-7 pass on exponents 0-3 of row lane, lanes 8-15 exponents 4-6 of row lane - 8.
+            const uint32_t my_sub = L::M1 ? ((lane & 8) ? sc8.y : sc8.x) : ((sc > 0.f) ? shift_bytes_of_ratio(sc * inv_half) : 0u);
+            const uint32_t e_grp = __float_as_uint(s_half) >> 23;
+            const int bk = lane >> 2;                            // MODEL1: 64-value block of this lane's piece (0-6 in the lanes that store)
+            if (t_it >= NK) ok = mbar_wait_hot(bar(BAR_KEMPTY + ks), ((t_it / NK) - 1) & 1u, abort_flag, W_KEMPTY);
+            if (STAGE_Q && ok && t_it == NK - 1 && first_work) ok = mbar_wait_hot(bar(BAR_QFREE), 0u, abort_flag, W_QFREE);   // K stage 1 held Q until now
+            TRACE(63, t_it);
+            if (!ok) break;
+            uint8_t* kp = sm + KS_OFF + ks * KS_BYTES;
 #pragma unroll
-                    for (int u = 0; u < RPW / 4; ++u) rp[u] = make_uint4(0, 0, 0, 0);
-                }
-                float wm = sc;
+            for (int i = 0; i < RPW; ++i) {
+                uint32_t sub;
                 if (L::M1) {
-                    // The group's scale as a biased exponent: the largest of the rows' 7 scale bytes (0 for a row without
-                    // an entry) and of what the rows' RoPE needs to fit e4m3 (2^ceil(log2(amax / 448))).
-                    uint32_t e = __vmaxu4(sc8.x, sc8.y & 0x00ffffffu);
-                    e = max(max(e & 0xffu, (e >> 8) & 0xffu), max((e >> 16) & 0xffu, e >> 24));
-                    auto absmax8 = [](const uint4& a) {
-                        return fmaxf(fmaxf(fmaxf(fabsf(bf16lo(a.x)), fabsf(bf16hi(a.x))), fmaxf(fabsf(bf16lo(a.y)), fabsf(bf16hi(a.y)))),
-                                     fmaxf(fmaxf(fabsf(bf16lo(a.z)), fabsf(bf16hi(a.z))), fmaxf(fabsf(bf16lo(a.w)), fabsf(bf16hi(a.w)))));
-                    };
-                    float am = 0.f;
-#pragma unroll
-                    for (int u = 0; u < RPW / 4; ++u) am = fmaxf(am, absmax8(rp[u]));
-                    const uint32_t ab = __float_as_uint(am * (1.f / 448.f));
-                    e = max(e, (ab >> 23) + ((ab & 0x007fffffu) ? 1u : 0u));
-                    if (vbits != 0u) e = max(e, 1u);
-                    wm = __uint_as_float(min(e, 254u) << 23);
+                    const uint32_t ew = __shfl_sync(0xffffffffu, my_sub, i + ((bk & 4) ? 8 : 0));
+                    sub = min(e_grp - ((ew >> (8 * (bk & 3))) & 0xffu), 15u) * 0x08080808u;
+                } else {
+                    sub = __shfl_sync(0xffffffffu, my_sub, 4 * i + blk);
                 }
-#pragma unroll
-                for (int o = 16; o >= 1; o >>= 1) wm = fmaxf(wm, __shfl_xor_sync(0xffffffffu, wm, o));
-                // the maximum needed the last shared-memory load of every lane (they return in order): the warp's rows
-                // have left the raw stage
-                if (lane == 0) mbar_arrive(bar(BAR_RAWEMPTY + rs * N_P_WARPS + gw * RPW / 16));
-                PROF(2);
-                TRACE(62, t_it);
-                if (ok && t_it >= NK) ok = mbar_wait_hot(bar(BAR_KEMPTY + ks), ((t_it / NK) - 1) & 1u, abort_flag, W_KEMPTY);
-                if (STAGE_Q && ok && t_it < NK && ks != 0 && first_work) ok = mbar_wait_hot(bar(BAR_QFREE), 0u, abort_flag, W_QFREE);   // K stage 1 held Q until now
-                PROF(3);
-                TRACE(63, t_it);
-                if (!ok) { stop = true; break; }
-                PROF(4);
-                TRACE(64, t_it);
-                // one scale for the warp's RPW rows: the largest of their 4 x RPW scales
-                const float s_half = wm;
-                const float inv_half = (s_half > 0.f) ? __uint_as_float(0x7f000000u - __float_as_uint(s_half)) : 0.f;
-                const __nv_bfloat162 rope_f = __float2bfloat162_rn(inv_half);
-                uint8_t* kp = sm + KS_OFF + ks * KS_BYTES;
-                // V32: exponent shift of the block whose scale this lane loaded (row lane / 4, block lane % 4): 0 for a block at the scale.
-                // MODEL1: lanes 0-7 pass on exponents 0-3 of row lane, lanes 8-15 exponents 4-6 of row lane - 8.
-                const uint32_t my_sub = L::M1 ? ((lane & 8) ? sc8.y : sc8.x) : ((sc > 0.f) ? shift_bytes_of_ratio(sc * inv_half) : 0u);
-                const uint32_t e_grp = __float_as_uint(s_half) >> 23;
-                const int bk = lane >> 2;                            // MODEL1: 64-value block of this lane's piece (0-6 in the lanes that store)
-#pragma unroll
-                for (int i = 0; i < RPW; ++i) {
-                    uint32_t sub;
-                    if (L::M1) {
-                        const uint32_t ew = __shfl_sync(0xffffffffu, my_sub, i + ((bk & 4) ? 8 : 0));
-                        sub = min(e_grp - ((ew >> (8 * (bk & 3))) & 0xffu), 15u) * 0x08080808u;
-                    } else {
-                        sub = __shfl_sync(0xffffffffu, my_sub, 4 * i + blk);
-                    }
-                    uint4 v = nope[i];      // no branch on sub: a shift by 0 is the identity, and a branch would keep the rows' chains apart
-                    v.x = shift_down_e4m3x4(v.x, sub); v.y = shift_down_e4m3x4(v.y, sub);
-                    v.z = shift_down_e4m3x4(v.z, sub); v.w = shift_down_e4m3x4(v.w, sub);
-                    if (!L::M1 || lane < L::NOPE / 16)
-                        *reinterpret_cast<uint4*>(kp + blk * CHUNK + swz((uint32_t)(gw * RPW + i), (uint32_t)lane & 7u)) = v;
-                }
-                if (L::M1) {      // V's RoPE columns: e4m3(rope / s) into dims [448, 512) of the rows, the upper half of chunk 3
-#pragma unroll
-                    for (int u = 0; u < RPW / 4; ++u) {
-                        const uint4 v = rp[u];
-                        const uint32_t lo = pack_e4m3x4(bf16lo(v.x) * inv_half, bf16hi(v.x) * inv_half, bf16lo(v.y) * inv_half, bf16hi(v.y) * inv_half);
-                        const uint32_t hi = pack_e4m3x4(bf16lo(v.z) * inv_half, bf16hi(v.z) * inv_half, bf16lo(v.w) * inv_half, bf16hi(v.w) * inv_half);
-                        const uint32_t pc = (uint32_t)lane & 7u;      // piece of 8 values
-                        *reinterpret_cast<uint2*>(kp + 3 * CHUNK + swz((uint32_t)(gw * RPW + (lane >> 3) + 4 * u), 4u + (pc >> 1)) + (pc & 1u) * 8u) =
-                            make_uint2(lo, hi);
-                    }
-                }
+                uint4 v = nope[i];      // no branch on sub: a shift by 0 is the identity, and a branch would keep the rows' chains apart
+                v.x = shift_down_e4m3x4(v.x, sub); v.y = shift_down_e4m3x4(v.y, sub);
+                v.z = shift_down_e4m3x4(v.z, sub); v.w = shift_down_e4m3x4(v.w, sub);
+                if (!L::M1 || lane < L::NOPE / 16)
+                    *reinterpret_cast<uint4*>(kp + blk * CHUNK + swz((uint32_t)(gw * RPW + i), (uint32_t)lane & 7u)) = v;
+            }
+            if (L::M1) {      // V's RoPE columns: e4m3(rope / s) into dims [448, 512) of the rows, the upper half of chunk 3
 #pragma unroll
                 for (int u = 0; u < RPW / 4; ++u) {
-                    uint4 v = rp[u];
-                    v.x = mul_bf16x2(v.x, rope_f); v.y = mul_bf16x2(v.y, rope_f);
-                    v.z = mul_bf16x2(v.z, rope_f); v.w = mul_bf16x2(v.w, rope_f);
-                    *reinterpret_cast<uint4*>(kp + KS_ROPE + swz((uint32_t)(gw * RPW + (lane >> 3) + 4 * u), (uint32_t)lane & 7u)) = v;
+                    const uint4 v = rp[u];
+                    const uint32_t lo = pack_e4m3x4(bf16lo(v.x) * inv_half, bf16hi(v.x) * inv_half, bf16lo(v.y) * inv_half, bf16hi(v.y) * inv_half);
+                    const uint32_t hi = pack_e4m3x4(bf16lo(v.z) * inv_half, bf16hi(v.z) * inv_half, bf16lo(v.w) * inv_half, bf16hi(v.w) * inv_half);
+                    const uint32_t pc = (uint32_t)lane & 7u;      // piece of 8 values
+                    *reinterpret_cast<uint2*>(kp + 3 * CHUNK + swz((uint32_t)(gw * RPW + (lane >> 3) + 4 * u), 4u + (pc >> 1)) + (pc & 1u) * 8u) =
+                        make_uint2(lo, hi);
                 }
-                if (lane == 0) {      // the record of the warp's rows: read by this CTA's softmax warps and sent to the partner's
-                    uint8_t* rec = sm + INFO_OFF + (t_it & (INFO_RING - 1)) * (2 * INFO_HALF) + rank * INFO_HALF + gw * 16;
-                    *reinterpret_cast<float4*>(rec) =
-                        make_float4(s_half, (s_half > 0.f) ? (float)((int)(__float_as_uint(s_half) >> 23) - 127) : -INFINITY, inv_half,
-                                    __uint_as_float(vbits));
-                }
-                PROF(5);
-                TRACE(65, t_it);
-                fence_proxy_async();
-                __syncwarp();
-                if (lane == 0) {
-                    mbar_arrive(bar(BAR_KSTORED + ks));
-                    mbar_arrive_remote(barp(BAR_KFULLP + ks));
-                }
-                PROF(6);
             }
-            it += nst;
+#pragma unroll
+            for (int u = 0; u < RPW / 4; ++u) {
+                uint4 v = rp[u];
+                v.x = mul_bf16x2(v.x, rope_f); v.y = mul_bf16x2(v.y, rope_f);
+                v.z = mul_bf16x2(v.z, rope_f); v.w = mul_bf16x2(v.w, rope_f);
+                *reinterpret_cast<uint4*>(kp + KS_ROPE + swz((uint32_t)(gw * RPW + (lane >> 3) + 4 * u), (uint32_t)lane & 7u)) = v;
+            }
+            if (lane == 0) {      // the record of the group: read by this CTA's softmax warps and sent to the partner's
+                uint8_t* rec = sm + INFO_OFF + (t_it & (INFO_RING - 1)) * (2 * INFO_HALF) + rank * INFO_HALF + gw * 16;
+                *reinterpret_cast<float4*>(rec) =
+                    make_float4(s_half, (s_half > 0.f) ? (float)((int)(__float_as_uint(s_half) >> 23) - 127) : -INFINITY, inv_half,
+                                __uint_as_float(vbits));
+            }
+            TRACE(64, t_it);
+            fence_proxy_async();
+            __syncwarp();
+            if (lane == 0) {
+                mbar_arrive(bar(BAR_KSTORED + ks));
+                mbar_arrive_remote(barp(BAR_KFULLP + ks));
+            }
+            TRACE(65, t_it);
+            item += N_G_WARPS;
         }
-    } else if (warp == MMA_WARP && lane == 0 && rank == 0) {
+    } else if (warp == MMA_WARP && rank == 0) {
         // =================================================================== score MMA issue (even CTA)
         uint32_t it = 0, rq = 0;
         bool ok = true;
@@ -881,47 +921,50 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) att
             Work w;
             if (!get_work(p, meta, req, w)) continue;
             const int nst = (w.nblk + 1) >> 1;
-            ok = mbar_wait_thread(bar(BAR_QREADYP), rq & 1u, abort_flag, W_QREADY);
+            ok = mbar_wait_hot(bar(BAR_QREADYP), rq & 1u, abort_flag, W_QREADY);
             if (!ok) break;
             ++rq;
             for (int j = 0; j < nst && ok; ++j, ++it) {
                 const uint32_t ks = it % NK, b = it & 1u;
                 PROF(0);
                 if (it >= 2) {
-                    ok = mbar_wait_thread(bar(BAR_SFREEP + b), ((it - 2) >> 1) & 1u, abort_flag, W_SFREE);
+                    ok = mbar_wait_hot(bar(BAR_SFREEP + b), ((it - 2) >> 1) & 1u, abort_flag, W_SFREE);
                     if (!ok) break;
                 }
                 PROF(1);
-                ok = mbar_wait_thread(bar(BAR_KFULLP + ks), (it / NK) & 1u, abort_flag, W_KFULL);
+                ok = mbar_wait_hot(bar(BAR_KFULLP + ks), (it / NK) & 1u, abort_flag, W_KFULL);
                 if (!ok) break;
                 PROF(2);
                 tc_fence_after();
                 TRACE(40, it);
                 const uint32_t kb_lo = desc_lo(base + KS_OFF + ks * KS_BYTES, 16);
                 const uint32_t d = tmem + TM_S + 64 * b;
+                if (elect_one()) {
 #pragma unroll
-                for (int kc = 0; kc < 4; ++kc) {
+                    for (int kc = 0; kc < 4; ++kc) {
+#pragma unroll
+                        for (int s = 0; s < 4; ++s) {
+                            if (32 * (4 * kc + s) < L::NOPE)      // MODEL1: the last 64 bytes of chunk 3 are V's RoPE columns
+                                mma_pair_f8_ts(d, tmem + TM_Q + 32 * kc + 8 * s,
+                                               make_desc(kb_lo + ((kc * CHUNK + s * 32) >> 4), DESC_HI_SW128), IDESC_QK_F8, (kc | s) != 0);
+                        }
+                    }
 #pragma unroll
                     for (int s = 0; s < 4; ++s) {
-                        if (32 * (4 * kc + s) < L::NOPE)      // MODEL1: the last 64 bytes of chunk 3 are V's RoPE columns
-                            mma_pair_f8_ts(d, tmem + TM_Q + 32 * kc + 8 * s,
-                                           make_desc(kb_lo + ((kc * CHUNK + s * 32) >> 4), DESC_HI_SW128), IDESC_QK_F8, (kc | s) != 0);
+                        mma_pair_f16(d, make_desc(qr_lo + ((s * 32) >> 4), DESC_HI_SW128),
+                                     make_desc(kb_lo + ((KS_ROPE + s * 32) >> 4), DESC_HI_SW128), IDESC_QK_BF16, true);
                     }
+                    tc_commit_pair(bar(BAR_SREADY + b));
+                    tc_commit_pair(mapa_shared(bar(BAR_SREADY + b), 1));
+                    tc_commit_pair(bar(BAR_KEMPTY + ks));
+                    tc_commit_pair(mapa_shared(bar(BAR_KEMPTY + ks), 1));
                 }
-#pragma unroll
-                for (int s = 0; s < 4; ++s) {
-                    mma_pair_f16(d, make_desc(qr_lo + ((s * 32) >> 4), DESC_HI_SW128),
-                                 make_desc(kb_lo + ((KS_ROPE + s * 32) >> 4), DESC_HI_SW128), IDESC_QK_BF16, true);
-                }
-                tc_commit_pair(bar(BAR_SREADY + b));
-                tc_commit_pair(mapa_shared(bar(BAR_SREADY + b), 1));
-                tc_commit_pair(bar(BAR_KEMPTY + ks));
-                tc_commit_pair(mapa_shared(bar(BAR_KEMPTY + ks), 1));
+                __syncwarp();
                 PROF(3);
                 TRACE(41, it);
             }
         }
-    } else if (warp == MMA_WARP + 1 && lane == 0 && rank == 0) {
+    } else if (warp == MMA_WARP + 1 && rank == 0) {
         // =================================================================== P.V MMA issue (even CTA)
         uint32_t it = 0;
         bool ok = true;
@@ -932,39 +975,42 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) att
             for (int j = 0; j < nst && ok; ++j, ++it) {
                 const uint32_t vs = it % NV, b = it & 1u;
                 PROF(0);
-                ok = mbar_wait_thread(bar(BAR_PREADYP + b), (it >> 1) & 1u, abort_flag, W_PREADY);
+                ok = mbar_wait_hot(bar(BAR_PREADYP + b), (it >> 1) & 1u, abort_flag, W_PREADY);
                 if (!ok) break;
                 PROF(1);
                 TRACE(50, it);
-                ok = mbar_wait_thread(bar(BAR_VFULLP + vs), (it / NV) & 1u, abort_flag, W_VFULL);
+                ok = mbar_wait_hot(bar(BAR_VFULLP + vs), (it / NV) & 1u, abort_flag, W_VFULL);
                 if (!ok) break;
                 PROF(2);
                 tc_fence_after();
                 TRACE(51, it);
                 const uint32_t pa_lo = desc_lo(base + PB_OFF + b * CHUNK, 16);
                 const uint32_t vb_lo = desc_lo(base + VS_OFF + vs * VS_BYTES, VSLOT);
+                if (elect_one()) {
 #pragma unroll
-                for (int kb = 0; kb < 4; ++kb) {
+                    for (int kb = 0; kb < 4; ++kb) {
 #pragma unroll
-                    for (int nb = 0; nb < 2; ++nb) {
-                        mma_pair_f8(tmem + TM_O + 128 * nb, make_desc(pa_lo + ((kb * 32) >> 4), DESC_HI_SW128),
-                                    make_desc(vb_lo + (((4 * nb + kb) * VSLOT) >> 4), DESC_HI_SW128), IDESC_PV_F8, (j | kb) != 0);
+                        for (int nb = 0; nb < 2; ++nb) {
+                            mma_pair_f8(tmem + TM_O + 128 * nb, make_desc(pa_lo + ((kb * 32) >> 4), DESC_HI_SW128),
+                                        make_desc(vb_lo + (((4 * nb + kb) * VSLOT) >> 4), DESC_HI_SW128), IDESC_PV_F8, (j | kb) != 0);
+                        }
                     }
+                    tc_commit_pair(bar(BAR_VEMPTY + vs));
+                    tc_commit_pair(mapa_shared(bar(BAR_VEMPTY + vs), 1));
+                    tc_commit_pair(bar(BAR_PVDONE + b));
+                    tc_commit_pair(mapa_shared(bar(BAR_PVDONE + b), 1));
                 }
-                tc_commit_pair(bar(BAR_VEMPTY + vs));
-                tc_commit_pair(mapa_shared(bar(BAR_VEMPTY + vs), 1));
-                tc_commit_pair(bar(BAR_PVDONE + b));
-                tc_commit_pair(mapa_shared(bar(BAR_PVDONE + b), 1));
+                __syncwarp();
                 PROF(3);
                 TRACE(52, it);
             }
         }
-    } else if (warp == FWD_WARP && lane == 0) {
+    } else if (warp == FWD_WARP) {
         // =================================================================== K stage -> V slots (both CTAs)
         // The no-PE bytes of this CTA's 64 rows lie in the K stage as four chunks of [64 rows x 128 dims], which is
         // two V slots each (rows 0-31 and 32-63) in the slots' own layout.  Chunks 2 r and 2 r + 1 go to CTA r: the
         // chunks of the own dims stay in this CTA, the others cross to the partner.  The destination's barrier
-        // counts the bytes.  The half tile's scale records travel the same way.  When this CTA's slots are full
+        // counts the bytes.  When this CTA's slots are full
         // (its own copies and the partner's have landed) the thread passes that on: V full to the even CTA,
         // K stage free to both.
         const uint32_t peer = 1u - rank;
@@ -975,97 +1021,102 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) att
             if (!get_work(p, meta, req, w)) continue;
             const int nst = (w.nblk + 1) >> 1;
             for (int j = 0; j < nst && ok; ++j, ++it) {
-                const uint32_t ks = it % NK, vs = it % NV, ir = it & (INFO_RING - 1);
+                const uint32_t ks = it % NK, vs = it % NV;
                 TRACE(70, it);
-                ok = mbar_wait_thread(bar(BAR_KSTORED + ks), (it / NK) & 1u, abort_flag, W_KSTORED);
+                ok = mbar_wait_hot(bar(BAR_KSTORED + ks), (it / NK) & 1u, abort_flag, W_KSTORED);
                 if (!ok) break;
                 TRACE(71, it);
-                mbar_arrive_expect_tx(bar(BAR_INFO + ir), INFO_HALF);
-                bulk_copy_to_cluster(mapa_shared(base + INFO_OFF + ir * (2 * INFO_HALF) + rank * INFO_HALF, peer),
-                                     base + INFO_OFF + ir * (2 * INFO_HALF) + rank * INFO_HALF, INFO_HALF, mapa_shared(bar(BAR_INFO + ir), peer));
                 if (it >= NV) {
-                    ok = mbar_wait_thread(bar(BAR_VEMPTY + vs), ((it / NV) - 1) & 1u, abort_flag, W_VEMPTY);
+                    ok = mbar_wait_hot(bar(BAR_VEMPTY + vs), ((it / NV) - 1) & 1u, abort_flag, W_VEMPTY);
                     if (!ok) break;
                 } else if (STAGE_Q && first_work) {    // the V stages of both CTAs held Q until the softmax warps had read it
-                    ok = mbar_wait_thread(bar(BAR_QFREE), 0u, abort_flag, W_QFREE);
+                    ok = mbar_wait_hot(bar(BAR_QFREE), 0u, abort_flag, W_QFREE);
                     if (!ok) break;
                 }
                 TRACE(72, it);
-                mbar_arrive_expect_tx(bar(BAR_VFULL + vs), 4 * CHUNK);
+                if (elect_one()) {
+                    mbar_arrive_expect_tx(bar(BAR_VFULL + vs), 4 * CHUNK);
 #pragma unroll
-                for (uint32_t r = 0; r < 2; ++r) {
+                    for (uint32_t r = 0; r < 2; ++r) {
 #pragma unroll
-                    for (uint32_t nb = 0; nb < 2; ++nb) {
-                        bulk_copy_to_cluster(mapa_shared(base + VS_OFF + vs * VS_BYTES + (4 * nb + 2 * rank) * VSLOT, r),
-                                             base + KS_OFF + ks * KS_BYTES + (2 * r + nb) * CHUNK, CHUNK,
-                                             mapa_shared(bar(BAR_VFULL + vs), r));
+                        for (uint32_t nb = 0; nb < 2; ++nb) {
+                            bulk_copy_to_cluster(mapa_shared(base + VS_OFF + vs * VS_BYTES + (4 * nb + 2 * rank) * VSLOT, r),
+                                                 base + KS_OFF + ks * KS_BYTES + (2 * r + nb) * CHUNK, CHUNK,
+                                                 mapa_shared(bar(BAR_VFULL + vs), r));
+                        }
                     }
                 }
+                __syncwarp();
                 TRACE(73, it);
-                ok = mbar_wait_thread(bar(BAR_VFULL + vs), (it / NV) & 1u, abort_flag, W_VFULL_CTA);
+                ok = mbar_wait_hot(bar(BAR_VFULL + vs), (it / NV) & 1u, abort_flag, W_VFULL_CTA);
                 if (!ok) break;
                 TRACE(74, it);
-                mbar_arrive_remote(barp(BAR_VFULLP + vs));
-                // the copies out of this CTA's K stage into its own slots and the partner's copies into them are done
-                mbar_arrive(bar(BAR_KEMPTY + ks));
-                mbar_arrive_remote(mapa_shared(bar(BAR_KEMPTY + ks), peer));
+                if (lane == 0) {
+                    mbar_arrive_remote(barp(BAR_VFULLP + vs));
+                    // the copies out of this CTA's K stage into its own slots and the partner's copies into them are done
+                    mbar_arrive(bar(BAR_KEMPTY + ks));
+                    mbar_arrive_remote(mapa_shared(bar(BAR_KEMPTY + ks), peer));
+                }
+                __syncwarp();
             }
         }
-    }
-    else if (warp >= PROD_WARP0) {
-        // =================================================================== global -> raw stage (both CTAs)
-        // Copy warp pw brings rows [16 pw, +16) of every tile of this CTA into the raw stage, one bulk copy per row
-        // (lanes 0-15; no load/store unit and no registers involved, two tiles of the CTA are in flight).  Nothing
-        // is copied for a row without an entry.  The tile NR ahead is issued as soon as the gather warps that read
-        // these rows have taken the tile out of the stage; the warp's barrier of the stage counts the bytes.
-        // Issuing a copy blocks while the copy unit is busy, which is why no working warp does it.
-        const int pw = warp - PROD_WARP0;
-        const CacheGeom main_c = cache_geom(p.kv, p.block_stride, p.page_block_size);
-        const CacheGeom extra_c = cache_geom(p.extra_kv, p.extra_block_stride, p.extra_topk > 0 ? p.extra_page_block_size : 1);
+    } else if (warp == INFO_WARP) {
+        // =================================================================== scale records -> partner (both CTAs)
+        // A warp of its own: the softmax warps need the records as soon as they have the scores, long before the
+        // V copies of the tile can start.
+        const uint32_t peer = 1u - rank;
         uint32_t it = 0;
         bool ok = true;
         for (int req = meta.begin_req; req <= last_req && ok; ++req) {
             Work w;
             if (!get_work(p, meta, req, w)) continue;
             const int nst = (w.nblk + 1) >> 1;
-            // tile j of this CTA is block blk0 + 2 j + rank of the request; row 16 pw + lane % 16
-            const int lim = min(w.len, (w.blk0 + w.nblk) * BLOCK_N);
-            auto fetch_idx = [&](int j) -> int { return tile_entry<EXTRA>(p, w, j, (int)rank, pw * 16 + (lane & 15), nst, lim); };
-            auto issue_rows = [&](int idx, int j, uint32_t t_it) {   // idx: lanes 0-15 hold the indices of the rows of tile j
-                const uint32_t stage = t_it % NR;
-                unsigned long long src = 0ull;
-                if (idx >= 0) {
-                    const CacheGeom& c = (!EXTRA || w.blk0 + 2 * j + (int)rank < w.main_blocks) ? main_c : extra_c;
-                    unsigned in;
-                    const uint8_t* pg = cache_page(c, idx, in);
-                    src = reinterpret_cast<unsigned long long>(pg + (int64_t)in * L::DATA);
-                }
-                const uint32_t dst0 = base + RAW_OFF + stage * RAW_BYTES + (pw * 16) * ROW_BYTES;
-                const uint32_t fb = bar(BAR_RAWFULL + stage * N_P_WARPS + pw);
-                const uint32_t nvalid = __popc(__ballot_sync(0xffffffffu, src != 0ull) & 0xffffu);
-                if (lane == 0) mbar_arrive_expect_tx(fb, nvalid * L::DATA);
-                __syncwarp();
-                if (lane < 16 && src != 0ull) bulk_copy_g2s(dst0 + lane * ROW_BYTES, src, L::DATA, fb);
-            };
-            // The raw stages that the first NR tiles of a request go to are free once the gather warps have taken the
-            // last NR tiles before them out (for the very first tiles of the CTA there is nothing to wait for).
-#pragma unroll 1
-            for (int j = 0; j < NR && j < nst && ok; ++j) {
-                const uint32_t t_it = it + j;
-                const int idx = fetch_idx(j);
-                if (t_it >= NR) ok = mbar_wait_hot(bar(BAR_RAWEMPTY + (t_it % NR) * N_P_WARPS + pw), ((t_it / NR) - 1) & 1u, abort_flag, W_RAWEMPTY);
-                if (ok) issue_rows(idx, j, t_it);
-            }
-            int idx_ahead = fetch_idx(NR);               // read one tile before it is turned into addresses
-#pragma unroll 1
-            for (int j = 0; j + NR < nst && ok; ++j) {   // the tile NR ahead goes into the raw stage that has just been emptied
-                const uint32_t t_it = it + j;
-                ok = mbar_wait_hot(bar(BAR_RAWEMPTY + (t_it % NR) * N_P_WARPS + pw), (t_it / NR) & 1u, abort_flag, W_RAWEMPTY);
+            for (int j = 0; j < nst && ok; ++j, ++it) {
+                const uint32_t ks = it % NK, ir = it & (INFO_RING - 1);
+                ok = mbar_wait_hot(bar(BAR_KSTORED + ks), (it / NK) & 1u, abort_flag, W_KSTORED);
                 if (!ok) break;
-                issue_rows(idx_ahead, j + NR, t_it + NR);
-                idx_ahead = fetch_idx(j + NR + 1);
+                if (elect_one()) {
+                    mbar_arrive_expect_tx(bar(BAR_INFO + ir), INFO_HALF);
+                    bulk_copy_to_cluster(mapa_shared(base + INFO_OFF + ir * (2 * INFO_HALF) + rank * INFO_HALF, peer),
+                                         base + INFO_OFF + ir * (2 * INFO_HALF) + rank * INFO_HALF, INFO_HALF, mapa_shared(bar(BAR_INFO + ir), peer));
+                    mbar_arrive(bar(BAR_KEMPTY + ks));      // this warp has seen the stage's phase: it cannot run two phases ahead of it
+                }
+                __syncwarp();
             }
-            it += nst;
+        }
+    } else if (warp >= PROD_WARP0) {
+        // =================================================================== global -> raw slots (both CTAs)
+        // Copy warp pw brings in the groups pw, pw + 4, ... of the CTA's sequence of groups (eight per tile, whatever
+        // request they belong to), one bulk copy per row (lanes 0-7; no load/store unit and no registers involved).
+        // Nothing is copied for a row without an entry.  A slot is refilled as soon as the gather warp that read it has
+        // its rows in registers; the slot's barrier counts the bytes.  Issuing a copy blocks while the copy unit is
+        // busy, which is why no working warp does it.
+        const CacheGeom main_c = cache_geom(p.kv, p.block_stride, p.page_block_size);
+        const CacheGeom extra_c = cache_geom(p.extra_kv, p.extra_block_stride, p.extra_topk > 0 ? p.extra_page_block_size : 1);
+        ItemWalk<EXTRA> walk(meta.begin_req);
+        uint32_t item = (uint32_t)(warp - PROD_WARP0);
+        auto fetch = [&](uint32_t i) { return walk.entry(p, meta, last_req, i, (int)rank, lane & (RPW - 1)); };
+        Entry cur = fetch(item);
+        bool ok = true;
+#pragma unroll 1
+        while (cur.have && ok) {
+            const Entry nxt = fetch(item + N_P_WARPS);          // read an item before it is turned into addresses
+            const uint32_t slot = item % NR;
+            unsigned long long src = 0ull;
+            if (cur.idx >= 0) {
+                const CacheGeom& c = EXTRA && cur.extra ? extra_c : main_c;
+                unsigned in;
+                const uint8_t* pg = cache_page(c, cur.idx, in);
+                src = reinterpret_cast<unsigned long long>(pg + (int64_t)in * L::DATA);
+            }
+            const uint32_t nvalid = __popc(__ballot_sync(0xffffffffu, src != 0ull) & ((1u << RPW) - 1u));
+            if (item >= NR) ok = mbar_wait_hot(bar(BAR_RAWEMPTY + slot), ((item / NR) - 1) & 1u, abort_flag, W_RAWEMPTY);
+            if (!ok) break;
+            if (lane == 0) mbar_arrive_expect_tx(bar(BAR_RAWFULL + slot), nvalid * L::DATA);
+            __syncwarp();
+            if (lane < RPW && src != 0ull) bulk_copy_g2s(base + RAW_OFF + slot * RAW_BYTES + lane * ROW_BYTES, src, L::DATA, bar(BAR_RAWFULL + slot));
+            cur = nxt;
+            item += N_P_WARPS;
         }
     }
 

@@ -82,6 +82,17 @@ __device__ __forceinline__ bool mbar_wait_hot(uint32_t bar, uint32_t parity, vol
     return __all_sync(0xffffffffu, ok != 0);
 }
 
+// True in one lane of the (converged) warp, the same one every time.  Instructions whose operands live in uniform
+// registers (tcgen05.mma and its commit, bulk copies) are issued under this predicate: the compiler then knows that
+// one lane runs them and keeps descriptors and addresses in uniform registers.  Under `lane == 0` it does not, and every
+// such instruction pays a transfer of its operands (measured: 46 cycles per pair MMA instead of 23 on an idle SM, about
+// 90 on a busy one).
+__device__ __forceinline__ bool elect_one() {
+    uint32_t r;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
+    return r != 0;
+}
+
 // ------------------------------------------------------------------ thread-block cluster
 __device__ __forceinline__ uint32_t cluster_ctarank() {
     uint32_t r;
@@ -110,7 +121,16 @@ __device__ __forceinline__ void unpack_f32x2(uint64_t v, float& lo, float& hi) {
 __device__ __forceinline__ void fma_f32x2(uint64_t& acc, uint64_t a, uint64_t b) {   // acc += a * b, per lane
     asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
 }
+__device__ __forceinline__ void add_f32x2(uint64_t& acc, uint64_t a) {               // acc += a, per lane
+    asm("add.rn.f32x2 %0, %0, %1;" : "+l"(acc) : "l"(a));
+}
 
+// 16 bytes of read-only global memory that are used once.
+__device__ __forceinline__ uint4 ld_row16(const void* p) {
+    uint4 v;
+    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
 // 256-bit global store (sm_100): one full 32-byte sector per lane; p must be 32-byte aligned.
 __device__ __forceinline__ void st_global_v8(void* p, const uint32_t (&v)[8]) {
     asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]),
