@@ -82,11 +82,11 @@ def kv_geometry(kv_cache: torch.Tensor) -> Tuple[int, int]:
     raise ValueError(f"unsupported kv_cache rank {kv_cache.dim()}")
 
 
-# What IMPL_AUTO means for a MODEL1 cache.  The tensor-core kernel rounds V's RoPE columns to e4m3 (the reference
-# keeps them in bf16), which costs up to about 2e-3 on rows with few entries and fails some of the reference's own
-# V4 tests by a small margin; the default is therefore the exact fp32 kernel.  A deployment that accepts FP8-class
-# error in those 64 columns sets SMLA_MODEL1_IMPL=tc in the environment (or assigns _lib.IMPL_TC here) and gets the
-# tensor-core kernel, about two orders of magnitude faster.
+# What IMPL_AUTO means for a MODEL1 cache.  The FP8-class tensor-core kernel rounds V's RoPE columns to e4m3 (the reference
+# keeps them in bf16), which costs up to about 2e-3 on rows with few entries and fails some of the reference's own V4
+# tests by a small margin; the default is therefore exact numerics (IMPL_SCALAR: attn_exact_kernel, bf16 operands and fp32
+# sums).  A deployment that accepts FP8-class error in those 64 columns sets SMLA_MODEL1_IMPL=tc in the environment (or
+# assigns _lib.IMPL_TC here).
 MODEL1_DEFAULT_IMPL = _lib.IMPL_TC if os.environ.get("SMLA_MODEL1_IMPL", "").lower() in ("tc", "2") else _lib.IMPL_SCALAR
 
 
@@ -113,6 +113,22 @@ def pick_num_sm_parts_fp32(num_tokens: int, num_heads: int, sms: int) -> int:
     if num_tokens * tiles >= 2 * sms:
         return num_tokens
     return max(2 * sms // tiles, 1)
+
+
+# attn_exact_kernel (exact numerics over MODEL1, aligned caches): microseconds of a partition's fixed part (q, epilogue),
+# of a 128-token tile, and of what a split adds (scheduler and combine launches, partial records).
+_EXACT_US_FIXED, _EXACT_US_TILE, _EXACT_US_SPLIT = 6.0, 4.0, 9.0
+
+
+def pick_num_sm_parts_exact(num_tokens: int, num_heads: int, sms: int, blocks_per_token: int) -> int:
+    """Partitions for attn_exact_kernel, which runs one CTA per partition and 64 heads: whole requests when their tiles in
+    full waves take no longer than cutting the work evenly over the machine and merging the pieces."""
+    most = max(sms // -(-num_heads // 64), 1)
+    tiles = max(-(-blocks_per_token // 2), 1)
+    whole = -(-num_tokens // most) * (_EXACT_US_FIXED + tiles * _EXACT_US_TILE)
+    parts = min(most, num_tokens * tiles)
+    cut = _EXACT_US_FIXED + -(-num_tokens * tiles // parts) * _EXACT_US_TILE + _EXACT_US_SPLIT
+    return num_tokens if whole <= cut else parts
 
 
 BLOCKS_PER_PARTITION = 4  # a partition should be worth at least two 128-token tiles: below that the partials cost more than the split gains

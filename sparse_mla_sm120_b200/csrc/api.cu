@@ -64,6 +64,8 @@ const char* smla_status_string(int code) {
         case 30: return "attention p_ready"; case 31: return "attention pv_done"; case 32: return "attention q_ready";
         case 33: return "attention q_staged"; case 34: return "attention q_free"; case 35: return "attention raw_empty";
         case 36: return "attention raw_full";
+        case 41: return "exact attention rows free"; case 42: return "exact attention rows stored"; case 43: return "exact attention s_ready";
+        case 44: return "exact attention p_ready"; case 45: return "exact attention pv_done"; case 46: return "exact attention q_ready";
         default: return "unknown";
     }
 }
@@ -315,16 +317,18 @@ static int check_ext(const char* fn, const void* q, const void* kv, const int32_
     return 0;
 }
 
-// impl AUTO: V32 (with a second cache) runs the tensor-core kernel when the caches are aligned for its bulk copies,
-// else the fp32 kernel.  MODEL1 runs the fp32 kernel unless the tensor-core kernel is asked for by name: there V
-// includes the row's RoPE, which the tensor-core kernel rounds to e4m3 like the rest of V, while the reference keeps
-// it in bf16 (csrc/kernel/common/xv_rope_mma.cuh:23-93) and bounds the error of short rows in its own tests
-// (tests/test_prefill.py:95-107, tests/test_v4_features.py:28-47) below what that rounding costs.
+// impl AUTO: V32 (with a second cache) runs the FP8-class tensor-core kernel when the caches are aligned for its bulk
+// copies, else the CUDA-core fp32 kernel.  MODEL1 runs exact numerics unless the FP8-class kernel is asked for by name:
+// there V includes the row's RoPE, which that kernel rounds to e4m3 like the rest of V, while the reference keeps it in
+// bf16 (csrc/kernel/common/xv_rope_mma.cuh:23-93) and bounds the error of short rows in its own tests
+// (tests/test_prefill.py:95-107, tests/test_v4_features.py:28-47) below what that rounding costs.  Exact numerics over
+// MODEL1 mean attn_exact_kernel, which loads rows 16 bytes at a time; caches that are only 4-byte aligned stay on the
+// CUDA-core kernel.
 static int launch_ext(const char* fn, const AttnParams& p, int impl, cudaStream_t stream) {
     if (impl != SMLA_IMPL_AUTO && impl != SMLA_IMPL_SCALAR && impl != SMLA_IMPL_TC)
         return set_error(SMLA_E_SHAPE, "%s: unknown impl %d", fn, impl);
     if (impl == SMLA_IMPL_SCALAR || (impl == SMLA_IMPL_AUTO && p.layout == SMLA_LAYOUT_MODEL1))
-        return launch_attn_scalar(p, stream);
+        return p.layout == SMLA_LAYOUT_MODEL1 && attn_pair_takes(p) ? launch_attn_exact(p, stream) : launch_attn_scalar(p, stream);
     if (attn_pair_takes(p)) return launch_attn_pair(p, stream);
     if (impl == SMLA_IMPL_TC)
         return set_error(SMLA_E_ALIGN, "%s: the tensor-core kernel needs 16-byte aligned caches and page strides", fn);

@@ -12,7 +12,8 @@
 // 8 tokens: dequantise 8 rows to shared memory, 64 dot products of length 576 (4 threads each),
 // online softmax per head, then P.V with one thread per (head, 16 output dims).
 //
-// It is also the kernel that serves the second cache layout and the second ("extra") cache:
+// It also knows the second cache layout (served by attn_exact_kernel unless the caches are only 4-byte aligned) and the
+// second ("extra") cache:
 //  * layout MODEL1 (csrc/model/kv_cache_traits.cuh:61-111): a page of `block` tokens is
 //    block x 576 data bytes (448 e4m3 + 64 bf16 RoPE per token) followed by a footer of
 //    block x 8 bytes (7 UE8M0 scales, one per 64 values, + 1 pad); q has 512 dims and V is the

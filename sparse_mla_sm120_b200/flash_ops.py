@@ -7,8 +7,8 @@ reference exposes as ``flash_mla_sm120.cuda`` (csrc/binding.cpp:250-292) are the
 
 Two cache layouts are served, told apart as the reference does by the width of q and of a cache row:
 V32 (q 576 wide, 656-byte rows) and MODEL1 (q 512 wide, 584 bytes per token with the scales in a footer
-of the page; V is the whole row).  V32 without a second cache runs on the tcgen05 kernels; MODEL1 and the
-second ("extra") cache run on the exact fp32 kernel.
+of the page; V is the whole row).  V32 runs on the FP8-class tcgen05 kernel, MODEL1 on the exact one (bf16 operands)
+unless the FP8-class kernel is asked for; caches that are not 16-byte aligned run on the CUDA-core fp32 kernel.
 """
 from __future__ import annotations
 
@@ -18,7 +18,7 @@ import torch
 
 from . import _lib
 from ._lib import IMPL_AUTO, IMPL_SCALAR, LAYOUT_MODEL1, LAYOUT_V32, check
-from ._runtime import (BLOCK_N, FIXED_OVERHEAD, kv_geometry, kv_layout, num_sms, pick_num_sm_parts_fp32, pick_split, ptr,
+from ._runtime import (BLOCK_N, FIXED_OVERHEAD, kv_geometry, kv_layout, num_sms, pick_num_sm_parts_exact, pick_num_sm_parts_fp32, pick_split, ptr,
                        require_cuda, resolve_impl, scratch, status_buffer, stream_ptr, tc_aligned)
 
 
@@ -180,8 +180,10 @@ def sparse_mla_decode_fwd(
 
     fixed_overhead = FIXED_OVERHEAD
     if num_sm_parts is None:
-        fp32 = use_ext and (impl == IMPL_SCALAR or not tc_aligned(kv_cache, ex.kv))
-        if fp32:
+        aligned = not use_ext or tc_aligned(kv_cache, ex.kv)
+        if aligned and layout == LAYOUT_MODEL1 and impl == IMPL_SCALAR:
+            num_sm_parts = pick_num_sm_parts_exact(num_tokens, num_heads, num_sms(q.device), blocks)
+        elif use_ext and (impl == IMPL_SCALAR or not aligned):
             num_sm_parts = pick_num_sm_parts_fp32(num_tokens, num_heads, num_sms(q.device))
         else:   # requests of equal length (no topk_length, no second cache) may be cut into equal partitions
             num_sm_parts, fixed_overhead = pick_split(num_tokens, num_sms(q.device), blocks,

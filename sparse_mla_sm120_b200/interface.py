@@ -24,8 +24,8 @@ from typing import Optional, Tuple
 import torch
 
 from . import _lib
-from ._lib import IMPL_AUTO, IMPL_SCALAR, LAYOUT_V32, check
-from ._runtime import (BLOCK_N, FIXED_OVERHEAD, kv_geometry, num_sms, pick_num_sm_parts_fp32, pick_split, ptr,
+from ._lib import IMPL_AUTO, IMPL_SCALAR, LAYOUT_MODEL1, LAYOUT_V32, check
+from ._runtime import (BLOCK_N, FIXED_OVERHEAD, kv_geometry, num_sms, pick_num_sm_parts_exact, pick_num_sm_parts_fp32, pick_split, ptr,
                        require_cuda, resolve_impl, status_buffer, stream_ptr, tc_aligned)
 from .flash_ops import _check_q, _Extra, _layout, sparse_mla_prefill_fwd
 
@@ -128,9 +128,11 @@ def flash_mla_with_kvcache(
     if not meta.have_initialized:
         meta.have_initialized = True
         meta.config = cfg
-        fp32 = use_ext and (impl == IMPL_SCALAR or not tc_aligned(k_cache, ex.kv))
+        aligned = not use_ext or tc_aligned(k_cache, ex.kv)
         fixed_overhead = FIXED_OVERHEAD
-        if fp32:
+        if aligned and layout == LAYOUT_MODEL1 and impl == IMPL_SCALAR:
+            meta.num_sm_parts = pick_num_sm_parts_exact(num_tokens, num_heads, num_sms(q.device), blocks)
+        elif use_ext and (impl == IMPL_SCALAR or not aligned):
             meta.num_sm_parts = pick_num_sm_parts_fp32(num_tokens, num_heads, num_sms(q.device))
         else:
             meta.num_sm_parts, fixed_overhead = pick_split(num_tokens, num_sms(q.device), blocks,
