@@ -1,12 +1,12 @@
-"""ctypes binding of libsmla_b200.so.  There is no CPU fallback: if the library is missing
-the import of any op raises."""
+"""Binding of libsmla_b200.so: ctypes prototypes of every entry point, and the extension _smla_native through which the ops
+call it.  There is no CPU fallback: if either is missing the first op raises ImportError."""
 from __future__ import annotations
 
 import ctypes
 import os
 from ctypes import c_char_p, c_float, c_int, c_int64, c_size_t, c_void_p
 
-from .build import LIB_PATH
+from .build import LIB_PATH, NATIVE_PATH
 
 IMPL_AUTO, IMPL_SCALAR, IMPL_TC = 0, 1, 2
 LAYOUT_V32, LAYOUT_MODEL1 = 0, 1
@@ -82,6 +82,22 @@ def load():
 
 class SmlaError(RuntimeError):
     pass
+
+
+_native = None
+
+
+def native():
+    """The extension that holds the host side of the ops (csrc/native.cpp), bound to the loaded library."""
+    global _native
+    if _native is None:
+        lib = load()
+        if not os.path.exists(NATIVE_PATH):
+            raise ImportError(f"{NATIVE_PATH} is missing: build it with `python -m sparse_mla_sm120_b200.build`")
+        from . import _runtime, _smla_native
+        _smla_native.init(lib._handle, _runtime, SmlaError)
+        _native = _smla_native
+    return _native
 
 
 def check(rc: int) -> None:

@@ -190,6 +190,25 @@ def pick_split(num_tokens: int, sms: int, blocks_per_token: Optional[int] = None
     return best[1], best[2]
 
 
+def split_plan(device: int, num_tokens: int, num_heads: int, blocks: int, uniform: int, layout: int, ext: int, aligned: int,
+               impl: int) -> Tuple[int, int, int]:
+    """(partitions, the scheduler's fixed overhead, equal partitions per request) of a decode step: the one choice that
+    the ops make.  A third value above 1 means that requests of equal length are cut into that many equal partitions each
+    and the attention kernel derives the schedule itself (smla_decode_uniform).  ``ext``: MODEL1 or a second cache."""
+    if num_tokens == 0:
+        return 0, FIXED_OVERHEAD, 0
+    sms = num_sms(torch.device("cuda", device))
+    if ext and aligned and layout == _lib.LAYOUT_MODEL1 and impl == _lib.IMPL_SCALAR:
+        return pick_num_sm_parts_exact(num_tokens, num_heads, sms, blocks), FIXED_OVERHEAD, 0
+    if ext and (impl == _lib.IMPL_SCALAR or not aligned):
+        return pick_num_sm_parts_fp32(num_tokens, num_heads, sms), FIXED_OVERHEAD, 0
+    parts, overhead = pick_split(num_tokens, sms, blocks, uniform=bool(uniform))
+    k = parts // num_tokens
+    equal = (uniform and not ext and impl != _lib.IMPL_SCALAR and overhead == 0 and k > 1 and k * num_tokens == parts
+             and blocks % k == 0)
+    return parts, overhead, k if equal else 0
+
+
 _SCRATCH_LIMIT = 64      # cached call shapes per process before the least recently used one is dropped
 
 
@@ -233,6 +252,10 @@ def status_buffer(device: torch.device) -> torch.Tensor:
     if idx not in _status:
         _status[idx] = torch.zeros(4, dtype=torch.int32, device=device)
     return _status[idx]
+
+
+def status_pointer(index: int) -> int:
+    return status_buffer(torch.device("cuda", index)).data_ptr()
 
 
 def check_status(device: Optional[torch.device] = None) -> None:

@@ -17,9 +17,8 @@ from typing import Optional, Tuple
 import torch
 
 from . import _lib
-from ._lib import IMPL_AUTO, IMPL_SCALAR, LAYOUT_MODEL1, LAYOUT_V32, check
-from ._runtime import (BLOCK_N, FIXED_OVERHEAD, kv_geometry, kv_layout, num_sms, pick_num_sm_parts_exact, pick_num_sm_parts_fp32, pick_split, ptr,
-                       require_cuda, resolve_impl, scratch, status_buffer, stream_ptr, tc_aligned)
+from ._lib import IMPL_AUTO, LAYOUT_MODEL1, LAYOUT_V32, check, native
+from ._runtime import kv_geometry, kv_layout, ptr, require_cuda, resolve_impl, status_buffer, stream_ptr
 
 
 def _check_q(q: torch.Tensor):
@@ -164,87 +163,8 @@ def sparse_mla_decode_fwd(
     extra_topk_length name a second cache whose rows join the same softmax.
     Returns (out [T, H, 512] bf16, lse [T, H] fp32, base-2 LSE of the scaled logits).
     Signature and results follow flash_mla_sm120/ops.py:48-119."""
-    _check_q(q)
-    layout = _layout(q, kv_cache)
-    impl = resolve_impl(impl, layout)
-    page_block_size, page_stride = kv_geometry(kv_cache)
-    if d_v != 512:
-        raise ValueError(f"d_v must be 512, got {d_v}")
-    num_tokens, num_heads, _ = q.shape
-    topk = indices.shape[-1]
-    assert indices.dtype == torch.int32 and indices.is_contiguous()
-    ex = _Extra(layout, num_tokens, extra_k_cache, extra_indices, extra_topk, extra_topk_length)
-    require_cuda(q, kv_cache, indices)
-    use_ext = layout != LAYOUT_V32 or ex.topk > 0
-    blocks = max(-(-topk // BLOCK_N), 1) + -(-ex.topk // BLOCK_N)
-
-    fixed_overhead = FIXED_OVERHEAD
-    if num_sm_parts is None:
-        aligned = not use_ext or tc_aligned(kv_cache, ex.kv)
-        if aligned and layout == LAYOUT_MODEL1 and impl == IMPL_SCALAR:
-            num_sm_parts = pick_num_sm_parts_exact(num_tokens, num_heads, num_sms(q.device), blocks)
-        elif use_ext and (impl == IMPL_SCALAR or not aligned):
-            num_sm_parts = pick_num_sm_parts_fp32(num_tokens, num_heads, num_sms(q.device))
-        else:   # requests of equal length (no topk_length, no second cache) may be cut into equal partitions
-            num_sm_parts, fixed_overhead = pick_split(num_tokens, num_sms(q.device), blocks,
-                                                      uniform=topk_length is None and ex.topk == 0)
-    lib = _lib.load()
-    stream = stream_ptr(q.device)
-    if out is not None:
-        output = out.view(num_tokens, num_heads, d_v)
-    else:
-        output = torch.empty((num_tokens, num_heads, d_v), dtype=torch.bfloat16, device=q.device)
-    out_lse = torch.empty((num_tokens, num_heads), dtype=torch.float32, device=q.device)
-    if use_ext:
-        st = ptr(status_buffer(q.device))
-        if num_sm_parts == num_tokens:
-            check(lib.smla_prefill_ext(
-                ptr(q), ptr(kv_cache), ptr(indices), ptr(ex.kv), ptr(ex.indices), ptr(output), ptr(out_lse), None,
-                num_tokens, num_heads, topk, ex.topk, float(sm_scale), layout, page_block_size, page_stride,
-                ex.block, ex.stride, ptr(attn_sink), ptr(topk_length), ptr(ex.length), impl, st, stream))
-            return output, out_lse
-        ws = scratch(q.device, num_tokens + num_sm_parts, num_heads, num_tokens, num_sm_parts)
-        check(lib.smla_sched_meta(num_tokens, topk, ex.topk, num_sm_parts, fixed_overhead, ptr(topk_length),
-                                  ptr(ex.length), ptr(ws["sched_meta"]), ptr(ws["num_splits"]), stream))
-        check(lib.smla_decode_splitkv_ext(
-            ptr(q), ptr(kv_cache), ptr(indices), ptr(ex.kv), ptr(ex.indices), ptr(ws["o_accum"]),
-            ptr(ws["lse_accum"]), ptr(output), ptr(out_lse), ptr(ws["sched_meta"]), ptr(ws["num_splits"]),
-            num_tokens, num_heads, topk, ex.topk, float(sm_scale), layout, page_block_size, page_stride,
-            ex.block, ex.stride, num_sm_parts, ptr(attn_sink), ptr(topk_length), ptr(ex.length), impl, st, stream))
-        check(lib.smla_combine(ptr(ws["o_accum"]), ptr(ws["lse_accum"]), ptr(output), ptr(out_lse),
-                               ptr(ws["num_splits"]), num_tokens, num_heads, min(blocks, num_sm_parts),
-                               ptr(attn_sink), stream))
-        return output, out_lse
-    if num_sm_parts == num_tokens:
-        # One partition per request: nothing is split, so neither the scheduler nor the combine
-        # has anything to decide; the attention kernel derives the trivial schedule itself.
-        check(lib.smla_prefill(
-            ptr(q), ptr(kv_cache), ptr(indices), ptr(output), ptr(out_lse), None, num_tokens, num_heads,
-            topk, float(sm_scale), page_block_size, page_stride, ptr(attn_sink), ptr(topk_length), impl,
-            ptr(status_buffer(q.device)), stream))
-        return output, out_lse
-    total_splits = num_tokens + num_sm_parts
-    ws = scratch(q.device, total_splits, num_heads, num_tokens, num_sm_parts)
-    if (fixed_overhead == 0 and topk_length is None and impl != IMPL_SCALAR and num_sm_parts % num_tokens == 0
-            and blocks % (num_sm_parts // num_tokens) == 0):
-        # requests of equal length in equal partitions: the attention kernel derives the schedule itself, the step is
-        # two launches (attention, combine)
-        check(lib.smla_decode_uniform(
-            ptr(q), ptr(kv_cache), ptr(indices), ptr(ws["o_accum"]), ptr(ws["lse_accum"]), ptr(output), ptr(out_lse),
-            num_tokens, num_heads, topk, float(sm_scale), page_block_size, page_stride, num_sm_parts // num_tokens,
-            ptr(attn_sink), impl, ptr(status_buffer(q.device)), stream))
-        return output, out_lse
-    check(lib.smla_sched_meta(num_tokens, topk, 0, num_sm_parts, fixed_overhead, ptr(topk_length), None,
-                              ptr(ws["sched_meta"]), ptr(ws["num_splits"]), stream))
-    check(lib.smla_decode_splitkv(
-        ptr(q), ptr(kv_cache), ptr(indices), ptr(ws["o_accum"]), ptr(ws["lse_accum"]), ptr(output), ptr(out_lse),
-        ptr(ws["sched_meta"]), ptr(ws["num_splits"]), num_tokens, num_heads, topk, float(sm_scale),
-        page_block_size, page_stride, num_sm_parts, ptr(attn_sink), ptr(topk_length), impl,
-        ptr(status_buffer(q.device)), stream))
-    max_nsplits = min(max(-(-topk // BLOCK_N), 1), num_sm_parts)
-    check(lib.smla_combine(ptr(ws["o_accum"]), ptr(ws["lse_accum"]), ptr(output), ptr(out_lse),
-                           ptr(ws["num_splits"]), num_tokens, num_heads, max_nsplits, ptr(attn_sink), stream))
-    return output, out_lse
+    return native().decode(q, kv_cache, indices, sm_scale, d_v, attn_sink, extra_k_cache, extra_indices, topk_length,
+                           extra_topk_length, extra_topk or 0, out, impl, num_sm_parts)
 
 
 def sparse_mla_prefill_fwd(
@@ -266,31 +186,5 @@ def sparse_mla_prefill_fwd(
 
     Returns (out [T, H, 512] bf16, max_logits [T, H] fp32, lse [T, H] fp32), as
     flash_mla_sm120/ops.py:122-165."""
-    _check_q(q)
-    layout = _layout(q, kv_cache)
-    impl = resolve_impl(impl, layout)
-    page_block_size, page_stride = kv_geometry(kv_cache)
-    require_cuda(q, kv_cache, indices)
-    if d_v != 512:
-        raise ValueError(f"d_v must be 512, got {d_v}")
-    num_tokens, num_heads, _ = q.shape
-    topk = indices.shape[-1]
-    assert indices.dtype == torch.int32 and indices.is_contiguous()
-    if out is not None:
-        output = out.view(num_tokens, num_heads, d_v)
-    else:
-        output = torch.empty((num_tokens, num_heads, d_v), dtype=torch.bfloat16, device=q.device)
-    lse = torch.empty((num_tokens, num_heads), dtype=torch.float32, device=q.device)
-    max_logits = torch.empty((num_tokens, num_heads), dtype=torch.float32, device=q.device)
-    ex = _Extra(layout, num_tokens, extra_k_cache, extra_indices, extra_topk)
-    if layout != LAYOUT_V32 or ex.topk:
-        check(_lib.load().smla_prefill_ext(
-            ptr(q), ptr(kv_cache), ptr(indices), ptr(ex.kv), ptr(ex.indices), ptr(output), ptr(lse), ptr(max_logits),
-            num_tokens, num_heads, topk, ex.topk, float(sm_scale), layout, page_block_size, page_stride, ex.block,
-            ex.stride, ptr(attn_sink), ptr(topk_length), None, impl, ptr(status_buffer(q.device)), stream_ptr(q.device)))
-        return output, max_logits, lse
-    check(_lib.load().smla_prefill(
-        ptr(q), ptr(kv_cache), ptr(indices), ptr(output), ptr(lse), ptr(max_logits), num_tokens, num_heads,
-        topk, float(sm_scale), page_block_size, page_stride, ptr(attn_sink), ptr(topk_length), impl,
-        ptr(status_buffer(q.device)), stream_ptr(q.device)))
-    return output, max_logits, lse
+    return native().prefill(q, kv_cache, indices, sm_scale, d_v, attn_sink, topk_length, out, extra_k_cache, extra_indices,
+                            extra_topk or 0, impl)

@@ -10,9 +10,7 @@ from typing import Optional
 
 import torch
 
-from . import _lib
-from ._lib import IMPL_AUTO, check
-from ._runtime import ptr, require_cuda, status_buffer, stream_ptr
+from ._lib import IMPL_AUTO, native
 
 
 def fp8_mqa_logits(q: torch.Tensor, k: torch.Tensor, k_scale: torch.Tensor, weights: torch.Tensor,
@@ -22,21 +20,7 @@ def fp8_mqa_logits(q: torch.Tensor, k: torch.Tensor, k_scale: torch.Tensor, weig
 
     q [s_q, H, 128] float8_e4m3fn, k [s_k, 128] float8_e4m3fn, k_scale [s_k] fp32,
     weights [s_q, H] fp32, ks / ke [s_q] int32 -> logits [s_q, s_k] fp32."""
-    require_cuda(q, k, k_scale, weights, ks, ke, out)
-    if q.dtype != torch.float8_e4m3fn or k.dtype != torch.float8_e4m3fn:
-        raise ValueError("q and k must be float8_e4m3fn")
-    if q.dim() != 3 or k.dim() != 2 or q.shape[-1] != 128 or k.shape[-1] != 128:
-        raise ValueError("q must be [s_q, H, 128] and k [s_k, 128]")
-    assert q.is_contiguous() and k.is_contiguous() and weights.is_contiguous() and k_scale.is_contiguous()
-    assert ks.dtype == torch.int32 and ke.dtype == torch.int32
-    s_q, h, _ = q.shape
-    s_k = k.shape[0]
-    if out is None:
-        out = torch.empty((s_q, s_k), dtype=torch.float32, device=q.device)
-    check(_lib.load().smla_mqa_logits(ptr(q), ptr(k), ptr(k_scale), ptr(weights), ptr(ks), ptr(ke), ptr(out),
-                                      s_q, h, s_k, out.stride(0), impl, ptr(status_buffer(q.device)),
-                                      stream_ptr(q.device)))
-    return out
+    return native().mqa_logits(q, k, k_scale, weights, ks, ke, out, impl)
 
 
 def topk_indices(logits: torch.Tensor, ks: Optional[torch.Tensor], ke: Optional[torch.Tensor],
@@ -45,20 +29,9 @@ def topk_indices(logits: torch.Tensor, ks: Optional[torch.Tensor], ke: Optional[
     padded with -1 when fewer than k candidates exist.  Ties at the k-th value go to the lowest
     columns.  The order inside a row is a fixed function of the input but not ascending, and not
     part of the contract.  Rows of any width."""
-    require_cuda(logits, ks, ke)
-    assert logits.dim() == 2 and logits.dtype == torch.float32 and logits.stride(1) == 1
-    rows, cols = logits.shape
-    out = torch.empty((rows, k), dtype=torch.int32, device=logits.device)
-    check(_lib.load().smla_topk(ptr(logits), ptr(ks), ptr(ke), ptr(out), rows, cols, logits.stride(0), k,
-                                stream_ptr(logits.device)))
-    return out
+    return native().topk(logits, ks, ke, k)
 
 
 def pack_kv_cache(kv_bf16: torch.Tensor) -> torch.Tensor:
     """bf16 [..., 576] -> packed uint8 [..., 656] (512 e4m3 | 4 fp32 power-of-two scales | 64 bf16)."""
-    require_cuda(kv_bf16)
-    assert kv_bf16.dtype == torch.bfloat16 and kv_bf16.shape[-1] == 576 and kv_bf16.is_contiguous()
-    rows = kv_bf16.numel() // 576
-    out = torch.empty(kv_bf16.shape[:-1] + (656,), dtype=torch.uint8, device=kv_bf16.device)
-    check(_lib.load().smla_pack_kv(ptr(kv_bf16), ptr(out), rows, stream_ptr(kv_bf16.device)))
-    return out
+    return native().pack_kv(kv_bf16)

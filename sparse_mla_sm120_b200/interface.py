@@ -24,9 +24,9 @@ from typing import Optional, Tuple
 import torch
 
 from . import _lib
-from ._lib import IMPL_AUTO, IMPL_SCALAR, LAYOUT_MODEL1, LAYOUT_V32, check
-from ._runtime import (BLOCK_N, FIXED_OVERHEAD, kv_geometry, num_sms, pick_num_sm_parts_exact, pick_num_sm_parts_fp32, pick_split, ptr,
-                       require_cuda, resolve_impl, status_buffer, stream_ptr, tc_aligned)
+from ._lib import IMPL_AUTO, IMPL_SCALAR, LAYOUT_V32, check
+from ._runtime import (BLOCK_N, kv_geometry, ptr, require_cuda, resolve_impl, split_plan, status_buffer, stream_ptr,
+                       tc_aligned)
 from .flash_ops import _check_q, _Extra, _layout, sparse_mla_prefill_fwd
 
 
@@ -129,18 +129,9 @@ def flash_mla_with_kvcache(
         meta.have_initialized = True
         meta.config = cfg
         aligned = not use_ext or tc_aligned(k_cache, ex.kv)
-        fixed_overhead = FIXED_OVERHEAD
-        if aligned and layout == LAYOUT_MODEL1 and impl == IMPL_SCALAR:
-            meta.num_sm_parts = pick_num_sm_parts_exact(num_tokens, num_heads, num_sms(q.device), blocks)
-        elif use_ext and (impl == IMPL_SCALAR or not aligned):
-            meta.num_sm_parts = pick_num_sm_parts_fp32(num_tokens, num_heads, num_sms(q.device))
-        else:
-            meta.num_sm_parts, fixed_overhead = pick_split(num_tokens, num_sms(q.device), blocks,
-                                                           uniform=topk_length is None and ex.topk == 0)
+        meta.num_sm_parts, fixed_overhead, meta.uniform_k = split_plan(
+            q.device.index, num_tokens, num_heads, blocks, topk_length is None and ex.topk == 0, layout, use_ext, aligned, impl)
         meta.max_nsplits = min(blocks, meta.num_sm_parts)
-        if (not use_ext and fixed_overhead == 0 and impl != IMPL_SCALAR and meta.num_sm_parts > num_tokens
-                and meta.num_sm_parts % num_tokens == 0 and blocks % (meta.num_sm_parts // num_tokens) == 0):
-            meta.uniform_k = meta.num_sm_parts // num_tokens
         if meta.num_sm_parts != num_tokens:
             meta.tile_scheduler_metadata = torch.empty(meta.num_sm_parts * 8, dtype=torch.int32, device=q.device)
             meta.num_splits = torch.empty(num_tokens + 1, dtype=torch.int32, device=q.device)
