@@ -213,6 +213,22 @@ int smla_topk(const float* logits, const int32_t* ks, const int32_t* ke, int32_t
               int num_rows, int num_cols, int64_t logits_stride, int k, void* stream);
 
 /*
+ * The same selection written as physical cache rows: column c of row i becomes
+ * block_table[i * table_stride + c / page_size] * page_size + c % page_size (-1 for a position past the table's
+ * table_pages pages, and as padding).
+ */
+int smla_topk_paged(const float* logits, const int32_t* ks, const int32_t* ke, int32_t* out_rows, int num_rows, int num_cols,
+                    int64_t logits_stride, int k, const int32_t* block_table, int64_t table_stride, int table_pages,
+                    int page_size, void* stream);
+
+/*
+ * Up to SMLA_COPY_BATCH_MAX device-to-device copies as one launch (the inputs of a step into the buffers of its captured
+ * graph).  The ranges must not overlap.
+ */
+#define SMLA_COPY_BATCH_MAX 8
+int smla_copy_batch(int n, void* const* dst, const void* const* src, const int64_t* bytes, void* stream);
+
+/*
  * Context-parallel index partition: keeps, in order, the entries of each row that fall in
  * [lo, hi), rebases them to lo, pads with -1 and writes the count to local_length.  No
  * counterpart in the reference (it has no multi-GPU path).

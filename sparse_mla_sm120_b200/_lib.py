@@ -51,6 +51,9 @@ _SIGS = {
     "smla_mqa_logits": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                 c_int, c_int, c_int, c_int64, c_int, c_void_p, c_void_p]),
     "smla_topk": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int64, c_int, c_void_p]),
+    "smla_topk_paged": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int64, c_int, c_void_p, c_int64, c_int,
+                                c_int, c_void_p]),
+    "smla_copy_batch": (c_int, [c_int, c_void_p, c_void_p, c_void_p, c_void_p]),
     "smla_cp_partition_indices": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p]),
     "smla_cp_local_window": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p]),
     "smla_cp_candidates": (c_int, [c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p]),

@@ -422,7 +422,27 @@ int smla_topk(const float* logits, const int32_t* ks, const int32_t* ke, int32_t
     if (num_rows < 0 || num_cols < 0 || k < 0 || logits_stride < num_cols)
         return set_error(SMLA_E_SHAPE, "smla_topk: rows=%d cols=%d k=%d stride=%lld", num_rows, num_cols, k,
                          (long long)logits_stride);
-    return launch_topk(logits, ks, ke, out_indices, num_rows, num_cols, logits_stride, k, (cudaStream_t)stream);
+    return launch_topk(logits, ks, ke, out_indices, num_rows, num_cols, logits_stride, k, nullptr, 0, 0, 1, (cudaStream_t)stream);
+}
+
+int smla_topk_paged(const float* logits, const int32_t* ks, const int32_t* ke, int32_t* out_rows, int num_rows, int num_cols,
+                    int64_t logits_stride, int k, const int32_t* block_table, int64_t table_stride, int table_pages,
+                    int page_size, void* stream) {
+    if (!logits || !out_rows || !block_table) return set_error(SMLA_E_NULL, "smla_topk_paged: null pointer argument");
+    if (num_rows < 0 || num_cols < 0 || k < 0 || logits_stride < num_cols || table_pages < 0 || table_stride < table_pages || page_size < 1)
+        return set_error(SMLA_E_SHAPE, "smla_topk_paged: rows=%d cols=%d k=%d stride=%lld pages=%d of %d", num_rows, num_cols, k,
+                         (long long)logits_stride, table_pages, page_size);
+    return launch_topk(logits, ks, ke, out_rows, num_rows, num_cols, logits_stride, k, block_table, table_stride, table_pages, page_size,
+                       (cudaStream_t)stream);
+}
+
+int smla_copy_batch(int n, void* const* dst, const void* const* src, const int64_t* bytes, void* stream) {
+    if (n < 0 || n > SMLA_COPY_BATCH_MAX) return set_error(SMLA_E_SHAPE, "smla_copy_batch: %d copies, supported 0..%d", n, SMLA_COPY_BATCH_MAX);
+    for (int i = 0; i < n; ++i) {
+        if (bytes[i] < 0) return set_error(SMLA_E_SHAPE, "smla_copy_batch: negative size");
+        if (bytes[i] > 0 && (!dst[i] || !src[i])) return set_error(SMLA_E_NULL, "smla_copy_batch: null pointer argument");
+    }
+    return launch_copy_batch(n, dst, src, bytes, (cudaStream_t)stream);
 }
 
 int smla_cp_partition_indices(const int32_t* indices, int32_t* local_indices, int32_t* local_length,

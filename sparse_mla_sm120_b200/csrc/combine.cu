@@ -222,4 +222,34 @@ int launch_cp_unslice(const void* gathered, __nv_bfloat16* out, float* lse, int 
     return check_launch("cp_unslice_kernel");
 }
 
+namespace {
+struct CopyBatch {
+    uint8_t* dst[SMLA_COPY_BATCH_MAX];
+    const uint8_t* src[SMLA_COPY_BATCH_MAX];
+    int64_t bytes[SMLA_COPY_BATCH_MAX];
+};
+// blockIdx.y: which copy.  16 bytes per thread and step where both sides are aligned for it, single bytes otherwise and at the end.
+__global__ void __launch_bounds__(256) copy_batch_kernel(const CopyBatch c) {
+    const int k = blockIdx.y;
+    const int64_t n = c.bytes[k], step = (int64_t)gridDim.x * blockDim.x, t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const bool wide = ((reinterpret_cast<uintptr_t>(c.dst[k]) | reinterpret_cast<uintptr_t>(c.src[k])) & 15u) == 0;
+    const int64_t n16 = wide ? n >> 4 : 0;
+    for (int64_t i = t; i < n16; i += step) reinterpret_cast<uint4*>(c.dst[k])[i] = __ldg(reinterpret_cast<const uint4*>(c.src[k]) + i);
+    for (int64_t i = (n16 << 4) + t; i < n; i += step) c.dst[k][i] = c.src[k][i];
+}
+}  // namespace
+
+int launch_copy_batch(int n, void* const* dst, const void* const* src, const int64_t* bytes, cudaStream_t stream) {
+    CopyBatch c{};
+    int64_t most = 0;
+    for (int i = 0; i < n; ++i) {
+        c.dst[i] = static_cast<uint8_t*>(dst[i]); c.src[i] = static_cast<const uint8_t*>(src[i]); c.bytes[i] = bytes[i];
+        most = bytes[i] > most ? bytes[i] : most;
+    }
+    if (most == 0) return 0;
+    const int64_t blocks = (most + 256 * 16 * 2 - 1) / (256 * 16 * 2);      // two steps per thread of the largest copy
+    copy_batch_kernel<<<dim3((unsigned)(blocks < 1184 ? blocks : 1184), n), 256, 0, stream>>>(c);
+    return check_launch("copy_batch_kernel");
+}
+
 }  // namespace smla

@@ -140,7 +140,9 @@ int launch_mqa_logits_tc(const uint8_t* q, const uint8_t* k, const float* k_scal
                          const int32_t* ks, const int32_t* ke, float* logits, int s_q, int num_heads,
                          int s_k, int64_t logits_stride, int32_t* status, cudaStream_t stream);
 int launch_topk(const float* logits, const int32_t* ks, const int32_t* ke, int32_t* out, int num_rows,
-                int num_cols, int64_t logits_stride, int k, cudaStream_t stream);
+                int num_cols, int64_t logits_stride, int k, const int32_t* table, int64_t table_stride, int table_pages,
+                int page_size, cudaStream_t stream);
+int launch_copy_batch(int n, void* const* dst, const void* const* src, const int64_t* bytes, cudaStream_t stream);
 int launch_cp_partition(const int32_t* indices, int32_t* local_indices, int32_t* local_length,
                         int num_tokens, int topk, int lo, int hi, cudaStream_t stream);
 

@@ -55,8 +55,6 @@ mqa_logits_scalar_kernel(const uint8_t* __restrict__ q, const uint8_t* __restric
 
 // ---------------------------------------------------------------- top-k: radix select per row
 constexpr int TK_THREADS = 1024;
-constexpr int TK_WARPS = TK_THREADS / 32;
-constexpr int32_t TK_REDO = INT32_MIN;     // first output of a row that has more: the multi-pass kernel redoes the row
 
 __device__ __forceinline__ uint32_t order_key(float f) {   // larger float <=> larger key
     const uint32_t b = __float_as_uint(f);
@@ -90,20 +88,28 @@ __device__ __forceinline__ void for_each_key(const float* __restrict__ x, int lo
     for (int j = a1 + tid; j < hi; j += nthreads) fn(j, order_key(x[j]));
 }
 
-// One CTA of 1024 threads per row, so at most two rows per SM are in flight: a row of 65536
-// logits is 256 KB, the rows in flight (76 MB on 148 SMs) fit the L2 and only the first of the
-// passes over a row reaches DRAM.
-__global__ void __launch_bounds__(TK_THREADS, 1)
-topk_kernel(const float* __restrict__ logits, const int32_t* __restrict__ ks,
-            const int32_t* __restrict__ ke, int32_t* __restrict__ out, int num_cols,
-            int64_t logits_stride, int k, int only_flagged) {
-    // only_flagged: redo the rows that topk_select_kernel gave up on
-    if (only_flagged && out[(size_t)blockIdx.x * k] != TK_REDO) return;
+// What a selected column is written as: itself, or the physical cache row of that position through a page table.
+struct Emit {
+    const int32_t* table;      // [rows, table_stride] page numbers, or null
+    int64_t table_stride;
+    int table_pages, page_size;
+    __device__ __forceinline__ int32_t operator()(int row, int col) const {
+        if (table == nullptr) return col;
+        const int page = col / page_size;
+        return page < table_pages ? __ldg(table + (size_t)row * table_stride + page) * page_size + (col - page * page_size) : -1;
+    }
+};
+
+// Multi-pass radix select of one row by the whole CTA: any k, any distribution.  A row of 65536 logits is 256 KB; the rows in
+// flight fit the L2 and only the first of the passes over a row reaches DRAM.
+template <int THREADS>
+__device__ void topk_multipass(const float* __restrict__ logits, const int32_t* __restrict__ ks, const int32_t* __restrict__ ke,
+                               int32_t* __restrict__ out, int num_cols, int64_t logits_stride, int k, int row, const Emit& emit) {
+    constexpr int WARPS = THREADS / 32;
     __shared__ int hist[256];
     __shared__ int sel_bin, sel_need;
-    __shared__ int seg_gt[TK_WARPS], seg_eq[TK_WARPS];
-
-    const int row = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    __shared__ int seg_gt[WARPS], seg_eq[WARPS];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const float* x = logits + (size_t)row * logits_stride;
     int lo = ks ? max(ks[row], 0) : 0;
     int hi = ke ? min(ke[row], num_cols) : num_cols;
@@ -119,13 +125,13 @@ topk_kernel(const float* __restrict__ logits, const int32_t* __restrict__ ks,
     bool take_all = false;
     for (int pass = 0; pass < 4; ++pass) {
         const int shift = 24 - 8 * pass;
-        for (int b = tid; b < 256; b += TK_THREADS) hist[b] = 0;
+        for (int b = tid; b < 256; b += THREADS) hist[b] = 0;
         __syncthreads();
         auto count = [&](int, uint32_t key) {
             if (key > NEG_INF_KEY && (key & prefix_mask) == prefix) atomicAdd(&hist[(key >> shift) & 255], 1);
         };
-        if (vec_ok) for_each_key(x, lo, hi, tid, TK_THREADS, count);
-        else for (int j = lo + tid; j < hi; j += TK_THREADS) count(j, order_key(x[j]));
+        if (vec_ok) for_each_key(x, lo, hi, tid, THREADS, count);
+        else for (int j = lo + tid; j < hi; j += THREADS) count(j, order_key(x[j]));
         __syncthreads();
         if (tid == 0) {
             int cum = 0, b = 255;
@@ -150,7 +156,7 @@ topk_kernel(const float* __restrict__ logits, const int32_t* __restrict__ ks,
     // at the threshold, and after a scan over the warps writes them in column order: positions
     // [0, n_gt) hold the greater ones, [n_gt, n_gt + need_eq) the first need_eq ties.
     const int span = hi - lo;
-    const int seg = ((span + TK_WARPS - 1) / TK_WARPS + 31) & ~31;
+    const int seg = ((span + WARPS - 1) / WARPS + 31) & ~31;
     const int s0 = min(lo + warp * seg, hi), s1 = min(s0 + seg, hi);
     int c_gt = 0, c_eq = 0;
     for (int j = s0 + lane; j < s1; j += 32) {
@@ -163,7 +169,7 @@ topk_kernel(const float* __restrict__ logits, const int32_t* __restrict__ ks,
     if (lane == 0) { seg_gt[warp] = c_gt; seg_eq[warp] = c_eq; }
     __syncthreads();
     int off_gt = 0, off_eq = 0, n_gt = 0, n_eq = 0;
-    for (int w = 0; w < TK_WARPS; ++w) {
+    for (int w = 0; w < WARPS; ++w) {
         if (w < warp) { off_gt += seg_gt[w]; off_eq += seg_eq[w]; }
         n_gt += seg_gt[w]; n_eq += seg_eq[w];
     }
@@ -175,15 +181,22 @@ topk_kernel(const float* __restrict__ logits, const int32_t* __restrict__ ks,
         const bool gt = key > thr;
         const bool eq = (!take_all) && key == thr && j < s1;
         const uint32_t mg = __ballot_sync(0xffffffffu, gt), me = __ballot_sync(0xffffffffu, eq);
-        if (gt) o[off_gt + __popc(mg & below)] = j;
+        if (gt) o[off_gt + __popc(mg & below)] = emit(row, j);
         if (eq) {
             const int r = off_eq + __popc(me & below);
-            if (r < need_eq) o[n_gt + r] = j;
+            if (r < need_eq) o[n_gt + r] = emit(row, j);
         }
         off_gt += __popc(mg); off_eq += __popc(me);
     }
     const int filled = n_gt + (take_all ? 0 : min(need_eq, n_eq));
-    for (int r = filled + tid; r < k; r += TK_THREADS) o[r] = -1;
+    for (int r = filled + tid; r < k; r += THREADS) o[r] = -1;
+}
+
+// For k beyond the one-read selection.
+__global__ void __launch_bounds__(TK_THREADS, 1)
+topk_kernel(const float* __restrict__ logits, const int32_t* __restrict__ ks, const int32_t* __restrict__ ke,
+            int32_t* __restrict__ out, int num_cols, int64_t logits_stride, int k, const Emit emit) {
+    topk_multipass<TK_THREADS>(logits, ks, ke, out, num_cols, logits_stride, k, blockIdx.x, emit);
 }
 
 // Warp 0: the highest of 256 bins at which the count cumulated from the top reaches `need`
@@ -224,7 +237,7 @@ __device__ __forceinline__ void pick_bin(const int* hist, int need, int lane, in
 // but the candidates is kept on chip), and two CTAs fit an SM, so the read of one row overlaps
 // the selection of another.  When the guess fails -- fewer than k candidates, a list overflows
 // (heavy ties, logits that cluster far more than the sample saw), too many entries in the bin of
-// the k-th -- the row is marked for the multi-pass kernel.
+// the k-th -- the CTA selects by multi-pass radix select instead.
 //
 // The pass over the row is kept free of warp-wide votes: a lane compares its logits as floats
 // (NaNs never become candidates) and only notes a bit per entry; after a stretch of eight rounds
@@ -264,7 +277,7 @@ template <int TS_THREADS>
 __global__ void __launch_bounds__(TS_THREADS, 1024 / TS_THREADS)
 topk_select_kernel(const float* __restrict__ logits, const int32_t* __restrict__ ks,
                    const int32_t* __restrict__ ke, int32_t* __restrict__ out, int num_cols,
-                   int64_t logits_stride, int k) {
+                   int64_t logits_stride, int k, const Emit emit) {
     constexpr int TS_WARPS = TS_THREADS / 32;
     constexpr int TS_LIST = TS_CAND / TS_WARPS;        // candidates per warp
     constexpr int TS_BPT = TS_BINS / TS_THREADS;       // histogram bins per thread in the suffix sums
@@ -397,8 +410,8 @@ topk_select_kernel(const float* __restrict__ logits, const int32_t* __restrict__
     bool overflow = false;
 #pragma unroll
     for (int w = 0; w < TS_WARPS; ++w) { total += cw[w]; overflow |= cw[w] > TS_LIST; }
-    if (overflow || (sampled && total < k)) {  // (uniform) the guess failed: the multi-pass kernel redoes the row
-        if (tid == 0) o[0] = TK_REDO;
+    if (overflow || (sampled && total < k)) {  // (uniform) the guess failed
+        topk_multipass<TS_THREADS>(logits, ks, ke, out, num_cols, logits_stride, k, row, emit);
         return;
     }
     const int mycount = cnt;
@@ -475,7 +488,7 @@ topk_select_kernel(const float* __restrict__ logits, const int32_t* __restrict__
         }
         __syncthreads();
         if (n_eq_s > TS_EQ) {                  // (uniform)
-            if (tid == 0) o[0] = TK_REDO;
+            topk_multipass<TS_THREADS>(logits, ks, ke, out, num_cols, logits_stride, k, row, emit);
             return;
         }
     }
@@ -517,10 +530,334 @@ topk_select_kernel(const float* __restrict__ logits, const int32_t* __restrict__
     for (int i0 = 0; i0 < mycount; i0 += 32) {
         const bool ch = (i0 + lane < mycount) && chosen(i0 + lane);
         const uint32_t mc = __ballot_sync(0xffffffffu, ch);
-        if (ch) o[off + __popc(mc & below)] = mine[i0 + lane];
+        if (ch) o[off + __popc(mc & below)] = emit(row, mine[i0 + lane]);
         off += __popc(mc);
     }
     for (int r = filled + tid; r < k; r += TS_THREADS) o[r] = -1;
+}
+
+// One row on a cluster of eight CTAs, for the few rows of a decode step (16 rows x 131072 columns: 23.7 us with one CTA per
+// row).  Same selection and same order of the output as topk_select_kernel<1024>: its 32 warps are "virtual warps" here,
+// four per CTA, each worked on by four warps that take two of the eight rounds of a stretch, so a lane has all of its share
+// of a 131072-column row (eight 16-byte loads) in flight at once.  Candidates and their keys stay in the CTA; the
+// histogram's 4096 bins are spread over the cluster (512 per CTA, counted by remote atomics), as are the suffix sum over
+// them and the output.  A handful of cluster barriers takes the place of reading the row with one SM's bandwidth.
+constexpr int TC_CTAS = 8, TC_THREADS = 512, TC_WARPS = TC_THREADS / 32;
+constexpr int TC_VW = 32 / TC_CTAS;              // virtual warps per CTA
+constexpr int TC_SUB = TC_WARPS / TC_VW;         // warps per virtual warp
+constexpr int TC_RPS = TS_ROUNDS / TC_SUB;       // rounds of a stretch per warp
+constexpr int TC_LIST = 1024;                    // candidates a virtual warp may have
+constexpr int TC_BINS = TS_BINS / TC_CTAS;       // bins per CTA: one per thread
+constexpr int TC_SMEM = TC_VW * TC_LIST * 8 + TC_BINS * 4 + TS_EQ * 8;
+static_assert(TC_BINS == TC_THREADS && TC_SUB * TC_RPS == TS_ROUNDS, "work split of the cluster kernel");
+
+__device__ __forceinline__ uint32_t smem_addr(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
+__device__ __forceinline__ uint32_t peer_addr(const void* p, uint32_t rank) {       // the same shared-memory location in another CTA
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr(p)), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void st_peer(uint32_t a, int v) { asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(a), "r"(v) : "memory"); }
+__device__ __forceinline__ int ld_peer(uint32_t a) {
+    int v;
+    asm volatile("ld.shared::cluster.b32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ int atom_add_peer(uint32_t a, int v) {
+    int old;
+    asm volatile("atom.shared::cluster.add.u32 %0, [%1], %2;" : "=r"(old) : "r"(a), "r"(v) : "memory");
+    return old;
+}
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+__global__ void __cluster_dims__(TC_CTAS, 1, 1) __launch_bounds__(TC_THREADS, 2)
+topk_cluster_kernel(const float* __restrict__ logits, const int32_t* __restrict__ ks, const int32_t* __restrict__ ke,
+                    int32_t* __restrict__ out, int num_cols, int64_t logits_stride, int k, const Emit emit) {
+    extern __shared__ __align__(16) uint8_t ts_smem[];
+    int* lists = reinterpret_cast<int*>(ts_smem);                               // [TC_VW][TC_LIST] candidate columns
+    uint32_t* keys = reinterpret_cast<uint32_t*>(lists + TC_VW * TC_LIST);      // their keys
+    int* hist = reinterpret_cast<int*>(keys + TC_VW * TC_LIST);                 // this CTA's bins (before that: the sample's two histograms)
+    uint32_t* eq_key = reinterpret_cast<uint32_t*>(hist + TC_BINS);             // entries of the k-th key's bin (CTA 0)
+    int* eq_col = reinterpret_cast<int*>(eq_key + TS_EQ);
+    __shared__ int sel_bin, sel_need;
+    __shared__ int part[TC_CTAS][4];             // of every CTA: candidates (-1: a list overflowed), smallest and largest key, then bin total
+    __shared__ int slice[TC_CTAS], chosen_in[TC_CTAS], found[2], n_eq_s;        // bin sums and chosen entries of every CTA; (bin, needed); entries of that bin (CTA 0)
+    __shared__ int lane_cnt[TC_WARPS][32], vw_cnt[TC_VW], vw_sel[TC_VW], wsum[TC_WARPS];
+    __shared__ uint32_t kmin_s, kmax_s, last_key_s;
+    __shared__ int last_col_s;
+
+    const int row = blockIdx.x / TC_CTAS, rank = blockIdx.x % TC_CTAS;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int vw = warp / TC_SUB, sub = warp % TC_SUB, vwarp = rank * TC_VW + vw;
+    const float* x = logits + (size_t)row * logits_stride;
+    int lo = ks ? max(ks[row], 0) : 0;
+    int hi = ke ? min(ke[row], num_cols) : num_cols;
+    if (hi < lo) hi = lo;
+    int32_t* o = out + (size_t)row * k;
+    const uint32_t NEG_INF_KEY = order_key(-INFINITY);
+    constexpr uint32_t VALID16 = 0x007fu;
+    const bool vec_ok = ((reinterpret_cast<size_t>(x) & 15) == 0);
+    const int base = lo & ~3, span = hi - lo;
+    const uint32_t below = (1u << lane) - 1u;
+
+    // ---- threshold from the sample of topk_select_kernel, by every CTA for itself
+    uint32_t t_lo = NEG_INF_KEY + 1u;
+    const bool sampled = (hi - base) > TS_DIRECT;
+    if (tid == 0) { n_eq_s = 0; kmin_s = 0xffffffffu; kmax_s = 0u; }
+    if (tid < TC_VW) vw_cnt[tid] = 0;
+    hist[tid] = 0;
+    __syncthreads();
+    if (sampled) {
+        const int run_stride = span / (TS_SAMPLE / 8);
+        uint32_t h[TS_SAMPLE / TC_THREADS];
+#pragma unroll
+        for (int r = 0; r < TS_SAMPLE / TC_THREADS; ++r) {
+            const int i = tid + TC_THREADS * r;
+            h[r] = order_key(x[lo + (i >> 3) * run_stride + (i & 7)]) >> 16;
+        }
+#pragma unroll
+        for (int r = 0; r < TS_SAMPLE / TC_THREADS; ++r)
+            if (h[r] > VALID16) atomicAdd(&hist[h[r] >> 8], 1);
+        __syncthreads();
+        const float m = (float)k * (float)TS_SAMPLE / (float)span;
+        const int need_s = (int)(m + 4.f * sqrtf(m)) + 4;
+        if (warp == 0) pick_bin(hist, need_s, lane, &sel_bin, &sel_need);
+        __syncthreads();
+        if (sel_bin >= 0) {
+            const uint32_t b1 = (uint32_t)sel_bin;
+            const int need1 = sel_need;
+#pragma unroll
+            for (int r = 0; r < TS_SAMPLE / TC_THREADS; ++r)
+                if (h[r] > VALID16 && (h[r] >> 8) == b1) atomicAdd(&hist[256 + (h[r] & 255u)], 1);
+            __syncthreads();
+            if (warp == 0) pick_bin(hist + 256, need1, lane, &sel_bin, &sel_need);
+            __syncthreads();
+            t_lo = max(((b1 << 8) | (uint32_t)sel_bin) << 16, NEG_INF_KEY + 1u);
+        }
+        __syncthreads();
+        hist[tid] = 0;
+    }
+    const float t_f = key_to_float(t_lo);
+
+    // ---- the pass over the CTA's part of the row
+    const int nblk = (hi - base + 127) >> 7;
+    int* mine = lists + vw * TC_LIST;
+    uint32_t* mykeys = keys + vw * TC_LIST;
+    const float4 none = make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
+    uint32_t vmin = 0xffffffffu, vmax = 0u;
+    int cnt = 0;                                 // entries of the virtual warp so far (beyond TC_LIST they are only counted)
+    for (int stretch = 0; stretch < nblk; stretch += TS_ROUNDS * 4 * 32) {
+        float4 f[TC_RPS * 4];
+        const int blk0 = stretch + sub * TC_RPS * 4 * 32 + vwarp;
+#pragma unroll
+        for (int u = 0; u < TC_RPS * 4; ++u) {
+            const int blk = blk0 + u * 32;
+            f[u] = blk < nblk ? load_row4(x, base + blk * 128 + 4 * lane, num_cols, vec_ok) : none;
+        }
+        uint32_t m = 0;                          // bit 4 u + e: entry e of the lane's float4 in block u
+#pragma unroll
+        for (int u = 0; u < TC_RPS * 4; ++u)
+            m |= (uint32_t)(f[u].x >= t_f) << (4 * u) | (uint32_t)(f[u].y >= t_f) << (4 * u + 1) |
+                 (uint32_t)(f[u].z >= t_f) << (4 * u + 2) | (uint32_t)(f[u].w >= t_f) << (4 * u + 3);
+        if (m != 0 && (blk0 == 0 || blk0 + (TC_RPS * 4 - 1) * 32 >= nblk - 1)) {      // the window's edges
+#pragma unroll
+            for (int b = 0; b < TC_RPS * 16; ++b) {
+                const int j = base + (blk0 + (b >> 2) * 32) * 128 + 4 * lane + (b & 3);
+                if (j < lo || j >= hi) m &= ~(1u << b);
+            }
+        }
+        const int c = __popc(m);
+        lane_cnt[warp][lane] = c;
+        asm volatile("bar.sync %0, %1;" ::"r"(1 + vw), "r"(TC_SUB * 32) : "memory");   // the warps of the virtual warp
+        int all = 0, before = 0;                 // this lane's entries in all of them, and in those of earlier rounds
+#pragma unroll
+        for (int q = 0; q < TC_SUB; ++q) {
+            const int n = lane_cnt[vw * TC_SUB + q][lane];
+            all += n;
+            before += q < sub ? n : 0;
+        }
+        int incl = all;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, incl, d);
+            if (lane >= d) incl += t;
+        }
+        int at = cnt + incl - all + before;
+#pragma unroll
+        for (int b = 0; b < TC_RPS * 16; ++b) {
+            if ((m >> b) & 1u) {
+                const float4 v = f[b >> 2];
+                const uint32_t key = order_key((b & 3) == 0 ? v.x : (b & 3) == 1 ? v.y : (b & 3) == 2 ? v.z : v.w);
+                if (at < TC_LIST) { mine[at] = base + (blk0 + (b >> 2) * 32) * 128 + 4 * lane + (b & 3); mykeys[at] = key; }
+                vmin = min(vmin, key); vmax = max(vmax, key);
+                ++at;
+            }
+        }
+        cnt += __shfl_sync(0xffffffffu, incl, 31);
+        asm volatile("bar.sync %0, %1;" ::"r"(1 + vw), "r"(TC_SUB * 32) : "memory");   // lane_cnt may be overwritten, the list is complete so far
+    }
+    vmin = __reduce_min_sync(0xffffffffu, vmin);
+    vmax = __reduce_max_sync(0xffffffffu, vmax);
+    if (lane == 0) {
+        if (vmin <= vmax) { atomicMin(&kmin_s, vmin); atomicMax(&kmax_s, vmax); }
+        if (sub == 0) vw_cnt[vw] = cnt;
+    }
+    cluster_barrier();                           // also: every CTA of the cluster runs, its shared memory may be written
+
+    // ---- what every CTA found, to every CTA
+    if (tid < TC_CTAS) {
+        int n = 0;
+        bool over = false;
+#pragma unroll
+        for (int v = 0; v < TC_VW; ++v) { n += vw_cnt[v]; over |= vw_cnt[v] > TC_LIST; }
+        const uint32_t a = peer_addr(&part[rank][0], (uint32_t)tid);
+        st_peer(a, over ? -1 : n);
+        st_peer(a + 4, (int)kmin_s);
+        st_peer(a + 8, (int)kmax_s);
+    }
+    cluster_barrier();
+    int total = 0;
+    bool overflow = false;
+    uint32_t kmin = 0xffffffffu, kmax = 0u;
+#pragma unroll
+    for (int r = 0; r < TC_CTAS; ++r) {
+        const int n = part[r][0];
+        overflow |= n < 0;
+        total += n;
+        kmin = min(kmin, (uint32_t)part[r][1]); kmax = max(kmax, (uint32_t)part[r][2]);
+    }
+    if (overflow || (sampled && total < k)) {    // (the same in all CTAs) the guess failed
+        if (rank == 0) topk_multipass<TC_THREADS>(logits, ks, ke, out, num_cols, logits_stride, k, row, emit);
+        return;
+    }
+    const bool take_all = total <= k;
+    const int mycount = vw_cnt[vw];
+    int thr_bin = -1, need_eq = 0, n_eq = 0, shift = 0;
+    bool by_value = false;
+    float vmin_f = 0.f, vscale = 0.f;
+    auto bin_of = [&](uint32_t key) -> int {
+        if (!by_value) return (int)((key - kmin) >> shift);
+        return min((int)((key_to_float(key) - vmin_f) * vscale), TS_BINS - 1);
+    };
+    if (!take_all) {
+        shift = max(0, 20 - (int)__clz((kmax - kmin) | 1u));
+        vmin_f = key_to_float(kmin);
+        const float vmax_f = key_to_float(kmax);
+        by_value = vmin_f < 0.f && vmax_f > 0.f && (vmax_f - vmin_f) < INFINITY;
+        vscale = by_value ? (float)TS_BINS / (vmax_f - vmin_f) : 0.f;
+        // ---- histogram: bin b is counted by CTA b / TC_BINS
+        for (int i = sub * 32 + lane; i < mycount; i += TC_SUB * 32) {
+            const int b = bin_of(mykeys[i]);
+            atom_add_peer(peer_addr(hist + b % TC_BINS, (uint32_t)(b / TC_BINS)), 1);
+        }
+        cluster_barrier();
+        // ---- the bin of the k-th: suffix sums over this CTA's bins, the sums of the CTAs above it added
+        const int h1 = hist[tid];
+        int suf = h1;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const int t = __shfl_down_sync(0xffffffffu, suf, d);
+            if (lane + d < 32) suf += t;
+        }
+        if (lane == 0) wsum[warp] = suf;
+        __syncthreads();
+        int above = suf - h1;
+#pragma unroll
+        for (int w = 0; w < TC_WARPS; ++w) above += (w > warp) ? wsum[w] : 0;
+        if (tid < TC_CTAS) {
+            int n = 0;
+#pragma unroll
+            for (int w = 0; w < TC_WARPS; ++w) n += wsum[w];
+            st_peer(peer_addr(&slice[rank], (uint32_t)tid), n);
+        }
+        cluster_barrier();
+#pragma unroll
+        for (int r = 0; r < TC_CTAS; ++r) above += (r > rank) ? slice[r] : 0;
+        if (above < k && above + h1 >= k) {      // exactly one thread of the cluster: total > k
+            for (uint32_t r = 0; r < TC_CTAS; ++r) {
+                const uint32_t a = peer_addr(&found[0], r);
+                st_peer(a, rank * TC_BINS + tid);
+                st_peer(a + 4, k - above);
+            }
+        }
+        cluster_barrier();
+        thr_bin = found[0];
+        need_eq = found[1];
+        // ---- the entries of that bin, listed in CTA 0
+        for (int i = sub * 32 + lane; i < mycount; i += TC_SUB * 32) {
+            const uint32_t key = mykeys[i];
+            if (bin_of(key) == thr_bin) {
+                const int at = atom_add_peer(peer_addr(&n_eq_s, 0), 1);
+                if (at < TS_EQ) { st_peer(peer_addr(eq_key + at, 0), (int)key); st_peer(peer_addr(eq_col + at, 0), mine[i]); }
+            }
+        }
+        cluster_barrier();
+        n_eq = ld_peer(peer_addr(&n_eq_s, 0));
+        if (n_eq > TS_EQ) {                      // (the same in all CTAs)
+            cluster_barrier();                   // CTA 0's counter has been read by everybody
+            if (rank == 0) topk_multipass<TC_THREADS>(logits, ks, ke, out, num_cols, logits_stride, k, row, emit);
+            return;
+        }
+        if (need_eq < n_eq) {                    // the last of them to be taken, in the order (key descending, column ascending)
+            if (rank != 0) {
+                for (int i = tid; i < n_eq; i += TC_THREADS) {
+                    eq_key[i] = (uint32_t)ld_peer(peer_addr(eq_key + i, 0));
+                    eq_col[i] = ld_peer(peer_addr(eq_col + i, 0));
+                }
+            }
+            __syncthreads();
+            for (int i = tid; i < n_eq; i += TC_THREADS) {
+                const uint32_t key = eq_key[i];
+                const int c = eq_col[i];
+                int rk = 0;
+                for (int j = 0; j < n_eq; ++j) rk += (eq_key[j] > key) || (eq_key[j] == key && eq_col[j] < c);
+                if (rk == need_eq - 1) { last_key_s = key; last_col_s = c; }
+            }
+            __syncthreads();
+        }
+    }
+    const bool all_eq = need_eq >= n_eq;
+    const uint32_t last_key = all_eq ? 0u : last_key_s;
+    const int last_col = all_eq ? 0x7fffffff : last_col_s;
+    auto chosen = [&](int i) -> bool {
+        if (take_all) return true;
+        const uint32_t key = mykeys[i];
+        const int bin = bin_of(key);
+        if (bin != thr_bin) return bin > thr_bin;
+        return key > last_key || (key == last_key && mine[i] <= last_col);
+    };
+    // ---- write: the virtual warps' lists one after the other, each by its first warp
+    if (sub == 0) {
+        int nsel = 0;
+        for (int i0 = 0; i0 < mycount; i0 += 32) {
+            const bool ch = (i0 + lane < mycount) && chosen(i0 + lane);
+            nsel += __popc(__ballot_sync(0xffffffffu, ch));
+        }
+        if (lane == 0) vw_sel[vw] = nsel;
+    }
+    __syncthreads();
+    if (tid < TC_CTAS) {
+        int n = 0;
+#pragma unroll
+        for (int v = 0; v < TC_VW; ++v) n += vw_sel[v];
+        st_peer(peer_addr(&chosen_in[rank], (uint32_t)tid), n);
+    }
+    cluster_barrier();                           // the last access to another CTA's shared memory lies before it
+    int off = 0, filled = 0;
+#pragma unroll
+    for (int r = 0; r < TC_CTAS; ++r) { if (r < rank) off += chosen_in[r]; filled += chosen_in[r]; }
+    if (sub == 0) {
+        for (int v = 0; v < vw; ++v) off += vw_sel[v];
+        for (int i0 = 0; i0 < mycount; i0 += 32) {
+            const bool ch = (i0 + lane < mycount) && chosen(i0 + lane);
+            const uint32_t mc = __ballot_sync(0xffffffffu, ch);
+            if (ch) o[off + __popc(mc & below)] = emit(row, mine[i0 + lane]);
+            off += __popc(mc);
+        }
+    }
+    for (int r = filled + rank * TC_THREADS + tid; r < k; r += TC_CTAS * TC_THREADS) o[r] = -1;
 }
 
 // ---------------------------------------------------------------- context-parallel partition
@@ -615,10 +952,12 @@ int launch_mqa_logits_scalar(const uint8_t* q, const uint8_t* k, const float* k_
 }
 
 int launch_topk(const float* logits, const int32_t* ks, const int32_t* ke, int32_t* out, int num_rows,
-                int num_cols, int64_t logits_stride, int k, cudaStream_t stream) {
+                int num_cols, int64_t logits_stride, int k, const int32_t* table, int64_t table_stride, int table_pages,
+                int page_size, cudaStream_t stream) {
     if (num_rows == 0 || k == 0) return 0;
+    const Emit emit{table, table_stride, table_pages, page_size};
     if (k > TS_KMAX) {
-        topk_kernel<<<num_rows, TK_THREADS, 0, stream>>>(logits, ks, ke, out, num_cols, logits_stride, k, 0);
+        topk_kernel<<<num_rows, TK_THREADS, 0, stream>>>(logits, ks, ke, out, num_cols, logits_stride, k, emit);
         return check_launch("topk_kernel");
     }
     static bool attr_set[64] = {};
@@ -628,18 +967,19 @@ int launch_topk(const float* logits, const int32_t* ks, const int32_t* ke, int32
     if (dev < 64 && !attr_set[dev]) {
         cudaError_t e = cudaFuncSetAttribute(topk_select_kernel<512>, cudaFuncAttributeMaxDynamicSharedMemorySize, TS_SMEM);
         if (e == cudaSuccess) e = cudaFuncSetAttribute(topk_select_kernel<1024>, cudaFuncAttributeMaxDynamicSharedMemorySize, TS_SMEM);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(topk_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM);
         if (e != cudaSuccess) return set_error((int)e, "topk_select_kernel: shared memory: %s", cudaGetErrorString(e));
         cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev);
         attr_set[dev] = true;
     }
-    if (num_rows <= sms[dev < 64 ? dev : 0])       // every row has an SM to itself
-        topk_select_kernel<1024><<<num_rows, 1024, TS_SMEM, stream>>>(logits, ks, ke, out, num_cols, logits_stride, k);
+    const int n = sms[dev < 64 ? dev : 0];
+    if (num_rows * TC_CTAS <= 2 * n)               // few rows: two CTAs of eight-CTA clusters per SM
+        topk_cluster_kernel<<<num_rows * TC_CTAS, TC_THREADS, TC_SMEM, stream>>>(logits, ks, ke, out, num_cols, logits_stride, k, emit);
+    else if (num_rows <= n)                        // every row has an SM to itself
+        topk_select_kernel<1024><<<num_rows, 1024, TS_SMEM, stream>>>(logits, ks, ke, out, num_cols, logits_stride, k, emit);
     else
-        topk_select_kernel<512><<<num_rows, 512, TS_SMEM, stream>>>(logits, ks, ke, out, num_cols, logits_stride, k);
-    if (const int rc = check_launch("topk_select_kernel")) return rc;
-    // rows the one-read kernel gave up on (it marks them) are redone by the multi-pass kernel
-    topk_kernel<<<num_rows, TK_THREADS, 0, stream>>>(logits, ks, ke, out, num_cols, logits_stride, k, 1);
-    return check_launch("topk_kernel");
+        topk_select_kernel<512><<<num_rows, 512, TS_SMEM, stream>>>(logits, ks, ke, out, num_cols, logits_stride, k, emit);
+    return check_launch("topk_select_kernel");
 }
 
 int launch_cp_partition(const int32_t* indices, int32_t* local_indices, int32_t* local_length,

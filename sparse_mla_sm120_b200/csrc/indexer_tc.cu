@@ -31,9 +31,9 @@ using namespace ptx;
 constexpr int LX_D = 128;            // head dim of the indexer (bytes per row)
 constexpr int LX_KT = 128;           // keys per tile
 constexpr int LX_QG = 4;             // queries per group
-constexpr int LX_EPI_WARPS = 16;
-constexpr int LX_LOAD_WARP = 16, LX_MMA_WARP = 17;
-constexpr int LX_THREADS = 18 * 32;
+constexpr int LX_EPI_WARPS = 16, LX_QPW = 2;   // epilogue warps: one set of eight per accumulator; queries per warp
+constexpr int LX_LOAD_WARP = LX_EPI_WARPS, LX_MMA_WARP = LX_EPI_WARPS + 1;
+constexpr int LX_THREADS = (LX_EPI_WARPS + 2) * 32;
 constexpr int LX_KSTAGE = 4;
 
 constexpr uint32_t LX_Q_OFF = 0;                              // q group: [<=256 rows x 128 B] K-major 128B swizzle
@@ -56,6 +56,8 @@ struct LogitsParams {
     int chunk_tiles;   // key tiles per work item (a work item: one query group x one run of key tiles)
 };
 
+// HEADS: 64 or 32 indexer heads.
+template <int HEADS>
 __global__ void __launch_bounds__(LX_THREADS, 1) mqa_logits_tc_kernel(const LogitsParams p, const __grid_constant__ CUtensorMap qmap,
                                                                       const __grid_constant__ CUtensorMap kmap) {
     extern __shared__ uint8_t smem_raw[];
@@ -66,11 +68,11 @@ __global__ void __launch_bounds__(LX_THREADS, 1) mqa_logits_tc_kernel(const Logi
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(sm + LX_MISC_OFF);
     auto bar = [&](int i) -> uint32_t { return base + LX_BAR_OFF + 8u * i; };
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int H = p.heads, N = LX_QG * H;
+    constexpr int H = HEADS, N = LX_QG * H;
 
     if (tid == 0) {
         for (int s = 0; s < LX_KSTAGE; ++s) { mbar_init(bar(LXB_KFULL + s), 1); mbar_init(bar(LXB_KEMPTY + s), 1); }
-        for (int b = 0; b < 2; ++b) { mbar_init(bar(LXB_DFULL + b), 1); mbar_init(bar(LXB_DEMPTY + b), LX_EPI_WARPS * 32); }
+        for (int b = 0; b < 2; ++b) { mbar_init(bar(LXB_DFULL + b), 1); mbar_init(bar(LXB_DEMPTY + b), LX_EPI_WARPS / 2); }
         mbar_init(bar(LXB_QFULL), 32);
         mbar_init(bar(LXB_QEMPTY), 1 + LX_EPI_WARPS);   // the MMAs have read q and every epilogue warp has seen the group's phase
         *abort_flag = 0;
@@ -112,72 +114,86 @@ __global__ void __launch_bounds__(LX_THREADS, 1) mqa_logits_tc_kernel(const Logi
 
     if (warp < LX_EPI_WARPS) {
         // =================================================================== epilogue
-        const int quarter = warp & 3, qp = warp >> 2;
-        const uint32_t lane_addr = tmem + ((uint32_t)(quarter * 32) << 16);
+        // Warp: TMEM lane quarter (32 keys of a tile), two queries of the group, and the accumulator (every other tile) that
+        // its set of eight looks after.
+        const int quarter = warp & 3, qh = (warp >> 2) & 1;
+        const uint32_t set = (uint32_t)warp >> 3;
+        const uint32_t lane_addr = tmem + ((uint32_t)(quarter * 32) << 16) + LX_QPW * qh * H + 256 * set;
         uint32_t it = 0, qn = 0;   // tiles and non-empty groups seen by this CTA
         bool ok = true;
         for (int w = blockIdx.x; w < num_items && ok; w += gridDim.x) {
             int g, t0, t1, j0, j1;
             item_range(w, g, t0, t1, j0, j1);
-            const float* wsm = reinterpret_cast<const float*>(sm + LX_W_OFF + (qn & 3u) * LX_W_BYTES);
-            const int q0 = g * LX_QG + qp;
-            const int ks0 = q0 < p.s_q ? p.ks[q0] : 0, ke0 = q0 < p.s_q ? p.ke[q0] : 0;
-            // columns of the item outside every tile the group needs are -inf: written here, 128 keys per pass
-            if (q0 < p.s_q) {
-                float* row = p.logits + (size_t)q0 * p.stride;
-                for (int j = j0 + quarter * 32 + lane; j < j1; j += 128)
-                    if (j < t0 * LX_KT || j >= t1 * LX_KT) row[j] = -INFINITY;
+            int ks_q[LX_QPW], ke_q[LX_QPW];
+            float* row[LX_QPW];
+#pragma unroll
+            for (int u = 0; u < LX_QPW; ++u) {
+                const int qi = g * LX_QG + LX_QPW * qh + u;
+                const bool have = qi < p.s_q;
+                ks_q[u] = have ? p.ks[qi] : 0;
+                ke_q[u] = have ? p.ke[qi] : 0;
+                row[u] = have ? p.logits + (size_t)qi * p.stride : nullptr;
+                // columns of the item outside every tile the group needs are -inf: written here, 128 keys per pass
+                if (have) {
+                    for (int j = j0 + quarter * 32 + lane; j < j1; j += 128)
+                        if (j < t0 * LX_KT || j >= t1 * LX_KT) row[u][j] = -INFINITY;
+                }
             }
-            if (t1 > t0) {
-                ok = mbar_wait(bar(LXB_QFULL), qn & 1u, abort_flag, 11);   // weights of the group are in shared memory
-                if (!ok) break;
-                // The loader may arm the next group only after this warp has seen this one: otherwise two phases
-                // of QFULL could complete before a slow epilogue warp waits for the first (a group of one or two
-                // tiles needs nothing from the epilogue), and its parity wait would then refer to a later phase.
-                __syncwarp();
-                if (lane == 0) mbar_arrive(bar(LXB_QEMPTY));
-                ++qn;
-            }
-            for (int t = t0; t < t1 && ok; ++t, ++it) {
-                const uint32_t b = it & 1u;
-                ok = mbar_wait_hot(bar(LXB_DFULL + b), (it >> 1) & 1u, abort_flag, 12);
+            if (t1 <= t0) continue;
+            ok = mbar_wait(bar(LXB_QFULL), qn & 1u, abort_flag, 11);   // weights of the group are in shared memory
+            if (!ok) break;
+            const float* wq = reinterpret_cast<const float*>(sm + LX_W_OFF + (qn & 3u) * LX_W_BYTES) + LX_QPW * qh * 64;
+            // The loader may arm the next group only after this warp has seen this one: otherwise two phases
+            // of QFULL could complete before a slow epilogue warp waits for the first (a group of one or two
+            // tiles needs nothing from the epilogue), and its parity wait would then refer to a later phase.
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar(LXB_QEMPTY));
+            ++qn;
+            // Chunks of 32 score columns; the tensor-memory load of the next chunk is in flight while one is reduced.
+            constexpr int NCH = LX_QPW * H / 32;
+#pragma unroll 1
+            for (int t = t0 + (int)((set ^ it) & 1u); t < t1; t += 2) {
+                const uint32_t n = it + (uint32_t)(t - t0);
+                ok = mbar_wait_hot(bar(LXB_DFULL + set), (n >> 1) & 1u, abort_flag, 12);
                 if (!ok) break;
                 tc_fence_after();
+                uint32_t d[2][32];
+                tmem_ld32(lane_addr, d[0]);
                 const int key = t * LX_KT + quarter * 32 + lane;
                 const float sc = key < p.s_k ? __ldg(p.k_scale + key) : 0.f;
-                // Chunks of 32 score columns of this warp's query (heads [0,32), [32,64)); the
-                // tensor-memory load of the next chunk is in flight while the current one is reduced,
-                // and four partial sums per chunk keep the FMA chains short.
-                float acc = 0.f;
-                const int nch = H >> 5;                          // 1 or 2 chunks
-                const uint32_t col0 = lane_addr + 256 * b + qp * H;
-                const float* wq = wsm + qp * 64;
-                uint32_t d0[32], d1[32];
-                tmem_ld32(col0, d0);
-                // two scores per instruction: packed fp32 FMAs (same products, same four partial sums
-                // as four scalar FMA chains)
-                auto reduce = [&](const uint32_t (&d)[32], int c) {
-                    uint64_t a01 = 0ull, a23 = 0ull;
+                float acc[LX_QPW];
+                uint64_t a01 = 0ull, a23 = 0ull;
 #pragma unroll
-                    for (int i = 0; i < 32; i += 4) {
-                        const ulonglong2 w4 = *reinterpret_cast<const ulonglong2*>(wq + c + i);      // (w0, w1), (w2, w3)
-                        fma_f32x2(a01, pack_f32x2(fmaxf(__uint_as_float(d[i + 0]), 0.f), fmaxf(__uint_as_float(d[i + 1]), 0.f)), w4.x);
-                        fma_f32x2(a23, pack_f32x2(fmaxf(__uint_as_float(d[i + 2]), 0.f), fmaxf(__uint_as_float(d[i + 3]), 0.f)), w4.y);
+                for (int c = 0; c < NCH; ++c) {
+                    tmem_wait_ld();
+                    if (c + 1 < NCH) {
+                        tmem_ld32(lane_addr + 32 * (c + 1), d[(c + 1) & 1]);
+                    } else {
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(bar(LXB_DEMPTY + set));     // every column of the tile is in registers
                     }
-                    float a0, a1, a2, a3;
-                    unpack_f32x2(a01, a0, a1);
-                    unpack_f32x2(a23, a2, a3);
-                    acc += (a0 + a1) + (a2 + a3);
-                };
-                tmem_wait_ld();
-                if (nch > 1) tmem_ld32(col0 + 32, d1);
-                reduce(d0, 0);
-                if (nch > 1) { tmem_wait_ld(); reduce(d1, 32); }
-                tc_fence_before();
-                mbar_arrive(bar(LXB_DEMPTY + b));
-                if (key < p.s_k && q0 < p.s_q)
-                    p.logits[(size_t)q0 * p.stride + key] = (key >= ks0 && key < ke0) ? acc * sc : -INFINITY;
+                    const uint32_t* v = d[c & 1];
+                    const float* wc = wq + (c / (H / 32)) * 64 + (c % (H / 32)) * 32;
+#pragma unroll
+                    for (int i = 0; i < 32; i += 4) {       // two scores per FMA
+                        const ulonglong2 w4 = *reinterpret_cast<const ulonglong2*>(wc + i);      // (w0, w1), (w2, w3)
+                        fma_f32x2(a01, pack_f32x2(fmaxf(__uint_as_float(v[i + 0]), 0.f), fmaxf(__uint_as_float(v[i + 1]), 0.f)), w4.x);
+                        fma_f32x2(a23, pack_f32x2(fmaxf(__uint_as_float(v[i + 2]), 0.f), fmaxf(__uint_as_float(v[i + 3]), 0.f)), w4.y);
+                    }
+                    if ((c + 1) % (H / 32) == 0) {
+                        float a0, a1, a2, a3;
+                        unpack_f32x2(a01, a0, a1);
+                        unpack_f32x2(a23, a2, a3);
+                        acc[c / (H / 32)] = (a0 + a1) + (a2 + a3);
+                        a01 = a23 = 0ull;
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < LX_QPW; ++u)
+                    if (key < p.s_k && row[u] != nullptr) row[u][key] = (key >= ks_q[u] && key < ke_q[u]) ? acc[u] * sc : -INFINITY;
             }
+            it += (uint32_t)(t1 - t0);
         }
     } else if (warp == LX_LOAD_WARP) {
         // =================================================================== loader
@@ -210,14 +226,14 @@ __global__ void __launch_bounds__(LX_THREADS, 1) mqa_logits_tc_kernel(const Logi
                     ok = mbar_wait_hot(bar(LXB_KEMPTY + st), ((it / LX_KSTAGE) - 1) & 1u, abort_flag, 14);
                     if (!ok) break;
                 }
-                if (lane == 0) {
+                if (elect_one()) {
                     mbar_arrive_expect_tx(bar(LXB_KFULL + st), LX_KT * LX_D);
                     tma_load_2d(base + LX_K_OFF + st * (LX_KT * 128), &kmap, 0, t * LX_KT, bar(LXB_KFULL + st));
                 }
             }
         }
-    } else if (warp == LX_MMA_WARP && lane == 0) {
-        // =================================================================== MMA issue (one thread)
+    } else if (warp == LX_MMA_WARP) {
+        // =================================================================== MMA issue (one elected lane)
         constexpr uint32_t HI = desc_hi(1024, (uint32_t)SWIZZLE_128B);
         const uint32_t idesc = instr_desc(FMT_E4M3, FMT_E4M3, false, false, 128, (uint32_t)N);
         const uint32_t q_lo = desc_lo(base + LX_Q_OFF, 16);
@@ -227,26 +243,30 @@ __global__ void __launch_bounds__(LX_THREADS, 1) mqa_logits_tc_kernel(const Logi
             int g, t0, t1, j0, j1;
             item_range(w, g, t0, t1, j0, j1);
             if (t1 <= t0) continue;
-            ok = mbar_wait_thread(bar(LXB_QFULL), qn & 1u, abort_flag, 15);
+            ok = mbar_wait_hot(bar(LXB_QFULL), qn & 1u, abort_flag, 15);
             if (!ok) break;
             ++qn;
             for (int t = t0; t < t1; ++t, ++it) {
                 const uint32_t st = it % LX_KSTAGE, b = it & 1u;
-                ok = mbar_wait_thread(bar(LXB_KFULL + st), (it / LX_KSTAGE) & 1u, abort_flag, 16);
+                ok = mbar_wait_hot(bar(LXB_KFULL + st), (it / LX_KSTAGE) & 1u, abort_flag, 16);
                 if (!ok) break;
                 if (it >= 2) {
-                    ok = mbar_wait_thread(bar(LXB_DEMPTY + b), ((it >> 1) - 1) & 1u, abort_flag, 17);
+                    ok = mbar_wait_hot(bar(LXB_DEMPTY + b), ((it >> 1) - 1) & 1u, abort_flag, 17);
                     if (!ok) break;
                 }
                 tc_fence_after();
                 const uint32_t k_lo = desc_lo(base + LX_K_OFF + st * (LX_KT * 128), 16);
+                if (elect_one()) {
 #pragma unroll
-                for (int ks = 0; ks < 4; ++ks)
-                    mma_f8(tmem + 256 * b, make_desc(k_lo + ks * 2, HI), make_desc(q_lo + ks * 2, HI), idesc, ks != 0);
-                tc_commit(bar(LXB_KEMPTY + st));
-                tc_commit(bar(LXB_DFULL + b));
+                    for (int ks = 0; ks < 4; ++ks)
+                        mma_f8(tmem + 256 * b, make_desc(k_lo + ks * 2, HI), make_desc(q_lo + ks * 2, HI), idesc, ks != 0);
+                    tc_commit(bar(LXB_KEMPTY + st));
+                    tc_commit(bar(LXB_DFULL + b));
+                }
+                __syncwarp();
             }
-            if (ok) tc_commit(bar(LXB_QEMPTY));
+            if (ok && elect_one()) tc_commit(bar(LXB_QEMPTY));
+            __syncwarp();
         }
     }
 
@@ -274,7 +294,8 @@ int launch_mqa_logits_tc(const uint8_t* q, const uint8_t* k, const float* k_scal
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 64 && !attr_set[dev]) {
-        const cudaError_t e = cudaFuncSetAttribute(mqa_logits_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LX_SMEM);
+        cudaError_t e = cudaFuncSetAttribute(mqa_logits_tc_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LX_SMEM);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(mqa_logits_tc_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LX_SMEM);
         if (e != cudaSuccess) return set_error((int)e, "mqa_logits_tc_kernel: shared memory: %s", cudaGetErrorString(e));
         cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev);
         attr_set[dev] = true;
@@ -319,7 +340,8 @@ int launch_mqa_logits_tc(const uint8_t* q, const uint8_t* k, const float* k_scal
     const int items = groups * ((tiles + chunk_tiles - 1) / chunk_tiles);
     LogitsParams p{q, k, k_scale, weights, ks, ke, logits, status, s_q, num_heads, s_k, logits_stride, chunk_tiles};
     const int grid = items < nsm ? items : nsm;
-    mqa_logits_tc_kernel<<<grid, LX_THREADS, LX_SMEM, stream>>>(p, qmap, kmap);
+    if (num_heads == 64) mqa_logits_tc_kernel<64><<<grid, LX_THREADS, LX_SMEM, stream>>>(p, qmap, kmap);
+    else mqa_logits_tc_kernel<32><<<grid, LX_THREADS, LX_SMEM, stream>>>(p, qmap, kmap);
     return check_launch("mqa_logits_tc_kernel");
 }
 

@@ -16,6 +16,7 @@
 #include <cstdarg>
 #include <map>
 #include <tuple>
+#include <vector>
 
 #include "../../include/smla.h"
 
@@ -33,6 +34,8 @@ struct Api {
     decltype(&smla_pack_kv) pack_kv;
     decltype(&smla_mqa_logits) mqa_logits;
     decltype(&smla_topk) topk;
+    decltype(&smla_topk_paged) topk_paged;
+    decltype(&smla_copy_batch) copy_batch;
 } api;
 PyObject* g_runtime = nullptr;      // module _runtime: split policy, status buffer, default numerics of MODEL1
 PyObject* g_error = nullptr;        // SmlaError
@@ -358,13 +361,20 @@ PyObject* mqa_logits(const Args& x) {
     return THPVariable_Wrap(out);
 }
 
-// (logits, ks, ke, k) -> indices
+// (logits, ks, ke, k, block_table, page_size) -> indices, or physical rows where there is a block table
 PyObject* topk(const Args& x) {
-    const at::Tensor logits = x.needed(0), ks = x.tensor(1), ke = x.tensor(2);
+    const at::Tensor logits = x.needed(0), ks = x.tensor(1), ke = x.tensor(2), table = x.tensor(4);
     const int64_t k = x.integer(3);
-    require_cuda({&logits, &ks, &ke});
+    require_cuda({&logits, &ks, &ke, &table});
     require(logits.dim() == 2 && logits.scalar_type() == at::kFloat && logits.stride(1) == 1);
     const at::Tensor out = at::empty({logits.size(0), k}, logits.options().dtype(at::kInt));
+    if (table.defined()) {
+        require(table.dim() == 2 && table.scalar_type() == at::kInt && table.stride(1) == 1 && table.size(0) == logits.size(0));
+        check(api.topk_paged(ptr_as<float>(logits), ptr_as<int32_t>(ks), ptr_as<int32_t>(ke), ptr_as<int32_t>(out), (int)logits.size(0),
+                             (int)logits.size(1), logits.stride(0), (int)k, ptr_as<int32_t>(table), table.size(0) > 1 ? table.stride(0) : table.size(1),
+                             (int)table.size(1), (int)x.integer(5), stream_of(logits)));
+        return THPVariable_Wrap(out);
+    }
     check(api.topk(ptr_as<float>(logits), ptr_as<int32_t>(ks), ptr_as<int32_t>(ke), ptr_as<int32_t>(out), (int)logits.size(0),
                    (int)logits.size(1), logits.stride(0), (int)k, stream_of(logits)));
     return THPVariable_Wrap(out);
@@ -382,6 +392,42 @@ PyObject* pack_kv(const Args& x) {
     return THPVariable_Wrap(out);
 }
 
+// (destinations, sources): sequences of tensors, each source copied into its destination as Tensor.copy_ does.  Those
+// that are plain device copies (same type, shape and device, contiguous) go as one launch.
+PyObject* copy_into(const Args& x) {
+    PyObject* d = PySequence_Fast(x.a[0], "destinations must be a sequence");
+    if (d == nullptr) throw Failure();
+    PyObject* s = PySequence_Fast(x.a[1], "sources must be a sequence");
+    if (s == nullptr) { Py_DECREF(d); throw Failure(); }
+    std::vector<at::Tensor> dt, st;
+    bool ok = PySequence_Fast_GET_SIZE(d) == PySequence_Fast_GET_SIZE(s);
+    for (Py_ssize_t i = 0; ok && i < PySequence_Fast_GET_SIZE(d); ++i) {
+        PyObject *a = PySequence_Fast_GET_ITEM(d, i), *b = PySequence_Fast_GET_ITEM(s, i);
+        ok = THPVariable_Check(a) && THPVariable_Check(b);
+        if (ok) { dt.push_back(THPVariable_Unpack(a)); st.push_back(THPVariable_Unpack(b)); }
+    }
+    Py_DECREF(d);
+    Py_DECREF(s);
+    if (!ok) fail(PyExc_TypeError, "expected as many source tensors as destination tensors");
+    void* dst[SMLA_COPY_BATCH_MAX];
+    const void* src[SMLA_COPY_BATCH_MAX];
+    int64_t bytes[SMLA_COPY_BATCH_MAX];
+    int n = 0;
+    for (size_t i = 0; i < dt.size(); ++i) {
+        const at::Tensor &a = dt[i], &b = st[i];
+        if (n < SMLA_COPY_BATCH_MAX && a.is_cuda() && b.is_cuda() && a.device() == b.device() && a.device() == dt[0].device() &&
+            a.scalar_type() == b.scalar_type() && a.sizes() == b.sizes() && a.is_contiguous() && b.is_contiguous() &&
+            a.data_ptr() != b.data_ptr()) {
+            dst[n] = a.data_ptr(); src[n] = b.data_ptr(); bytes[n] = (int64_t)a.nbytes();
+            ++n;
+        } else {
+            a.copy_(b);
+        }
+    }
+    if (n > 0) check(api.copy_batch(n, dst, src, bytes, stream_of(dt[0])));
+    Py_RETURN_NONE;
+}
+
 // (handle of the loaded library, module _runtime, SmlaError)
 PyObject* init(const Args& x) {
     void* lib = reinterpret_cast<void*>((uintptr_t)x.integer(0));
@@ -393,6 +439,7 @@ PyObject* init(const Args& x) {
     get(api.decode_splitkv_ext, "smla_decode_splitkv_ext"); get(api.decode_uniform, "smla_decode_uniform"); get(api.prefill, "smla_prefill");
     get(api.prefill_ext, "smla_prefill_ext"); get(api.combine, "smla_combine"); get(api.pack_kv, "smla_pack_kv");
     get(api.mqa_logits, "smla_mqa_logits"); get(api.topk, "smla_topk");
+    get(api.topk_paged, "smla_topk_paged"); get(api.copy_batch, "smla_copy_batch");
     g_runtime = x.a[1]; Py_INCREF(g_runtime);
     g_error = x.a[2]; Py_INCREF(g_error);
     Py_RETURN_NONE;
@@ -414,7 +461,8 @@ PyObject* entry(PyObject*, PyObject* const* args, Py_ssize_t n) {
 #define SMLA_FN(name, f, n, ...) {name, reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(&entry<f, n, ##__VA_ARGS__>)), METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {
     SMLA_FN("init", init, 3, false), SMLA_FN("decode", decode, 14), SMLA_FN("prefill", prefill, 12),
-    SMLA_FN("mqa_logits", mqa_logits, 8), SMLA_FN("topk", topk, 4), SMLA_FN("pack_kv", pack_kv, 1),
+    SMLA_FN("mqa_logits", mqa_logits, 8), SMLA_FN("topk", topk, 6), SMLA_FN("pack_kv", pack_kv, 1),
+    SMLA_FN("copy_into", copy_into, 2),
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_smla_native", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 

@@ -29,7 +29,7 @@ def topk_indices(logits: torch.Tensor, ks: Optional[torch.Tensor], ke: Optional[
     padded with -1 when fewer than k candidates exist.  Ties at the k-th value go to the lowest
     columns.  The order inside a row is a fixed function of the input but not ascending, and not
     part of the contract.  Rows of any width."""
-    return native().topk(logits, ks, ke, k)
+    return native().topk(logits, ks, ke, k, None, 0)
 
 
 def pack_kv_cache(kv_bf16: torch.Tensor) -> torch.Tensor:

@@ -11,7 +11,7 @@ from typing import Optional, Tuple
 import torch
 
 from . import indexer
-from ._lib import IMPL_AUTO
+from ._lib import IMPL_AUTO, native
 from .flash_ops import sparse_mla_decode_fwd
 
 
@@ -34,9 +34,12 @@ def sparse_mla_indexed_decode_fwd(q: torch.Tensor, kv_cache: torch.Tensor, qi: t
     indexer queries, ``ki`` [s_k, 128] e4m3 / ``k_scale`` [s_k] indexer keys, ``ks`` / ``ke`` [T]
     the window of each token.  Returns (out [T, H, 512] bf16, lse [T, H], rows [T, topk] int32)."""
     logits = indexer.fp8_mqa_logits(qi, ki, k_scale, weights, ks, ke)
-    rows = indexer.topk_indices(logits, ks, ke, topk)
-    if block_table is not None:
-        rows = positions_to_rows(rows, block_table, kv_cache.shape[1])
+    if block_table is not None and block_table.dtype == torch.int32 and block_table.stride(1) == 1:
+        rows = native().topk(logits, ks, ke, topk, block_table, kv_cache.shape[1])     # written as rows by the selection
+    else:
+        rows = indexer.topk_indices(logits, ks, ke, topk)
+        if block_table is not None:
+            rows = positions_to_rows(rows, block_table, kv_cache.shape[1])
     out, lse = sparse_mla_decode_fwd(q, kv_cache, rows, sm_scale, attn_sink=attn_sink, impl=impl)
     return out, lse, rows
 
@@ -78,11 +81,7 @@ class GraphedIndexedDecode:
 
     def __call__(self, q, qi, weights, ks, ke) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
         """Returns (out, lse, rows): static tensors, overwritten by the next call."""
-        self.q.copy_(q)
-        self.qi.copy_(qi)
-        self.weights.copy_(weights)
-        self.ks.copy_(ks)
-        self.ke.copy_(ke)
+        native().copy_into((self.q, self.qi, self.weights, self.ks, self.ke), (q, qi, weights, ks, ke))
         return self.replay()
 
     def replay(self) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
