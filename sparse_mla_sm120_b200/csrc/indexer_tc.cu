@@ -11,12 +11,18 @@
 //
 // One CTA walks query groups (4 queries) round-robin and, per group, the key tiles up to the
 // largest ke of the group.  Warps: 0-15 epilogue (warp w: TMEM lane quarter w % 4, query w / 4
-// of the group; the epilogue is bound by instruction issue, so it gets four warps per scheduler),
+// of the group, its 64 head weights in registers),
 // 16 loader (one TMA tile load per key tile and per q group: both are contiguous rows of 128
 // bytes in global memory and land 128B-swizzled, K-major; rows past the end arrive as zeros),
-// 17 MMA issue (one thread).
-// The kernel is tensor-bound at the benchmark shape (4.26 TFLOP) with the logits write
-// (1.07 GB) as the second term.  Every wait is bounded.
+// 17 MMA issue (one elected lane).
+// What bounds it: 4096 queries x 65536 keys x 64 heads (4.26 TFLOP) take 2.05 ms at 1965 MHz, about 1080 cycles per tile of
+// 128 keys x 256 scores, of which the MMAs are 520 and the epilogue's instructions 660 (the rate of a loop of nothing but
+// tensor-memory loads, maxima and packed FMAs); in a long run the 1000 W limit holds the clock at 1665 MHz and a call takes
+// 2.36 ms.  Before: weights read from shared memory for every tile, 2.43-2.69 ms.  Measured and not kept: the ReLU as a
+// saturating multiplication on the FMA pipe for half of the scores (2.13 ms), accumulators of two queries each that are
+// refilled separately (2.48 ms: N = 128 MMAs read their A operand twice and are bound by shared memory), eight epilogue
+// warps of two queries (2.40 ms), tensor-memory loads across tiles (3.0 ms, registers).
+// Every wait is bounded.
 #include <cuda.h>
 
 #include "common.cuh"
@@ -31,9 +37,13 @@ using namespace ptx;
 constexpr int LX_D = 128;            // head dim of the indexer (bytes per row)
 constexpr int LX_KT = 128;           // keys per tile
 constexpr int LX_QG = 4;             // queries per group
-constexpr int LX_EPI_WARPS = 16, LX_QPW = 2;   // epilogue warps: one set of eight per accumulator; queries per warp
+constexpr int LX_EPI_WARPS = 16;      // epilogue warps: four tensor-memory lane quarters x the four queries of a group
 constexpr int LX_LOAD_WARP = LX_EPI_WARPS, LX_MMA_WARP = LX_EPI_WARPS + 1;
-constexpr int LX_THREADS = (LX_EPI_WARPS + 2) * 32;
+constexpr int LX_THREADS = (LX_EPI_WARPS + 4) * 32;
+// The epilogue warps keep 64 head weights in registers; the loader's and MMA warp's warpgroup gives up registers for it (what
+// setmaxnreg.inc draws on is what the CTA was launched with; the launcher checks the compiled count).
+constexpr int LX_REGS_LAUNCH = 96, LX_REGS_EPI = 112, LX_REGS_REST = 32;
+static_assert(LX_EPI_WARPS * 32 * LX_REGS_EPI + 128 * LX_REGS_REST <= LX_THREADS * LX_REGS_LAUNCH, "register budgets exceed what the CTA owns");
 constexpr int LX_KSTAGE = 4;
 
 constexpr uint32_t LX_Q_OFF = 0;                              // q group: [<=256 rows x 128 B] K-major 128B swizzle
@@ -72,7 +82,7 @@ __global__ void __launch_bounds__(LX_THREADS, 1) mqa_logits_tc_kernel(const Logi
 
     if (tid == 0) {
         for (int s = 0; s < LX_KSTAGE; ++s) { mbar_init(bar(LXB_KFULL + s), 1); mbar_init(bar(LXB_KEMPTY + s), 1); }
-        for (int b = 0; b < 2; ++b) { mbar_init(bar(LXB_DFULL + b), 1); mbar_init(bar(LXB_DEMPTY + b), LX_EPI_WARPS / 2); }
+        for (int b = 0; b < 2; ++b) { mbar_init(bar(LXB_DFULL + b), 1); mbar_init(bar(LXB_DEMPTY + b), LX_EPI_WARPS); }
         mbar_init(bar(LXB_QFULL), 32);
         mbar_init(bar(LXB_QEMPTY), 1 + LX_EPI_WARPS);   // the MMAs have read q and every epilogue warp has seen the group's phase
         *abort_flag = 0;
@@ -112,88 +122,81 @@ __global__ void __launch_bounds__(LX_THREADS, 1) mqa_logits_tc_kernel(const Logi
         j1 = min(p.s_k, (c + 1) * p.chunk_tiles * LX_KT);
     };
 
+    if (warp < LX_EPI_WARPS) setmaxnreg_inc<LX_REGS_EPI>();
+    else setmaxnreg_dec<LX_REGS_REST>();
     if (warp < LX_EPI_WARPS) {
         // =================================================================== epilogue
-        // Warp: TMEM lane quarter (32 keys of a tile), two queries of the group, and the accumulator (every other tile) that
-        // its set of eight looks after.
-        const int quarter = warp & 3, qh = (warp >> 2) & 1;
-        const uint32_t set = (uint32_t)warp >> 3;
-        const uint32_t lane_addr = tmem + ((uint32_t)(quarter * 32) << 16) + LX_QPW * qh * H + 256 * set;
+        const int quarter = warp & 3, qp = warp >> 2;
+        const uint32_t lane_addr = tmem + ((uint32_t)(quarter * 32) << 16) + qp * H;
         uint32_t it = 0, qn = 0;   // tiles and non-empty groups seen by this CTA
         bool ok = true;
         for (int w = blockIdx.x; w < num_items && ok; w += gridDim.x) {
             int g, t0, t1, j0, j1;
             item_range(w, g, t0, t1, j0, j1);
-            int ks_q[LX_QPW], ke_q[LX_QPW];
-            float* row[LX_QPW];
-#pragma unroll
-            for (int u = 0; u < LX_QPW; ++u) {
-                const int qi = g * LX_QG + LX_QPW * qh + u;
-                const bool have = qi < p.s_q;
-                ks_q[u] = have ? p.ks[qi] : 0;
-                ke_q[u] = have ? p.ke[qi] : 0;
-                row[u] = have ? p.logits + (size_t)qi * p.stride : nullptr;
-                // columns of the item outside every tile the group needs are -inf: written here, 128 keys per pass
-                if (have) {
-                    for (int j = j0 + quarter * 32 + lane; j < j1; j += 128)
-                        if (j < t0 * LX_KT || j >= t1 * LX_KT) row[u][j] = -INFINITY;
-                }
+            const int qi = g * LX_QG + qp;
+            const bool have = qi < p.s_q;
+            const int ks_q = have ? p.ks[qi] : 0, ke_q = have ? p.ke[qi] : 0;
+            float* row = p.logits + (size_t)(have ? qi : 0) * p.stride;
+            // columns of the item outside every tile the group needs are -inf: written here, 128 keys per pass
+            if (have) {
+                for (int j = j0 + quarter * 32 + lane; j < j1; j += 128)
+                    if (j < t0 * LX_KT || j >= t1 * LX_KT) row[j] = -INFINITY;
             }
             if (t1 <= t0) continue;
             ok = mbar_wait(bar(LXB_QFULL), qn & 1u, abort_flag, 11);   // weights of the group are in shared memory
             if (!ok) break;
-            const float* wq = reinterpret_cast<const float*>(sm + LX_W_OFF + (qn & 3u) * LX_W_BYTES) + LX_QPW * qh * 64;
+            // The head weights of the warp's query stay in registers for the whole run of tiles, as pairs for the packed FMAs:
+            // read from shared memory for every tile they cost 16 wide loads per warp and tile, and the 16 warps together
+            // were bound by the bytes those return.
+            uint64_t wreg[H / 2];
+            {
+                const float* wq = reinterpret_cast<const float*>(sm + LX_W_OFF + (qn & 3u) * LX_W_BYTES) + qp * 64;
+#pragma unroll
+                for (int i = 0; i < H / 4; ++i) {
+                    const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(wq + 4 * i);
+                    wreg[2 * i] = v.x;
+                    wreg[2 * i + 1] = v.y;
+                }
+            }
             // The loader may arm the next group only after this warp has seen this one: otherwise two phases
             // of QFULL could complete before a slow epilogue warp waits for the first (a group of one or two
             // tiles needs nothing from the epilogue), and its parity wait would then refer to a later phase.
             __syncwarp();
             if (lane == 0) mbar_arrive(bar(LXB_QEMPTY));
             ++qn;
-            // Chunks of 32 score columns; the tensor-memory load of the next chunk is in flight while one is reduced.
-            constexpr int NCH = LX_QPW * H / 32;
+            int key = t0 * LX_KT + quarter * 32 + lane;
+            const int last = min(ke_q, p.s_k);
 #pragma unroll 1
-            for (int t = t0 + (int)((set ^ it) & 1u); t < t1; t += 2) {
-                const uint32_t n = it + (uint32_t)(t - t0);
-                ok = mbar_wait_hot(bar(LXB_DFULL + set), (n >> 1) & 1u, abort_flag, 12);
+            for (int t = t0; t < t1; ++t, ++it, key += LX_KT) {
+                const uint32_t b = it & 1u;
+                const float sc = key < p.s_k ? __ldg(p.k_scale + key) : 0.f;
+                ok = mbar_wait_hot(bar(LXB_DFULL + b), (it >> 1) & 1u, abort_flag, 12);
                 if (!ok) break;
                 tc_fence_after();
-                uint32_t d[2][32];
-                tmem_ld32(lane_addr, d[0]);
-                const int key = t * LX_KT + quarter * 32 + lane;
-                const float sc = key < p.s_k ? __ldg(p.k_scale + key) : 0.f;
-                float acc[LX_QPW];
                 uint64_t a01 = 0ull, a23 = 0ull;
 #pragma unroll
-                for (int c = 0; c < NCH; ++c) {
+                for (int c = 0; c < H / 16; ++c) {
+                    uint32_t d[16];
+                    tmem_ld16(lane_addr + 256 * b + 16 * c, d);
                     tmem_wait_ld();
-                    if (c + 1 < NCH) {
-                        tmem_ld32(lane_addr + 32 * (c + 1), d[(c + 1) & 1]);
-                    } else {
+                    if (c + 1 == H / 16) {
                         tc_fence_before();
                         __syncwarp();
-                        if (lane == 0) mbar_arrive(bar(LXB_DEMPTY + set));     // every column of the tile is in registers
+                        if (lane == 0) mbar_arrive(bar(LXB_DEMPTY + b));       // every column of the tile is in registers
                     }
-                    const uint32_t* v = d[c & 1];
-                    const float* wc = wq + (c / (H / 32)) * 64 + (c % (H / 32)) * 32;
 #pragma unroll
-                    for (int i = 0; i < 32; i += 4) {       // two scores per FMA
-                        const ulonglong2 w4 = *reinterpret_cast<const ulonglong2*>(wc + i);      // (w0, w1), (w2, w3)
-                        fma_f32x2(a01, pack_f32x2(fmaxf(__uint_as_float(v[i + 0]), 0.f), fmaxf(__uint_as_float(v[i + 1]), 0.f)), w4.x);
-                        fma_f32x2(a23, pack_f32x2(fmaxf(__uint_as_float(v[i + 2]), 0.f), fmaxf(__uint_as_float(v[i + 3]), 0.f)), w4.y);
-                    }
-                    if ((c + 1) % (H / 32) == 0) {
-                        float a0, a1, a2, a3;
-                        unpack_f32x2(a01, a0, a1);
-                        unpack_f32x2(a23, a2, a3);
-                        acc[c / (H / 32)] = (a0 + a1) + (a2 + a3);
-                        a01 = a23 = 0ull;
+                    for (int i = 0; i < 16; i += 4) {       // two scores per FMA
+                        const int wi = (16 * c + i) / 2;
+                        fma_f32x2(a01, pack_f32x2(fmaxf(__uint_as_float(d[i + 0]), 0.f), fmaxf(__uint_as_float(d[i + 1]), 0.f)), wreg[wi]);
+                        fma_f32x2(a23, pack_f32x2(fmaxf(__uint_as_float(d[i + 2]), 0.f), fmaxf(__uint_as_float(d[i + 3]), 0.f)), wreg[wi + 1]);
                     }
                 }
-#pragma unroll
-                for (int u = 0; u < LX_QPW; ++u)
-                    if (key < p.s_k && row[u] != nullptr) row[u][key] = (key >= ks_q[u] && key < ke_q[u]) ? acc[u] * sc : -INFINITY;
+                float a0, a1, a2, a3;
+                unpack_f32x2(a01, a0, a1);
+                unpack_f32x2(a23, a2, a3);
+                const float sum = (a0 + a1) + (a2 + a3);
+                if (have && key < p.s_k) row[key] = (key >= ks_q && key < last) ? sum * sc : -INFINITY;
             }
-            it += (uint32_t)(t1 - t0);
         }
     } else if (warp == LX_LOAD_WARP) {
         // =================================================================== loader
@@ -294,6 +297,11 @@ int launch_mqa_logits_tc(const uint8_t* q, const uint8_t* k, const float* k_scal
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 64 && !attr_set[dev]) {
+        cudaFuncAttributes fa[2];
+        if (cudaFuncGetAttributes(&fa[0], mqa_logits_tc_kernel<64>) != cudaSuccess || cudaFuncGetAttributes(&fa[1], mqa_logits_tc_kernel<32>) != cudaSuccess ||
+            fa[0].numRegs != LX_REGS_LAUNCH || fa[1].numRegs != LX_REGS_LAUNCH)
+            return set_error(SMLA_E_DEVICE, "mqa_logits_tc_kernel: compiled with %d and %d registers per thread, the warpgroup budgets assume %d",
+                             fa[0].numRegs, fa[1].numRegs, LX_REGS_LAUNCH);
         cudaError_t e = cudaFuncSetAttribute(mqa_logits_tc_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LX_SMEM);
         if (e == cudaSuccess) e = cudaFuncSetAttribute(mqa_logits_tc_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LX_SMEM);
         if (e != cudaSuccess) return set_error((int)e, "mqa_logits_tc_kernel: shared memory: %s", cudaGetErrorString(e));
