@@ -961,7 +961,7 @@ int launch_topk(const float* logits, const int32_t* ks, const int32_t* ke, int32
         return check_launch("topk_kernel");
     }
     static bool attr_set[64] = {};
-    static int sms[64] = {};
+    static int sms[64] = {}, clusters[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 64 && !attr_set[dev]) {
@@ -970,10 +970,21 @@ int launch_topk(const float* logits, const int32_t* ks, const int32_t* ke, int32
         if (e == cudaSuccess) e = cudaFuncSetAttribute(topk_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM);
         if (e != cudaSuccess) return set_error((int)e, "topk_select_kernel: shared memory: %s", cudaGetErrorString(e));
         cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev);
+        // clusters of eight that the device holds at once (a cluster stays inside one GPC, so it is fewer than the SMs suggest)
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(TC_CTAS); cfg.blockDim = dim3(TC_THREADS); cfg.dynamicSmemBytes = TC_SMEM;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = TC_CTAS; attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr; cfg.numAttrs = 1;
+        if (cudaOccupancyMaxActiveClusters(&clusters[dev], topk_cluster_kernel, &cfg) != cudaSuccess) {
+            cudaGetLastError();
+            clusters[dev] = 0;
+        }
         attr_set[dev] = true;
     }
     const int n = sms[dev < 64 ? dev : 0];
-    if (num_rows * TC_CTAS <= 2 * n)               // few rows: two CTAs of eight-CTA clusters per SM
+    if (num_rows <= clusters[dev < 64 ? dev : 0])  // a cluster per row, all at once (one row more takes a second wave: 17 -> 26 us)
         topk_cluster_kernel<<<num_rows * TC_CTAS, TC_THREADS, TC_SMEM, stream>>>(logits, ks, ke, out, num_cols, logits_stride, k, emit);
     else if (num_rows <= n)                        // every row has an SM to itself
         topk_select_kernel<1024><<<num_rows, 1024, TS_SMEM, stream>>>(logits, ks, ke, out, num_cols, logits_stride, k, emit);
