@@ -65,6 +65,9 @@ const char* smla_status_string(int code) {
         case 33: return "attention q_staged"; case 34: return "attention q_free"; case 35: return "attention raw_empty";
         case 36: return "attention raw_full";
         case 41: return "exact attention rows free"; case 42: return "exact attention rows stored"; case 43: return "exact attention s_ready";
+        case 51: return "attention tile k_full"; case 52: return "attention tile rope_full"; case 53: return "attention tile k_free";
+        case 54: return "attention tile s_ready"; case 55: return "attention tile s_free"; case 56: return "attention tile scales";
+        case 57: return "attention tile p_ready"; case 58: return "attention tile pv_done"; case 59: return "attention tile q_ready";
         case 44: return "exact attention p_ready"; case 45: return "exact attention pv_done"; case 46: return "exact attention q_ready";
         default: return "unknown";
     }

@@ -1,0 +1,736 @@
+// Sparse-MLA attention over packed 656-byte rows, one CTA per 64 query heads (sm_100a): split-KV decode and prefill.
+//
+// Work unit: one partition (a run of 64-token blocks of consecutive requests, see sched.cu; without a scheduler every
+// parts-th request) for 64 query heads; up to 128 heads are two CTAs next to each other in the grid, which read the same
+// rows at about the same time (the second read comes from L2).
+//
+// The gathered rows are never touched by a thread.  TMA gather4 loads bring the 512 e4m3 values of a row, as four
+// pieces of 128 dims, and its 64 RoPE values straight into the 128B-swizzled tiles that the MMAs read; a row without an
+// entry is named by an index outside the tensor and arrives as zeros.  Both contractions run transposed, with the tile of
+// rows as the A operand of both (M = 128 whatever the number of heads, and V needs no second copy):
+//   * S^T [128 tokens x 64 heads] = K . Q^T, K-major.  The four fp32 scales of a row (powers of two, one per 128 dims) and
+//     the scale of a head's quantised q are applied by the tensor core: kind::mxf8f6f4 takes one power of two per row and 32
+//     values, and the scale bytes of a row's four blocks are the four bytes of one scale word.  RoPE goes into the same
+//     accumulator by bf16 MMAs, so that it holds q . k itself.
+//   * O^T [4 x 128 dims x 64 heads] += V^T . P_b, the same tile read MN-major.  V's scale is a factor of the token inside a
+//     block of 128 dims, so it goes into the weights: block b uses P_b = P * 2^(e_b - e_max), rounded to e4m3, with
+//     e_max the largest of the row's four exponents.
+// Numerics (the FP8 class of the reference's V32 kernels, which quantise Q and P to e4m3:
+// csrc/kernel/common/fp8_quant.cuh:44-103, csrc/kernel/decode/decode_v2_kernel.cuh:414-493): q no-PE e4m3 with one power of
+// two per head, q RoPE bf16 as given, K and V bytes as stored, P' = 2^(z - m) in e4m3 (times 2^T_P_SHIFT) with
+// z = logit * log2(e) + e_max and m its lazily updated running maximum per head; the denominator sums P' / 2^e_max in fp32.
+// Entries without a row (index < 0, position >= topk_length) have weight exactly 0.
+//
+// Warp roles (896 threads):
+//   warps 0-15   softmax, epilogue, Q: warp w holds tokens [32 (w % 4), +32) and heads [16 (w / 4), +16) of a tile, a thread
+//                one token; the four warps of a head group meet once per tile at a barrier that also ORs "a weight has
+//                outgrown the running maximum".  Groups without heads only quantise Q.
+//   warps 16-19  producers: warp 16 + i gathers rows [32 i, +32) of every tile; a quarter of a stage is refilled as soon as
+//                P.V has read it, and the score MMAs of a block of dims start when that block has landed.
+//   warps 20-23  scales: the rows' scale words into tensor memory (each warp the 32 lanes it can reach) and shared memory.
+//   warp 24      issues the score MMAs, warp 25 the P.V MMAs (one elected lane each).
+// Every wait is bounded; a wait that gives up records a code in status[] and the CTA drains and exits.
+#include <cuda.h>
+
+#include "attn_common.cuh"
+#include "sm100_ptx.cuh"
+
+namespace smla {
+
+namespace {
+
+using namespace ptx;
+using namespace attn;
+
+constexpr int T_HEADS = 64;                    // heads per CTA
+constexpr int T_TILE = 128;                    // tokens per tile: two scheduler blocks
+constexpr int T_SM_WARPS = 16, T_PROD = 16, T_SCALE = 20, T_QK = 24, T_PV = 25;
+constexpr int T_THREADS = 28 * 32;
+constexpr int T_HPW = 16;                      // heads per softmax warp
+constexpr int T_REGS_LAUNCH = 72, T_REGS_SOFTMAX = 88, T_REGS_REST = 48;
+static_assert(T_SM_WARPS * 32 * T_REGS_SOFTMAX + (T_THREADS - T_SM_WARPS * 32) * T_REGS_REST <= T_THREADS * T_REGS_LAUNCH,
+              "register budgets exceed what the CTA owns");
+constexpr int T_P_SHIFT = 5;                   // P' is stored as e4m3(P' * 2^T_P_SHIFT)
+constexpr float T_TAU = 3.0f;                  // lazy-rescale threshold (log2 units); P' <= 2^T_TAU
+constexpr float T_NO_MAX = 1e30f;              // minus the running maximum of a head that has seen no entry (finite: -inf minus it is -inf)
+constexpr int NSTAGE = 2;
+
+constexpr uint32_t K_CHUNK = T_TILE * 128;                 // 128 dims (or the RoPE) of all rows
+constexpr uint32_t Q_CHUNK = T_HEADS * 128;
+constexpr uint32_t K_STAGE = 4 * K_CHUNK;
+constexpr uint32_t K_OFF = 0;
+constexpr uint32_t R_OFF = K_OFF + NSTAGE * K_STAGE;       // RoPE of the rows: one stage, free again when the scores are done
+constexpr uint32_t Q_OFF = R_OFF + K_CHUNK;                // q e4m3, four chunks of [64 heads x 128 dims]
+constexpr uint32_t QR_OFF = Q_OFF + 4 * Q_CHUNK;           // q RoPE bf16
+constexpr uint32_t P_OFF = QR_OFF + Q_CHUNK;               // P_b: [128 tokens x 64 heads] e4m3, 64B swizzle
+constexpr uint32_t P_BYTES = T_TILE * T_HEADS;
+constexpr int SW_RING = 4;
+constexpr uint32_t SW_OFF = P_OFF + 4 * P_BYTES;           // scale words of a tile's tokens (0: no entry), [SW_RING][128]
+constexpr uint32_t NM_OFF = SW_OFF + SW_RING * T_TILE * 4; // -m of the 64 heads
+constexpr uint32_t QW_OFF = NM_OFF + T_HEADS * 4;          // the heads' scale words
+constexpr uint32_t XX_OFF = QW_OFF + T_HEADS * 4;          // exchange between the four warps of a head group: [2][4][64] fp32
+constexpr uint32_t B_OFF = XX_OFF + 2 * 4 * T_HEADS * 4;
+constexpr int B_KFULL = 0, B_RFULL = B_KFULL + 4 * NSTAGE, B_KFREE = B_RFULL + 1, B_SREADY = B_KFREE + 4 * NSTAGE, B_SFREE = B_SREADY + 2,
+              B_SCALES = B_SFREE + 2, B_PREADY = B_SCALES + SW_RING, B_PVDONE = B_PREADY + 1, B_QREADY = B_PVDONE + 1, B_N = B_QREADY + 1;
+constexpr uint32_t MISC_OFF = B_OFF + B_N * 8;
+constexpr uint32_t T_SMEM = MISC_OFF + 16 + 1024;
+static_assert(T_SMEM <= 227 * 1024, "shared memory budget");
+static_assert(R_OFF % 1024 == 0 && Q_OFF % 1024 == 0 && P_OFF % 1024 == 0 && B_OFF % 8 == 0, "alignment");
+
+// tensor memory: dims block b of O^T at 64 b, score buffers, scale words of the rows (4 columns per tile) and of the heads
+constexpr uint32_t TM_O = 0, TM_S = 256, TM_SFA = 384, TM_SFB = 400;
+// Instruction descriptors.  kind::mxf8f6f4: scale type UE8M0 (bit 23), which byte of the scale word A uses (bits 29-30); the
+// head's word has the same byte four times.
+__host__ __device__ constexpr uint32_t idesc_mx(uint32_t a_byte) {
+    return (FMT_E4M3 << 7) | (FMT_E4M3 << 10) | ((T_HEADS >> 3) << 17) | (1u << 23) | ((T_TILE >> 7) << 27) | (a_byte << 29);
+}
+constexpr uint32_t IDESC_ROPE = instr_desc(FMT_BF16, FMT_BF16, false, false, T_TILE, T_HEADS);
+constexpr uint32_t IDESC_PV = instr_desc(FMT_E4M3, FMT_E4M3, true, true, 128, T_HEADS);
+constexpr uint32_t HI_128 = desc_hi(1024, (uint32_t)SWIZZLE_128B), HI_P = desc_hi(512, (uint32_t)SWIZZLE_64B);
+constexpr int NO_ROW = 0x7fffffff;             // outside the tensor map: arrives as zeros
+
+enum { WT_KFULL = 51, WT_RFULL = 52, WT_KFREE = 53, WT_SREADY = 54, WT_SFREE = 55, WT_SCALES = 56, WT_PREADY = 57, WT_PVDONE = 58, WT_QREADY = 59 };
+
+__device__ __forceinline__ uint32_t swz128(uint32_t row, uint32_t piece) { return row * 128u + ((piece ^ (row & 7u)) << 4); }
+__device__ __forceinline__ uint32_t swz64(uint32_t row, uint32_t piece) { return row * 64u + ((piece ^ ((row >> 1) & 3u)) << 4); }
+
+__device__ __forceinline__ float lanes_max(float v) {
+    float r;
+    asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
+}
+
+// The requests of a CTA and their tiles, in the order in which every role walks them.
+struct Tiles {
+    Work w;
+    int req, step, last, j, nst;
+    __device__ __forceinline__ Tiles(int first, int step_, int last_) : req(first - step_), step(step_), last(last_), j(0), nst(0) {}
+    __device__ __forceinline__ bool next_request(const AttnParams& p, const SchedMeta& m) {
+        do {
+            if (req + step > last) return false;
+            req += step;
+        } while (!get_work(p, m, req, w));
+        nst = (w.nblk + 1) >> 1;
+        j = 0;
+        return true;
+    }
+    __device__ __forceinline__ bool next_tile(const AttnParams& p, const SchedMeta& m) {
+        if (++j < nst) return true;
+        return next_request(p, m);
+    }
+    // Row r of the current tile: its index in the cache, -1 where there is no entry.
+    __device__ __forceinline__ int row_index(const AttnParams& p, int r) const {
+        const int pos = (w.blk0 + 2 * j) * BLOCK_N + r, lim = min(w.len, (w.blk0 + w.nblk) * BLOCK_N);
+        return pos < lim ? __ldg(p.indices + (size_t)w.req * p.topk + pos) : -1;
+    }
+};
+
+template <bool MAXL>
+__global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParams p, const int halves, const __grid_constant__ CUtensorMap kv_map) {
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t raw = smem_u32(smem_raw);
+    const uint32_t base = (raw + 1023u) & ~1023u;
+    uint8_t* sm = smem_raw + (base - raw);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(sm + MISC_OFF + 4);
+    auto bar = [&](int i) -> uint32_t { return base + B_OFF + 8u * i; };
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int part = blockIdx.x / halves, head0 = (blockIdx.x - part * halves) * T_HEADS;
+    const int my_heads = min(p.num_heads - head0, T_HEADS);
+    const int act = 4 * ((my_heads + T_HPW - 1) / T_HPW);  // softmax warps with live heads
+
+    if (tid == 0) {
+        for (int s = 0; s < NSTAGE; ++s) {
+            for (int i = 0; i < 4; ++i) {
+                mbar_init(bar(B_KFULL + 4 * s + i), 4);    // dims block i of the stage: + the bytes of the four producers
+                mbar_init(bar(B_KFREE + 4 * s + i), 1);    // its rows [32 i, +32) have been read
+            }
+        }
+        mbar_init(bar(B_RFULL), 4);
+        for (int b = 0; b < 2; ++b) { mbar_init(bar(B_SREADY + b), 1); mbar_init(bar(B_SFREE + b), act); }
+        for (int i = 0; i < SW_RING; ++i) mbar_init(bar(B_SCALES + i), 4);
+        mbar_init(bar(B_PREADY), act);
+        mbar_init(bar(B_PVDONE), 1);
+        mbar_init(bar(B_QREADY), T_SM_WARPS);
+        *abort_flag = 0;
+        mbar_init_fence();
+    }
+    if (act < T_SM_WARPS)                                  // the weights of heads that do not exist stay zero
+        for (int i = tid; i < (int)(4 * P_BYTES / 16); i += T_THREADS) reinterpret_cast<uint4*>(sm + P_OFF)[i] = make_uint4(0, 0, 0, 0);
+    if (warp == T_QK) { tmem_alloc(base + MISC_OFF, 512); tmem_relinquish(); }
+    fence_proxy_async();
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(sm + MISC_OFF);
+    grid_dep_wait();
+    grid_dep_launch();
+    SchedMeta meta;
+    int first, step, last;
+    if (p.sched != nullptr || p.uniform_k > 1) {
+        meta = load_meta(p, part);
+        first = meta.begin_req; step = 1; last = min(meta.end_req, p.num_tokens - 1);
+    } else {                                               // whole requests; neighbours differ little in length, so every CTA takes each parts-th
+        meta.begin_block = 0; meta.end_block = 0x7fffffff;
+        meta.begin_split = 0; meta.first_split = meta.last_split = 0; meta.pad = 0;
+        first = part; step = (int)gridDim.x / halves; last = p.num_tokens - 1;
+        meta.begin_req = 0; meta.end_req = last;
+    }
+    if (warp < T_SM_WARPS) setmaxnreg_inc<T_REGS_SOFTMAX>();
+    else setmaxnreg_dec<T_REGS_REST>();
+
+    if (warp < T_SM_WARPS) {
+        // =================================================================== softmax + epilogue + Q
+        const int quarter = warp & 3, grp = warp >> 2, h0 = grp * T_HPW;
+        const int token = quarter * 32 + lane;             // of the tile; in O^T: output dim inside a block of 128
+        const int hl = h0 + (lane & (T_HPW - 1));          // the head whose state this lane keeps (the same in four warps)
+        const bool live = hl < my_heads, active = h0 < my_heads;
+        const uint32_t lane_addr = tmem + ((uint32_t)(quarter * 32) << 16);
+        float* nm = reinterpret_cast<float*>(sm + NM_OFF);
+        float* xx = reinterpret_cast<float*>(sm + XX_OFF);
+        uint32_t* qw = reinterpret_cast<uint32_t*>(sm + QW_OFF);
+        // logits in log2 units are scores times a positive number: the sign of the softmax scale goes into q
+        const float c = fabsf(p.sm_scale) * LOG2E;
+        const uint32_t scale_sign = __float_as_uint(p.sm_scale) & 0x80000000u;
+        Tiles tiles(first, step, last);
+        uint32_t it = 0;
+        bool dead = false;
+        bool prev = false, prev_no_split = false;          // a request's epilogue runs after the next request's Q phase
+        int prev_req = 0, prev_split = 0;
+        float prev_m = 0.f, prev_l = 0.f, prev_x = 0.f;
+        while (true) {
+            const bool have = tiles.next_request(p, meta);
+            // Every score of the request before has been read, by all warps, and so has its state: q, its scales and the maxima may
+            // be overwritten.  The sixteen warps leave the loop here together when one of them has given up.
+            if (named_bar_or(5, T_SM_WARPS * 32, dead || *abort_flag != 0)) break;
+            if (have) {
+                // ---- Q: warp w quantises heads [4 w, +4), a lane 16 of the 512 no-PE dims of each
+                const __nv_bfloat16* q0 = p.q + ((size_t)tiles.w.req * p.num_heads + head0) * D_QK;
+                {
+                    uint4 v[8];
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        const int h = 4 * warp + k;
+                        v[2 * k] = v[2 * k + 1] = make_uint4(0, 0, 0, 0);
+                        if (h < my_heads) {
+                            v[2 * k] = __ldg(reinterpret_cast<const uint4*>(q0 + (size_t)h * D_QK + lane * 16));
+                            v[2 * k + 1] = __ldg(reinterpret_cast<const uint4*>(q0 + (size_t)h * D_QK + lane * 16 + 8));
+                        }
+                    }
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        const int h = 4 * warp + k;
+                        const uint32_t x[8] = {v[2 * k].x, v[2 * k].y, v[2 * k].z, v[2 * k].w, v[2 * k + 1].x, v[2 * k + 1].y, v[2 * k + 1].z, v[2 * k + 1].w};
+                        uint32_t am = 0u;                  // magnitudes of bf16 numbers order as integers do
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) am = __vmaxu2(am, x[i] & 0x7fff7fffu);
+                        am = __reduce_max_sync(0xffffffffu, max(am & 0xffffu, am >> 16));
+                        const float sq = pow2_ceil(fmaxf(__uint_as_float(am << 16), 1e-4f) * (1.f / 448.f));
+                        const float is = __uint_as_float((0x7f000000u - __float_as_uint(sq)) | scale_sign);   // 1/sq, sq a power of two
+                        uint32_t o[4];
+#pragma unroll
+                        for (int i = 0; i < 4; ++i)
+                            o[i] = pack_e4m3x4(bf16lo(x[2 * i]) * is, bf16hi(x[2 * i]) * is, bf16lo(x[2 * i + 1]) * is, bf16hi(x[2 * i + 1]) * is);
+                        *reinterpret_cast<uint4*>(sm + Q_OFF + (lane >> 3) * Q_CHUNK + swz128((uint32_t)h, (uint32_t)lane & 7u)) = make_uint4(o[0], o[1], o[2], o[3]);
+                        if (lane == 0) qw[h] = (__float_as_uint(sq) >> 23) * 0x01010101u;
+                    }
+                }
+                {                                          // RoPE
+                    const int h = 4 * warp + (lane >> 3);
+                    uint4 v = make_uint4(0, 0, 0, 0);
+                    if (h < my_heads) v = __ldg(reinterpret_cast<const uint4*>(q0 + (size_t)h * D_QK + D_NOPE + (lane & 7) * 8));
+                    const uint32_t flip = scale_sign | (scale_sign >> 16);
+                    v.x ^= flip; v.y ^= flip; v.z ^= flip; v.w ^= flip;
+                    *reinterpret_cast<uint4*>(sm + QR_OFF + swz128((uint32_t)h, (uint32_t)lane & 7u)) = v;
+                }
+                fence_proxy_async();
+                if (warp < 2) nm[warp * 32 + lane] = T_NO_MAX;
+                named_bar_sync(5, T_SM_WARPS * 32);
+                if (grp == 0) {                            // the heads' scale words, in the lanes that this warp reaches
+                    const uint32_t w2[2] = {qw[lane], qw[32 + lane]};
+                    tmem_st2(lane_addr + TM_SFB, w2);
+                    tmem_wait_st();
+                }
+                tc_fence_before();                         // also orders the previous epilogue's reads of the accumulator
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar(B_QREADY));
+                // ask L2 for the next request's q, a whole request of tiles ahead of its use
+                if (tiles.req + tiles.step <= tiles.last) {
+                    const uint8_t* qn = reinterpret_cast<const uint8_t*>(p.q + ((size_t)(tiles.req + tiles.step) * p.num_heads + head0) * D_QK);
+                    for (int i = tid; i < (my_heads * D_QK * 2 + 127) >> 7; i += T_SM_WARPS * 32)
+                        asm volatile("prefetch.global.L2 [%0];" ::"l"(qn + (size_t)i * 128));
+                }
+            }
+            // ---- epilogue of the request before
+            auto epilogue = [&]() {
+                if (!dead) dead = !mbar_wait_hot(bar(B_PVDONE), (it - 1) & 1u, abort_flag, WT_PVDONE);
+                tc_fence_after();
+                xx[quarter * T_HEADS + hl] = prev_l;
+                if (MAXL) xx[(4 + quarter) * T_HEADS + hl] = prev_x;
+                if (named_bar_or(1 + grp, 128, dead || *abort_flag != 0)) { dead = true; return; }
+                const float l_all = (xx[hl] + xx[T_HEADS + hl]) + (xx[2 * T_HEADS + hl] + xx[3 * T_HEADS + hl]);
+                float x_all = -INFINITY;
+                if (MAXL) x_all = fmaxf(fmaxf(xx[4 * T_HEADS + hl], xx[5 * T_HEADS + hl]), fmaxf(xx[6 * T_HEADS + hl], xx[7 * T_HEADS + hl]));
+                float lse = (l_all > 0.f) ? (log2f(l_all) - (float)T_P_SHIFT + prev_m) : NEG_BIG;
+                float denom = l_all;
+                if (prev_no_split && p.attn_sink != nullptr && live) {
+                    const float sink2 = p.attn_sink[head0 + hl] * LOG2E;
+                    denom = l_all + ((prev_m == -T_NO_MAX) ? INFINITY : exp2f(sink2 - prev_m + (float)T_P_SHIFT));
+                    if (lse != NEG_BIG) lse += log2f(1.f + exp2f(sink2 - lse));
+                    else lse = sink2;
+                }
+                const float inv = (denom > 0.f) ? 1.f / denom : 0.f;
+                const size_t row0 = (size_t)(prev_no_split ? prev_req : prev_split) * p.num_heads + head0 + h0;
+                const int n_live = min(my_heads - h0, T_HPW);
+#pragma unroll 1
+                for (int b = 0; b < 4; ++b) {
+                    uint32_t o[T_HPW];
+                    tmem_ld16(lane_addr + TM_O + 64 * b + h0, o);
+                    tmem_wait_ld();
+#pragma unroll
+                    for (int i = 0; i < T_HPW; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * __shfl_sync(0xffffffffu, inv, i));
+                    if (!prev_no_split && p.uniform_k <= 1) {      // fp32 records: a head's 32 dims of the warp are one store of 128 bytes
+                        float* dst = p.o_accum + row0 * D_V + 128 * b + token;
+#pragma unroll
+                        for (int i = 0; i < T_HPW; ++i)
+                            if (i < n_live) dst[i * D_V] = __uint_as_float(o[i]);
+                        continue;
+                    }
+                    // 16-bit results (bf16 outputs; fp16 records of equal partitions, the library's own scratch): neighbouring lanes
+                    // exchange halves, so that a lane has two dims of eight heads (even lanes heads 0-7, odd lanes 8-15)
+                    const bool odd = (lane & 1) != 0;
+                    uint32_t pk[8];
+#pragma unroll
+                    for (int i = 0; i < 8; i += 2) {
+                        auto pack = [&](float a, float bb) -> uint32_t {
+                            if (prev_no_split) { const __nv_bfloat162 t = __floats2bfloat162_rn(a, bb); return *reinterpret_cast<const uint32_t*>(&t); }
+                            const __half2 t = __floats2half2_rn(a, bb);
+                            return *reinterpret_cast<const uint32_t*>(&t);
+                        };
+                        const uint32_t lo = pack(__uint_as_float(o[i]), __uint_as_float(o[i + 1])), hi = pack(__uint_as_float(o[8 + i]), __uint_as_float(o[9 + i]));
+                        const uint32_t got = __shfl_xor_sync(0xffffffffu, odd ? lo : hi, 1), own = odd ? hi : lo;
+                        // own: this lane's dim of two heads; got: the neighbour's
+                        pk[i] = __byte_perm(odd ? got : own, odd ? own : got, 0x5410);
+                        pk[i + 1] = __byte_perm(odd ? got : own, odd ? own : got, 0x7632);
+                    }
+                    uint32_t* dst = reinterpret_cast<uint32_t*>(prev_no_split ? reinterpret_cast<void*>(p.out) : reinterpret_cast<void*>(p.o_accum)) +
+                                    (row0 + (odd ? 8 : 0)) * (D_V / 2) + 64 * b + (token >> 1);
+                    const int n = n_live - (odd ? 8 : 0);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i)
+                        if (i < n) dst[i * (D_V / 2)] = pk[i];
+                }
+                if (live && quarter == 0 && lane < T_HPW) {
+                    if (prev_no_split) {
+                        p.out_lse[row0 + lane] = lse;
+                        if (MAXL) p.out_max_logits[row0 + lane] = (x_all == -INFINITY) ? NEG_BIG : x_all;
+                    } else {
+                        p.lse_accum[row0 + lane] = lse;
+                    }
+                }
+                tc_fence_before();                         // the accumulator's reads precede the next request's first P.V
+                named_bar_sync(1 + grp, 128);              // xx is free again
+            };
+            if (prev && active) epilogue();
+            prev = false;
+            if (!have) break;
+            if (!active) continue;                         // no heads here
+            uint64_t l2[T_HPW / 2];                        // this token's share of the denominators of the warp's heads
+            float xm[MAXL ? T_HPW : 1];
+#pragma unroll
+            for (int i = 0; i < T_HPW / 2; ++i) l2[i] = 0ull;
+#pragma unroll
+            for (int i = 0; i < (MAXL ? T_HPW : 1); ++i) xm[i] = -INFINITY;
+            for (int j = 0; j < tiles.nst; ++j, ++it) {
+                const uint32_t b = it & 1u;
+                uint32_t z[T_HPW];
+                uint32_t sw = 0u, em = 0u;
+                bool grow = false;
+                float off = 0.f;                           // e_max + T_P_SHIFT: weights carry the shift
+                auto load_scores = [&]() {
+                    tmem_ld16(lane_addr + TM_S + 64 * b + h0, z);
+                    tmem_wait_ld();
+                };
+                // exponents: two per packed addition and FMA
+                auto exponents = [&]() {
+                    const uint64_t c2 = pack_f32x2(c, c), off2 = pack_f32x2(off, off);
+                    float mx = -INFINITY;
+#pragma unroll
+                    for (int i = 0; i < T_HPW; i += 4) {
+                        const ulonglong2 m4 = *reinterpret_cast<const ulonglong2*>(nm + h0 + i);
+                        uint64_t a = m4.x, d = m4.y;
+                        add_f32x2(a, off2);
+                        add_f32x2(d, off2);
+                        fma_f32x2(a, pack_f32x2(__uint_as_float(z[i]), __uint_as_float(z[i + 1])), c2);
+                        fma_f32x2(d, pack_f32x2(__uint_as_float(z[i + 2]), __uint_as_float(z[i + 3])), c2);
+                        float e0, e1, e2, e3;
+                        unpack_f32x2(a, e0, e1);
+                        unpack_f32x2(d, e2, e3);
+                        mx = fmaxf(mx, fmaxf(fmaxf(e0, e1), fmaxf(e2, e3)));
+                        z[i] = __float_as_uint(e0); z[i + 1] = __float_as_uint(e1); z[i + 2] = __float_as_uint(e2); z[i + 3] = __float_as_uint(e3);
+                    }
+                    if (!__all_sync(0xffffffffu, sw != 0u) && sw == 0u) {
+#pragma unroll
+                        for (int i = 0; i < T_HPW; ++i) z[i] = 0xff800000u;      // no entry: weight exactly 0
+                    }
+                    return mx;
+                };
+                if (!dead) dead = !mbar_wait_hot(bar(B_SCALES + (it & (SW_RING - 1))), (it / SW_RING) & 1u, abort_flag, WT_SCALES);
+                if (!dead) {
+                    sw = *reinterpret_cast<const uint32_t*>(sm + SW_OFF + ((it & (SW_RING - 1)) * T_TILE + token) * 4);
+                    const uint32_t em2 = __vmaxu4(sw, sw >> 16);
+                    em = max(em2 & 0xffu, (em2 >> 8) & 0xffu);
+                    off = (float)((int)em - 127 + T_P_SHIFT);
+                    dead = !mbar_wait_hot(bar(B_SREADY + b), (it >> 1) & 1u, abort_flag, WT_SREADY);
+                }
+                if (!dead) {
+                    tc_fence_after();
+                    load_scores();
+                    if (MAXL && sw != 0u) {
+#pragma unroll
+                        for (int i = 0; i < T_HPW; ++i) xm[i] = fmaxf(xm[i], __uint_as_float(z[i]));
+                    }
+                    grow = exponents() > T_TAU + (float)T_P_SHIFT && sw != 0u;
+                }
+                // Some weight of the group has outgrown the running maximum (or a wait gave up): rare after the first tiles of a
+                // request, so only then the maxima over the tokens are taken, exchanged and the accumulator rescaled.
+                if (named_bar_or(1 + grp, 128, grow || dead || *abort_flag != 0)) {
+                    if (*abort_flag != 0) dead = true;
+                    float mine = -INFINITY;
+                    if (!dead) {
+                        load_scores();
+#pragma unroll
+                        for (int i = 0; i < T_HPW; ++i) {
+                            const float r = lanes_max(sw != 0u ? fmaf(__uint_as_float(z[i]), c, off - (float)T_P_SHIFT) : -INFINITY);
+                            if ((lane & (T_HPW - 1)) == i) mine = r;
+                        }
+                        xx[quarter * T_HEADS + hl] = mine;
+                        if (j > 0) dead = !mbar_wait_hot(bar(B_PVDONE), (it - 1) & 1u, abort_flag, WT_PVDONE);
+                    }
+                    const float m_old = -nm[hl];
+                    if (named_bar_or(1 + grp, 128, dead || *abort_flag != 0)) { dead = true; break; }
+                    const float mx = fmaxf(fmaxf(xx[hl], xx[T_HEADS + hl]), fmaxf(xx[2 * T_HEADS + hl], xx[3 * T_HEADS + hl]));
+                    const bool up = mx > m_old;            // false while the head has seen no entry
+                    const float alpha = up ? ex2(m_old - mx) : 1.f;       // 0 for the first entries
+                    if (up) nm[hl] = -mx;                  // the four warps of the head write the same value
+                    tc_fence_after();
+                    if (__any_sync(0xffffffffu, up)) {
+#pragma unroll
+                        for (int i = 0; i < T_HPW / 2; ++i) {
+                            float a, d;
+                            unpack_f32x2(l2[i], a, d);
+                            l2[i] = pack_f32x2(a * __shfl_sync(0xffffffffu, alpha, 2 * i), d * __shfl_sync(0xffffffffu, alpha, 2 * i + 1));
+                        }
+                        if (j > 0) {
+#pragma unroll 1
+                            for (int bb = 0; bb < 4; ++bb) {
+                                uint32_t o[T_HPW];
+                                tmem_ld16(lane_addr + TM_O + 64 * bb + h0, o);
+                                tmem_wait_ld();
+#pragma unroll
+                                for (int i = 0; i < T_HPW; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * __shfl_sync(0xffffffffu, alpha, i));
+                                tmem_st16(lane_addr + TM_O + 64 * bb + h0, o);
+                            }
+                            tmem_wait_st();
+                        }
+                    }
+                    named_bar_sync(1 + grp, 128);          // xx is free again, the new maxima are in place
+                    load_scores();
+                    exponents();
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar(B_SFREE + b));      // the score buffer may be overwritten
+                const float is = sw != 0u ? __uint_as_float((254u - em) << 23) : 0.f;      // 1 / 2^e_max
+                const uint64_t is2 = pack_f32x2(is, is);
+#pragma unroll
+                for (int i = 0; i < T_HPW; i += 2) {
+                    const float p0 = ex2(__uint_as_float(z[i])), p1 = ex2(__uint_as_float(z[i + 1]));
+                    fma_f32x2(l2[i / 2], pack_f32x2(p0, p1), is2);
+                    z[i] = __float_as_uint(p0); z[i + 1] = __float_as_uint(p1);
+                }
+                // The weights of a block of dims are those of the row's largest scale times 2^(e_b - e_max).
+                auto packed = [&](float r) -> uint4 {
+                    uint32_t w[4];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                        w[i] = pack_e4m3x4(__uint_as_float(z[4 * i]) * r, __uint_as_float(z[4 * i + 1]) * r, __uint_as_float(z[4 * i + 2]) * r,
+                                           __uint_as_float(z[4 * i + 3]) * r);
+                    return make_uint4(w[0], w[1], w[2], w[3]);
+                };
+                const uint32_t down = __vsubus4(em * 0x01010101u, sw);      // e_max - e_b of the four blocks
+                const bool near = __all_sync(0xffffffffu, (down & 0xfefefefeu) == 0u || sw == 0u);
+                const uint4 w0 = packed(1.f);
+                uint4 w1 = w0;
+                if (near) w1 = packed(0.5f);
+                if (it > 0 && !dead) dead = !mbar_wait_hot(bar(B_PVDONE), (it - 1) & 1u, abort_flag, WT_PVDONE);   // the weights of the last tile have been read
+                if (dead) continue;
+                uint8_t* pb = sm + P_OFF + swz64((uint32_t)token, (uint32_t)grp);
+                if (near) {                                // the blocks' scales of the rows differ by a factor of two at most: two versions serve
+#pragma unroll
+                    for (int bb = 0; bb < 4; ++bb) {
+                        const bool h = (down >> (8 * bb)) & 1u;
+                        *reinterpret_cast<uint4*>(pb + bb * P_BYTES) = make_uint4(h ? w1.x : w0.x, h ? w1.y : w0.y, h ? w1.z : w0.z, h ? w1.w : w0.w);
+                    }
+                } else {
+#pragma unroll
+                    for (int bb = 0; bb < 4; ++bb) {
+                        const uint32_t d = min((down >> (8 * bb)) & 0xffu, 100u);
+                        *reinterpret_cast<uint4*>(pb + bb * P_BYTES) = d == 0u ? w0 : packed(__uint_as_float((127u - d) << 23));
+                    }
+                }
+                fence_proxy_async();
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar(B_PREADY));
+            }
+            if (dead) continue;
+            // sums over the warp's tokens: halve the list at every exchange, lanes i and i + 16 end with head i
+            float s[T_HPW];
+#pragma unroll
+            for (int i = 0; i < T_HPW / 2; ++i) unpack_f32x2(l2[i], s[2 * i], s[2 * i + 1]);
+#pragma unroll
+            for (int i = 0; i < T_HPW; ++i) s[i] += __shfl_xor_sync(0xffffffffu, s[i], 16);
+#pragma unroll
+            for (int o = T_HPW / 2; o >= 1; o >>= 1) {
+#pragma unroll
+                for (int i = 0; i < o; ++i) {
+                    const bool up = (lane & o) != 0;
+                    const float send = up ? s[i] : s[i + o], keep = up ? s[i + o] : s[i];
+                    s[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+                }
+            }
+            prev_l = s[0];
+            if (MAXL) {
+#pragma unroll
+                for (int i = 0; i < T_HPW; ++i) {
+                    const float r = lanes_max(xm[i]);
+                    if ((lane & (T_HPW - 1)) == i) prev_x = r * c;
+                }
+            }
+            prev_m = -nm[hl];
+            prev = true; prev_no_split = tiles.w.no_split; prev_req = tiles.w.req; prev_split = tiles.w.split_idx;
+        }
+    } else if (warp < T_SCALE) {
+        // =================================================================== rows -> K stages (TMA gather)
+        const int quarter = warp - T_PROD;
+        Tiles tiles(first, step, last);
+        bool have = tiles.next_tile(p, meta), ok = true;
+        int idx = have ? tiles.row_index(p, quarter * 32 + lane) : -1;
+        for (uint32_t it = 0; have; ++it) {
+            const uint32_t st = it % NSTAGE;
+            const int row = idx >= 0 ? idx : NO_ROW;
+            have = tiles.next_tile(p, meta);
+            const int idx_next = have ? tiles.row_index(p, quarter * 32 + lane) : -1;     // read ahead of its use
+            auto gather = [&](uint32_t dst, int x, uint32_t full) {                  // 128 bytes of each of the warp's 32 rows
+                if (elect_one()) mbar_arrive_expect_tx(full, 32 * 128);
+                __syncwarp();
+#pragma unroll
+                for (int q = 0; q < 8; ++q) {
+                    const int r0 = __shfl_sync(0xffffffffu, row, 4 * q), r1 = __shfl_sync(0xffffffffu, row, 4 * q + 1);
+                    const int r2 = __shfl_sync(0xffffffffu, row, 4 * q + 2), r3 = __shfl_sync(0xffffffffu, row, 4 * q + 3);
+                    if (elect_one()) tma_gather4(dst + quarter * (32 * 128) + q * 512, &kv_map, x, r0, r1, r2, r3, full);
+                    __syncwarp();
+                }
+            };
+            // the RoPE stage is free when the scores of the tile before are done, earlier than this tile's stage
+            if (it >= 1) ok = mbar_wait_hot(bar(B_SREADY + ((it - 1) & 1u)), ((it - 1) >> 1) & 1u, abort_flag, WT_SREADY);
+            if (!ok) break;
+            gather(base + R_OFF, ROPE_OFF / 4, bar(B_RFULL));
+            if (it >= NSTAGE) ok = mbar_wait_hot(bar(B_KFREE + 4 * st + quarter), ((it / NSTAGE) - 1) & 1u, abort_flag, WT_KFREE);
+            if (!ok) break;
+#pragma unroll 1
+            for (int b = 0; b < 4; ++b) gather(base + K_OFF + st * K_STAGE + b * K_CHUNK, 32 * b, bar(B_KFULL + 4 * st + b));
+            idx = idx_next;
+        }
+    } else if (warp < T_QK) {
+        // =================================================================== scale words
+        // Lane i reads the scales of tokens i, 32 + i, 64 + i, 96 + i: row r's word belongs into column r / 32 of lane r % 32, in
+        // all four lane quarters.
+        const int quarter = warp - T_SCALE;
+        const uint32_t lane_addr = tmem + ((uint32_t)(quarter * 32) << 16);
+        Tiles tiles(first, step, last);
+        bool have = tiles.next_tile(p, meta), ok = true;
+        int idx[4];
+        uint4 sc[4];
+        auto fetch = [&]() {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) idx[k] = have ? tiles.row_index(p, 32 * k + lane) : -1;
+        };
+        auto load = [&]() {                                // (exponent 0 marks a token without an entry)
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                sc[k] = make_uint4(0u, 0u, 0u, 0u);
+                if (idx[k] >= 0) sc[k] = __ldg(reinterpret_cast<const uint4*>(p.kv + (size_t)idx[k] * ROW_BYTES + SCALE_OFF));
+            }
+        };
+        uint32_t some = 0u;                                // which of the four tokens of the loaded tile have an entry
+        auto mark = [&]() {
+            some = 0u;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) some |= (idx[k] >= 0 ? 1u : 0u) << k;
+        };
+        fetch();
+        load();
+        mark();
+        bool cur = have;
+        have = have && tiles.next_tile(p, meta);
+        fetch();
+        for (uint32_t it = 0; cur; ++it) {
+            uint32_t word[4], mx[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                auto e = [](uint32_t s) { return max((s >> 23) & 0xffu, 1u); };
+                word[k] = ((some >> k) & 1u) ? e(sc[k].x) | (e(sc[k].y) << 8) | (e(sc[k].z) << 16) | (e(sc[k].w) << 24) : 0u;
+                mx[k] = word[k] != 0u ? word[k] : 0x7f7f7f7fu;
+            }
+            load();                                        // of the next tile
+            mark();
+            cur = have;
+            have = have && tiles.next_tile(p, meta);
+            fetch();
+            if (it >= 2) ok = mbar_wait_hot(bar(B_SREADY + (it & 1u)), ((it >> 1) - 1) & 1u, abort_flag, WT_SREADY);   // the scores two tiles ago are done
+            if (!ok) break;
+            tc_fence_after();
+            tmem_st4(lane_addr + TM_SFA + 4 * (it & 1u), mx);
+            const uint32_t mine = quarter == 0 ? word[0] : quarter == 1 ? word[1] : quarter == 2 ? word[2] : word[3];
+            *reinterpret_cast<uint32_t*>(sm + SW_OFF + ((it & (SW_RING - 1)) * T_TILE + quarter * 32 + lane) * 4) = mine;
+            tmem_wait_st();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar(B_SCALES + (it & (SW_RING - 1))));
+        }
+    } else if (warp == T_QK) {
+        // =================================================================== score MMAs
+        const uint32_t q_lo = desc_lo(base + Q_OFF, 16), qr_lo = desc_lo(base + QR_OFF, 16), r_lo = desc_lo(base + R_OFF, 16);
+        Tiles tiles(first, step, last);
+        uint32_t it = 0, rq = 0;
+        bool ok = true;
+        while (ok && tiles.next_request(p, meta)) {
+            ok = mbar_wait_hot(bar(B_QREADY), rq & 1u, abort_flag, WT_QREADY);
+            ++rq;
+            for (int j = 0; j < tiles.nst && ok; ++j, ++it) {
+                const uint32_t st = it % NSTAGE, b = it & 1u;
+                if (it >= 2) ok = mbar_wait_hot(bar(B_SFREE + b), ((it >> 1) - 1) & 1u, abort_flag, WT_SFREE);
+                if (ok) ok = mbar_wait_hot(bar(B_SCALES + (it & (SW_RING - 1))), (it / SW_RING) & 1u, abort_flag, WT_SCALES);
+                if (ok) ok = mbar_wait_hot(bar(B_RFULL), it & 1u, abort_flag, WT_RFULL);
+                if (!ok) break;
+                tc_fence_after();
+                const uint32_t k_lo = desc_lo(base + K_OFF + st * K_STAGE, 16), d = tmem + TM_S + 64 * b;
+                if (elect_one()) {
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)
+                        mma_f16(d, make_desc(r_lo + ((k * 32) >> 4), HI_128), make_desc(qr_lo + ((k * 32) >> 4), HI_128), IDESC_ROPE, k != 0);
+                }
+                __syncwarp();
+#pragma unroll
+                for (int bb = 0; bb < 4; ++bb) {
+                    if (ok) ok = mbar_wait_hot(bar(B_KFULL + 4 * st + bb), (it / NSTAGE) & 1u, abort_flag, WT_KFULL);
+                    if (!ok) break;
+                    if (elect_one()) {
+#pragma unroll
+                        for (int k = 0; k < 4; ++k)
+                            mma_mxf8(d, make_desc(k_lo + ((bb * K_CHUNK + k * 32) >> 4), HI_128), make_desc(q_lo + ((bb * Q_CHUNK + k * 32) >> 4), HI_128),
+                                     idesc_mx(bb), tmem + TM_SFA + 4 * b, tmem + TM_SFB, true);
+                        if (bb == 3) tc_commit(bar(B_SREADY + b));
+                    }
+                    __syncwarp();
+                }
+            }
+        }
+    } else if (warp == T_PV) {
+        // =================================================================== P.V MMAs
+        Tiles tiles(first, step, last);
+        const uint32_t p_lo = desc_lo(base + P_OFF, 16);
+        uint32_t it = 0;
+        bool ok = true;
+        while (ok && tiles.next_request(p, meta)) {
+            for (int j = 0; j < tiles.nst && ok; ++j, ++it) {
+                const uint32_t st = it % NSTAGE;
+                ok = mbar_wait_hot(bar(B_PREADY), it & 1u, abort_flag, WT_PREADY);
+                if (!ok) break;
+                tc_fence_after();
+                const uint32_t v_lo = desc_lo(base + K_OFF + st * K_STAGE, 16);
+                if (elect_one()) {
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {          // 32 tokens: their rows may be overwritten as soon as they have been read
+#pragma unroll
+                        for (int b = 0; b < 4; ++b)
+                            mma_f8(tmem + TM_O + 64 * b, make_desc(v_lo + ((b * K_CHUNK + k * 4096) >> 4), HI_128),
+                                   make_desc(p_lo + ((b * P_BYTES + k * 2048) >> 4), HI_P), IDESC_PV, (j | k) != 0);
+                        tc_commit(bar(B_KFREE + 4 * st + k));
+                    }
+                    tc_commit(bar(B_PVDONE));
+                }
+                __syncwarp();
+            }
+        }
+    }
+
+    if (*abort_flag != 0) {        // a wait gave up: copies and MMAs may still be in flight; give them time to finish
+        const long long t0 = clock64();
+        while (clock64() - t0 < 200000) { }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (tid == 0 && *abort_flag != 0 && p.status != nullptr) {
+        atomicCAS(p.status, 0, *abort_flag);
+        atomicAdd(p.status + 1, 1);
+        p.status[2] = blockIdx.x;
+    }
+    if (warp == T_QK) { tc_fence_after(); tmem_dealloc(tmem, 512); }
+}
+
+typedef CUresult (*EncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
+                             const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+}  // namespace
+
+// One linear array of 656-byte rows: pages without padding between them.
+bool attn_tile_takes(const AttnParams& p) {
+    return p.layout == SMLA_LAYOUT_V32 && p.extra_topk == 0 && p.block_stride == (int64_t)p.page_block_size * ROW_BYTES &&
+           (reinterpret_cast<uintptr_t>(p.kv) & 15u) == 0;
+}
+
+int launch_attn_tile(const AttnParams& p, cudaStream_t stream) {
+    if (p.num_tokens == 0) return 0;
+    static bool attr_set[64] = {};
+    static int sm_count[64] = {};
+    static EncodeFn encode = nullptr;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 0 || dev >= 64) return set_error(SMLA_E_SHAPE, "attn_tile_kernel: device ordinal %d not supported", dev);
+    if (!attr_set[dev]) {
+        cudaDriverEntryPointQueryResult qres;
+        void* fn = nullptr;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &qres) != cudaSuccess || fn == nullptr)
+            return set_error(SMLA_E_DEVICE, "attn_tile_kernel: the driver has no cuTensorMapEncodeTiled");
+        encode = (EncodeFn)fn;
+        cudaFuncAttributes fa[2];
+        if (cudaFuncGetAttributes(&fa[0], attn_tile_kernel<false>) != cudaSuccess || cudaFuncGetAttributes(&fa[1], attn_tile_kernel<true>) != cudaSuccess ||
+            fa[0].numRegs != T_REGS_LAUNCH || fa[1].numRegs != T_REGS_LAUNCH)
+            return set_error(SMLA_E_DEVICE, "attn_tile_kernel: compiled with %d and %d registers per thread, the warpgroup budgets assume %d",
+                             fa[0].numRegs, fa[1].numRegs, T_REGS_LAUNCH);
+        cudaError_t e = cudaFuncSetAttribute(attn_tile_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T_SMEM);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(attn_tile_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T_SMEM);
+        if (e != cudaSuccess) return set_error((int)e, "attn_tile_kernel: cannot reserve %u bytes of shared memory: %s", T_SMEM, cudaGetErrorString(e));
+        cudaDeviceGetAttribute(&sm_count[dev], cudaDevAttrMultiProcessorCount, dev);
+        attr_set[dev] = true;
+    }
+    // the cache as 32-bit words, 164 per row; boxes of 32 words (128 bytes) of one row
+    CUtensorMap map;
+    const cuuint64_t dims[2] = {ROW_BYTES / 4, (cuuint64_t)NO_ROW}, strides[1] = {ROW_BYTES};
+    const cuuint32_t box[2] = {32, 1}, estr[2] = {1, 1};
+    const CUresult r = encode(&map, CU_TENSOR_MAP_DATA_TYPE_INT32, 2, const_cast<uint8_t*>(p.kv), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return set_error(SMLA_E_DEVICE, "attn_tile_kernel: cuTensorMapEncodeTiled failed (%d)", (int)r);
+    const int halves = (p.num_heads + T_HEADS - 1) / T_HEADS;
+    const int most = sm_count[dev] / halves > 0 ? sm_count[dev] / halves : 1;
+    const int parts = p.sched ? p.num_parts : p.uniform_k > 1 ? p.uniform_k * p.num_tokens : (p.num_tokens < most ? p.num_tokens : most);
+    const dim3 grid(parts * halves);
+    auto* kernel = p.out_max_logits != nullptr ? attn_tile_kernel<true> : attn_tile_kernel<false>;
+    if (p.sched != nullptr) launch_dependent(kernel, grid, dim3(T_THREADS), T_SMEM, stream, p, halves, map);
+    else kernel<<<grid, T_THREADS, T_SMEM, stream>>>(p, halves, map);
+    return check_launch("attn_tile_kernel");
+}
+
+}  // namespace smla
