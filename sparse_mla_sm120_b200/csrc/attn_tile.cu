@@ -25,8 +25,9 @@
 //   warps 0-15   softmax, epilogue, Q: warp w holds tokens [32 (w % 4), +32) and heads [16 (w / 4), +16) of a tile, a thread
 //                one token; the four warps of a head group meet once per tile at a barrier that also ORs "a weight has
 //                outgrown the running maximum".  Groups without heads only quantise Q.
-//   warps 16-19  producers: warp 16 + i gathers rows [32 i, +32) of every tile; a quarter of a stage is refilled as soon as
-//                P.V has read it, and the score MMAs of a block of dims start when that block has landed.
+//   warps 16-19  producers: warp 16 + i gathers the no-PE dims of rows [32 i, +32) of every tile, the four pieces of a quad of
+//                rows one after the other (piece by piece over all rows takes twice as long); a quarter of a stage is
+//                refilled as soon as P.V has read it.  Warps 26 and 27 gather the RoPE as soon as its one stage is free.
 //   warps 20-23  scales: the rows' scale words into tensor memory (each warp the 32 lanes it can reach) and shared memory.
 //   warp 24      issues the score MMAs, warp 25 the P.V MMAs (one elected lane each).
 // Every wait is bounded; a wait that gives up records a code in status[] and the CTA drains and exits.
@@ -44,14 +45,14 @@ using namespace attn;
 
 constexpr int T_HEADS = 64;                    // heads per CTA
 constexpr int T_TILE = 128;                    // tokens per tile: two scheduler blocks
-constexpr int T_SM_WARPS = 16, T_PROD = 16, T_SCALE = 20, T_QK = 24, T_PV = 25;
+constexpr int T_SM_WARPS = 16, T_PROD = 16, T_SCALE = 20, T_QK = 24, T_PV = 25, T_ROPE = 26;
 constexpr int T_THREADS = 28 * 32;
 constexpr int T_HPW = 16;                      // heads per softmax warp
 constexpr int T_REGS_LAUNCH = 72, T_REGS_SOFTMAX = 88, T_REGS_REST = 48;
 static_assert(T_SM_WARPS * 32 * T_REGS_SOFTMAX + (T_THREADS - T_SM_WARPS * 32) * T_REGS_REST <= T_THREADS * T_REGS_LAUNCH,
               "register budgets exceed what the CTA owns");
-constexpr int T_P_SHIFT = 5;                   // P' is stored as e4m3(P' * 2^T_P_SHIFT)
-constexpr float T_TAU = 3.0f;                  // lazy-rescale threshold (log2 units); P' <= 2^T_TAU
+constexpr int T_P_SHIFT = 7;                   // P' is stored as e4m3(P' * 2^T_P_SHIFT)
+constexpr float T_TAU = 1.0f;                  // lazy-rescale threshold (log2 units); P' <= 2^T_TAU
 constexpr float T_NO_MAX = 1e30f;              // minus the running maximum of a head that has seen no entry (finite: -inf minus it is -inf)
 constexpr int NSTAGE = 2;
 
@@ -70,7 +71,7 @@ constexpr uint32_t NM_OFF = SW_OFF + SW_RING * T_TILE * 4; // -m of the 64 heads
 constexpr uint32_t QW_OFF = NM_OFF + T_HEADS * 4;          // the heads' scale words
 constexpr uint32_t XX_OFF = QW_OFF + T_HEADS * 4;          // exchange between the four warps of a head group: [2][4][64] fp32
 constexpr uint32_t B_OFF = XX_OFF + 2 * 4 * T_HEADS * 4;
-constexpr int B_KFULL = 0, B_RFULL = B_KFULL + 4 * NSTAGE, B_KFREE = B_RFULL + 1, B_SREADY = B_KFREE + 4 * NSTAGE, B_SFREE = B_SREADY + 2,
+constexpr int B_KFULL = 0, B_RFULL = B_KFULL + NSTAGE, B_KFREE = B_RFULL + 1, B_SREADY = B_KFREE + 4 * NSTAGE, B_SFREE = B_SREADY + 2,
               B_SCALES = B_SFREE + 2, B_PREADY = B_SCALES + SW_RING, B_PVDONE = B_PREADY + 1, B_QREADY = B_PVDONE + 1, B_N = B_QREADY + 1;
 constexpr uint32_t MISC_OFF = B_OFF + B_N * 8;
 constexpr uint32_t T_SMEM = MISC_OFF + 16 + 1024;
@@ -140,12 +141,10 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
 
     if (tid == 0) {
         for (int s = 0; s < NSTAGE; ++s) {
-            for (int i = 0; i < 4; ++i) {
-                mbar_init(bar(B_KFULL + 4 * s + i), 4);    // dims block i of the stage: + the bytes of the four producers
-                mbar_init(bar(B_KFREE + 4 * s + i), 1);    // its rows [32 i, +32) have been read
-            }
+            mbar_init(bar(B_KFULL + s), 4);                // + the bytes of the four producers
+            for (int i = 0; i < 4; ++i) mbar_init(bar(B_KFREE + 4 * s + i), 1);    // its rows [32 i, +32) have been read
         }
-        mbar_init(bar(B_RFULL), 4);
+        mbar_init(bar(B_RFULL), 2);
         for (int b = 0; b < 2; ++b) { mbar_init(bar(B_SREADY + b), 1); mbar_init(bar(B_SFREE + b), act); }
         for (int i = 0; i < SW_RING; ++i) mbar_init(bar(B_SCALES + i), 4);
         mbar_init(bar(B_PREADY), act);
@@ -350,29 +349,49 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
                     tmem_ld16(lane_addr + TM_S + 64 * b + h0, z);
                     tmem_wait_ld();
                 };
-                // exponents: two per packed addition and FMA
-                auto exponents = [&]() {
-                    const uint64_t c2 = pack_f32x2(c, c), off2 = pack_f32x2(off, off);
-                    float mx = -INFINITY;
+                // exponents: two per FMA, onto e_max + T_P_SHIFT - m
+                uint64_t e2[T_HPW / 2];
+                auto offsets = [&]() {
+                    const uint64_t off2 = pack_f32x2(off, off);
 #pragma unroll
                     for (int i = 0; i < T_HPW; i += 4) {
                         const ulonglong2 m4 = *reinterpret_cast<const ulonglong2*>(nm + h0 + i);
-                        uint64_t a = m4.x, d = m4.y;
-                        add_f32x2(a, off2);
-                        add_f32x2(d, off2);
-                        fma_f32x2(a, pack_f32x2(__uint_as_float(z[i]), __uint_as_float(z[i + 1])), c2);
-                        fma_f32x2(d, pack_f32x2(__uint_as_float(z[i + 2]), __uint_as_float(z[i + 3])), c2);
-                        float e0, e1, e2, e3;
-                        unpack_f32x2(a, e0, e1);
-                        unpack_f32x2(d, e2, e3);
-                        mx = fmaxf(mx, fmaxf(fmaxf(e0, e1), fmaxf(e2, e3)));
-                        z[i] = __float_as_uint(e0); z[i + 1] = __float_as_uint(e1); z[i + 2] = __float_as_uint(e2); z[i + 3] = __float_as_uint(e3);
+                        e2[i / 2] = m4.x; e2[i / 2 + 1] = m4.y;
+                        add_f32x2(e2[i / 2], off2);
+                        add_f32x2(e2[i / 2 + 1], off2);
+                    }
+                };
+                auto exponents = [&]() {
+                    const uint64_t c2 = pack_f32x2(c, c);
+#pragma unroll
+                    for (int i = 0; i < T_HPW; i += 2) {
+                        fma_f32x2(e2[i / 2], pack_f32x2(__uint_as_float(z[i]), __uint_as_float(z[i + 1])), c2);
+                        float a, d;
+                        unpack_f32x2(e2[i / 2], a, d);
+                        z[i] = __float_as_uint(a); z[i + 1] = __float_as_uint(d);
                     }
                     if (!__all_sync(0xffffffffu, sw != 0u) && sw == 0u) {
 #pragma unroll
                         for (int i = 0; i < T_HPW; ++i) z[i] = 0xff800000u;      // no entry: weight exactly 0
                     }
-                    return mx;
+                };
+                // The weights of a block of dims are those of the row's largest scale times 2^(e_b - e_max).
+                auto packed = [&](float r) -> uint4 {
+                    uint32_t w[4];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                        w[i] = pack_e4m3x4(__uint_as_float(z[4 * i]) * r, __uint_as_float(z[4 * i + 1]) * r, __uint_as_float(z[4 * i + 2]) * r,
+                                           __uint_as_float(z[4 * i + 3]) * r);
+                    return make_uint4(w[0], w[1], w[2], w[3]);
+                };
+                uint4 w0 = make_uint4(0u, 0u, 0u, 0u), w1 = w0;
+                uint32_t down = 0u;                        // e_max - e_b of the four blocks
+                bool near = true;
+                auto weights = [&]() {
+#pragma unroll
+                    for (int i = 0; i < T_HPW; ++i) z[i] = __float_as_uint(ex2(__uint_as_float(z[i])));
+                    w0 = packed(1.f);
+                    if (near) w1 = packed(0.5f);
                 };
                 if (!dead) dead = !mbar_wait_hot(bar(B_SCALES + (it & (SW_RING - 1))), (it / SW_RING) & 1u, abort_flag, WT_SCALES);
                 if (!dead) {
@@ -380,6 +399,9 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
                     const uint32_t em2 = __vmaxu4(sw, sw >> 16);
                     em = max(em2 & 0xffu, (em2 >> 8) & 0xffu);
                     off = (float)((int)em - 127 + T_P_SHIFT);
+                    down = __vsubus4(em * 0x01010101u, sw);
+                    near = __all_sync(0xffffffffu, (down & 0xfefefefeu) == 0u || sw == 0u);
+                    offsets();
                     dead = !mbar_wait_hot(bar(B_SREADY + b), (it >> 1) & 1u, abort_flag, WT_SREADY);
                 }
                 if (!dead) {
@@ -389,7 +411,12 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
 #pragma unroll
                         for (int i = 0; i < T_HPW; ++i) xm[i] = fmaxf(xm[i], __uint_as_float(z[i]));
                     }
-                    grow = exponents() > T_TAU + (float)T_P_SHIFT && sw != 0u;
+                    exponents();
+                    float mx = __uint_as_float(z[0]);
+#pragma unroll
+                    for (int i = 1; i < T_HPW; ++i) mx = fmaxf(mx, __uint_as_float(z[i]));
+                    grow = mx > T_TAU + (float)T_P_SHIFT;
+                    weights();                             // before the barrier: they are rarely computed again
                 }
                 // Some weight of the group has outgrown the running maximum (or a wait gave up): rare after the first tiles of a
                 // request, so only then the maxima over the tokens are taken, exchanged and the accumulator rescaled.
@@ -435,7 +462,9 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
                     }
                     named_bar_sync(1 + grp, 128);          // xx is free again, the new maxima are in place
                     load_scores();
+                    offsets();
                     exponents();
+                    weights();
                 }
                 tc_fence_before();
                 __syncwarp();
@@ -443,25 +472,8 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
                 const float is = sw != 0u ? __uint_as_float((254u - em) << 23) : 0.f;      // 1 / 2^e_max
                 const uint64_t is2 = pack_f32x2(is, is);
 #pragma unroll
-                for (int i = 0; i < T_HPW; i += 2) {
-                    const float p0 = ex2(__uint_as_float(z[i])), p1 = ex2(__uint_as_float(z[i + 1]));
-                    fma_f32x2(l2[i / 2], pack_f32x2(p0, p1), is2);
-                    z[i] = __float_as_uint(p0); z[i + 1] = __float_as_uint(p1);
-                }
-                // The weights of a block of dims are those of the row's largest scale times 2^(e_b - e_max).
-                auto packed = [&](float r) -> uint4 {
-                    uint32_t w[4];
-#pragma unroll
-                    for (int i = 0; i < 4; ++i)
-                        w[i] = pack_e4m3x4(__uint_as_float(z[4 * i]) * r, __uint_as_float(z[4 * i + 1]) * r, __uint_as_float(z[4 * i + 2]) * r,
-                                           __uint_as_float(z[4 * i + 3]) * r);
-                    return make_uint4(w[0], w[1], w[2], w[3]);
-                };
-                const uint32_t down = __vsubus4(em * 0x01010101u, sw);      // e_max - e_b of the four blocks
-                const bool near = __all_sync(0xffffffffu, (down & 0xfefefefeu) == 0u || sw == 0u);
-                const uint4 w0 = packed(1.f);
-                uint4 w1 = w0;
-                if (near) w1 = packed(0.5f);
+                for (int i = 0; i < T_HPW; i += 2)
+                    fma_f32x2(l2[i / 2], pack_f32x2(__uint_as_float(z[i]), __uint_as_float(z[i + 1])), is2);
                 if (it > 0 && !dead) dead = !mbar_wait_hot(bar(B_PVDONE), (it - 1) & 1u, abort_flag, WT_PVDONE);   // the weights of the last tile have been read
                 if (dead) continue;
                 uint8_t* pb = sm + P_OFF + swz64((uint32_t)token, (uint32_t)grp);
@@ -511,7 +523,7 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
             prev = true; prev_no_split = tiles.w.no_split; prev_req = tiles.w.req; prev_split = tiles.w.split_idx;
         }
     } else if (warp < T_SCALE) {
-        // =================================================================== rows -> K stages (TMA gather)
+        // =================================================================== no-PE dims -> K stages (TMA gather)
         const int quarter = warp - T_PROD;
         Tiles tiles(first, step, last);
         bool have = tiles.next_tile(p, meta), ok = true;
@@ -521,25 +533,21 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
             const int row = idx >= 0 ? idx : NO_ROW;
             have = tiles.next_tile(p, meta);
             const int idx_next = have ? tiles.row_index(p, quarter * 32 + lane) : -1;     // read ahead of its use
-            auto gather = [&](uint32_t dst, int x, uint32_t full) {                  // 128 bytes of each of the warp's 32 rows
-                if (elect_one()) mbar_arrive_expect_tx(full, 32 * 128);
-                __syncwarp();
-#pragma unroll
-                for (int q = 0; q < 8; ++q) {
-                    const int r0 = __shfl_sync(0xffffffffu, row, 4 * q), r1 = __shfl_sync(0xffffffffu, row, 4 * q + 1);
-                    const int r2 = __shfl_sync(0xffffffffu, row, 4 * q + 2), r3 = __shfl_sync(0xffffffffu, row, 4 * q + 3);
-                    if (elect_one()) tma_gather4(dst + quarter * (32 * 128) + q * 512, &kv_map, x, r0, r1, r2, r3, full);
-                    __syncwarp();
-                }
-            };
-            // the RoPE stage is free when the scores of the tile before are done, earlier than this tile's stage
-            if (it >= 1) ok = mbar_wait_hot(bar(B_SREADY + ((it - 1) & 1u)), ((it - 1) >> 1) & 1u, abort_flag, WT_SREADY);
-            if (!ok) break;
-            gather(base + R_OFF, ROPE_OFF / 4, bar(B_RFULL));
             if (it >= NSTAGE) ok = mbar_wait_hot(bar(B_KFREE + 4 * st + quarter), ((it / NSTAGE) - 1) & 1u, abort_flag, WT_KFREE);
             if (!ok) break;
-#pragma unroll 1
-            for (int b = 0; b < 4; ++b) gather(base + K_OFF + st * K_STAGE + b * K_CHUNK, 32 * b, bar(B_KFULL + 4 * st + b));
+            const uint32_t dst = base + K_OFF + st * K_STAGE + quarter * (32 * 128), full = bar(B_KFULL + st);
+            if (elect_one()) mbar_arrive_expect_tx(full, 4 * 32 * 128);
+            __syncwarp();
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                const int r0 = __shfl_sync(0xffffffffu, row, 4 * q), r1 = __shfl_sync(0xffffffffu, row, 4 * q + 1);
+                const int r2 = __shfl_sync(0xffffffffu, row, 4 * q + 2), r3 = __shfl_sync(0xffffffffu, row, 4 * q + 3);
+                if (elect_one()) {
+#pragma unroll
+                    for (int b = 0; b < 4; ++b) tma_gather4(dst + b * K_CHUNK + q * 512, &kv_map, 32 * b, r0, r1, r2, r3, full);
+                }
+                __syncwarp();
+            }
             idx = idx_next;
         }
     } else if (warp < T_QK) {
@@ -622,19 +630,20 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
                         mma_f16(d, make_desc(r_lo + ((k * 32) >> 4), HI_128), make_desc(qr_lo + ((k * 32) >> 4), HI_128), IDESC_ROPE, k != 0);
                 }
                 __syncwarp();
+                ok = mbar_wait_hot(bar(B_KFULL + st), (it / NSTAGE) & 1u, abort_flag, WT_KFULL);
+                if (!ok) break;
+                tc_fence_after();
+                if (elect_one()) {
 #pragma unroll
-                for (int bb = 0; bb < 4; ++bb) {
-                    if (ok) ok = mbar_wait_hot(bar(B_KFULL + 4 * st + bb), (it / NSTAGE) & 1u, abort_flag, WT_KFULL);
-                    if (!ok) break;
-                    if (elect_one()) {
+                    for (int bb = 0; bb < 4; ++bb) {
 #pragma unroll
                         for (int k = 0; k < 4; ++k)
                             mma_mxf8(d, make_desc(k_lo + ((bb * K_CHUNK + k * 32) >> 4), HI_128), make_desc(q_lo + ((bb * Q_CHUNK + k * 32) >> 4), HI_128),
                                      idesc_mx(bb), tmem + TM_SFA + 4 * b, tmem + TM_SFB, true);
-                        if (bb == 3) tc_commit(bar(B_SREADY + b));
                     }
-                    __syncwarp();
+                    tc_commit(bar(B_SREADY + b));
                 }
+                __syncwarp();
             }
         }
     } else if (warp == T_PV) {
@@ -662,6 +671,37 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
                     tc_commit(bar(B_PVDONE));
                 }
                 __syncwarp();
+            }
+        }
+    } else {
+        // =================================================================== RoPE -> its stage (TMA gather)
+        const int half = warp - T_ROPE;                    // rows [64 half, +64), two per lane
+        Tiles tiles(first, step, last);
+        bool have = tiles.next_tile(p, meta), ok = true;
+        int idx[2] = {-1, -1};
+        auto fetch = [&]() {
+#pragma unroll
+            for (int k = 0; k < 2; ++k) idx[k] = have ? tiles.row_index(p, 64 * half + 32 * k + lane) : -1;
+        };
+        fetch();
+        for (uint32_t it = 0; have; ++it) {
+            const int row[2] = {idx[0] >= 0 ? idx[0] : NO_ROW, idx[1] >= 0 ? idx[1] : NO_ROW};
+            have = tiles.next_tile(p, meta);
+            fetch();
+            // the stage is free when the scores of the tile before are done
+            if (it >= 1) ok = mbar_wait_hot(bar(B_SREADY + ((it - 1) & 1u)), ((it - 1) >> 1) & 1u, abort_flag, WT_SREADY);
+            if (!ok) break;
+            if (elect_one()) mbar_arrive_expect_tx(bar(B_RFULL), 64 * 128);
+            __syncwarp();
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+#pragma unroll
+                for (int q = 0; q < 8; ++q) {
+                    const int r0 = __shfl_sync(0xffffffffu, row[k], 4 * q), r1 = __shfl_sync(0xffffffffu, row[k], 4 * q + 1);
+                    const int r2 = __shfl_sync(0xffffffffu, row[k], 4 * q + 2), r3 = __shfl_sync(0xffffffffu, row[k], 4 * q + 3);
+                    if (elect_one()) tma_gather4(base + R_OFF + (64 * half + 32 * k) * 128 + q * 512, &kv_map, ROPE_OFF / 4, r0, r1, r2, r3, bar(B_RFULL));
+                    __syncwarp();
+                }
             }
         }
     }
