@@ -106,6 +106,13 @@ def tc_aligned(kv_cache: torch.Tensor, extra_kv: Optional[torch.Tensor] = None) 
     return True
 
 
+def one_array(kv_cache: torch.Tensor) -> bool:
+    """Whether the 656-byte rows of a cache are one linear, 16-byte aligned array (pages without padding between them):
+    what attn_tile_kernel needs to name rows by their index (the library checks the same)."""
+    block, stride = kv_geometry(kv_cache)
+    return stride == block * 656 and kv_cache.data_ptr() % 16 == 0
+
+
 def pick_num_sm_parts_fp32(num_tokens: int, num_heads: int, sms: int) -> int:
     """Partitions for the fp32 kernel, which runs ceil(heads / 8) CTAs per partition: requests stay
     whole when they already give two CTAs per SM, otherwise the work is cut so that they do."""
@@ -190,11 +197,37 @@ def pick_split(num_tokens: int, sms: int, blocks_per_token: Optional[int] = None
     return best[1], best[2]
 
 
+# attn_tile_kernel (up to 64 heads over one linear array of rows): microseconds of a partition's fixed part, of a 128-token
+# tile, and of what a split adds: a part that grows with the pieces of a request, and the records that are written and
+# read back.  Fitted to 1 to 64 requests of top-k 512, 1024 and 2048 in up to 16 equal partitions each, 16 and 64 heads (48
+# requests of top-k 2048 at 16 heads: 40 us whole, 28.6 us in two partitions each; one: 38.5, 25.3, 18.5, 17.9 and 19.9 us in
+# 1, 2, 4, 8 and 16); the cut that it names is the fastest measured one or within a microsecond of it.
+def _tile_us(num_tokens: int, num_heads: int, blocks: int, k: int) -> float:
+    t = 7.3 + 0.022 * num_heads + -(-(blocks // k) // 2) * (1.78 + 0.0077 * num_heads)
+    return t if k == 1 else t + 1.9 + 0.45 * k + 0.03 * k * num_tokens
+
+
+def pick_split_tile(num_tokens: int, num_heads: int, sms: int, blocks_per_token: int, uniform: bool) -> Tuple[int, int]:
+    """(partitions, fixed overhead) for attn_tile_kernel, which runs one CTA per partition.  Requests of equal length are
+    cut into as many equal partitions as pay off while all of them run at once.  Where no equal cut exists the rule is the
+    general one: a partition that straddles two requests pays its fixed part twice, so that more of them, one per SM,
+    are slower than half as many (16 requests of top-k 2048: 34 us in 148 partitions, 28 us in 74)."""
+    n = max(blocks_per_token, 1)
+    if not uniform:
+        return pick_num_sm_parts(num_tokens, sms, blocks_per_token), FIXED_OVERHEAD
+    cuts = [k for k in range(2, n // 2 + 1) if n % k == 0 and k * num_tokens <= sms]
+    if not cuts and n >= 2 * BLOCKS_PER_PARTITION:
+        return pick_num_sm_parts(num_tokens, sms, blocks_per_token), FIXED_OVERHEAD
+    k = min([1] + cuts, key=lambda c: _tile_us(num_tokens, num_heads, n, c))
+    return (num_tokens, FIXED_OVERHEAD) if k == 1 else (k * num_tokens, 0)
+
+
 def split_plan(device: int, num_tokens: int, num_heads: int, blocks: int, uniform: int, layout: int, ext: int, aligned: int,
                impl: int) -> Tuple[int, int, int]:
     """(partitions, the scheduler's fixed overhead, equal partitions per request) of a decode step: the one choice that
     the ops make.  A third value above 1 means that requests of equal length are cut into that many equal partitions each
-    and the attention kernel derives the schedule itself (smla_decode_uniform).  ``ext``: MODEL1 or a second cache."""
+    and the attention kernel derives the schedule itself (smla_decode_uniform).  ``ext``: MODEL1 or a second cache;
+    ``aligned``: tc_aligned of the caches there, one_array of the cache otherwise."""
     if num_tokens == 0:
         return 0, FIXED_OVERHEAD, 0
     sms = num_sms(torch.device("cuda", device))
@@ -202,7 +235,10 @@ def split_plan(device: int, num_tokens: int, num_heads: int, blocks: int, unifor
         return pick_num_sm_parts_exact(num_tokens, num_heads, sms, blocks), FIXED_OVERHEAD, 0
     if ext and (impl == _lib.IMPL_SCALAR or not aligned):
         return pick_num_sm_parts_fp32(num_tokens, num_heads, sms), FIXED_OVERHEAD, 0
-    parts, overhead = pick_split(num_tokens, sms, blocks, uniform=bool(uniform))
+    if not ext and aligned and num_heads <= 64 and impl != _lib.IMPL_SCALAR:
+        parts, overhead = pick_split_tile(num_tokens, num_heads, sms, blocks, bool(uniform))
+    else:
+        parts, overhead = pick_split(num_tokens, sms, blocks, uniform=bool(uniform))
     k = parts // num_tokens
     equal = (uniform and not ext and impl != _lib.IMPL_SCALAR and overhead == 0 and k > 1 and k * num_tokens == parts
              and blocks % k == 0)

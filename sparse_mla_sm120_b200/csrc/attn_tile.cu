@@ -10,8 +10,8 @@
 // rows as the A operand of both (M = 128 whatever the number of heads, and V needs no second copy):
 //   * S^T [128 tokens x 64 heads] = K . Q^T, K-major.  The four fp32 scales of a row (powers of two, one per 128 dims) and
 //     the scale of a head's quantised q are applied by the tensor core: kind::mxf8f6f4 takes one power of two per row and 32
-//     values, and the scale bytes of a row's four blocks are the four bytes of one scale word.  RoPE goes into the same
-//     accumulator by bf16 MMAs, so that it holds q . k itself.
+//     values, and the scale bytes of a row's four blocks are the four bytes of one scale word.  RoPE follows as bf16 MMAs
+//     into the same accumulator, so the accumulator holds q . k itself.
 //   * O^T [4 x 128 dims x 64 heads] += V^T . P_b, the same tile read MN-major.  V's scale is a factor of the token inside a
 //     block of 128 dims, so it goes into the weights: block b uses P_b = P * 2^(e_b - e_max), rounded to e4m3, with
 //     e_max the largest of the row's four exponents.
@@ -21,15 +21,14 @@
 // z = logit * log2(e) + e_max and m its lazily updated running maximum per head; the denominator sums P' / 2^e_max in fp32.
 // Entries without a row (index < 0, position >= topk_length) have weight exactly 0.
 //
-// Warp roles (896 threads):
-//   warps 0-15   softmax, epilogue, Q: warp w holds tokens [32 (w % 4), +32) and heads [16 (w / 4), +16) of a tile, a thread
-//                one token; the four warps of a head group meet once per tile at a barrier that also ORs "a weight has
-//                outgrown the running maximum".  Groups without heads only quantise Q.
-//   warps 16-19  producers: warp 16 + i gathers the no-PE dims of rows [32 i, +32) of every tile, the four pieces of a quad of
-//                rows one after the other (piece by piece over all rows takes twice as long); a quarter of a stage is
-//                refilled as soon as P.V has read it.  Warps 26 and 27 gather the RoPE as soon as its one stage is free.
-//   warps 20-23  scales: the rows' scale words into tensor memory (each warp the 32 lanes it can reach) and shared memory.
-//   warp 24      issues the score MMAs, warp 25 the P.V MMAs (one elected lane each).
+// Warp roles (640 threads):
+//   warps 0-7    softmax, epilogue, Q: warp w holds tokens [32 (w % 4), +32) and heads [32 (w / 4), +32) of a tile, a thread
+//                one token; the four warps of a head half meet once per tile at a barrier that also ORs "a weight has outgrown
+//                the running maximum".  Warps 4-7 only quantise Q when there are 32 heads or fewer.
+//   warps 8-11   producers: warp 8 + i gathers rows [32 i, +32) of every tile; a quarter of a stage is refilled as soon as
+//                P.V has read it.
+//   warps 12-15  scales: the rows' scale words into tensor memory (each warp the 32 lanes it can reach) and shared memory.
+//   warp 16      issues the score MMAs, warp 17 the P.V MMAs (one elected lane each).
 // Every wait is bounded; a wait that gives up records a code in status[] and the CTA drains and exits.
 #include <cuda.h>
 
@@ -45,15 +44,14 @@ using namespace attn;
 
 constexpr int T_HEADS = 64;                    // heads per CTA
 constexpr int T_TILE = 128;                    // tokens per tile: two scheduler blocks
-constexpr int T_SM_WARPS = 16, T_PROD = 16, T_SCALE = 20, T_QK = 24, T_PV = 25, T_ROPE = 26;
-constexpr int T_THREADS = 28 * 32;
-constexpr int T_HPW = 16;                      // heads per softmax warp
-constexpr int T_REGS_LAUNCH = 72, T_REGS_SOFTMAX = 88, T_REGS_REST = 48;
+constexpr int T_SM_WARPS = 8, T_PROD = 8, T_SCALE = 12, T_QK = 16, T_PV = 17;
+constexpr int T_THREADS = 20 * 32;
+constexpr int T_REGS_LAUNCH = 96, T_REGS_SOFTMAX = 152, T_REGS_REST = 56;
 static_assert(T_SM_WARPS * 32 * T_REGS_SOFTMAX + (T_THREADS - T_SM_WARPS * 32) * T_REGS_REST <= T_THREADS * T_REGS_LAUNCH,
               "register budgets exceed what the CTA owns");
-constexpr int T_P_SHIFT = 7;                   // P' is stored as e4m3(P' * 2^T_P_SHIFT)
-constexpr float T_TAU = 1.0f;                  // lazy-rescale threshold (log2 units); P' <= 2^T_TAU
+constexpr int T_P_SHIFT = 5;                   // P' is stored as e4m3(P' * 2^T_P_SHIFT)
 constexpr float T_NO_MAX = 1e30f;              // minus the running maximum of a head that has seen no entry (finite: -inf minus it is -inf)
+constexpr float T_TAU = 3.0f;                  // lazy-rescale threshold (log2 units); P' <= 2^T_TAU
 constexpr int NSTAGE = 2;
 
 constexpr uint32_t K_CHUNK = T_TILE * 128;                 // 128 dims (or the RoPE) of all rows
@@ -69,7 +67,7 @@ constexpr int SW_RING = 4;
 constexpr uint32_t SW_OFF = P_OFF + 4 * P_BYTES;           // scale words of a tile's tokens (0: no entry), [SW_RING][128]
 constexpr uint32_t NM_OFF = SW_OFF + SW_RING * T_TILE * 4; // -m of the 64 heads
 constexpr uint32_t QW_OFF = NM_OFF + T_HEADS * 4;          // the heads' scale words
-constexpr uint32_t XX_OFF = QW_OFF + T_HEADS * 4;          // exchange between the four warps of a head group: [2][4][64] fp32
+constexpr uint32_t XX_OFF = QW_OFF + T_HEADS * 4;          // exchange between the four warps of a head half: [2][4][64] fp32
 constexpr uint32_t B_OFF = XX_OFF + 2 * 4 * T_HEADS * 4;
 constexpr int B_KFULL = 0, B_RFULL = B_KFULL + NSTAGE, B_KFREE = B_RFULL + 1, B_SREADY = B_KFREE + 4 * NSTAGE, B_SFREE = B_SREADY + 2,
               B_SCALES = B_SFREE + 2, B_PREADY = B_SCALES + SW_RING, B_PVDONE = B_PREADY + 1, B_QREADY = B_PVDONE + 1, B_N = B_QREADY + 1;
@@ -105,7 +103,7 @@ __device__ __forceinline__ float lanes_max(float v) {
 struct Tiles {
     Work w;
     int req, step, last, j, nst;
-    __device__ __forceinline__ Tiles(int first, int step_, int last_) : req(first - step_), step(step_), last(last_), j(0), nst(0) {}
+    __device__ __forceinline__ Tiles(const SchedMeta& m, int first, int step_, int last_) : req(first - step_), step(step_), last(last_), j(0), nst(0) {}
     __device__ __forceinline__ bool next_request(const AttnParams& p, const SchedMeta& m) {
         do {
             if (req + step > last) return false;
@@ -137,14 +135,14 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int part = blockIdx.x / halves, head0 = (blockIdx.x - part * halves) * T_HEADS;
     const int my_heads = min(p.num_heads - head0, T_HEADS);
-    const int act = 4 * ((my_heads + T_HPW - 1) / T_HPW);  // softmax warps with live heads
+    const int act = my_heads > 32 ? 8 : 4;                 // softmax warps with live heads
 
     if (tid == 0) {
         for (int s = 0; s < NSTAGE; ++s) {
             mbar_init(bar(B_KFULL + s), 4);                // + the bytes of the four producers
-            for (int i = 0; i < 4; ++i) mbar_init(bar(B_KFREE + 4 * s + i), 1);    // its rows [32 i, +32) have been read
+            for (int i = 0; i < 4; ++i) mbar_init(bar(B_KFREE + 4 * s + i), 1);
         }
-        mbar_init(bar(B_RFULL), 2);
+        mbar_init(bar(B_RFULL), 4);
         for (int b = 0; b < 2; ++b) { mbar_init(bar(B_SREADY + b), 1); mbar_init(bar(B_SFREE + b), act); }
         for (int i = 0; i < SW_RING; ++i) mbar_init(bar(B_SCALES + i), 4);
         mbar_init(bar(B_PREADY), act);
@@ -153,7 +151,7 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
         *abort_flag = 0;
         mbar_init_fence();
     }
-    if (act < T_SM_WARPS)                                  // the weights of heads that do not exist stay zero
+    if (act == 4)                                          // the weights of heads that do not exist stay zero
         for (int i = tid; i < (int)(4 * P_BYTES / 16); i += T_THREADS) reinterpret_cast<uint4*>(sm + P_OFF)[i] = make_uint4(0, 0, 0, 0);
     if (warp == T_QK) { tmem_alloc(base + MISC_OFF, 512); tmem_relinquish(); }
     fence_proxy_async();
@@ -179,10 +177,10 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
 
     if (warp < T_SM_WARPS) {
         // =================================================================== softmax + epilogue + Q
-        const int quarter = warp & 3, grp = warp >> 2, h0 = grp * T_HPW;
+        const int quarter = warp & 3, half = warp >> 2;
         const int token = quarter * 32 + lane;             // of the tile; in O^T: output dim inside a block of 128
-        const int hl = h0 + (lane & (T_HPW - 1));          // the head whose state this lane keeps (the same in four warps)
-        const bool live = hl < my_heads, active = h0 < my_heads;
+        const int hl = half * 32 + lane;                   // the head whose state this lane keeps (the same in four warps)
+        const bool live = hl < my_heads, active = half * 32 < my_heads;
         const uint32_t lane_addr = tmem + ((uint32_t)(quarter * 32) << 16);
         float* nm = reinterpret_cast<float*>(sm + NM_OFF);
         float* xx = reinterpret_cast<float*>(sm + XX_OFF);
@@ -190,7 +188,7 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
         // logits in log2 units are scores times a positive number: the sign of the softmax scale goes into q
         const float c = fabsf(p.sm_scale) * LOG2E;
         const uint32_t scale_sign = __float_as_uint(p.sm_scale) & 0x80000000u;
-        Tiles tiles(first, step, last);
+        Tiles tiles(meta, first, step, last);
         uint32_t it = 0;
         bool dead = false;
         bool prev = false, prev_no_split = false;          // a request's epilogue runs after the next request's Q phase
@@ -199,16 +197,17 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
         while (true) {
             const bool have = tiles.next_request(p, meta);
             // Every score of the request before has been read, by all warps, and so has its state: q, its scales and the maxima may
-            // be overwritten.  The sixteen warps leave the loop here together when one of them has given up.
-            if (named_bar_or(5, T_SM_WARPS * 32, dead || *abort_flag != 0)) break;
+            // be overwritten.  The eight warps leave the loop here together when one of them has given up.
+            if (named_bar_or(3, T_SM_WARPS * 32, dead || *abort_flag != 0)) break;
             if (have) {
-                // ---- Q: warp w quantises heads [4 w, +4), a lane 16 of the 512 no-PE dims of each
+                // ---- Q: warp w quantises heads [8 w, +8), a lane 16 of the 512 no-PE dims of each
                 const __nv_bfloat16* q0 = p.q + ((size_t)tiles.w.req * p.num_heads + head0) * D_QK;
-                {
+#pragma unroll
+                for (int u = 0; u < 8; u += 4) {
                     uint4 v[8];
 #pragma unroll
                     for (int k = 0; k < 4; ++k) {
-                        const int h = 4 * warp + k;
+                        const int h = 8 * warp + u + k;
                         v[2 * k] = v[2 * k + 1] = make_uint4(0, 0, 0, 0);
                         if (h < my_heads) {
                             v[2 * k] = __ldg(reinterpret_cast<const uint4*>(q0 + (size_t)h * D_QK + lane * 16));
@@ -217,7 +216,7 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
                     }
 #pragma unroll
                     for (int k = 0; k < 4; ++k) {
-                        const int h = 4 * warp + k;
+                        const int h = 8 * warp + u + k;
                         const uint32_t x[8] = {v[2 * k].x, v[2 * k].y, v[2 * k].z, v[2 * k].w, v[2 * k + 1].x, v[2 * k + 1].y, v[2 * k + 1].z, v[2 * k + 1].w};
                         uint32_t am = 0u;                  // magnitudes of bf16 numbers order as integers do
 #pragma unroll
@@ -233,8 +232,9 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
                         if (lane == 0) qw[h] = (__float_as_uint(sq) >> 23) * 0x01010101u;
                     }
                 }
-                {                                          // RoPE
-                    const int h = 4 * warp + (lane >> 3);
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {              // RoPE
+                    const int h = 8 * warp + 4 * u + (lane >> 3);
                     uint4 v = make_uint4(0, 0, 0, 0);
                     if (h < my_heads) v = __ldg(reinterpret_cast<const uint4*>(q0 + (size_t)h * D_QK + D_NOPE + (lane & 7) * 8));
                     const uint32_t flip = scale_sign | (scale_sign >> 16);
@@ -243,8 +243,8 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
                 }
                 fence_proxy_async();
                 if (warp < 2) nm[warp * 32 + lane] = T_NO_MAX;
-                named_bar_sync(5, T_SM_WARPS * 32);
-                if (grp == 0) {                            // the heads' scale words, in the lanes that this warp reaches
+                named_bar_sync(3, T_SM_WARPS * 32);
+                if (half == 0) {                           // the heads' scale words, in the lanes that this warp reaches
                     const uint32_t w2[2] = {qw[lane], qw[32 + lane]};
                     tmem_st2(lane_addr + TM_SFB, w2);
                     tmem_wait_st();
@@ -265,10 +265,10 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
                 tc_fence_after();
                 xx[quarter * T_HEADS + hl] = prev_l;
                 if (MAXL) xx[(4 + quarter) * T_HEADS + hl] = prev_x;
-                if (named_bar_or(1 + grp, 128, dead || *abort_flag != 0)) { dead = true; return; }
+                if (named_bar_or(1 + half, 128, dead || *abort_flag != 0)) { dead = true; return; }
                 const float l_all = (xx[hl] + xx[T_HEADS + hl]) + (xx[2 * T_HEADS + hl] + xx[3 * T_HEADS + hl]);
                 float x_all = -INFINITY;
-                if (MAXL) x_all = fmaxf(fmaxf(xx[4 * T_HEADS + hl], xx[5 * T_HEADS + hl]), fmaxf(xx[6 * T_HEADS + hl], xx[7 * T_HEADS + hl]));
+                if (MAXL) x_all = fmaxf(fmaxf(xx[256 + hl], xx[256 + T_HEADS + hl]), fmaxf(xx[256 + 2 * T_HEADS + hl], xx[256 + 3 * T_HEADS + hl]));
                 float lse = (l_all > 0.f) ? (log2f(l_all) - (float)T_P_SHIFT + prev_m) : NEG_BIG;
                 float denom = l_all;
                 if (prev_no_split && p.attn_sink != nullptr && live) {
@@ -278,47 +278,47 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
                     else lse = sink2;
                 }
                 const float inv = (denom > 0.f) ? 1.f / denom : 0.f;
-                const size_t row0 = (size_t)(prev_no_split ? prev_req : prev_split) * p.num_heads + head0 + h0;
-                const int n_live = min(my_heads - h0, T_HPW);
+                const size_t row0 = (size_t)(prev_no_split ? prev_req : prev_split) * p.num_heads + head0 + half * 32;
+                const int n_live = min(my_heads - half * 32, 32);
 #pragma unroll 1
                 for (int b = 0; b < 4; ++b) {
-                    uint32_t o[T_HPW];
-                    tmem_ld16(lane_addr + TM_O + 64 * b + h0, o);
+                    uint32_t o[32];
+                    tmem_ld32(lane_addr + TM_O + 64 * b + 32 * half, o);
                     tmem_wait_ld();
 #pragma unroll
-                    for (int i = 0; i < T_HPW; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * __shfl_sync(0xffffffffu, inv, i));
+                    for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * __shfl_sync(0xffffffffu, inv, i));
                     if (!prev_no_split && p.uniform_k <= 1) {      // fp32 records: a head's 32 dims of the warp are one store of 128 bytes
                         float* dst = p.o_accum + row0 * D_V + 128 * b + token;
 #pragma unroll
-                        for (int i = 0; i < T_HPW; ++i)
+                        for (int i = 0; i < 32; ++i)
                             if (i < n_live) dst[i * D_V] = __uint_as_float(o[i]);
                         continue;
                     }
                     // 16-bit results (bf16 outputs; fp16 records of equal partitions, the library's own scratch): neighbouring lanes
-                    // exchange halves, so that a lane has two dims of eight heads (even lanes heads 0-7, odd lanes 8-15)
+                    // exchange halves, so that a lane has two dims of 16 heads (even lanes heads 0-15, odd lanes 16-31)
                     const bool odd = (lane & 1) != 0;
-                    uint32_t pk[8];
+                    uint32_t pk[16];
 #pragma unroll
-                    for (int i = 0; i < 8; i += 2) {
+                    for (int i = 0; i < 16; i += 2) {
                         auto pack = [&](float a, float bb) -> uint32_t {
                             if (prev_no_split) { const __nv_bfloat162 t = __floats2bfloat162_rn(a, bb); return *reinterpret_cast<const uint32_t*>(&t); }
                             const __half2 t = __floats2half2_rn(a, bb);
                             return *reinterpret_cast<const uint32_t*>(&t);
                         };
-                        const uint32_t lo = pack(__uint_as_float(o[i]), __uint_as_float(o[i + 1])), hi = pack(__uint_as_float(o[8 + i]), __uint_as_float(o[9 + i]));
+                        const uint32_t lo = pack(__uint_as_float(o[i]), __uint_as_float(o[i + 1])), hi = pack(__uint_as_float(o[16 + i]), __uint_as_float(o[17 + i]));
                         const uint32_t got = __shfl_xor_sync(0xffffffffu, odd ? lo : hi, 1), own = odd ? hi : lo;
                         // own: this lane's dim of two heads; got: the neighbour's
                         pk[i] = __byte_perm(odd ? got : own, odd ? own : got, 0x5410);
                         pk[i + 1] = __byte_perm(odd ? got : own, odd ? own : got, 0x7632);
                     }
                     uint32_t* dst = reinterpret_cast<uint32_t*>(prev_no_split ? reinterpret_cast<void*>(p.out) : reinterpret_cast<void*>(p.o_accum)) +
-                                    (row0 + (odd ? 8 : 0)) * (D_V / 2) + 64 * b + (token >> 1);
-                    const int n = n_live - (odd ? 8 : 0);
+                                    (row0 + (odd ? 16 : 0)) * (D_V / 2) + 64 * b + (token >> 1);
+                    const int n = n_live - (odd ? 16 : 0);
 #pragma unroll
-                    for (int i = 0; i < 8; ++i)
+                    for (int i = 0; i < 16; ++i)
                         if (i < n) dst[i * (D_V / 2)] = pk[i];
                 }
-                if (live && quarter == 0 && lane < T_HPW) {
+                if (live && quarter == 0) {
                     if (prev_no_split) {
                         p.out_lse[row0 + lane] = lse;
                         if (MAXL) p.out_max_logits[row0 + lane] = (x_all == -INFINITY) ? NEG_BIG : x_all;
@@ -327,81 +327,57 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
                     }
                 }
                 tc_fence_before();                         // the accumulator's reads precede the next request's first P.V
-                named_bar_sync(1 + grp, 128);              // xx is free again
+                named_bar_sync(1 + half, 128);             // xx is free again
             };
             if (prev && active) epilogue();
             prev = false;
             if (!have) break;
             if (!active) continue;                         // no heads here
-            uint64_t l2[T_HPW / 2];                        // this token's share of the denominators of the warp's heads
-            float xm[MAXL ? T_HPW : 1];
+            uint64_t l2[16];                               // this token's share of the denominators of the warp's 32 heads
+            float xm[MAXL ? 32 : 1];
 #pragma unroll
-            for (int i = 0; i < T_HPW / 2; ++i) l2[i] = 0ull;
+            for (int i = 0; i < 16; ++i) l2[i] = 0ull;
 #pragma unroll
-            for (int i = 0; i < (MAXL ? T_HPW : 1); ++i) xm[i] = -INFINITY;
+            for (int i = 0; i < (MAXL ? 32 : 1); ++i) xm[i] = -INFINITY;
             for (int j = 0; j < tiles.nst; ++j, ++it) {
                 const uint32_t b = it & 1u;
-                uint32_t z[T_HPW];
-                uint32_t sw = 0u, em = 0u;
+                uint32_t z[32];
+                uint32_t sw = 0u;
                 bool grow = false;
                 float off = 0.f;                           // e_max + T_P_SHIFT: weights carry the shift
                 auto load_scores = [&]() {
-                    tmem_ld16(lane_addr + TM_S + 64 * b + h0, z);
+                    tmem_ld32(lane_addr + TM_S + 64 * b + 32 * half, z);
                     tmem_wait_ld();
                 };
-                // exponents: two per FMA, onto e_max + T_P_SHIFT - m
-                uint64_t e2[T_HPW / 2];
-                auto offsets = [&]() {
-                    const uint64_t off2 = pack_f32x2(off, off);
-#pragma unroll
-                    for (int i = 0; i < T_HPW; i += 4) {
-                        const ulonglong2 m4 = *reinterpret_cast<const ulonglong2*>(nm + h0 + i);
-                        e2[i / 2] = m4.x; e2[i / 2 + 1] = m4.y;
-                        add_f32x2(e2[i / 2], off2);
-                        add_f32x2(e2[i / 2 + 1], off2);
-                    }
-                };
+                // exponents: two per packed addition and FMA
                 auto exponents = [&]() {
-                    const uint64_t c2 = pack_f32x2(c, c);
+                    const uint64_t c2 = pack_f32x2(c, c), off2 = pack_f32x2(off, off);
+                    float mx = -INFINITY;
 #pragma unroll
-                    for (int i = 0; i < T_HPW; i += 2) {
-                        fma_f32x2(e2[i / 2], pack_f32x2(__uint_as_float(z[i]), __uint_as_float(z[i + 1])), c2);
-                        float a, d;
-                        unpack_f32x2(e2[i / 2], a, d);
-                        z[i] = __float_as_uint(a); z[i + 1] = __float_as_uint(d);
+                    for (int i = 0; i < 32; i += 4) {
+                        const ulonglong2 m4 = *reinterpret_cast<const ulonglong2*>(nm + half * 32 + i);
+                        uint64_t a = m4.x, d = m4.y;
+                        add_f32x2(a, off2);
+                        add_f32x2(d, off2);
+                        fma_f32x2(a, pack_f32x2(__uint_as_float(z[i]), __uint_as_float(z[i + 1])), c2);
+                        fma_f32x2(d, pack_f32x2(__uint_as_float(z[i + 2]), __uint_as_float(z[i + 3])), c2);
+                        float e0, e1, e2, e3;
+                        unpack_f32x2(a, e0, e1);
+                        unpack_f32x2(d, e2, e3);
+                        mx = fmaxf(mx, fmaxf(fmaxf(e0, e1), fmaxf(e2, e3)));
+                        z[i] = __float_as_uint(e0); z[i + 1] = __float_as_uint(e1); z[i + 2] = __float_as_uint(e2); z[i + 3] = __float_as_uint(e3);
                     }
                     if (!__all_sync(0xffffffffu, sw != 0u) && sw == 0u) {
 #pragma unroll
-                        for (int i = 0; i < T_HPW; ++i) z[i] = 0xff800000u;      // no entry: weight exactly 0
+                        for (int i = 0; i < 32; ++i) z[i] = 0xff800000u;      // no entry: weight exactly 0
                     }
-                };
-                // The weights of a block of dims are those of the row's largest scale times 2^(e_b - e_max).
-                auto packed = [&](float r) -> uint4 {
-                    uint32_t w[4];
-#pragma unroll
-                    for (int i = 0; i < 4; ++i)
-                        w[i] = pack_e4m3x4(__uint_as_float(z[4 * i]) * r, __uint_as_float(z[4 * i + 1]) * r, __uint_as_float(z[4 * i + 2]) * r,
-                                           __uint_as_float(z[4 * i + 3]) * r);
-                    return make_uint4(w[0], w[1], w[2], w[3]);
-                };
-                uint4 w0 = make_uint4(0u, 0u, 0u, 0u), w1 = w0;
-                uint32_t down = 0u;                        // e_max - e_b of the four blocks
-                bool near = true;
-                auto weights = [&]() {
-#pragma unroll
-                    for (int i = 0; i < T_HPW; ++i) z[i] = __float_as_uint(ex2(__uint_as_float(z[i])));
-                    w0 = packed(1.f);
-                    if (near) w1 = packed(0.5f);
+                    return mx;
                 };
                 if (!dead) dead = !mbar_wait_hot(bar(B_SCALES + (it & (SW_RING - 1))), (it / SW_RING) & 1u, abort_flag, WT_SCALES);
                 if (!dead) {
                     sw = *reinterpret_cast<const uint32_t*>(sm + SW_OFF + ((it & (SW_RING - 1)) * T_TILE + token) * 4);
                     const uint32_t em2 = __vmaxu4(sw, sw >> 16);
-                    em = max(em2 & 0xffu, (em2 >> 8) & 0xffu);
-                    off = (float)((int)em - 127 + T_P_SHIFT);
-                    down = __vsubus4(em * 0x01010101u, sw);
-                    near = __all_sync(0xffffffffu, (down & 0xfefefefeu) == 0u || sw == 0u);
-                    offsets();
+                    off = (float)((int)max(em2 & 0xffu, (em2 >> 8) & 0xffu) - 127 + T_P_SHIFT);
                     dead = !mbar_wait_hot(bar(B_SREADY + b), (it >> 1) & 1u, abort_flag, WT_SREADY);
                 }
                 if (!dead) {
@@ -409,32 +385,27 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
                     load_scores();
                     if (MAXL && sw != 0u) {
 #pragma unroll
-                        for (int i = 0; i < T_HPW; ++i) xm[i] = fmaxf(xm[i], __uint_as_float(z[i]));
+                        for (int i = 0; i < 32; ++i) xm[i] = fmaxf(xm[i], __uint_as_float(z[i]));
                     }
-                    exponents();
-                    float mx = __uint_as_float(z[0]);
-#pragma unroll
-                    for (int i = 1; i < T_HPW; ++i) mx = fmaxf(mx, __uint_as_float(z[i]));
-                    grow = mx > T_TAU + (float)T_P_SHIFT;
-                    weights();                             // before the barrier: they are rarely computed again
+                    grow = exponents() > T_TAU + (float)T_P_SHIFT && sw != 0u;
                 }
-                // Some weight of the group has outgrown the running maximum (or a wait gave up): rare after the first tiles of a
+                // Some weight of the 32 heads has outgrown the running maximum (or a wait gave up): rare after the first tiles of a
                 // request, so only then the maxima over the tokens are taken, exchanged and the accumulator rescaled.
-                if (named_bar_or(1 + grp, 128, grow || dead || *abort_flag != 0)) {
+                if (named_bar_or(1 + half, 128, grow || dead || *abort_flag != 0)) {
                     if (*abort_flag != 0) dead = true;
                     float mine = -INFINITY;
                     if (!dead) {
                         load_scores();
 #pragma unroll
-                        for (int i = 0; i < T_HPW; ++i) {
+                        for (int i = 0; i < 32; ++i) {
                             const float r = lanes_max(sw != 0u ? fmaf(__uint_as_float(z[i]), c, off - (float)T_P_SHIFT) : -INFINITY);
-                            if ((lane & (T_HPW - 1)) == i) mine = r;
+                            if (lane == i) mine = r;
                         }
                         xx[quarter * T_HEADS + hl] = mine;
                         if (j > 0) dead = !mbar_wait_hot(bar(B_PVDONE), (it - 1) & 1u, abort_flag, WT_PVDONE);
                     }
                     const float m_old = -nm[hl];
-                    if (named_bar_or(1 + grp, 128, dead || *abort_flag != 0)) { dead = true; break; }
+                    if (named_bar_or(1 + half, 128, dead || *abort_flag != 0)) { dead = true; break; }
                     const float mx = fmaxf(fmaxf(xx[hl], xx[T_HEADS + hl]), fmaxf(xx[2 * T_HEADS + hl], xx[3 * T_HEADS + hl]));
                     const bool up = mx > m_old;            // false while the head has seen no entry
                     const float alpha = up ? ex2(m_old - mx) : 1.f;       // 0 for the first entries
@@ -442,7 +413,7 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
                     tc_fence_after();
                     if (__any_sync(0xffffffffu, up)) {
 #pragma unroll
-                        for (int i = 0; i < T_HPW / 2; ++i) {
+                        for (int i = 0; i < 16; ++i) {
                             float a, d;
                             unpack_f32x2(l2[i], a, d);
                             l2[i] = pack_f32x2(a * __shfl_sync(0xffffffffu, alpha, 2 * i), d * __shfl_sync(0xffffffffu, alpha, 2 * i + 1));
@@ -450,45 +421,50 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
                         if (j > 0) {
 #pragma unroll 1
                             for (int bb = 0; bb < 4; ++bb) {
-                                uint32_t o[T_HPW];
-                                tmem_ld16(lane_addr + TM_O + 64 * bb + h0, o);
-                                tmem_wait_ld();
 #pragma unroll
-                                for (int i = 0; i < T_HPW; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * __shfl_sync(0xffffffffu, alpha, i));
-                                tmem_st16(lane_addr + TM_O + 64 * bb + h0, o);
+                                for (int hh = 0; hh < 2; ++hh) {
+                                    uint32_t o[16];
+                                    tmem_ld16(lane_addr + TM_O + 64 * bb + 32 * half + 16 * hh, o);
+                                    tmem_wait_ld();
+#pragma unroll
+                                    for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * __shfl_sync(0xffffffffu, alpha, 16 * hh + i));
+                                    tmem_st16(lane_addr + TM_O + 64 * bb + 32 * half + 16 * hh, o);
+                                }
                             }
                             tmem_wait_st();
                         }
                     }
-                    named_bar_sync(1 + grp, 128);          // xx is free again, the new maxima are in place
+                    named_bar_sync(1 + half, 128);         // xx is free again, the new maxima are in place
                     load_scores();
-                    offsets();
                     exponents();
-                    weights();
                 }
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(bar(B_SFREE + b));      // the score buffer may be overwritten
+                const uint32_t em2 = __vmaxu4(sw, sw >> 16);
+                const uint32_t em = max(em2 & 0xffu, (em2 >> 8) & 0xffu);
                 const float is = sw != 0u ? __uint_as_float((254u - em) << 23) : 0.f;      // 1 / 2^e_max
                 const uint64_t is2 = pack_f32x2(is, is);
 #pragma unroll
-                for (int i = 0; i < T_HPW; i += 2)
-                    fma_f32x2(l2[i / 2], pack_f32x2(__uint_as_float(z[i]), __uint_as_float(z[i + 1])), is2);
+                for (int i = 0; i < 32; i += 2) {
+                    const float p0 = ex2(__uint_as_float(z[i])), p1 = ex2(__uint_as_float(z[i + 1]));
+                    fma_f32x2(l2[i / 2], pack_f32x2(p0, p1), is2);
+                    z[i] = __float_as_uint(p0); z[i + 1] = __float_as_uint(p1);
+                }
                 if (it > 0 && !dead) dead = !mbar_wait_hot(bar(B_PVDONE), (it - 1) & 1u, abort_flag, WT_PVDONE);   // the weights of the last tile have been read
                 if (dead) continue;
-                uint8_t* pb = sm + P_OFF + swz64((uint32_t)token, (uint32_t)grp);
-                if (near) {                                // the blocks' scales of the rows differ by a factor of two at most: two versions serve
 #pragma unroll
-                    for (int bb = 0; bb < 4; ++bb) {
-                        const bool h = (down >> (8 * bb)) & 1u;
-                        *reinterpret_cast<uint4*>(pb + bb * P_BYTES) = make_uint4(h ? w1.x : w0.x, h ? w1.y : w0.y, h ? w1.z : w0.z, h ? w1.w : w0.w);
-                    }
-                } else {
+                for (int bb = 0; bb < 4; ++bb) {           // the weights of dims block bb
+                    const int d = max((int)((sw >> (8 * bb)) & 0xffu) - (int)em, -100);
+                    const float r = __uint_as_float((uint32_t)(127 + d) << 23);
+                    uint32_t w8[8];
 #pragma unroll
-                    for (int bb = 0; bb < 4; ++bb) {
-                        const uint32_t d = min((down >> (8 * bb)) & 0xffu, 100u);
-                        *reinterpret_cast<uint4*>(pb + bb * P_BYTES) = d == 0u ? w0 : packed(__uint_as_float((127u - d) << 23));
-                    }
+                    for (int i = 0; i < 8; ++i)
+                        w8[i] = pack_e4m3x4(__uint_as_float(z[4 * i]) * r, __uint_as_float(z[4 * i + 1]) * r, __uint_as_float(z[4 * i + 2]) * r,
+                                            __uint_as_float(z[4 * i + 3]) * r);
+                    uint8_t* pb = sm + P_OFF + bb * P_BYTES;
+                    *reinterpret_cast<uint4*>(pb + swz64((uint32_t)token, (uint32_t)(2 * half))) = make_uint4(w8[0], w8[1], w8[2], w8[3]);
+                    *reinterpret_cast<uint4*>(pb + swz64((uint32_t)token, (uint32_t)(2 * half + 1))) = make_uint4(w8[4], w8[5], w8[6], w8[7]);
                 }
                 fence_proxy_async();
                 tc_fence_before();
@@ -496,14 +472,12 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
                 if (lane == 0) mbar_arrive(bar(B_PREADY));
             }
             if (dead) continue;
-            // sums over the warp's tokens: halve the list at every exchange, lanes i and i + 16 end with head i
-            float s[T_HPW];
+            // sums over the warp's tokens: halve the list at every exchange, lane i ends with head i
+            float s[32];
 #pragma unroll
-            for (int i = 0; i < T_HPW / 2; ++i) unpack_f32x2(l2[i], s[2 * i], s[2 * i + 1]);
+            for (int i = 0; i < 16; ++i) unpack_f32x2(l2[i], s[2 * i], s[2 * i + 1]);
 #pragma unroll
-            for (int i = 0; i < T_HPW; ++i) s[i] += __shfl_xor_sync(0xffffffffu, s[i], 16);
-#pragma unroll
-            for (int o = T_HPW / 2; o >= 1; o >>= 1) {
+            for (int o = 16; o >= 1; o >>= 1) {
 #pragma unroll
                 for (int i = 0; i < o; ++i) {
                     const bool up = (lane & o) != 0;
@@ -514,29 +488,29 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
             prev_l = s[0];
             if (MAXL) {
 #pragma unroll
-                for (int i = 0; i < T_HPW; ++i) {
+                for (int i = 0; i < 32; ++i) {
                     const float r = lanes_max(xm[i]);
-                    if ((lane & (T_HPW - 1)) == i) prev_x = r * c;
+                    if (lane == i) prev_x = r * c;
                 }
             }
             prev_m = -nm[hl];
             prev = true; prev_no_split = tiles.w.no_split; prev_req = tiles.w.req; prev_split = tiles.w.split_idx;
         }
     } else if (warp < T_SCALE) {
-        // =================================================================== no-PE dims -> K stages (TMA gather)
+        // =================================================================== rows -> K stages (TMA gather)
         const int quarter = warp - T_PROD;
-        Tiles tiles(first, step, last);
+        Tiles tiles(meta, first, step, last);
         bool have = tiles.next_tile(p, meta), ok = true;
         int idx = have ? tiles.row_index(p, quarter * 32 + lane) : -1;
         for (uint32_t it = 0; have; ++it) {
             const uint32_t st = it % NSTAGE;
             const int row = idx >= 0 ? idx : NO_ROW;
             have = tiles.next_tile(p, meta);
-            const int idx_next = have ? tiles.row_index(p, quarter * 32 + lane) : -1;     // read ahead of its use
+            int idx_next = have ? tiles.row_index(p, quarter * 32 + lane) : -1;     // read ahead of its use
             if (it >= NSTAGE) ok = mbar_wait_hot(bar(B_KFREE + 4 * st + quarter), ((it / NSTAGE) - 1) & 1u, abort_flag, WT_KFREE);
             if (!ok) break;
-            const uint32_t dst = base + K_OFF + st * K_STAGE + quarter * (32 * 128), full = bar(B_KFULL + st);
-            if (elect_one()) mbar_arrive_expect_tx(full, 4 * 32 * 128);
+            const uint32_t dst = base + K_OFF + st * K_STAGE + quarter * (32 * 128);
+            if (elect_one()) mbar_arrive_expect_tx(bar(B_KFULL + st), 4 * 32 * 128);
             __syncwarp();
 #pragma unroll
             for (int q = 0; q < 8; ++q) {
@@ -544,8 +518,20 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
                 const int r2 = __shfl_sync(0xffffffffu, row, 4 * q + 2), r3 = __shfl_sync(0xffffffffu, row, 4 * q + 3);
                 if (elect_one()) {
 #pragma unroll
-                    for (int b = 0; b < 4; ++b) tma_gather4(dst + b * K_CHUNK + q * 512, &kv_map, 32 * b, r0, r1, r2, r3, full);
+                    for (int b = 0; b < 4; ++b) tma_gather4(dst + b * K_CHUNK + q * 512, &kv_map, 32 * b, r0, r1, r2, r3, bar(B_KFULL + st));
                 }
+                __syncwarp();
+            }
+            // the RoPE stage is free when the scores of the tile before are done
+            if (it >= 1) ok = mbar_wait_hot(bar(B_SREADY + ((it - 1) & 1u)), ((it - 1) >> 1) & 1u, abort_flag, WT_SREADY);
+            if (!ok) break;
+            if (elect_one()) mbar_arrive_expect_tx(bar(B_RFULL), 32 * 128);
+            __syncwarp();
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                const int r0 = __shfl_sync(0xffffffffu, row, 4 * q), r1 = __shfl_sync(0xffffffffu, row, 4 * q + 1);
+                const int r2 = __shfl_sync(0xffffffffu, row, 4 * q + 2), r3 = __shfl_sync(0xffffffffu, row, 4 * q + 3);
+                if (elect_one()) tma_gather4(base + R_OFF + quarter * (32 * 128) + q * 512, &kv_map, ROPE_OFF / 4, r0, r1, r2, r3, bar(B_RFULL));
                 __syncwarp();
             }
             idx = idx_next;
@@ -556,7 +542,7 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
         // all four lane quarters.
         const int quarter = warp - T_SCALE;
         const uint32_t lane_addr = tmem + ((uint32_t)(quarter * 32) << 16);
-        Tiles tiles(first, step, last);
+        Tiles tiles(meta, first, step, last);
         bool have = tiles.next_tile(p, meta), ok = true;
         int idx[4];
         uint4 sc[4];
@@ -568,18 +554,15 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
                 sc[k] = make_uint4(0u, 0u, 0u, 0u);
-                if (idx[k] >= 0) sc[k] = __ldg(reinterpret_cast<const uint4*>(p.kv + (size_t)idx[k] * ROW_BYTES + SCALE_OFF));
+                if (idx[k] >= 0) {
+                    sc[k] = __ldg(reinterpret_cast<const uint4*>(p.kv + (size_t)idx[k] * ROW_BYTES + SCALE_OFF));
+                    sc[k].x = max(sc[k].x, 0x00800000u); sc[k].y = max(sc[k].y, 0x00800000u);
+                    sc[k].z = max(sc[k].z, 0x00800000u); sc[k].w = max(sc[k].w, 0x00800000u);
+                }
             }
-        };
-        uint32_t some = 0u;                                // which of the four tokens of the loaded tile have an entry
-        auto mark = [&]() {
-            some = 0u;
-#pragma unroll
-            for (int k = 0; k < 4; ++k) some |= (idx[k] >= 0 ? 1u : 0u) << k;
         };
         fetch();
         load();
-        mark();
         bool cur = have;
         have = have && tiles.next_tile(p, meta);
         fetch();
@@ -587,12 +570,10 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
             uint32_t word[4], mx[4];
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
-                auto e = [](uint32_t s) { return max((s >> 23) & 0xffu, 1u); };
-                word[k] = ((some >> k) & 1u) ? e(sc[k].x) | (e(sc[k].y) << 8) | (e(sc[k].z) << 16) | (e(sc[k].w) << 24) : 0u;
+                word[k] = ((sc[k].x >> 23) & 0xffu) | (((sc[k].y >> 23) & 0xffu) << 8) | (((sc[k].z >> 23) & 0xffu) << 16) | (((sc[k].w >> 23) & 0xffu) << 24);
                 mx[k] = word[k] != 0u ? word[k] : 0x7f7f7f7fu;
             }
             load();                                        // of the next tile
-            mark();
             cur = have;
             have = have && tiles.next_tile(p, meta);
             fetch();
@@ -610,7 +591,7 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
     } else if (warp == T_QK) {
         // =================================================================== score MMAs
         const uint32_t q_lo = desc_lo(base + Q_OFF, 16), qr_lo = desc_lo(base + QR_OFF, 16), r_lo = desc_lo(base + R_OFF, 16);
-        Tiles tiles(first, step, last);
+        Tiles tiles(meta, first, step, last);
         uint32_t it = 0, rq = 0;
         bool ok = true;
         while (ok && tiles.next_request(p, meta)) {
@@ -620,27 +601,26 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
                 const uint32_t st = it % NSTAGE, b = it & 1u;
                 if (it >= 2) ok = mbar_wait_hot(bar(B_SFREE + b), ((it >> 1) - 1) & 1u, abort_flag, WT_SFREE);
                 if (ok) ok = mbar_wait_hot(bar(B_SCALES + (it & (SW_RING - 1))), (it / SW_RING) & 1u, abort_flag, WT_SCALES);
-                if (ok) ok = mbar_wait_hot(bar(B_RFULL), it & 1u, abort_flag, WT_RFULL);
+                if (ok) ok = mbar_wait_hot(bar(B_KFULL + st), (it / NSTAGE) & 1u, abort_flag, WT_KFULL);
                 if (!ok) break;
                 tc_fence_after();
                 const uint32_t k_lo = desc_lo(base + K_OFF + st * K_STAGE, 16), d = tmem + TM_S + 64 * b;
-                if (elect_one()) {
-#pragma unroll
-                    for (int k = 0; k < 4; ++k)
-                        mma_f16(d, make_desc(r_lo + ((k * 32) >> 4), HI_128), make_desc(qr_lo + ((k * 32) >> 4), HI_128), IDESC_ROPE, k != 0);
-                }
-                __syncwarp();
-                ok = mbar_wait_hot(bar(B_KFULL + st), (it / NSTAGE) & 1u, abort_flag, WT_KFULL);
-                if (!ok) break;
-                tc_fence_after();
                 if (elect_one()) {
 #pragma unroll
                     for (int bb = 0; bb < 4; ++bb) {
 #pragma unroll
                         for (int k = 0; k < 4; ++k)
                             mma_mxf8(d, make_desc(k_lo + ((bb * K_CHUNK + k * 32) >> 4), HI_128), make_desc(q_lo + ((bb * Q_CHUNK + k * 32) >> 4), HI_128),
-                                     idesc_mx(bb), tmem + TM_SFA + 4 * b, tmem + TM_SFB, true);
+                                     idesc_mx(bb), tmem + TM_SFA + 4 * b, tmem + TM_SFB, (bb | k) != 0);
                     }
+                }
+                __syncwarp();
+                ok = mbar_wait_hot(bar(B_RFULL), it & 1u, abort_flag, WT_RFULL);
+                if (!ok) break;
+                if (elect_one()) {
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)
+                        mma_f16(d, make_desc(r_lo + ((k * 32) >> 4), HI_128), make_desc(qr_lo + ((k * 32) >> 4), HI_128), IDESC_ROPE, true);
                     tc_commit(bar(B_SREADY + b));
                 }
                 __syncwarp();
@@ -648,7 +628,7 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
         }
     } else if (warp == T_PV) {
         // =================================================================== P.V MMAs
-        Tiles tiles(first, step, last);
+        Tiles tiles(meta, first, step, last);
         const uint32_t p_lo = desc_lo(base + P_OFF, 16);
         uint32_t it = 0;
         bool ok = true;
@@ -673,37 +653,6 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
                 __syncwarp();
             }
         }
-    } else {
-        // =================================================================== RoPE -> its stage (TMA gather)
-        const int half = warp - T_ROPE;                    // rows [64 half, +64), two per lane
-        Tiles tiles(first, step, last);
-        bool have = tiles.next_tile(p, meta), ok = true;
-        int idx[2] = {-1, -1};
-        auto fetch = [&]() {
-#pragma unroll
-            for (int k = 0; k < 2; ++k) idx[k] = have ? tiles.row_index(p, 64 * half + 32 * k + lane) : -1;
-        };
-        fetch();
-        for (uint32_t it = 0; have; ++it) {
-            const int row[2] = {idx[0] >= 0 ? idx[0] : NO_ROW, idx[1] >= 0 ? idx[1] : NO_ROW};
-            have = tiles.next_tile(p, meta);
-            fetch();
-            // the stage is free when the scores of the tile before are done
-            if (it >= 1) ok = mbar_wait_hot(bar(B_SREADY + ((it - 1) & 1u)), ((it - 1) >> 1) & 1u, abort_flag, WT_SREADY);
-            if (!ok) break;
-            if (elect_one()) mbar_arrive_expect_tx(bar(B_RFULL), 64 * 128);
-            __syncwarp();
-#pragma unroll
-            for (int k = 0; k < 2; ++k) {
-#pragma unroll
-                for (int q = 0; q < 8; ++q) {
-                    const int r0 = __shfl_sync(0xffffffffu, row[k], 4 * q), r1 = __shfl_sync(0xffffffffu, row[k], 4 * q + 1);
-                    const int r2 = __shfl_sync(0xffffffffu, row[k], 4 * q + 2), r3 = __shfl_sync(0xffffffffu, row[k], 4 * q + 3);
-                    if (elect_one()) tma_gather4(base + R_OFF + (64 * half + 32 * k) * 128 + q * 512, &kv_map, ROPE_OFF / 4, r0, r1, r2, r3, bar(B_RFULL));
-                    __syncwarp();
-                }
-            }
-        }
     }
 
     if (*abort_flag != 0) {        // a wait gave up: copies and MMAs may still be in flight; give them time to finish
@@ -725,9 +674,9 @@ typedef CUresult (*EncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void
 
 }  // namespace
 
-// One linear array of 656-byte rows: pages without padding between them.
+// One linear array of 656-byte rows (pages without padding between them) and one CTA's worth of heads.
 bool attn_tile_takes(const AttnParams& p) {
-    return p.layout == SMLA_LAYOUT_V32 && p.extra_topk == 0 && p.block_stride == (int64_t)p.page_block_size * ROW_BYTES &&
+    return p.num_heads <= T_HEADS && p.layout == SMLA_LAYOUT_V32 && p.extra_topk == 0 && p.block_stride == (int64_t)p.page_block_size * ROW_BYTES &&
            (reinterpret_cast<uintptr_t>(p.kv) & 15u) == 0;
 }
 

@@ -200,6 +200,8 @@ struct Attn {
         if (ext) {
             auto al = [](const at::Tensor& t, const Cache& g) { return reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0 && g.stride % 16 == 0; };
             aligned = al(kv, c) && (!extra_kv.defined() || al(extra_kv, ec));
+        } else {
+            aligned = c.stride == c.block * SMLA_ROW_BYTES && (reinterpret_cast<uintptr_t>(kv.data_ptr()) & 15u) == 0;
         }
     }
     at::Tensor output() const {

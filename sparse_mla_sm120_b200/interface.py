@@ -25,7 +25,7 @@ import torch
 
 from . import _lib
 from ._lib import IMPL_AUTO, IMPL_SCALAR, LAYOUT_V32, check
-from ._runtime import (BLOCK_N, kv_geometry, ptr, require_cuda, resolve_impl, split_plan, status_buffer, stream_ptr,
+from ._runtime import (BLOCK_N, kv_geometry, one_array, ptr, require_cuda, resolve_impl, split_plan, status_buffer, stream_ptr,
                        tc_aligned)
 from .flash_ops import _check_q, _Extra, _layout, sparse_mla_prefill_fwd
 
@@ -128,7 +128,7 @@ def flash_mla_with_kvcache(
     if not meta.have_initialized:
         meta.have_initialized = True
         meta.config = cfg
-        aligned = not use_ext or tc_aligned(k_cache, ex.kv)
+        aligned = tc_aligned(k_cache, ex.kv) if use_ext else one_array(k_cache)
         meta.num_sm_parts, fixed_overhead, meta.uniform_k = split_plan(
             q.device.index, num_tokens, num_heads, blocks, topk_length is None and ex.topk == 0, layout, use_ext, aligned, impl)
         meta.max_nsplits = min(blocks, meta.num_sm_parts)
