@@ -160,8 +160,8 @@ int smla_prefill(const void* q, const void* kv, const int32_t* indices,
  * extra_topk 0 = no second cache; the scheduler must have been given the same extra_topk and
  * extra_topk_length.  impl as above, with two differences.  SMLA_IMPL_TC refuses caches whose base address or
  * page stride is not a multiple of 16 bytes (what the kernel's bulk copies need) with SMLA_E_ALIGN; SMLA_IMPL_AUTO
- * runs the fp32 kernel for them.  And SMLA_IMPL_AUTO runs the fp32 kernel for SMLA_LAYOUT_MODEL1: V includes the
- * row's RoPE there, which the tcgen05 kernel rounds to e4m3 with the rest of V (the reference multiplies it in
+ * runs the fp32 kernel for them.  And SMLA_IMPL_AUTO is exact (bf16 operands, fp32 sums) for SMLA_LAYOUT_MODEL1: V includes the
+ * row's RoPE there, which the FP8 kernel rounds to e4m3 with the rest of V (the reference multiplies it in
  * bf16, csrc/kernel/common/xv_rope_mma.cuh:23-93), so results of rows with few entries differ from the
  * reference's by up to about 2e-3 on its own test data; callers that accept this ask for SMLA_IMPL_TC.
  */

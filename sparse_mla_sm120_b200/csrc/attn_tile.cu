@@ -1,8 +1,16 @@
-// Sparse-MLA attention over packed 656-byte rows, one CTA per 64 query heads (sm_100a): split-KV decode and prefill.
+// Sparse-MLA attention of up to 64 query heads over packed 656-byte rows (sm_100a): split-KV decode and prefill, one CTA per
+// partition (a run of 64-token blocks of consecutive requests, see sched.cu; without a scheduler every parts-th request).
 //
-// Work unit: one partition (a run of 64-token blocks of consecutive requests, see sched.cu; without a scheduler every
-// parts-th request) for 64 query heads; up to 128 heads are two CTAs next to each other in the grid, which read the same
-// rows at about the same time (the second read comes from L2).
+// Why not the pair kernel: it spends two CTAs on a partition whatever the number of heads, copies every row through registers
+// and splits the work over half as many partitions.  48 requests of top-k 2048 at 16 heads: 45.1 us there, 32.8 us here; 1237
+// ragged prompt tokens of top-k 1024 at 64 heads: 371 us there, 176 us here.  At 128 heads two of these CTAs would gather every
+// row twice: 2400 us against 2238 us for 4096 tokens of top-k 2048, so the pair kernel keeps those.
+//
+// What bounds it (clock64 at 64 heads, 1.9 GHz): a tile of 128 tokens takes 4300 cycles, half of the way of a tile from the load
+// of its rows (2000 cycles: the gather delivers 35 bytes per cycle and SM) over its scores (2100, with the hand-overs) and its
+// weights (2700) to P.V (1300), because two tiles are all that shared memory holds.  A request costs another 16000 cycles for its
+// q and its epilogue, which the softmax warps do in between.  Tried without gain: sixteen softmax warps (2485 us where
+// eight take 2400), weights before the group's barrier (2483), a tighter rescale threshold (3350, more rescales).
 //
 // The gathered rows are never touched by a thread.  TMA gather4 loads bring the 512 e4m3 values of a row, as four
 // pieces of 128 dims, and its 64 RoPE values straight into the 128B-swizzled tiles that the MMAs read; a row without an
@@ -125,7 +133,7 @@ struct Tiles {
 };
 
 template <bool MAXL>
-__global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParams p, const int halves, const __grid_constant__ CUtensorMap kv_map) {
+__global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParams p, const __grid_constant__ CUtensorMap kv_map) {
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;
@@ -133,8 +141,7 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
     volatile int* abort_flag = reinterpret_cast<volatile int*>(sm + MISC_OFF + 4);
     auto bar = [&](int i) -> uint32_t { return base + B_OFF + 8u * i; };
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int part = blockIdx.x / halves, head0 = (blockIdx.x - part * halves) * T_HEADS;
-    const int my_heads = min(p.num_heads - head0, T_HEADS);
+    const int part = blockIdx.x, my_heads = p.num_heads;   // at most T_HEADS
     const int act = my_heads > 32 ? 8 : 4;                 // softmax warps with live heads
 
     if (tid == 0) {
@@ -169,7 +176,7 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
     } else {                                               // whole requests; neighbours differ little in length, so every CTA takes each parts-th
         meta.begin_block = 0; meta.end_block = 0x7fffffff;
         meta.begin_split = 0; meta.first_split = meta.last_split = 0; meta.pad = 0;
-        first = part; step = (int)gridDim.x / halves; last = p.num_tokens - 1;
+        first = part; step = (int)gridDim.x; last = p.num_tokens - 1;
         meta.begin_req = 0; meta.end_req = last;
     }
     if (warp < T_SM_WARPS) setmaxnreg_inc<T_REGS_SOFTMAX>();
@@ -201,7 +208,7 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
             if (named_bar_or(3, T_SM_WARPS * 32, dead || *abort_flag != 0)) break;
             if (have) {
                 // ---- Q: warp w quantises heads [8 w, +8), a lane 16 of the 512 no-PE dims of each
-                const __nv_bfloat16* q0 = p.q + ((size_t)tiles.w.req * p.num_heads + head0) * D_QK;
+                const __nv_bfloat16* q0 = p.q + ((size_t)tiles.w.req * my_heads) * D_QK;
 #pragma unroll
                 for (int u = 0; u < 8; u += 4) {
                     uint4 v[8];
@@ -254,7 +261,7 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
                 if (lane == 0) mbar_arrive(bar(B_QREADY));
                 // ask L2 for the next request's q, a whole request of tiles ahead of its use
                 if (tiles.req + tiles.step <= tiles.last) {
-                    const uint8_t* qn = reinterpret_cast<const uint8_t*>(p.q + ((size_t)(tiles.req + tiles.step) * p.num_heads + head0) * D_QK);
+                    const uint8_t* qn = reinterpret_cast<const uint8_t*>(p.q + ((size_t)(tiles.req + tiles.step) * my_heads) * D_QK);
                     for (int i = tid; i < (my_heads * D_QK * 2 + 127) >> 7; i += T_SM_WARPS * 32)
                         asm volatile("prefetch.global.L2 [%0];" ::"l"(qn + (size_t)i * 128));
                 }
@@ -272,13 +279,13 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
                 float lse = (l_all > 0.f) ? (log2f(l_all) - (float)T_P_SHIFT + prev_m) : NEG_BIG;
                 float denom = l_all;
                 if (prev_no_split && p.attn_sink != nullptr && live) {
-                    const float sink2 = p.attn_sink[head0 + hl] * LOG2E;
+                    const float sink2 = p.attn_sink[hl] * LOG2E;
                     denom = l_all + ((prev_m == -T_NO_MAX) ? INFINITY : exp2f(sink2 - prev_m + (float)T_P_SHIFT));
                     if (lse != NEG_BIG) lse += log2f(1.f + exp2f(sink2 - lse));
                     else lse = sink2;
                 }
                 const float inv = (denom > 0.f) ? 1.f / denom : 0.f;
-                const size_t row0 = (size_t)(prev_no_split ? prev_req : prev_split) * p.num_heads + head0 + half * 32;
+                const size_t row0 = (size_t)(prev_no_split ? prev_req : prev_split) * my_heads + half * 32;
                 const int n_live = min(my_heads - half * 32, 32);
 #pragma unroll 1
                 for (int b = 0; b < 4; ++b) {
@@ -712,13 +719,11 @@ int launch_attn_tile(const AttnParams& p, cudaStream_t stream) {
     const CUresult r = encode(&map, CU_TENSOR_MAP_DATA_TYPE_INT32, 2, const_cast<uint8_t*>(p.kv), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return set_error(SMLA_E_DEVICE, "attn_tile_kernel: cuTensorMapEncodeTiled failed (%d)", (int)r);
-    const int halves = (p.num_heads + T_HEADS - 1) / T_HEADS;
-    const int most = sm_count[dev] / halves > 0 ? sm_count[dev] / halves : 1;
-    const int parts = p.sched ? p.num_parts : p.uniform_k > 1 ? p.uniform_k * p.num_tokens : (p.num_tokens < most ? p.num_tokens : most);
-    const dim3 grid(parts * halves);
+    const int parts = p.sched ? p.num_parts : p.uniform_k > 1 ? p.uniform_k * p.num_tokens : (p.num_tokens < sm_count[dev] ? p.num_tokens : sm_count[dev]);
+    const dim3 grid(parts);
     auto* kernel = p.out_max_logits != nullptr ? attn_tile_kernel<true> : attn_tile_kernel<false>;
-    if (p.sched != nullptr) launch_dependent(kernel, grid, dim3(T_THREADS), T_SMEM, stream, p, halves, map);
-    else kernel<<<grid, T_THREADS, T_SMEM, stream>>>(p, halves, map);
+    if (p.sched != nullptr) launch_dependent(kernel, grid, dim3(T_THREADS), T_SMEM, stream, p, map);
+    else kernel<<<grid, T_THREADS, T_SMEM, stream>>>(p, map);
     return check_launch("attn_tile_kernel");
 }
 
