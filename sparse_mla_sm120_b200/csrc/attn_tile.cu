@@ -3,14 +3,16 @@
 //
 // Why not the pair kernel: it spends two CTAs on a partition whatever the number of heads, copies every row through registers
 // and splits the work over half as many partitions.  48 requests of top-k 2048 at 16 heads: 45.1 us there, 32.8 us here; 1237
-// ragged prompt tokens of top-k 1024 at 64 heads: 371 us there, 176 us here.  At 128 heads two of these CTAs would gather every
+// ragged prompt tokens of top-k 1024 at 64 heads: 371 us there, 172 us here.  At 128 heads two of these CTAs would gather every
 // row twice: 2400 us against 2238 us for 4096 tokens of top-k 2048, so the pair kernel keeps those.
 //
 // What bounds it (clock64 at 64 heads, 1.9 GHz): a tile of 128 tokens takes 4300 cycles, half of the way of a tile from the load
 // of its rows (2000 cycles: the gather delivers 35 bytes per cycle and SM) over its scores (2100, with the hand-overs) and its
-// weights (2700) to P.V (1300), because two tiles are all that shared memory holds.  A request costs another 16000 cycles for its
+// weights (2700) to P.V (1300), because two tiles are all that shared memory holds.  A request costs another 15000 cycles for its
 // q and its epilogue, which the softmax warps do in between.  Tried without gain: sixteen softmax warps (2485 us where
-// eight take 2400), weights before the group's barrier (2483), a tighter rescale threshold (3350, more rescales).
+// eight take 2400), q and epilogue on four warps of their own (169 us for the
+// ragged prompt, but 36.8 us for the 48 requests: every role's code grows, and code beyond the instruction caches slows all of
+// them; fully unrolled gathers and MMAs 188 us), weights before the group's barrier (2483), a tighter rescale threshold (3350, more rescales).
 //
 // The gathered rows are never touched by a thread.  TMA gather4 loads bring the 512 e4m3 values of a row, as four
 // pieces of 128 dims, and its 64 RoPE values straight into the 128B-swizzled tiles that the MMAs read; a row without an
@@ -284,16 +286,28 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
                     if (lse != NEG_BIG) lse += log2f(1.f + exp2f(sink2 - lse));
                     else lse = sink2;
                 }
-                const float inv = (denom > 0.f) ? 1.f / denom : 0.f;
+                named_bar_sync(1 + half, 128);             // the sums have been read: 1 / denominator takes the place of a quarter's
+                float* iv = xx + quarter * T_HEADS + half * 32;
+                iv[lane] = (denom > 0.f) ? 1.f / denom : 0.f;
+                __syncwarp();
                 const size_t row0 = (size_t)(prev_no_split ? prev_req : prev_split) * my_heads + half * 32;
                 const int n_live = min(my_heads - half * 32, 32);
+                const bool odd = (lane & 1) != 0;
+                const uint32_t sel0 = odd ? 0x1054u : 0x5410u, sel1 = odd ? 0x3276u : 0x7632u;
+                // 1 / denominator by broadcast reads instead of a shuffle per head, one conversion per type: 178 -> 172 us at 64 heads
 #pragma unroll 1
                 for (int b = 0; b < 4; ++b) {
                     uint32_t o[32];
                     tmem_ld32(lane_addr + TM_O + 64 * b + 32 * half, o);
                     tmem_wait_ld();
 #pragma unroll
-                    for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * __shfl_sync(0xffffffffu, inv, i));
+                    for (int i = 0; i < 32; i += 4) {
+                        const float4 f = *reinterpret_cast<const float4*>(iv + i);
+                        o[i] = __float_as_uint(__uint_as_float(o[i]) * f.x);
+                        o[i + 1] = __float_as_uint(__uint_as_float(o[i + 1]) * f.y);
+                        o[i + 2] = __float_as_uint(__uint_as_float(o[i + 2]) * f.z);
+                        o[i + 3] = __float_as_uint(__uint_as_float(o[i + 3]) * f.w);
+                    }
                     if (!prev_no_split && p.uniform_k <= 1) {      // fp32 records: a head's 32 dims of the warp are one store of 128 bytes
                         float* dst = p.o_accum + row0 * D_V + 128 * b + token;
 #pragma unroll
@@ -303,27 +317,28 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
                     }
                     // 16-bit results (bf16 outputs; fp16 records of equal partitions, the library's own scratch): neighbouring lanes
                     // exchange halves, so that a lane has two dims of 16 heads (even lanes heads 0-15, odd lanes 16-31)
-                    const bool odd = (lane & 1) != 0;
-                    uint32_t pk[16];
-#pragma unroll
-                    for (int i = 0; i < 16; i += 2) {
-                        auto pack = [&](float a, float bb) -> uint32_t {
-                            if (prev_no_split) { const __nv_bfloat162 t = __floats2bfloat162_rn(a, bb); return *reinterpret_cast<const uint32_t*>(&t); }
-                            const __half2 t = __floats2half2_rn(a, bb);
-                            return *reinterpret_cast<const uint32_t*>(&t);
-                        };
-                        const uint32_t lo = pack(__uint_as_float(o[i]), __uint_as_float(o[i + 1])), hi = pack(__uint_as_float(o[16 + i]), __uint_as_float(o[17 + i]));
-                        const uint32_t got = __shfl_xor_sync(0xffffffffu, odd ? lo : hi, 1), own = odd ? hi : lo;
-                        // own: this lane's dim of two heads; got: the neighbour's
-                        pk[i] = __byte_perm(odd ? got : own, odd ? own : got, 0x5410);
-                        pk[i + 1] = __byte_perm(odd ? got : own, odd ? own : got, 0x7632);
-                    }
+                    const int n = n_live - (odd ? 16 : 0);
                     uint32_t* dst = reinterpret_cast<uint32_t*>(prev_no_split ? reinterpret_cast<void*>(p.out) : reinterpret_cast<void*>(p.o_accum)) +
                                     (row0 + (odd ? 16 : 0)) * (D_V / 2) + 64 * b + (token >> 1);
-                    const int n = n_live - (odd ? 16 : 0);
+                    if (prev_no_split) {
 #pragma unroll
-                    for (int i = 0; i < 16; ++i)
-                        if (i < n) dst[i * (D_V / 2)] = pk[i];
+                        for (int i = 0; i < 16; ++i) {
+                            const __nv_bfloat162 t = __floats2bfloat162_rn(__uint_as_float(o[2 * i]), __uint_as_float(o[2 * i + 1]));
+                            o[i] = *reinterpret_cast<const uint32_t*>(&t);
+                        }
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) {
+                            const __half2 t = __floats2half2_rn(__uint_as_float(o[2 * i]), __uint_as_float(o[2 * i + 1]));
+                            o[i] = *reinterpret_cast<const uint32_t*>(&t);
+                        }
+                    }
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {          // own: this lane's dim of two heads; got: the neighbour's
+                        const uint32_t got = __shfl_xor_sync(0xffffffffu, odd ? o[i] : o[8 + i], 1), own = odd ? o[8 + i] : o[i];
+                        if (2 * i < n) dst[2 * i * (D_V / 2)] = __byte_perm(own, got, sel0);
+                        if (2 * i + 1 < n) dst[(2 * i + 1) * (D_V / 2)] = __byte_perm(own, got, sel1);
+                    }
                 }
                 if (live && quarter == 0) {
                     if (prev_no_split) {
