@@ -3,7 +3,7 @@
 //
 // Why not the pair kernel: it spends two CTAs on a partition whatever the number of heads, copies every row through registers
 // and splits the work over half as many partitions.  48 requests of top-k 2048 at 16 heads: 45.1 us there, 32.8 us here; 1237
-// ragged prompt tokens of top-k 1024 at 64 heads: 371 us there, 172 us here.  At 128 heads two of these CTAs would gather every
+// ragged prompt tokens of top-k 1024 at 64 heads: 395 us there, 176 us here.  At 128 heads two of these CTAs would gather every
 // row twice: 2400 us against 2238 us for 4096 tokens of top-k 2048, so the pair kernel keeps those.
 //
 // What bounds it (clock64 at 64 heads, 1.9 GHz): a tile of 128 tokens takes 4300 cycles, half of the way of a tile from the load
@@ -23,12 +23,17 @@
 //     values, and the scale bytes of a row's four blocks are the four bytes of one scale word.  RoPE follows as bf16 MMAs
 //     into the same accumulator, so the accumulator holds q . k itself.
 //   * O^T [4 x 128 dims x 64 heads] += V^T . P_b, the same tile read MN-major.  V's scale is a factor of the token inside a
-//     block of 128 dims, so it goes into the weights: block b uses P_b = P * 2^(e_b - e_max), rounded to e4m3, with
-//     e_max the largest of the row's four exponents.
+//     block of 128 dims, so it goes into the weights: block b uses P_b = P' * 2^(e_b - e_g + k_b), rounded to e4m3, with
+//     e_g the largest exponent of the token's group of eight (the group of the pair kernel, so that P' is its P') and k_b,
+//     the same for all tokens of a request, as large as it can be without lifting any P_b over P'.  A block whose scales
+//     are small throughout so has weights as precise as the largest block's: without k_b, scales 2^-9 below the row's
+//     largest leave weights in e4m3's subnormals (error of that block 12 % at logits of +-6 instead of 0.6 %).  k_b only
+//     ever falls; the block's part of the accumulator is then multiplied by the power of two (exactly), and the epilogue
+//     takes 2^k_b out again.  Price: 172 -> 176 us for 1237 ragged prompt tokens, nothing at longer lists.
 // Numerics (the FP8 class of the reference's V32 kernels, which quantise Q and P to e4m3:
 // csrc/kernel/common/fp8_quant.cuh:44-103, csrc/kernel/decode/decode_v2_kernel.cuh:414-493): q no-PE e4m3 with one power of
 // two per head, q RoPE bf16 as given, K and V bytes as stored, P' = 2^(z - m) in e4m3 (times 2^T_P_SHIFT) with
-// z = logit * log2(e) + e_max and m its lazily updated running maximum per head; the denominator sums P' / 2^e_max in fp32.
+// z = logit * log2(e) + e_g and m its lazily updated running maximum per head; the denominator sums P' / 2^e_g in fp32.
 // Entries without a row (index < 0, position >= topk_length) have weight exactly 0.
 //
 // Warp roles (640 threads):
@@ -74,11 +79,12 @@ constexpr uint32_t QR_OFF = Q_OFF + 4 * Q_CHUNK;           // q RoPE bf16
 constexpr uint32_t P_OFF = QR_OFF + Q_CHUNK;               // P_b: [128 tokens x 64 heads] e4m3, 64B swizzle
 constexpr uint32_t P_BYTES = T_TILE * T_HEADS;
 constexpr int SW_RING = 4;
-constexpr uint32_t SW_OFF = P_OFF + 4 * P_BYTES;           // scale words of a tile's tokens (0: no entry), [SW_RING][128]
-constexpr uint32_t NM_OFF = SW_OFF + SW_RING * T_TILE * 4; // -m of the 64 heads
+constexpr uint32_t SW_OFF = P_OFF + 4 * P_BYTES;           // TokenScale of a tile's tokens, [SW_RING][128]
+constexpr uint32_t NM_OFF = SW_OFF + SW_RING * T_TILE * 8; // -m of the 64 heads
 constexpr uint32_t QW_OFF = NM_OFF + T_HEADS * 4;          // the heads' scale words
 constexpr uint32_t XX_OFF = QW_OFF + T_HEADS * 4;          // exchange between the four warps of a head half: [2][4][64] fp32
-constexpr uint32_t B_OFF = XX_OFF + 2 * 4 * T_HEADS * 4;
+constexpr uint32_t KX_OFF = XX_OFF + 2 * 4 * T_HEADS * 4;  // the same for the blocks' shifts: [2 halves][4]
+constexpr uint32_t B_OFF = KX_OFF + 2 * 4 * 4;
 constexpr int B_KFULL = 0, B_RFULL = B_KFULL + NSTAGE, B_KFREE = B_RFULL + 1, B_SREADY = B_KFREE + 4 * NSTAGE, B_SFREE = B_SREADY + 2,
               B_SCALES = B_SFREE + 2, B_PREADY = B_SCALES + SW_RING, B_PVDONE = B_PREADY + 1, B_QREADY = B_PVDONE + 1, B_N = B_QREADY + 1;
 constexpr uint32_t MISC_OFF = B_OFF + B_N * 8;
@@ -108,6 +114,11 @@ __device__ __forceinline__ float lanes_max(float v) {
     asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
     return r;
 }
+
+// What the softmax needs of a token's scales: by how many powers of two each of its four blocks lies below e_g, the largest
+// exponent of the group of eight tokens (a byte per block, at most NO_SHIFT), and e_g itself (biased; 0: no entry).
+struct TokenScale { uint32_t below, e_g; };
+constexpr uint32_t NO_SHIFT = 0x7fu;
 
 // The requests of a CTA and their tiles, in the order in which every role walks them.
 struct Tiles {
@@ -193,6 +204,7 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
         const uint32_t lane_addr = tmem + ((uint32_t)(quarter * 32) << 16);
         float* nm = reinterpret_cast<float*>(sm + NM_OFF);
         float* xx = reinterpret_cast<float*>(sm + XX_OFF);
+        uint32_t* kx = reinterpret_cast<uint32_t*>(sm + KX_OFF);
         uint32_t* qw = reinterpret_cast<uint32_t*>(sm + QW_OFF);
         // logits in log2 units are scores times a positive number: the sign of the softmax scale goes into q
         const float c = fabsf(p.sm_scale) * LOG2E;
@@ -203,6 +215,7 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
         bool prev = false, prev_no_split = false;          // a request's epilogue runs after the next request's Q phase
         int prev_req = 0, prev_split = 0;
         float prev_m = 0.f, prev_l = 0.f, prev_x = 0.f;
+        uint32_t prev_shift = 0u;
         while (true) {
             const bool have = tiles.next_request(p, meta);
             // Every score of the request before has been read, by all warps, and so has its state: q, its scales and the maxima may
@@ -294,19 +307,20 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
                 const int n_live = min(my_heads - half * 32, 32);
                 const bool odd = (lane & 1) != 0;
                 const uint32_t sel0 = odd ? 0x1054u : 0x5410u, sel1 = odd ? 0x3276u : 0x7632u;
-                // 1 / denominator by broadcast reads instead of a shuffle per head, one conversion per type: 178 -> 172 us at 64 heads
+                // 1 / denominator by broadcast reads instead of a shuffle per head, one conversion per type: 6 us of 178 at 64 heads
 #pragma unroll 1
                 for (int b = 0; b < 4; ++b) {
                     uint32_t o[32];
                     tmem_ld32(lane_addr + TM_O + 64 * b + 32 * half, o);
+                    const float unshift = __uint_as_float((127u - ((prev_shift >> (8 * b)) & 0xffu)) << 23);
                     tmem_wait_ld();
 #pragma unroll
                     for (int i = 0; i < 32; i += 4) {
                         const float4 f = *reinterpret_cast<const float4*>(iv + i);
-                        o[i] = __float_as_uint(__uint_as_float(o[i]) * f.x);
-                        o[i + 1] = __float_as_uint(__uint_as_float(o[i + 1]) * f.y);
-                        o[i + 2] = __float_as_uint(__uint_as_float(o[i + 2]) * f.z);
-                        o[i + 3] = __float_as_uint(__uint_as_float(o[i + 3]) * f.w);
+                        o[i] = __float_as_uint(__uint_as_float(o[i]) * unshift * f.x);
+                        o[i + 1] = __float_as_uint(__uint_as_float(o[i + 1]) * unshift * f.y);
+                        o[i + 2] = __float_as_uint(__uint_as_float(o[i + 2]) * unshift * f.z);
+                        o[i + 3] = __float_as_uint(__uint_as_float(o[i + 3]) * unshift * f.w);
                     }
                     if (!prev_no_split && p.uniform_k <= 1) {      // fp32 records: a head's 32 dims of the warp are one store of 128 bytes
                         float* dst = p.o_accum + row0 * D_V + 128 * b + token;
@@ -361,12 +375,13 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
             for (int i = 0; i < 16; ++i) l2[i] = 0ull;
 #pragma unroll
             for (int i = 0; i < (MAXL ? 32 : 1); ++i) xm[i] = -INFINITY;
+            uint32_t shift = NO_SHIFT * 0x01010101u;       // of the four blocks; the same in all warps of the half
             for (int j = 0; j < tiles.nst; ++j, ++it) {
                 const uint32_t b = it & 1u;
                 uint32_t z[32];
-                uint32_t sw = 0u;
+                TokenScale ts{NO_SHIFT * 0x01010101u, 0u};
                 bool grow = false;
-                float off = 0.f;                           // e_max + T_P_SHIFT: weights carry the shift
+                float off = 0.f;                           // log2 of the group's scale + T_P_SHIFT: weights carry the shift
                 auto load_scores = [&]() {
                     tmem_ld32(lane_addr + TM_S + 64 * b + 32 * half, z);
                     tmem_wait_ld();
@@ -389,7 +404,7 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
                         mx = fmaxf(mx, fmaxf(fmaxf(e0, e1), fmaxf(e2, e3)));
                         z[i] = __float_as_uint(e0); z[i + 1] = __float_as_uint(e1); z[i + 2] = __float_as_uint(e2); z[i + 3] = __float_as_uint(e3);
                     }
-                    if (!__all_sync(0xffffffffu, sw != 0u) && sw == 0u) {
+                    if (!__all_sync(0xffffffffu, ts.e_g != 0u) && ts.e_g == 0u) {
 #pragma unroll
                         for (int i = 0; i < 32; ++i) z[i] = 0xff800000u;      // no entry: weight exactly 0
                     }
@@ -397,22 +412,24 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
                 };
                 if (!dead) dead = !mbar_wait_hot(bar(B_SCALES + (it & (SW_RING - 1))), (it / SW_RING) & 1u, abort_flag, WT_SCALES);
                 if (!dead) {
-                    sw = *reinterpret_cast<const uint32_t*>(sm + SW_OFF + ((it & (SW_RING - 1)) * T_TILE + token) * 4);
-                    const uint32_t em2 = __vmaxu4(sw, sw >> 16);
-                    off = (float)((int)max(em2 & 0xffu, (em2 >> 8) & 0xffu) - 127 + T_P_SHIFT);
+                    const uint2 t2 = *reinterpret_cast<const uint2*>(sm + SW_OFF + ((it & (SW_RING - 1)) * T_TILE + token) * 8);
+                    ts.below = t2.x; ts.e_g = t2.y;
+                    off = (float)((int)ts.e_g - 127 + T_P_SHIFT);
                     dead = !mbar_wait_hot(bar(B_SREADY + b), (it >> 1) & 1u, abort_flag, WT_SREADY);
                 }
                 if (!dead) {
                     tc_fence_after();
                     load_scores();
-                    if (MAXL && sw != 0u) {
+                    if (MAXL && ts.e_g != 0u) {
 #pragma unroll
                         for (int i = 0; i < 32; ++i) xm[i] = fmaxf(xm[i], __uint_as_float(z[i]));
                     }
-                    grow = exponents() > T_TAU + (float)T_P_SHIFT && sw != 0u;
+                    grow = exponents() > T_TAU + (float)T_P_SHIFT && ts.e_g != 0u;
+                    grow |= (((ts.below | 0x80808080u) - shift) & 0x80808080u) != 0x80808080u;     // some byte is smaller
                 }
-                // Some weight of the 32 heads has outgrown the running maximum (or a wait gave up): rare after the first tiles of a
-                // request, so only then the maxima over the tokens are taken, exchanged and the accumulator rescaled.
+                // Some weight of the 32 heads has outgrown the running maximum, or a block's scale the shift of its weights (or a
+                // wait gave up): rare after the first tiles of a request, so only then the maxima over the tokens and the shifts
+                // are taken, exchanged and the accumulator rescaled.
                 if (named_bar_or(1 + half, 128, grow || dead || *abort_flag != 0)) {
                     if (*abort_flag != 0) dead = true;
                     float mine = -INFINITY;
@@ -420,20 +437,28 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
                         load_scores();
 #pragma unroll
                         for (int i = 0; i < 32; ++i) {
-                            const float r = lanes_max(sw != 0u ? fmaf(__uint_as_float(z[i]), c, off - (float)T_P_SHIFT) : -INFINITY);
+                            const float r = lanes_max(ts.e_g != 0u ? fmaf(__uint_as_float(z[i]), c, off - (float)T_P_SHIFT) : -INFINITY);
                             if (lane == i) mine = r;
                         }
                         xx[quarter * T_HEADS + hl] = mine;
+                        uint32_t low = ts.below;
+#pragma unroll
+                        for (int o = 16; o >= 1; o >>= 1) low = __vminu4(low, __shfl_xor_sync(0xffffffffu, low, o));
+                        kx[half * 4 + quarter] = low;
                         if (j > 0) dead = !mbar_wait_hot(bar(B_PVDONE), (it - 1) & 1u, abort_flag, WT_PVDONE);
                     }
                     const float m_old = -nm[hl];
                     if (named_bar_or(1 + half, 128, dead || *abort_flag != 0)) { dead = true; break; }
                     const float mx = fmaxf(fmaxf(xx[hl], xx[T_HEADS + hl]), fmaxf(xx[2 * T_HEADS + hl], xx[3 * T_HEADS + hl]));
-                    const bool up = mx > m_old;            // false while the head has seen no entry
+                    const bool up = mx > m_old + T_TAU;    // false while the head has seen no entry
                     const float alpha = up ? ex2(m_old - mx) : 1.f;       // 0 for the first entries
                     if (up) nm[hl] = -mx;                  // the four warps of the head write the same value
+                    const uint32_t* kh = kx + half * 4;
+                    const uint32_t low = __vminu4(shift, __vminu4(__vminu4(kh[0], kh[1]), __vminu4(kh[2], kh[3])));
+                    const uint32_t drop = shift - low;     // (no borrows)
+                    shift = low;
                     tc_fence_after();
-                    if (__any_sync(0xffffffffu, up)) {
+                    if (__any_sync(0xffffffffu, up) || drop != 0u) {
 #pragma unroll
                         for (int i = 0; i < 16; ++i) {
                             float a, d;
@@ -443,13 +468,14 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
                         if (j > 0) {
 #pragma unroll 1
                             for (int bb = 0; bb < 4; ++bb) {
+                                const float alpha_b = alpha * __uint_as_float((127u - ((drop >> (8 * bb)) & 0xffu)) << 23);
 #pragma unroll
                                 for (int hh = 0; hh < 2; ++hh) {
                                     uint32_t o[16];
                                     tmem_ld16(lane_addr + TM_O + 64 * bb + 32 * half + 16 * hh, o);
                                     tmem_wait_ld();
 #pragma unroll
-                                    for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * __shfl_sync(0xffffffffu, alpha, 16 * hh + i));
+                                    for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * __shfl_sync(0xffffffffu, alpha_b, 16 * hh + i));
                                     tmem_st16(lane_addr + TM_O + 64 * bb + 32 * half + 16 * hh, o);
                                 }
                             }
@@ -463,9 +489,7 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(bar(B_SFREE + b));      // the score buffer may be overwritten
-                const uint32_t em2 = __vmaxu4(sw, sw >> 16);
-                const uint32_t em = max(em2 & 0xffu, (em2 >> 8) & 0xffu);
-                const float is = sw != 0u ? __uint_as_float((254u - em) << 23) : 0.f;      // 1 / 2^e_max
+                const float is = ts.e_g != 0u ? __uint_as_float((254u - ts.e_g) << 23) : 0.f;      // 1 / the group's scale
                 const uint64_t is2 = pack_f32x2(is, is);
 #pragma unroll
                 for (int i = 0; i < 32; i += 2) {
@@ -475,10 +499,10 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
                 }
                 if (it > 0 && !dead) dead = !mbar_wait_hot(bar(B_PVDONE), (it - 1) & 1u, abort_flag, WT_PVDONE);   // the weights of the last tile have been read
                 if (dead) continue;
+                const uint32_t under = ts.below - shift;   // (no borrows: the shifts are the smallest so far)
 #pragma unroll
                 for (int bb = 0; bb < 4; ++bb) {           // the weights of dims block bb
-                    const int d = max((int)((sw >> (8 * bb)) & 0xffu) - (int)em, -100);
-                    const float r = __uint_as_float((uint32_t)(127 + d) << 23);
+                    const float r = __uint_as_float((127u - ((under >> (8 * bb)) & 0xffu)) << 23);
                     uint32_t w8[8];
 #pragma unroll
                     for (int i = 0; i < 8; ++i)
@@ -516,6 +540,7 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
                 }
             }
             prev_m = -nm[hl];
+            prev_shift = shift;
             prev = true; prev_no_split = tiles.w.no_split; prev_req = tiles.w.req; prev_split = tiles.w.split_idx;
         }
     } else if (warp < T_SCALE) {
@@ -595,6 +620,12 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
                 word[k] = ((sc[k].x >> 23) & 0xffu) | (((sc[k].y >> 23) & 0xffu) << 8) | (((sc[k].z >> 23) & 0xffu) << 16) | (((sc[k].w >> 23) & 0xffu) << 24);
                 mx[k] = word[k] != 0u ? word[k] : 0x7f7f7f7fu;
             }
+            const uint32_t mine = quarter == 0 ? word[0] : quarter == 1 ? word[1] : quarter == 2 ? word[2] : word[3];
+            const uint32_t em2 = __vmaxu4(mine, mine >> 16);
+            uint32_t e_g = max(em2 & 0xffu, (em2 >> 8) & 0xffu);
+#pragma unroll
+            for (int o = 4; o >= 1; o >>= 1) e_g = max(e_g, __shfl_xor_sync(0xffffffffu, e_g, o));
+            const uint2 ts = mine != 0u ? make_uint2(__vminu4(e_g * 0x01010101u - mine, NO_SHIFT * 0x01010101u), e_g) : make_uint2(NO_SHIFT * 0x01010101u, 0u);
             load();                                        // of the next tile
             cur = have;
             have = have && tiles.next_tile(p, meta);
@@ -603,8 +634,7 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
             if (!ok) break;
             tc_fence_after();
             tmem_st4(lane_addr + TM_SFA + 4 * (it & 1u), mx);
-            const uint32_t mine = quarter == 0 ? word[0] : quarter == 1 ? word[1] : quarter == 2 ? word[2] : word[3];
-            *reinterpret_cast<uint32_t*>(sm + SW_OFF + ((it & (SW_RING - 1)) * T_TILE + quarter * 32 + lane) * 4) = mine;
+            *reinterpret_cast<uint2*>(sm + SW_OFF + ((it & (SW_RING - 1)) * T_TILE + quarter * 32 + lane) * 8) = ts;
             tmem_wait_st();
             tc_fence_before();
             __syncwarp();
