@@ -75,6 +75,11 @@ __device__ __forceinline__ int fetch_entry(const AttnParams& p, const Work& w, i
     return pos < w.extra_len ? __ldg(p.extra_indices + (size_t)w.req * p.extra_topk + pos) : -1;
 }
 
+// Smallest scale of a row, as a biased exponent: smaller ones (a zero-filled row has scales of 0) are taken for it.  The
+// denominator divides weights of up to 2^8 by the scale, and 2^95 times any number of rows is finite; what such a row
+// itself holds stays far below anything that matters (448 * 2^-87), and its weight is that of its logit.
+constexpr uint32_t MIN_SCALE_BITS = 40u << 23;
+
 __device__ __forceinline__ float pow2_ceil(float x) {
     uint32_t b = __float_as_uint(x);
     if (b & 0x007fffffu) b = (b + 0x00800000u) & 0x7f800000u;

@@ -843,15 +843,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) att
                 for (int u = 0; u < RPW / 4; ++u) am = fmaxf(am, absmax8(rp[u]));
                 const uint32_t ab = __float_as_uint(am * (1.f / 448.f));
                 e = max(e, (ab >> 23) + ((ab & 0x007fffffu) ? 1u : 0u));
-                if (vbits != 0u) e = max(e, 1u);
                 wm = __uint_as_float(min(e, 254u) << 23);
             }
             // scales are not negative, so their bits order as integers do: one reduction instead of five exchanges
-            const float s_half = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(wm)));
+            const float s_half = __uint_as_float(max(__reduce_max_sync(0xffffffffu, __float_as_uint(wm)), MIN_SCALE_BITS));
             // the maximum needed the last shared-memory load of every lane (they return in order): the rows have left the slot
             if (lane == 0) mbar_arrive(bar(BAR_RAWEMPTY + slot));
             TRACE(62, t_it);
-            const float inv_half = (s_half > 0.f) ? __uint_as_float(0x7f000000u - __float_as_uint(s_half)) : 0.f;
+            const float inv_half = __uint_as_float(0x7f000000u - __float_as_uint(s_half));
             const __nv_bfloat162 rope_f = __float2bfloat162_rn(inv_half);
             // V32: exponent shift of the block whose scale this lane loaded (row lane / 4, block lane % 4): 0 for a block at the scale.
             // MODEL1: lanes 0-7 pass on exponents 0-3 of row lane, lanes 8-15 exponents 4-6 of row lane - 8.
@@ -899,8 +898,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) att
             if (lane == 0) {      // the record of the group: read by this CTA's softmax warps and sent to the partner's
                 uint8_t* rec = sm + INFO_OFF + (t_it & (INFO_RING - 1)) * (2 * INFO_HALF) + rank * INFO_HALF + gw * 16;
                 *reinterpret_cast<float4*>(rec) =
-                    make_float4(s_half, (s_half > 0.f) ? (float)((int)(__float_as_uint(s_half) >> 23) - 127) : -INFINITY, inv_half,
-                                __uint_as_float(vbits));
+                    make_float4(s_half, (float)((int)(__float_as_uint(s_half) >> 23) - 127), inv_half, __uint_as_float(vbits));
             }
             TRACE(64, t_it);
             fence_proxy_async();

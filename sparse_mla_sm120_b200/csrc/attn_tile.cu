@@ -603,8 +603,8 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
                 sc[k] = make_uint4(0u, 0u, 0u, 0u);
                 if (idx[k] >= 0) {
                     sc[k] = __ldg(reinterpret_cast<const uint4*>(p.kv + (size_t)idx[k] * ROW_BYTES + SCALE_OFF));
-                    sc[k].x = max(sc[k].x, 0x00800000u); sc[k].y = max(sc[k].y, 0x00800000u);
-                    sc[k].z = max(sc[k].z, 0x00800000u); sc[k].w = max(sc[k].w, 0x00800000u);
+                    sc[k].x = max(sc[k].x, MIN_SCALE_BITS); sc[k].y = max(sc[k].y, MIN_SCALE_BITS);
+                    sc[k].z = max(sc[k].z, MIN_SCALE_BITS); sc[k].w = max(sc[k].w, MIN_SCALE_BITS);
                 }
             }
         };
