@@ -526,7 +526,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) att
                 for (int i = tid; i < lines; i += N_SM_WARPS * 32)
                     asm volatile("prefetch.global.L2 [%0];" ::"l"(qn + (size_t)i * 128));
             }
-            my_sqc = live ? sqv[hrow] * fabsf(p.sm_scale) * LOG2E : 1.f;
+            // Never 0, also times the smallest scale of a group (2^-87): the scores of entries without a row are -inf, and -inf
+            // times a softmax scale of 0 would be no number.  2^-62 times any score is far below one step of an exponent.
+            my_sqc = live ? fmaxf(sqv[hrow] * fabsf(p.sm_scale) * LOG2E, 0x1p-62f) : 1.f;
             __syncwarp();
             if (lane == 0) mbar_arrive_remote(barp(BAR_QREADYP));
 

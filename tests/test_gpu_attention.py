@@ -365,3 +365,17 @@ def test_uniform_split_derived_in_the_kernel(tokens, heads, topk, k):
                                    stream_ptr(dev)) == -2
     assert lib.smla_decode_uniform(ptr(q), ptr(kv), ptr(idx), ptr(o_accum), ptr(lse_accum), ptr(out), ptr(lse), tokens, heads,
                                    topk, ctypes.c_float(1.0), pbs, pstride, k, None, SCALAR, None, stream_ptr(dev)) == -2
+
+
+@pytest.mark.parametrize("impl", [SCALAR, TC])
+@pytest.mark.parametrize("heads", [16, 128])
+@pytest.mark.parametrize("scale", [0.0, -0.0, 1e-40])
+def test_softmax_scale_of_zero(heads, impl, scale):
+    """The plain mean of the rows that exist, with entries without a row among them."""
+    case = make_case(29, 3, heads, 320, 8, invalid_tail=0.1)
+    case["indices"][:, 2::7] = -1
+    case["indices"][1] = -1
+    case["sm_scale"] = scale
+    ref_out, ref_lse = oracle_attn(case)
+    for out, lse in (_decode(case, impl), _decode(case, impl, num_sm_parts=4), _prefill(case, impl)[::2]):
+        _check(out, lse, ref_out, ref_lse, impl)
