@@ -249,35 +249,30 @@ _SCRATCH_LIMIT = 64      # cached call shapes per process before the least recen
 
 
 def scratch(device: torch.device, total_splits: int, num_heads: int, num_tokens: int, num_parts: int):
-    """Cached scratch for one decode call shape on the current stream (the reference allocates
+    """Cached scratch for one call shape on the current stream (the reference allocates
     these on every call, flash_mla_sm120/ops.py:78-99).
 
     The key includes the stream: two calls of the same shape on different streams get different
-    buffers, so they cannot race on ``o_accum``.  An entry that is handed out while its stream is
-    being captured into a CUDA graph is pinned: the graph keeps raw pointers into it, so it is
-    never evicted.  Past _SCRATCH_LIMIT entries the least recently used unpinned one is dropped
+    buffers, so they cannot race on ``o_accum``.  A capture gets buffers of its own, from the graph's
+    memory, that never enter the cache: the graph may replay on any stream, beside eager calls on the
+    stream that it was captured on.  Past _SCRATCH_LIMIT entries the least recently used one is dropped
     (it was allocated on, and only ever used on, its own stream, so the caching allocator may
     reuse it in stream order)."""
-    stream = torch.cuda.current_stream(device)
-    key = (device.index, stream.cuda_stream, total_splits, num_heads, num_tokens, num_parts)
-    ws = _scratch.pop(key, None)
-    if ws is None:
-        ws = {
+    def fresh():
+        return {
             "o_accum": torch.empty((total_splits, 1, num_heads, 512), dtype=torch.float32, device=device),
             "lse_accum": torch.empty((total_splits, 1, num_heads), dtype=torch.float32, device=device),
             "sched_meta": torch.empty(num_parts * 8, dtype=torch.int32, device=device),
             "num_splits": torch.empty(num_tokens + 1, dtype=torch.int32, device=device),
-            "pinned": False,
         }
     if torch.cuda.is_current_stream_capturing():
-        ws["pinned"] = True
-    _scratch[key] = ws                      # most recently used last
+        return fresh()
+    key = (device.index, torch.cuda.current_stream(device).cuda_stream, total_splits, num_heads, num_tokens, num_parts)
+    ws = _scratch.pop(key, None)
+    _scratch[key] = fresh() if ws is None else ws                      # most recently used last
     if len(_scratch) > _SCRATCH_LIMIT:
-        for old in list(_scratch):
-            if not _scratch[old]["pinned"] and old != key:
-                del _scratch[old]
-                break
-    return ws
+        del _scratch[next(iter(_scratch))]
+    return _scratch[key]
 
 
 _status: Dict[int, torch.Tensor] = {}

@@ -3,8 +3,8 @@
 //
 // Why: a decode step of one request takes the GPU about 24 us, and the same host work in Python took 27 (argument
 // handling, the split policy's loop, dictionary look-ups, a 21-argument foreign call); here it is a few.
-// Kept between calls: the answers of the split policy (integers per call shape), the address of the device status words,
-// the library's entry points, and scratch for partial outputs (see Scratch).  Everything runs under the interpreter lock.
+// Kept between calls: the answers of the split policy (integers per call shape), the address of the device status words and
+// the library's entry points.  Everything runs under the interpreter lock.
 #include <Python.h>
 #include <ATen/ATen.h>
 #include <ATen/cuda/CUDAContext.h>
@@ -244,38 +244,6 @@ Plan plan_for(const Attn& a, int blocks, bool uniform) {
     return p;
 }
 
-// Scratch of a decode call, kept per (device, stream, size): calls of one stream run one after the other, calls of
-// different streams never share.  A buffer that is handed out while its stream is being captured stays for good, since the
-// graph holds its address; of the others the least recently used goes when there are more than 64 (it was only ever used on
-// its own stream, so the allocator may reuse it in stream order).  A capture that finds none takes one from the graph's own
-// pool instead of the cache.
-at::Tensor scratch(const at::Tensor& like, int64_t bytes, void* stream) {
-    struct Buffer { at::Tensor t; bool pinned; uint64_t used; };
-    using Key = std::tuple<int, void*, int64_t>;
-    static std::map<Key, Buffer> pool;
-    static uint64_t clock = 0;
-    constexpr size_t LIMIT = 64;
-    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-    cudaStreamIsCapturing(static_cast<cudaStream_t>(stream), &st);
-    const bool capturing = st != cudaStreamCaptureStatusNone;
-    const Key key{(int)like.get_device(), stream, bytes};
-    auto it = pool.find(key);
-    if (it == pool.end()) {
-        at::Tensor t = at::empty({bytes}, like.options().dtype(at::kByte));
-        if (capturing) return t;
-        it = pool.emplace(key, Buffer{t, false, 0}).first;
-        if (pool.size() > LIMIT) {
-            auto old = pool.end();
-            for (auto b = pool.begin(); b != pool.end(); ++b)
-                if (b != it && !b->second.pinned && (old == pool.end() || b->second.used < old->second.used)) old = b;
-            if (old != pool.end()) pool.erase(old);
-        }
-    }
-    it->second.used = ++clock;
-    it->second.pinned |= capturing;
-    return it->second.t;
-}
-
 PyObject* wrap2(const at::Tensor& a, const at::Tensor& b) {
     PyObject* r = PyTuple_New(2);
     PyTuple_SET_ITEM(r, 0, THPVariable_Wrap(a));
@@ -304,7 +272,10 @@ PyObject* decode(const Args& x) {
     // equal partitions write fp16 records, one each; the scheduler's write fp32 ones at the positions it gives
     const int64_t row = (int64_t)a.heads * (p.uniform > 1 ? p.parts : (int64_t)a.tokens + p.parts);
     const int64_t o_bytes = row * SMLA_D_V * (p.uniform > 1 ? 2 : 4), l_bytes = (row * 4 + 255) & ~255ll, m_bytes = ((int64_t)p.parts * SMLA_SCHED_META_INTS * 4 + 255) & ~255ll;
-    const at::Tensor ws = scratch(a.q, o_bytes + l_bytes + m_bytes + ((int64_t)a.tokens + 1) * 4, stream);
+    // Scratch of this call alone, from the allocator: of the current stream's memory, of the graph's own while a capture runs.
+    // (Kept between calls it would be shared by a graph, which may replay on any stream, and whoever else used the stream that
+    // it was captured on.)
+    const at::Tensor ws = at::empty({o_bytes + l_bytes + m_bytes + ((int64_t)a.tokens + 1) * 4}, a.q.options().dtype(at::kByte));
     char* w = static_cast<char*>(ws.data_ptr());
     float* o_accum = reinterpret_cast<float*>(w);
     float* lse_accum = reinterpret_cast<float*>(w + o_bytes);

@@ -73,7 +73,7 @@ class GraphedIndexedDecode:
         side = torch.cuda.Stream(device=dev)
         side.wait_stream(torch.cuda.current_stream(dev))
         with torch.cuda.stream(side):
-            step()                                   # warm-up: library load, scratch buffers, kernel attributes
+            step()                                   # warm-up: library load, kernel attributes
             self.graph = torch.cuda.CUDAGraph()
             with torch.cuda.graph(self.graph, stream=side):
                 self.out, self.lse, self.rows = step()
