@@ -3,7 +3,7 @@
 //
 // Why not the pair kernel: it spends two CTAs on a partition whatever the number of heads, copies every row through registers
 // and splits the work over half as many partitions.  48 requests of top-k 2048 at 16 heads: 45.1 us there, 32.8 us here; 1237
-// ragged prompt tokens of top-k 1024 at 64 heads: 395 us there, 176 us here.  At 128 heads two of these CTAs would gather every
+// ragged prompt tokens of top-k 1024 at 64 heads: 395 us there, 175 us here.  At 128 heads two of these CTAs would gather every
 // row twice: 2400 us against 2238 us for 4096 tokens of top-k 2048, so the pair kernel keeps those.
 //
 // What bounds it (clock64 at 64 heads, 1.9 GHz): a tile of 128 tokens takes 4300 cycles, half of the way of a tile from the load
@@ -29,7 +29,7 @@
 //     are small throughout so has weights as precise as the largest block's: without k_b, scales 2^-9 below the row's
 //     largest leave weights in e4m3's subnormals (error of that block 12 % at logits of +-6 instead of 0.6 %).  k_b only
 //     ever falls; the block's part of the accumulator is then multiplied by the power of two (exactly), and the epilogue
-//     takes 2^k_b out again.  Price: 172 -> 176 us for 1237 ragged prompt tokens, nothing at longer lists.
+//     takes 2^k_b out again.  Price: 172 -> 174.6 us for 1237 ragged prompt tokens, 2 % and less elsewhere.
 // Numerics (the FP8 class of the reference's V32 kernels, which quantise Q and P to e4m3:
 // csrc/kernel/common/fp8_quant.cuh:44-103, csrc/kernel/decode/decode_v2_kernel.cuh:414-493): q no-PE e4m3 with one power of
 // two per head, q RoPE bf16 as given, K and V bytes as stored, P' = 2^(z - m) in e4m3 (times 2^T_P_SHIFT) with
@@ -587,6 +587,7 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
         // =================================================================== scale words
         // Lane i reads the scales of tokens i, 32 + i, 64 + i, 96 + i: row r's word belongs into column r / 32 of lane r % 32, in
         // all four lane quarters.
+        // The next tile's scales are asked for when this tile's words have been handed over, and looked at a tile later.
         const int quarter = warp - T_SCALE;
         const uint32_t lane_addr = tmem + ((uint32_t)(quarter * 32) << 16);
         Tiles tiles(meta, first, step, last);
@@ -597,14 +598,15 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
 #pragma unroll
             for (int k = 0; k < 4; ++k) idx[k] = have ? tiles.row_index(p, 32 * k + lane) : -1;
         };
-        auto load = [&]() {                                // (exponent 0 marks a token without an entry)
+        uint32_t there = 0u;                               // bit k: token 32 k + lane has an entry
+        auto load = [&]() {
+            there = 0u;
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
                 sc[k] = make_uint4(0u, 0u, 0u, 0u);
                 if (idx[k] >= 0) {
                     sc[k] = __ldg(reinterpret_cast<const uint4*>(p.kv + (size_t)idx[k] * ROW_BYTES + SCALE_OFF));
-                    sc[k].x = max(sc[k].x, MIN_SCALE_BITS); sc[k].y = max(sc[k].y, MIN_SCALE_BITS);
-                    sc[k].z = max(sc[k].z, MIN_SCALE_BITS); sc[k].w = max(sc[k].w, MIN_SCALE_BITS);
+                    there |= 1u << k;
                 }
             }
         };
@@ -617,19 +619,20 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
             uint32_t word[4], mx[4];
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
-                word[k] = ((sc[k].x >> 23) & 0xffu) | (((sc[k].y >> 23) & 0xffu) << 8) | (((sc[k].z >> 23) & 0xffu) << 16) | (((sc[k].w >> 23) & 0xffu) << 24);
+                auto bits = [](uint32_t v) { return max(v, MIN_SCALE_BITS) << 1; };         // the exponent is the upper byte
+                const uint32_t lo = __byte_perm(bits(sc[k].x), bits(sc[k].y), 0x0073), hi = __byte_perm(bits(sc[k].z), bits(sc[k].w), 0x0073);
+                word[k] = ((there >> k) & 1u) != 0u ? __byte_perm(lo, hi, 0x5410) : 0u;
                 mx[k] = word[k] != 0u ? word[k] : 0x7f7f7f7fu;
             }
             const uint32_t mine = quarter == 0 ? word[0] : quarter == 1 ? word[1] : quarter == 2 ? word[2] : word[3];
-            const uint32_t em2 = __vmaxu4(mine, mine >> 16);
-            uint32_t e_g = max(em2 & 0xffu, (em2 >> 8) & 0xffu);
+            uint32_t e_g = max(max(mine & 0xffu, (mine >> 8) & 0xffu), max((mine >> 16) & 0xffu, mine >> 24));
 #pragma unroll
             for (int o = 4; o >= 1; o >>= 1) e_g = max(e_g, __shfl_xor_sync(0xffffffffu, e_g, o));
-            const uint2 ts = mine != 0u ? make_uint2(__vminu4(e_g * 0x01010101u - mine, NO_SHIFT * 0x01010101u), e_g) : make_uint2(NO_SHIFT * 0x01010101u, 0u);
-            load();                                        // of the next tile
-            cur = have;
-            have = have && tiles.next_tile(p, meta);
-            fetch();
+            uint2 ts = make_uint2(NO_SHIFT * 0x01010101u, 0u);
+            if (mine != 0u) {
+                ts = make_uint2(e_g * 0x01010101u - mine, e_g);
+                if ((ts.x & 0x80808080u) != 0u) ts.x = __vminu4(ts.x, NO_SHIFT * 0x01010101u);
+            }
             if (it >= 2) ok = mbar_wait_hot(bar(B_SREADY + (it & 1u)), ((it >> 1) - 1) & 1u, abort_flag, WT_SREADY);   // the scores two tiles ago are done
             if (!ok) break;
             tc_fence_after();
@@ -639,6 +642,10 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(bar(B_SCALES + (it & (SW_RING - 1))));
+            load();                                        // of the next tile
+            cur = have;
+            have = have && tiles.next_tile(p, meta);
+            fetch();
         }
     } else if (warp == T_QK) {
         // =================================================================== score MMAs
