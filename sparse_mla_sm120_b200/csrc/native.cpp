@@ -8,6 +8,7 @@
 #include <Python.h>
 #include <ATen/ATen.h>
 #include <ATen/cuda/CUDAContext.h>
+#include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <dlfcn.h>
 #include <torch/csrc/Exceptions.h>
@@ -88,6 +89,14 @@ struct Args {
 void require_cuda(std::initializer_list<const at::Tensor*> ts) {
     for (const at::Tensor* t : ts)
         if (t->defined() && !t->is_cuda()) fail(PyExc_ValueError, "sparse_mla_sm120_b200 runs on CUDA tensors only (there is no CPU path)");
+}
+
+// All CUDA tensors of a call lie on one device.  (Every launch is made with that device current, by a CUDAGuard: the library
+// asks for the current device's attributes, and a default stream's handle means the current device's.)
+void require_one_device(const at::Tensor& first, std::initializer_list<const at::Tensor*> ts) {
+    for (const at::Tensor* t : ts)
+        if (t->defined() && t->is_cuda() && t->device() != first.device())
+            fail(PyExc_ValueError, "tensors on different devices: %s and %s", first.device().str().c_str(), t->device().str().c_str());
 }
 
 void* ptr(const at::Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
@@ -196,6 +205,7 @@ struct Attn {
             ec = geometry(extra_kv);
         }
         require_cuda({&q, &kv, &indices});
+        require_one_device(q, {&kv, &indices, &sink, &topk_length, &extra_kv, &extra_indices, &extra_length, &out});
         ext = c.layout != SMLA_LAYOUT_V32 || extra_topk > 0;
         if (ext) {
             auto al = [](const at::Tensor& t, const Cache& g) { return reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0 && g.stride % 16 == 0; };
@@ -263,6 +273,7 @@ PyObject* decode(const Args& x) {
     Plan p{0, 5, 0};
     if (x.none(13)) p = plan_for(a, blocks, !a.topk_length.defined() && a.extra_topk == 0);
     else p.parts = (int)x.integer(13);
+    const c10::cuda::CUDAGuard on(a.q.device());
     const at::Tensor o = a.output(), lse = a.row_stats();
     if (p.parts == a.tokens) {      // one partition per request: nothing to schedule or to combine
         a.run_whole(o, lse, at::Tensor());
@@ -310,6 +321,7 @@ PyObject* prefill(const Args& x) {
     a.sink = x.tensor(5); a.topk_length = x.tensor(6); a.out = x.tensor(7); a.extra_kv = x.tensor(8); a.extra_indices = x.tensor(9);
     a.extra_topk = (int)x.integer(10); a.impl = (int)x.integer(11);
     a.init(x.integer(4));
+    const c10::cuda::CUDAGuard on(a.q.device());
     const at::Tensor o = a.output(), lse = a.row_stats(), mx = a.row_stats();
     a.run_whole(o, lse, mx);
     PyObject* r = PyTuple_New(3);
@@ -328,6 +340,8 @@ PyObject* mqa_logits(const Args& x) {
     if (q.dim() != 3 || k.dim() != 2 || q.size(2) != 128 || k.size(1) != 128) fail(PyExc_ValueError, "q must be [s_q, H, 128] and k [s_k, 128]");
     require(q.is_contiguous() && k.is_contiguous() && w.is_contiguous() && k_scale.is_contiguous());
     require(ks.scalar_type() == at::kInt && ke.scalar_type() == at::kInt);
+    require_one_device(q, {&k, &k_scale, &w, &ks, &ke, &out});
+    const c10::cuda::CUDAGuard on(q.device());
     if (!out.defined()) out = at::empty({q.size(0), k.size(0)}, q.options().dtype(at::kFloat));
     check(api.mqa_logits(ptr(q), ptr(k), ptr_as<float>(k_scale), ptr_as<float>(w), ptr_as<int32_t>(ks), ptr_as<int32_t>(ke), ptr_as<float>(out),
                          (int)q.size(0), (int)q.size(1), (int)k.size(0), out.stride(0), (int)x.integer(7), status_of(q), stream_of(q)));
@@ -340,6 +354,8 @@ PyObject* topk(const Args& x) {
     const int64_t k = x.integer(3);
     require_cuda({&logits, &ks, &ke, &table});
     require(logits.dim() == 2 && logits.scalar_type() == at::kFloat && logits.stride(1) == 1);
+    require_one_device(logits, {&ks, &ke, &table});
+    const c10::cuda::CUDAGuard on(logits.device());
     const at::Tensor out = at::empty({logits.size(0), k}, logits.options().dtype(at::kInt));
     if (table.defined()) {
         require(table.dim() == 2 && table.scalar_type() == at::kInt && table.stride(1) == 1 && table.size(0) == logits.size(0));
@@ -358,6 +374,7 @@ PyObject* pack_kv(const Args& x) {
     const at::Tensor kv = x.needed(0);
     require_cuda({&kv});
     require(kv.scalar_type() == at::kBFloat16 && kv.dim() >= 1 && kv.size(-1) == SMLA_D_QK && kv.is_contiguous());
+    const c10::cuda::CUDAGuard on(kv.device());
     auto shape = kv.sizes().vec();
     shape.back() = SMLA_ROW_BYTES;
     const at::Tensor out = at::empty(shape, kv.options().dtype(at::kByte));
@@ -397,7 +414,10 @@ PyObject* copy_into(const Args& x) {
             a.copy_(b);
         }
     }
-    if (n > 0) check(api.copy_batch(n, dst, src, bytes, stream_of(dt[0])));
+    if (n > 0) {
+        const c10::cuda::CUDAGuard on(dt[0].device());
+        check(api.copy_batch(n, dst, src, bytes, stream_of(dt[0])));
+    }
     Py_RETURN_NONE;
 }
 
