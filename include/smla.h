@@ -215,7 +215,7 @@ int smla_topk(const float* logits, const int32_t* ks, const int32_t* ke, int32_t
 /*
  * The same selection written as physical cache rows: column c of row i becomes
  * block_table[i * table_stride + c / page_size] * page_size + c % page_size (-1 for a position past the table's
- * table_pages pages, and as padding).
+ * table_pages pages, and as padding).  Rows of the table may overlap; table_stride 0 is one table for all rows.
  */
 int smla_topk_paged(const float* logits, const int32_t* ks, const int32_t* ke, int32_t* out_rows, int num_rows, int num_cols,
                     int64_t logits_stride, int k, const int32_t* block_table, int64_t table_stride, int table_pages,

@@ -432,7 +432,7 @@ int smla_topk_paged(const float* logits, const int32_t* ks, const int32_t* ke, i
                     int64_t logits_stride, int k, const int32_t* block_table, int64_t table_stride, int table_pages,
                     int page_size, void* stream) {
     if (!logits || !out_rows || !block_table) return set_error(SMLA_E_NULL, "smla_topk_paged: null pointer argument");
-    if (num_rows < 0 || num_cols < 0 || k < 0 || logits_stride < num_cols || table_pages < 0 || table_stride < table_pages || page_size < 1)
+    if (num_rows < 0 || num_cols < 0 || k < 0 || logits_stride < num_cols || table_pages < 0 || table_stride < 0 || page_size < 1)
         return set_error(SMLA_E_SHAPE, "smla_topk_paged: rows=%d cols=%d k=%d stride=%lld pages=%d of %d", num_rows, num_cols, k,
                          (long long)logits_stride, table_pages, page_size);
     return launch_topk(logits, ks, ke, out_rows, num_rows, num_cols, logits_stride, k, block_table, table_stride, table_pages, page_size,

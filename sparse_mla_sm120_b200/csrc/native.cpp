@@ -358,7 +358,7 @@ PyObject* topk(const Args& x) {
     const c10::cuda::CUDAGuard on(logits.device());
     const at::Tensor out = at::empty({logits.size(0), k}, logits.options().dtype(at::kInt));
     if (table.defined()) {
-        require(table.dim() == 2 && table.scalar_type() == at::kInt && table.stride(1) == 1 && table.size(0) == logits.size(0));
+        require(table.dim() == 2 && table.scalar_type() == at::kInt && (table.stride(1) == 1 || table.size(1) == 1) && table.size(0) >= logits.size(0));
         check(api.topk_paged(ptr_as<float>(logits), ptr_as<int32_t>(ks), ptr_as<int32_t>(ke), ptr_as<int32_t>(out), (int)logits.size(0),
                              (int)logits.size(1), logits.stride(0), (int)k, ptr_as<int32_t>(table), table.size(0) > 1 ? table.stride(0) : table.size(1),
                              (int)table.size(1), (int)x.integer(5), stream_of(logits)));

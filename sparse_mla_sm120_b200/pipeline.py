@@ -25,6 +25,15 @@ def positions_to_rows(positions: torch.Tensor, block_table: torch.Tensor, page_b
     return torch.where(valid, rows, torch.full_like(rows, -1)).to(torch.int32)
 
 
+def _selection_reads(block_table: torch.Tensor, logits: torch.Tensor, page_block_size: int) -> bool:
+    """Whether the selection can write its columns as rows through this table: int32 with adjacent columns, a row for every
+    token (any distance apart: one request's table may be expanded over its tokens) and a page for every column.  Any other
+    table goes through positions_to_rows, which refuses what it cannot serve: a position past a table that is
+    too short must not become an entry that is silently left out."""
+    return (block_table.dtype == torch.int32 and block_table.dim() == 2 and (block_table.stride(1) == 1 or block_table.shape[1] == 1)
+            and block_table.shape[0] >= logits.shape[0] and block_table.shape[1] * page_block_size >= logits.shape[1])
+
+
 def sparse_mla_indexed_decode_fwd(q: torch.Tensor, kv_cache: torch.Tensor, qi: torch.Tensor, ki: torch.Tensor,
                                   k_scale: torch.Tensor, weights: torch.Tensor, ks: torch.Tensor, ke: torch.Tensor,
                                   sm_scale: float, topk: int = 2048, block_table: Optional[torch.Tensor] = None,
@@ -34,7 +43,7 @@ def sparse_mla_indexed_decode_fwd(q: torch.Tensor, kv_cache: torch.Tensor, qi: t
     indexer queries, ``ki`` [s_k, 128] e4m3 / ``k_scale`` [s_k] indexer keys, ``ks`` / ``ke`` [T]
     the window of each token.  Returns (out [T, H, 512] bf16, lse [T, H], rows [T, topk] int32)."""
     logits = indexer.fp8_mqa_logits(qi, ki, k_scale, weights, ks, ke)
-    if block_table is not None and block_table.dtype == torch.int32 and block_table.stride(1) == 1:
+    if block_table is not None and _selection_reads(block_table, logits, kv_cache.shape[1]):
         rows = native().topk(logits, ks, ke, topk, block_table, kv_cache.shape[1])     # written as rows by the selection
     else:
         rows = indexer.topk_indices(logits, ks, ke, topk)

@@ -49,6 +49,9 @@ def test_argument_errors_do_not_launch(lib):
     assert lib.smla_combine(fake, fake, fake, fake, fake, 1, 128, 4096, None, None) == -2
     assert lib.smla_sched_meta(0, 2048, 0, 4, 5, None, None, fake, fake, None) == -2
     assert lib.smla_topk(None, None, None, None, 1, 1, 1, 1, None) == -1
+    paged = lambda stride, pages=3, page=64: lib.smla_topk_paged(fake, None, None, fake, 0, 9, 9, 4, fake, stride, pages, page, None)
+    assert paged(3) == 0 and paged(0) == 0 and paged(2) == 0      # rows of a page table may overlap (no rows: nothing is launched)
+    assert paged(-1) == -2 and paged(3, pages=-1) == -2 and paged(3, page=0) == -2
     assert lib.smla_workspace_bytes(64, 128, 74) == (64 + 74) * 128 * 513 * 4
     with pytest.raises(ValueError):
         _lib.check(-2)
