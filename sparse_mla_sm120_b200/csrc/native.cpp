@@ -383,7 +383,8 @@ PyObject* pack_kv(const Args& x) {
 }
 
 // (destinations, sources): sequences of tensors, each source copied into its destination as Tensor.copy_ does.  Those
-// that are plain device copies (same type, shape and device, contiguous) go as one launch.
+// that are plain device copies (same type, shape and device, contiguous) go as one launch, unless a destination overlaps some
+// source or another destination: then the order counts, and a copy onto part of itself is for Tensor.copy_ to refuse.
 PyObject* copy_into(const Args& x) {
     PyObject* d = PySequence_Fast(x.a[0], "destinations must be a sequence");
     if (d == nullptr) throw Failure();
@@ -403,11 +404,23 @@ PyObject* copy_into(const Args& x) {
     const void* src[SMLA_COPY_BATCH_MAX];
     int64_t bytes[SMLA_COPY_BATCH_MAX];
     int n = 0;
+    struct Range { uintptr_t lo, hi; };
+    auto range = [](const at::Tensor& t) {      // every byte between a tensor's first and last element
+        int64_t last = 0;
+        for (int64_t d = 0; d < t.dim(); ++d) last += (t.size(d) - 1) * t.stride(d);
+        const uintptr_t lo = t.is_cuda() && t.numel() > 0 ? reinterpret_cast<uintptr_t>(t.data_ptr()) : 0;
+        return Range{lo, lo == 0 ? 0 : lo + (uintptr_t)((last + 1) * (int64_t)t.element_size())};
+    };
+    std::vector<Range> rd, rs;
+    for (size_t i = 0; i < dt.size(); ++i) { rd.push_back(range(dt[i])); rs.push_back(range(st[i])); }
+    auto meet = [](const Range& u, const Range& v) { return u.lo < v.hi && v.lo < u.hi; };
+    bool apart = true;
+    for (size_t i = 0; i < rd.size(); ++i)
+        for (size_t j = 0; j < rd.size(); ++j) apart &= !meet(rd[i], rs[j]) && (i == j || !meet(rd[i], rd[j]));
     for (size_t i = 0; i < dt.size(); ++i) {
         const at::Tensor &a = dt[i], &b = st[i];
-        if (n < SMLA_COPY_BATCH_MAX && a.is_cuda() && b.is_cuda() && a.device() == b.device() && a.device() == dt[0].device() &&
-            a.scalar_type() == b.scalar_type() && a.sizes() == b.sizes() && a.is_contiguous() && b.is_contiguous() &&
-            a.data_ptr() != b.data_ptr()) {
+        if (apart && n < SMLA_COPY_BATCH_MAX && a.is_cuda() && b.is_cuda() && a.device() == b.device() && a.device() == dt[0].device() &&
+            a.scalar_type() == b.scalar_type() && a.sizes() == b.sizes() && a.is_contiguous() && b.is_contiguous()) {
             dst[n] = a.data_ptr(); src[n] = b.data_ptr(); bytes[n] = (int64_t)a.nbytes();
             ++n;
         } else {

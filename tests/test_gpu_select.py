@@ -78,3 +78,23 @@ def test_copies_of_a_step():
         assert torch.equal(a, b.to(DEV).to(a.dtype))
     with pytest.raises(TypeError):
         native().copy_into(dst, src[:-1])
+
+
+def test_copies_that_touch_each_other_run_in_order():
+    """A destination that is also a source, or another destination: as if copied one after the other; a copy onto part of itself is
+    refused, as Tensor.copy_ refuses it; a tensor onto itself is left alone."""
+    from sparse_mla_sm120_b200._lib import native
+    n = 1 << 22                                                        # many blocks per copy
+    a, b, c = (torch.arange(n, device=DEV, dtype=torch.int32) * k for k in (1, 3, 7))
+    want = a.clone()
+    native().copy_into((b, c, a), (a, b, c))                           # a chain: everything becomes a
+    for t in (a, b, c):
+        assert torch.equal(t, want)
+    native().copy_into((c, c), (torch.zeros_like(c), a * 5))           # the later one stays
+    assert torch.equal(c, a * 5)
+    native().copy_into((a, b), (a, c))
+    assert torch.equal(a, want) and torch.equal(b, c)
+    with pytest.raises(RuntimeError):
+        native().copy_into((a[1:],), (a[:-1],))
+    with pytest.raises(RuntimeError):
+        a[1:].copy_(a[:-1])
