@@ -86,7 +86,7 @@ int smla_device_status(int32_t* status, int32_t host_out[4], void* stream) {
 int smla_version(void) { return 100; }
 
 int smla_num_sms(void) {
-    static int cache[64] = {};
+    static std::atomic<int> cache[64];
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return set_error(SMLA_E_DEVICE, "smla_num_sms: no CUDA device");
     if (dev < 64 && cache[dev]) return cache[dev];

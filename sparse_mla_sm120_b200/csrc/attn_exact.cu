@@ -539,7 +539,7 @@ __global__ void __launch_bounds__(X_THREADS, 1) attn_exact_kernel(const AttnPara
 
 int launch_attn_exact(const AttnParams& p, cudaStream_t stream) {
     if (p.num_tokens == 0) return 0;
-    static bool attr_set[64] = {};
+    static std::atomic<bool> attr_set[64];
     static int sm_count[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);

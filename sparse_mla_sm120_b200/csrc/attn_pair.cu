@@ -1168,7 +1168,7 @@ namespace {
 
 template <int LAYOUT, bool EXTRA, bool STAGE_Q>
 int launch_pair_instance(const AttnParams& p, cudaStream_t stream) {
-    static bool attr_set[64] = {};
+    static std::atomic<bool> attr_set[64];
     static int sm_count[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);

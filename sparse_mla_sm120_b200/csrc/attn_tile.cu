@@ -741,9 +741,9 @@ bool attn_tile_takes(const AttnParams& p) {
 
 int launch_attn_tile(const AttnParams& p, cudaStream_t stream) {
     if (p.num_tokens == 0) return 0;
-    static bool attr_set[64] = {};
+    static std::atomic<bool> attr_set[64];
     static int sm_count[64] = {};
-    static EncodeFn encode = nullptr;
+    static std::atomic<EncodeFn> encode{nullptr};
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64) return set_error(SMLA_E_SHAPE, "attn_tile_kernel: device ordinal %d not supported", dev);
@@ -768,7 +768,7 @@ int launch_attn_tile(const AttnParams& p, cudaStream_t stream) {
     CUtensorMap map;
     const cuuint64_t dims[2] = {ROW_BYTES / 4, (cuuint64_t)NO_ROW}, strides[1] = {ROW_BYTES};
     const cuuint32_t box[2] = {32, 1}, estr[2] = {1, 1};
-    const CUresult r = encode(&map, CU_TENSOR_MAP_DATA_TYPE_INT32, 2, const_cast<uint8_t*>(p.kv), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+    const CUresult r = encode.load()(&map, CU_TENSOR_MAP_DATA_TYPE_INT32, 2, const_cast<uint8_t*>(p.kv), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return set_error(SMLA_E_DEVICE, "attn_tile_kernel: cuTensorMapEncodeTiled failed (%d)", (int)r);
     const int parts = p.sched ? p.num_parts : p.uniform_k > 1 ? p.uniform_k * p.num_tokens : (p.num_tokens < sm_count[dev] ? p.num_tokens : sm_count[dev]);

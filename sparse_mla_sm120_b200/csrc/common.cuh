@@ -7,6 +7,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>      // what a launcher finds out once per device: several threads may launch at a time
+
 #include "../../include/smla.h"
 
 namespace smla {

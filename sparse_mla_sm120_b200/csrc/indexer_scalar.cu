@@ -938,7 +938,7 @@ int launch_mqa_logits_scalar(const uint8_t* q, const uint8_t* k, const float* k_
                              int s_k, int64_t logits_stride, cudaStream_t stream) {
     if (s_q == 0 || s_k == 0) return 0;
     const size_t smem = (size_t)num_heads * LD * sizeof(float);
-    static bool attr_set[64] = {};
+    static std::atomic<bool> attr_set[64];
     int dev = 0;
     cudaGetDevice(&dev);
     if (smem > 48 * 1024 && dev < 64 && !attr_set[dev]) {
@@ -960,7 +960,7 @@ int launch_topk(const float* logits, const int32_t* ks, const int32_t* ke, int32
         topk_kernel<<<num_rows, TK_THREADS, 0, stream>>>(logits, ks, ke, out, num_cols, logits_stride, k, emit);
         return check_launch("topk_kernel");
     }
-    static bool attr_set[64] = {};
+    static std::atomic<bool> attr_set[64];
     static int sms[64] = {}, clusters[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);

@@ -292,7 +292,7 @@ int launch_mqa_logits_tc(const uint8_t* q, const uint8_t* k, const float* k_scal
     // the tensor-core kernel reads its accumulator 32 columns at a time: 32 or 64 heads
     if (num_heads % 32 != 0 || num_heads > 64)
         return launch_mqa_logits_scalar(q, k, k_scale, weights, ks, ke, logits, s_q, num_heads, s_k, logits_stride, stream);
-    static bool attr_set[64] = {};
+    static std::atomic<bool> attr_set[64];
     static int sms[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
@@ -312,7 +312,7 @@ int launch_mqa_logits_tc(const uint8_t* q, const uint8_t* k, const float* k_scal
     typedef CUresult (*EncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                                  const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-    static EncodeFn encode = nullptr;
+    static std::atomic<EncodeFn> encode{nullptr};
     if (encode == nullptr) {
         cudaDriverEntryPointQueryResult qres;
         void* fn = nullptr;
@@ -326,10 +326,10 @@ int launch_mqa_logits_tc(const uint8_t* q, const uint8_t* k, const float* k_scal
         const cuuint64_t strides[1] = {(cuuint64_t)LX_D};
         const cuuint32_t qbox[2] = {(cuuint32_t)LX_D, (cuuint32_t)(LX_QG * num_heads)}, kbox[2] = {(cuuint32_t)LX_D, (cuuint32_t)LX_KT};
         const cuuint32_t estr[2] = {1, 1};
-        const CUresult r1 = encode(&qmap, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<uint8_t*>(q), qdims, strides, qbox, estr,
+        const CUresult r1 = encode.load()(&qmap, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<uint8_t*>(q), qdims, strides, qbox, estr,
                                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
                                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-        const CUresult r2 = encode(&kmap, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<uint8_t*>(k), kdims, strides, kbox, estr,
+        const CUresult r2 = encode.load()(&kmap, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<uint8_t*>(k), kdims, strides, kbox, estr,
                                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
                                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
         if (r1 != CUDA_SUCCESS || r2 != CUDA_SUCCESS)

@@ -4,7 +4,8 @@
 // Why: a decode step of one request takes the GPU about 24 us, and the same host work in Python took 27 (argument
 // handling, the split policy's loop, dictionary look-ups, a 21-argument foreign call); here it is a few.
 // Kept between calls: the answers of the split policy (integers per call shape), the address of the device status words and
-// the library's entry points.  Everything runs under the interpreter lock.
+// the library's entry points; what is kept is read and written under the interpreter lock, which a launch gives up (a launch
+// waits when the queue of its stream is full, and other threads drive other streams meanwhile).
 #include <Python.h>
 #include <ATen/ATen.h>
 #include <ATen/cuda/CUDAContext.h>
@@ -56,6 +57,20 @@ void check(int rc) {
     if (rc == 0) return;
     if (rc < 0) fail(PyExc_ValueError, "smla error %d: %s", rc, api.last_error());
     fail(g_error, "CUDA error %d: %s", rc, api.last_error());
+}
+
+// The result of a call into the library, made without the interpreter lock.  (Its message is the calling thread's.)
+template <typename F>
+void launch(F&& f) {
+    int rc;
+    {
+        struct Unlocked {
+            PyThreadState* s = PyEval_SaveThread();
+            ~Unlocked() { PyEval_RestoreThread(s); }
+        } unlocked;
+        rc = f();
+    }
+    check(rc);
 }
 
 void require(bool ok) { if (!ok) fail(PyExc_AssertionError, "unsupported tensor: expected a contiguous one of the documented type"); }
@@ -221,15 +236,16 @@ struct Attn {
 
     // Attention alone, every request whole.
     void run_whole(const at::Tensor& o, const at::Tensor& lse, const at::Tensor& mx) const {
-        if (ext)
-            check(api.prefill_ext(ptr(q), ptr(kv), ptr_as<int32_t>(indices), ptr(extra_kv), ptr_as<int32_t>(extra_indices), ptr(o),
-                                  ptr_as<float>(lse), ptr_as<float>(mx), tokens, heads, topk, extra_topk, sm_scale, c.layout, (int)c.block,
-                                  c.stride, (int)ec.block, ec.stride, ptr_as<float>(sink), ptr_as<int32_t>(topk_length),
-                                  ptr_as<int32_t>(extra_length), impl, status_of(q), stream_of(q)));
-        else
-            check(api.prefill(ptr(q), ptr(kv), ptr_as<int32_t>(indices), ptr(o), ptr_as<float>(lse), ptr_as<float>(mx), tokens, heads, topk,
-                              sm_scale, (int)c.block, c.stride, ptr_as<float>(sink), ptr_as<int32_t>(topk_length), impl, status_of(q),
-                              stream_of(q)));
+        int32_t* status = status_of(q);
+        launch([&] {
+            if (ext)
+                return api.prefill_ext(ptr(q), ptr(kv), ptr_as<int32_t>(indices), ptr(extra_kv), ptr_as<int32_t>(extra_indices), ptr(o),
+                                       ptr_as<float>(lse), ptr_as<float>(mx), tokens, heads, topk, extra_topk, sm_scale, c.layout, (int)c.block,
+                                       c.stride, (int)ec.block, ec.stride, ptr_as<float>(sink), ptr_as<int32_t>(topk_length),
+                                       ptr_as<int32_t>(extra_length), impl, status, stream_of(q));
+            return api.prefill(ptr(q), ptr(kv), ptr_as<int32_t>(indices), ptr(o), ptr_as<float>(lse), ptr_as<float>(mx), tokens, heads, topk,
+                               sm_scale, (int)c.block, c.stride, ptr_as<float>(sink), ptr_as<int32_t>(topk_length), impl, status, stream_of(q));
+        });
     }
 };
 
@@ -292,25 +308,32 @@ PyObject* decode(const Args& x) {
     float* lse_accum = reinterpret_cast<float*>(w + o_bytes);
     int32_t* meta = reinterpret_cast<int32_t*>(w + o_bytes + l_bytes);
     int32_t* splits = reinterpret_cast<int32_t*>(w + o_bytes + l_bytes + m_bytes);
+    int32_t* status = status_of(a.q);
     if (p.uniform > 1) {
-        check(api.decode_uniform(ptr(a.q), ptr(a.kv), ptr_as<int32_t>(a.indices), o_accum, lse_accum, ptr(o), ptr_as<float>(lse), a.tokens,
-                                 a.heads, a.topk, a.sm_scale, (int)a.c.block, a.c.stride, p.uniform, ptr_as<float>(a.sink), a.impl,
-                                 status_of(a.q), stream));
+        launch([&] {
+            return api.decode_uniform(ptr(a.q), ptr(a.kv), ptr_as<int32_t>(a.indices), o_accum, lse_accum, ptr(o), ptr_as<float>(lse), a.tokens,
+                                      a.heads, a.topk, a.sm_scale, (int)a.c.block, a.c.stride, p.uniform, ptr_as<float>(a.sink), a.impl,
+                                      status, stream);
+        });
         return wrap2(o, lse);
     }
-    check(api.sched_meta(a.tokens, a.topk, a.extra_topk, p.parts, p.overhead, ptr_as<int32_t>(a.topk_length), ptr_as<int32_t>(a.extra_length),
-                         meta, splits, stream));
-    if (a.ext)
-        check(api.decode_splitkv_ext(ptr(a.q), ptr(a.kv), ptr_as<int32_t>(a.indices), ptr(a.extra_kv), ptr_as<int32_t>(a.extra_indices), o_accum,
-                                     lse_accum, ptr(o), ptr_as<float>(lse), meta, splits, a.tokens, a.heads, a.topk, a.extra_topk, a.sm_scale,
-                                     a.c.layout, (int)a.c.block, a.c.stride, (int)a.ec.block, a.ec.stride, p.parts, ptr_as<float>(a.sink),
-                                     ptr_as<int32_t>(a.topk_length), ptr_as<int32_t>(a.extra_length), a.impl, status_of(a.q), stream));
-    else
-        check(api.decode_splitkv(ptr(a.q), ptr(a.kv), ptr_as<int32_t>(a.indices), o_accum, lse_accum, ptr(o), ptr_as<float>(lse), meta, splits,
-                                 a.tokens, a.heads, a.topk, a.sm_scale, (int)a.c.block, a.c.stride, p.parts, ptr_as<float>(a.sink),
-                                 ptr_as<int32_t>(a.topk_length), a.impl, status_of(a.q), stream));
-    check(api.combine(o_accum, lse_accum, ptr(o), ptr_as<float>(lse), splits, a.tokens, a.heads, std::min(blocks, p.parts),
-                      ptr_as<float>(a.sink), stream));
+    launch([&] {
+        int rc = api.sched_meta(a.tokens, a.topk, a.extra_topk, p.parts, p.overhead, ptr_as<int32_t>(a.topk_length),
+                                ptr_as<int32_t>(a.extra_length), meta, splits, stream);
+        if (rc != 0) return rc;
+        if (a.ext)
+            rc = api.decode_splitkv_ext(ptr(a.q), ptr(a.kv), ptr_as<int32_t>(a.indices), ptr(a.extra_kv), ptr_as<int32_t>(a.extra_indices), o_accum,
+                                        lse_accum, ptr(o), ptr_as<float>(lse), meta, splits, a.tokens, a.heads, a.topk, a.extra_topk, a.sm_scale,
+                                        a.c.layout, (int)a.c.block, a.c.stride, (int)a.ec.block, a.ec.stride, p.parts, ptr_as<float>(a.sink),
+                                        ptr_as<int32_t>(a.topk_length), ptr_as<int32_t>(a.extra_length), a.impl, status, stream);
+        else
+            rc = api.decode_splitkv(ptr(a.q), ptr(a.kv), ptr_as<int32_t>(a.indices), o_accum, lse_accum, ptr(o), ptr_as<float>(lse), meta, splits,
+                                    a.tokens, a.heads, a.topk, a.sm_scale, (int)a.c.block, a.c.stride, p.parts, ptr_as<float>(a.sink),
+                                    ptr_as<int32_t>(a.topk_length), a.impl, status, stream);
+        if (rc != 0) return rc;
+        return api.combine(o_accum, lse_accum, ptr(o), ptr_as<float>(lse), splits, a.tokens, a.heads, std::min(blocks, p.parts),
+                           ptr_as<float>(a.sink), stream);
+    });
     return wrap2(o, lse);
 }
 
@@ -343,8 +366,12 @@ PyObject* mqa_logits(const Args& x) {
     require_one_device(q, {&k, &k_scale, &w, &ks, &ke, &out});
     const c10::cuda::CUDAGuard on(q.device());
     if (!out.defined()) out = at::empty({q.size(0), k.size(0)}, q.options().dtype(at::kFloat));
-    check(api.mqa_logits(ptr(q), ptr(k), ptr_as<float>(k_scale), ptr_as<float>(w), ptr_as<int32_t>(ks), ptr_as<int32_t>(ke), ptr_as<float>(out),
-                         (int)q.size(0), (int)q.size(1), (int)k.size(0), out.stride(0), (int)x.integer(7), status_of(q), stream_of(q)));
+    const int impl = (int)x.integer(7);
+    int32_t* status = status_of(q);
+    launch([&] {
+        return api.mqa_logits(ptr(q), ptr(k), ptr_as<float>(k_scale), ptr_as<float>(w), ptr_as<int32_t>(ks), ptr_as<int32_t>(ke), ptr_as<float>(out),
+                              (int)q.size(0), (int)q.size(1), (int)k.size(0), out.stride(0), impl, status, stream_of(q));
+    });
     return THPVariable_Wrap(out);
 }
 
@@ -359,13 +386,18 @@ PyObject* topk(const Args& x) {
     const at::Tensor out = at::empty({logits.size(0), k}, logits.options().dtype(at::kInt));
     if (table.defined()) {
         require(table.dim() == 2 && table.scalar_type() == at::kInt && (table.stride(1) == 1 || table.size(1) == 1) && table.size(0) >= logits.size(0));
-        check(api.topk_paged(ptr_as<float>(logits), ptr_as<int32_t>(ks), ptr_as<int32_t>(ke), ptr_as<int32_t>(out), (int)logits.size(0),
-                             (int)logits.size(1), logits.stride(0), (int)k, ptr_as<int32_t>(table), table.size(0) > 1 ? table.stride(0) : table.size(1),
-                             (int)table.size(1), (int)x.integer(5), stream_of(logits)));
+        const int page = (int)x.integer(5);
+        launch([&] {
+            return api.topk_paged(ptr_as<float>(logits), ptr_as<int32_t>(ks), ptr_as<int32_t>(ke), ptr_as<int32_t>(out), (int)logits.size(0),
+                                  (int)logits.size(1), logits.stride(0), (int)k, ptr_as<int32_t>(table),
+                                  table.size(0) > 1 ? table.stride(0) : table.size(1), (int)table.size(1), page, stream_of(logits));
+        });
         return THPVariable_Wrap(out);
     }
-    check(api.topk(ptr_as<float>(logits), ptr_as<int32_t>(ks), ptr_as<int32_t>(ke), ptr_as<int32_t>(out), (int)logits.size(0),
-                   (int)logits.size(1), logits.stride(0), (int)k, stream_of(logits)));
+    launch([&] {
+        return api.topk(ptr_as<float>(logits), ptr_as<int32_t>(ks), ptr_as<int32_t>(ke), ptr_as<int32_t>(out), (int)logits.size(0),
+                        (int)logits.size(1), logits.stride(0), (int)k, stream_of(logits));
+    });
     return THPVariable_Wrap(out);
 }
 
@@ -378,7 +410,7 @@ PyObject* pack_kv(const Args& x) {
     auto shape = kv.sizes().vec();
     shape.back() = SMLA_ROW_BYTES;
     const at::Tensor out = at::empty(shape, kv.options().dtype(at::kByte));
-    check(api.pack_kv(ptr(kv), ptr(out), kv.numel() / SMLA_D_QK, stream_of(kv)));
+    launch([&] { return api.pack_kv(ptr(kv), ptr(out), kv.numel() / SMLA_D_QK, stream_of(kv)); });
     return THPVariable_Wrap(out);
 }
 
@@ -429,7 +461,7 @@ PyObject* copy_into(const Args& x) {
     }
     if (n > 0) {
         const c10::cuda::CUDAGuard on(dt[0].device());
-        check(api.copy_batch(n, dst, src, bytes, stream_of(dt[0])));
+        launch([&] { return api.copy_batch(n, dst, src, bytes, stream_of(dt[0])); });
     }
     Py_RETURN_NONE;
 }

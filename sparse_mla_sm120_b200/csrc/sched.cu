@@ -112,7 +112,7 @@ int launch_sched_meta(int b, int topk, int extra_topk, int num_sm_parts, int fix
     SchedArgs a{b, topk, extra_topk, num_sm_parts, fixed_overhead, topk_length, extra_topk_length,
                 reinterpret_cast<SchedMeta*>(sched_meta), num_splits};
     const size_t smem = sizeof(int) * (2 * (size_t)b + 4 + 4 * ((size_t)num_sm_parts + 1));
-    static bool big_smem[64] = {};
+    static std::atomic<bool> big_smem[64];
     if (smem > 48 * 1024) {
         int dev = 0;
         cudaGetDevice(&dev);
