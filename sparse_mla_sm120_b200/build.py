@@ -41,10 +41,28 @@ def _run(cmd, verbose: bool) -> None:
         print(res.stdout)
 
 
+def _stamp_path() -> str:
+    return os.path.splitext(NATIVE_PATH)[0] + ".stamp"
+
+
+def _stamped(cmd) -> bool:
+    try:
+        with open(_stamp_path()) as f:
+            return f.read() == _stamp(cmd)
+    except OSError:
+        return False
+
+
+def _stamp(cmd) -> str:
+    import torch
+    # (the tree may be moved)
+    return "\n".join([f"torch {torch.__version__}", f"python {sys.version}"] + [os.path.relpath(c, PKG_DIR) if c in (NATIVE_PATH, NATIVE_SRC) else c for c in cmd])
+
+
 def build_native(force: bool = False, verbose: bool = False) -> str:
-    """Compile csrc/native.cpp; returns the extension's path."""
-    if not force and not _older(NATIVE_PATH, [NATIVE_SRC] + _headers()):
-        return NATIVE_PATH
+    """Compile csrc/native.cpp; returns the extension's path.  Compiled again too when the torch or the Python that it was
+    compiled against is another one, or the command: its layout of tensors is that torch's (the .stamp beside it says
+    which)."""
     import torch
     from torch.utils import cpp_extension
     cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
@@ -53,7 +71,11 @@ def build_native(force: bool = False, verbose: bool = False) -> str:
            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
            *(f"-I{p}" for p in cpp_extension.include_paths()), f"-I{sysconfig.get_paths()['include']}", f"-I{cuda}/include",
            "-o", NATIVE_PATH, NATIVE_SRC, f"-L{libs}", "-ltorch_python", "-ltorch_cpu", "-lc10_cuda", "-lc10", f"-L{cuda}/lib64", "-lcudart", "-ldl"]
+    if not force and not _older(NATIVE_PATH, [NATIVE_SRC] + _headers()) and _stamped(cmd):
+        return NATIVE_PATH
     _run(cmd, verbose)
+    with open(_stamp_path(), "w") as f:
+        f.write(_stamp(cmd))
     return NATIVE_PATH
 
 
