@@ -94,6 +94,8 @@ __device__ __forceinline__ void e4m3_as_bf16(uint32_t w, uint32_t& even, uint32_
     even = ((w * 256u) & 0x80008000u) | ((w * 16u) & 0x07f007f0u);
     odd = (w & 0x80008000u) | ((w >> 4) & 0x07f007f0u);
 }
+// Bit 7 of every byte: whether the e4m3 value is no number (all seven lower bits set).
+__device__ __forceinline__ uint32_t no_number_bytes(uint32_t w) { return (w & 0x7f7f7f7fu) + 0x01010101u; }
 __device__ __forceinline__ int exact_dim_at(int pos) {           // output dim of position pos of a row, and the reverse
     return (pos < X_NOPE && ((pos + 1) & 2)) ? pos ^ 3 : pos;
 }
@@ -422,6 +424,20 @@ __global__ void __launch_bounds__(X_THREADS, 1) attn_exact_kernel(const AttnPara
         for (uint32_t it = 0; have; ++it) {
             const bool have_after = have_next && walk.next(p, meta, last_req);
             int idx_after = fetch(have_after);              // read while this tile is stored
+            // A byte that is no number (the conversion would make 480 of it) makes its token's score none: one pair of the row's
+            // RoPE values, which every score and every weight's product meets, becomes NaN.  Looked for here, while P.V still
+            // reads the tile before; in the conversion it cost 2 us of 51.
+            uint32_t bad = 0u;
+#pragma unroll
+            for (int i = 0; i < X_RPW; ++i) {
+                const uint32_t none = no_number_bytes(nope[i].x) | no_number_bytes(nope[i].y) | no_number_bytes(nope[i].z) | no_number_bytes(nope[i].w);
+                bad |= __any_sync(0xffffffffu, (none & 0x80808080u) != 0u) ? 1u << i : 0u;
+            }
+            if (bad != 0u) {
+#pragma unroll
+                for (int u = 0; u < X_RPW / 4; ++u)
+                    if ((bad >> ((lane >> 3) + 4 * u)) & 1u) rp[u].x = 0x7fff7fffu;
+            }
 #pragma unroll
             for (int i = 0; i < X_RPW; ++i) {
                 if (it >= 1 && (i & 1) == 0 && ok) ok = mbar_wait_hot(bar(XB_KFREE + (i >> 1)), (it - 1) & 1u, abort_flag, WX_KFREE);
@@ -440,7 +456,8 @@ __global__ void __launch_bounds__(X_THREADS, 1) attn_exact_kernel(const AttnPara
                     d[2 * k + 1] = mul_bf16x2(d[2 * k + 1], f);
                 }
                 if (__any_sync(0xffffffffu, e > 134u)) {
-                    const __nv_bfloat162 f2 = pow2_bf16x2(e > 134u ? min(e - 134u, 127u) + 127u : 127u);
+                    // (255, no number in UE8M0, makes infinity here as in the fp32 kernel)
+                    const __nv_bfloat162 f2 = pow2_bf16x2(e == 255u ? 255u : e > 134u ? min(e - 134u, 127u) + 127u : 127u);
 #pragma unroll
                     for (int k = 0; k < 8; ++k) d[k] = mul_bf16x2(d[k], f2);
                 }

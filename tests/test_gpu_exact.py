@@ -41,3 +41,35 @@ def test_every_byte_and_scale():
     out, lse = _decode(c, impl=FP32)
     H.compare_out(out.cpu(), ref_out, 1e-4, H.SCALAR_REL)
     _compare(out[..., 128:], lse, ref_out[..., 128:], ref_lse, impl=FP32)
+
+
+@pytest.mark.parametrize("byte", [0x7F, 0xFF])
+@pytest.mark.parametrize("at", [0, 15, 16, 250, 447])
+def test_a_byte_that_is_no_number_stays_none(byte, at):
+    """A NaN in a row that a request selects makes all of that request's outputs NaN, and nobody else's; as the fp32 kernel has it,
+    which serves the same call over caches that are only 4-byte aligned."""
+    c = _m1_case(12, 3, 64, 200, nblk=8)
+    c["indices"][:, 0, 190:] = -1
+    c["indices"][c["indices"] == 77] = 78
+    c["indices"][1, 0, 131] = 77
+    base_out, base_lse = _decode(c, num_sm_parts=3, impl=FP32)
+    c["packed"].view(8, -1)[1, 13 * 576 + at] = byte           # row 77: token 13 of page 1
+    out, lse = _decode(c, num_sm_parts=3, impl=FP32)
+    assert torch.isnan(out[1].float()).all()
+    for r in (0, 2):
+        assert torch.equal(out[r], base_out[r]) and torch.equal(lse[r], base_lse[r])
+    buf = torch.zeros(c["packed"].numel() + 64, dtype=torch.uint8, device="cuda:0")
+    moved = buf[4:4 + c["packed"].numel()].view(c["packed"].shape)
+    moved.copy_(c["packed"])
+    slow, slow_lse = _decode(dict(c, packed=moved), num_sm_parts=3, impl=FP32)
+    assert torch.equal(torch.isnan(slow.float()), torch.isnan(out.float())) and torch.equal(slow_lse[1], lse[1])
+
+
+def test_a_scale_byte_of_255():
+    """No number in UE8M0: infinity times the block's values in both kernels."""
+    c = _m1_case(13, 2, 8, 64, nblk=8)
+    c["indices"][c["indices"] == 5] = 6
+    c["indices"][0, 0, 3] = 5
+    c["packed"].view(8, -1)[0, 64 * 576 + 5 * 8 + 2] = 255
+    out, lse = _decode(c, num_sm_parts=2, impl=FP32)
+    assert not torch.isfinite(out[0].float()).any() and torch.isfinite(out[1].float()).all()
