@@ -733,9 +733,23 @@ typedef CUresult (*EncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void
 
 }  // namespace
 
+// Whole requests that each get a pair of SMs to themselves take as long as one request does, and two CTAs walk a long list
+// faster than one.  us of this kernel / of the pair kernel, 8 to 74 requests that use all of their list:
+//     above 32 heads             512 entries 18.8-20.6 / 18.8-20.9, 768: 22.9-25.1 / 22.9-25.3, 1024: 27.7-31.2 / 27.0-30.6, 2048: 45.5-51.4 / 42.6-47.5
+//       with maximum logits      256: 16.2-16.7 / 16.7-16.8, 512: 20.8-21.3 / 18.8-20.8, 2048: 45.7-55.6 / 42.5-47.6
+//     up to 32 heads             512: 16.8-18.1 / 18.8-20.8, 2048: 40.2-44.9 / 41.4-47.4 (never)
+//       with maximum logits      768: 22.9-24.8 / 22.5-25.0, 1024: 27.0-29.2 / 25.4-29.1, 2048: 44.2-49.0 / 41.4-47.5
+// With more requests than pairs the pair kernel needs another round: 80 requests of 2048 entries 51.4 / 86.6.
+static bool pair_is_faster(const AttnParams& p) {
+    if (p.sched != nullptr || p.uniform_k > 1 || p.num_tokens > smla_num_sms() / 2) return false;
+    const int blocks = (p.topk + BLOCK_N - 1) / BLOCK_N;
+    if (p.num_heads > 32) return blocks >= (p.out_max_logits != nullptr ? 8 : 12);
+    return p.out_max_logits != nullptr && blocks >= 16;
+}
+
 // One linear array of 656-byte rows (pages without padding between them) and one CTA's worth of heads.
 bool attn_tile_takes(const AttnParams& p) {
-    return p.num_heads <= T_HEADS && p.layout == SMLA_LAYOUT_V32 && p.extra_topk == 0 && p.block_stride == (int64_t)p.page_block_size * ROW_BYTES &&
+    return !pair_is_faster(p) && p.num_heads <= T_HEADS && p.layout == SMLA_LAYOUT_V32 && p.extra_topk == 0 && p.block_stride == (int64_t)p.page_block_size * ROW_BYTES &&
            (reinterpret_cast<uintptr_t>(p.kv) & 15u) == 0;
 }
 

@@ -48,7 +48,7 @@ def test_small_blocks_keep_their_precision(heads, pattern):
     magnitude, held to the emulation's error on the same inputs as test_scale_spread_rows does (there at 128 heads, which
     run on the pair kernel).  steady: small in every row; late: rows of a later tile are the first with a large block, so
     what was accumulated for it has to come down; mixed: small in two rows of three."""
-    case = make_case(17, 3, heads, 640, 32, q_std=2.0, invalid_tail=0.0)
+    case = make_case(17, 80, heads, 640, 32, q_std=2.0, invalid_tail=0.0)     # (fewer whole requests run on the pair kernel)
     scales = case["packed"].view(-1, 656)[:, 512:528].view(torch.float32)
     if pattern == "steady":
         scales[:, 1] *= 2.0 ** -6
@@ -65,7 +65,7 @@ def test_small_blocks_keep_their_precision(heads, pattern):
         scales[1:, 2] *= 2.0 ** -8
     ref_out, ref_lse = oracle_attn(case)
     emu_out, _ = H.orc.emulate_fp8_attention(case["q"], case["packed"], case["indices"], case["sm_scale"])
-    results = [_prefill(case, TC)[0]] + [_decode(case, TC, num_sm_parts=parts)[0] for parts in (None, 2, 7)]
+    results = [_prefill(case, TC)[0]] + [_decode(case, TC, num_sm_parts=parts)[0] for parts in (None, 2, 90)]
     for out in results:
         for b in range(4):
             sl = slice(128 * b, 128 * b + 128)
@@ -92,9 +92,23 @@ def test_weights_are_rounded_as_by_the_pair_kernel(heads):
     """The same whole requests over pages with and without padding (the pair kernel and attn_tile_kernel): the same maxima and
     the same rounded weights, so the outputs differ by sums in another order and by values below 2^-6 that the pair
     kernel cuts when it moves them to its group's scale, not by another realisation of the roundings (3e-3 of the rms)."""
-    case = make_case(19, 6, heads, 512, 16, invalid_tail=0.1)
+    case = make_case(19, 80, heads, 512, 16, invalid_tail=0.1)
     a, mx_a, lse_a = _prefill(case, TC)
     b, mx_b, lse_b = _prefill_padded(case)
     d = (a.float() - b.float()).pow(2).mean().sqrt() / b.float().pow(2).mean().sqrt()
     assert float(d) <= 5e-4, float(d)
     assert float((lse_a - lse_b).abs().max()) <= 1e-4 and float((mx_a - mx_b).abs().max()) <= 1e-4
+
+
+@pytest.mark.parametrize("heads,topk,tokens", [(33, 448, 74), (33, 449, 74), (33, 704, 74), (33, 705, 74), (33, 705, 75), (32, 960, 74), (32, 961, 74),
+                                               (64, 1024, 1), (64, 1024, 76)])
+def test_whole_requests_on_either_side_of_the_line_to_the_pair_kernel(heads, topk, tokens):
+    """Lists and numbers of requests at which whole requests go to the other kernel, with and without maximum logits."""
+    case = make_case(31, tokens, heads, topk, 20, invalid_tail=0.1)
+    ref_out, ref_lse = oracle_attn(case)
+    out, mx, lse = _prefill(case, TC)
+    _check_hard(out, lse, ref_out, ref_lse, TC, case)
+    out2, lse2 = _decode(case, TC, num_sm_parts=tokens)
+    _check_hard(out2, lse2, ref_out, ref_lse, TC, case)
+    d = (out.float() - out2.float()).pow(2).mean().sqrt() / out.float().pow(2).mean().sqrt()
+    assert float(d) <= 5e-4 and float((lse - lse2).abs().max()) <= 1e-4      # the same roundings on both (see above)
