@@ -9,7 +9,6 @@ import torch
 
 from . import _lib
 
-HEADS_PER_TILE = 128     # one CTA covers every head of a query token
 CTAS_PER_PART = 2        # two CTAs (one per half of d_v) share a partition
 FIXED_OVERHEAD = 5       # scheduler cost of starting a request, in 64-token blocks
 BLOCK_N = 64

@@ -99,19 +99,6 @@ __device__ __forceinline__ uint32_t pack_e4m3x4(float a, float b, float c, float
     return (uint32_t)lo | ((uint32_t)hi << 16);
 }
 
-// Multiplies four packed e4m3 values by a power of two (given as half2) with rounding.
-__device__ __forceinline__ uint32_t rescale_e4m3x4(uint32_t w, __half2 ratio) {
-    uint32_t lo, hi;
-    asm("cvt.rn.f16x2.e4m3x2 %0, %1;" : "=r"(lo) : "h"((uint16_t)(w & 0xffffu)));
-    asm("cvt.rn.f16x2.e4m3x2 %0, %1;" : "=r"(hi) : "h"((uint16_t)(w >> 16)));
-    __half2 a = __hmul2(*reinterpret_cast<__half2*>(&lo), ratio);
-    __half2 b = __hmul2(*reinterpret_cast<__half2*>(&hi), ratio);
-    uint16_t ra, rb;
-    asm("cvt.rn.satfinite.e4m3x2.f16x2 %0, %1;" : "=h"(ra) : "r"(*reinterpret_cast<uint32_t*>(&a)));
-    asm("cvt.rn.satfinite.e4m3x2.f16x2 %0, %1;" : "=h"(rb) : "r"(*reinterpret_cast<uint32_t*>(&b)));
-    return (uint32_t)ra | ((uint32_t)rb << 16);
-}
-
 // Divides four packed e4m3 values by 2^d with integer arithmetic: the exponent field of every byte drops
 // by d (`sub` = d * 8 in every byte, d <= 15).  Exact while the result stays a normal number; a result
 // below 2^-6 is cut to the subnormal grid or to zero (off by at most 2^-7, i.e. 2^-15 of the largest

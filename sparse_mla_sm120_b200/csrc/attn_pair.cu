@@ -149,40 +149,6 @@ constexpr uint32_t DESC_HI_SW128 = desc_hi(1024, (uint32_t)SWIZZLE_128B);
 enum { W_QSTAGE = 33, W_QFREE = 34, W_RAWEMPTY = 35, W_RAWFULL = 36, W_KEMPTY = 21, W_KSTORED = 22, W_KFULL = 23, W_INFO = 24, W_VEMPTY = 25, W_VFULL_CTA = 26, W_VFULL = 27,
        W_SREADY = 28, W_SFREE = 29, W_PREADY = 30, W_PVDONE = 31, W_QREADY = 32 };
 
-#ifdef SMLA_TRACE
-// Timeline of one CTA (instrumented builds only): lane 0 of every warp appends (tag, tile, clock) records.
-__device__ long long* g_trace_buf = nullptr;   // [warps][cap][2]
-__device__ int g_trace_cap = 0;
-__device__ int g_trace_block = 0;
-struct TraceCursor { long long* at = nullptr; };     // looked up once: a trace point is a clock read and a store
-__device__ __forceinline__ void trace_open(TraceCursor& c) {
-    if (g_trace_buf != nullptr && (int)blockIdx.x == g_trace_block && (threadIdx.x & 31) == 0)
-        c.at = g_trace_buf + (size_t)(threadIdx.x >> 5) * g_trace_cap * 2;
-}
-__device__ __forceinline__ void trace(TraceCursor& c, int tag, int tile) {
-    if (c.at != nullptr) {
-        c.at[0] = ((long long)tag << 32) | (unsigned)tile;
-        c.at[1] = clock64();
-        c.at += 2;
-    }
-}
-#ifdef SMLA_TRACE_FROM             // only the trace points with tags in [SMLA_TRACE_FROM, SMLA_TRACE_TO): the other roles keep their registers
-#define TRACE(tag, tile) { if ((tag) >= SMLA_TRACE_FROM && (tag) < SMLA_TRACE_TO) trace(tcur, tag, (int)(tile)); }
-#else
-#define TRACE(tag, tile) trace(tcur, tag, (int)(tile))
-#endif
-#else
-#define TRACE(tag, tile)
-#endif
-#ifdef SMLA_PROF
-// Cycle sum of one phase (bin SMLA_PROF, chosen at compile time) per warp of one CTA, written once at the end:
-// PROF(i) adds the time since the last PROF point to the sum when i is the chosen bin.
-__device__ long long* g_prof_buf = nullptr;     // [warps][2]: the sum and the kernel's length
-__device__ int g_prof_block = 0;
-#define PROF(i) { const unsigned now_ = (unsigned)clock(); if ((i) == SMLA_PROF) prof_acc += now_ - prof_last; prof_last = now_; }
-#else
-#define PROF(i)
-#endif
 
 __device__ __forceinline__ uint32_t swz(uint32_t row, uint32_t chunk16) { return row * 128u + ((chunk16 ^ (row & 7u)) << 4); }
 
@@ -278,16 +244,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) att
     auto bar = [&](int i) -> uint32_t { return base + BAR_OFF + 8u * i; };
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-#ifdef SMLA_TRACE
-    TraceCursor tcur;
-    trace_open(tcur);
-#endif
-#ifdef SMLA_PROF
-    unsigned prof_acc = 0;
-    unsigned prof_last = (unsigned)clock();
-    const unsigned prof_start = prof_last;
-#endif
-    TRACE(1, 0);
     const uint32_t rank = cluster_ctarank();          // 0: the CTA that issues the MMAs
     const int part = blockIdx.x >> 1;
     const int heads_cta = (p.num_heads + 1) >> 1;     // heads per CTA
@@ -329,7 +285,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) att
     __syncthreads();
     cluster_sync_all();          // the partner's barriers exist before anything arrives on them
     tc_fence_after();
-    TRACE(6, 0);
     const uint32_t tmem = *tmem_slot;
     auto barp = [&](int i) -> uint32_t { return mapa_shared(bar(i), 0); };   // the even CTA's copy of barrier i
 
@@ -367,7 +322,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) att
     else if (warp < MMA_WARP) setmaxnreg_dec<REGS_GATHER>();
     else if (warp < PROD_WARP0) setmaxnreg_dec<REGS_MMA>();
     else setmaxnreg_dec<REGS_PROD>();
-    TRACE(7, 0);
 
     if (warp < N_SM_WARPS) {
         // =================================================================== softmax + epilogue
@@ -515,8 +469,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) att
                 }
             }
             if (named_bar_or(1 + grp, 128, dead || *abort_flag != 0)) { stop = true; break; }
-            TRACE(2, it);
-            PROF(11);
             // The next request's Q rows are read from global memory by the next Q phase, several dependent rounds of
             // loads with nothing else to do: ask L2 for them now (this CTA's heads, 128-byte lines), a whole request
             // of tiles ahead.
@@ -641,8 +593,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) att
                 }
                 tc_fence_before();                  // the accumulator reads precede the next request's first P.V
                 named_bar_sync(1 + grp, 128);       // xch is free again
-                PROF(12);
-                TRACE(4, it);
             }
             prev_valid = false;
             if (!have) break;
@@ -656,12 +606,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) att
                 float c_g[4], off_g[4], inv_g[4];          // of the four groups of eight tokens that this thread holds: z = s * c + off, 1/s
                 // the records of this thread's 32 tokens: half tile thalf, gather warps [4 ch, 4 ch + 4)
                 const uint8_t* info = sm + INFO_OFF + (it & (INFO_RING - 1)) * (2 * INFO_HALF) + thalf * INFO_HALF + ch * 64;
-                PROF(0);
                 if (!dead) dead = !mbar_wait_hot(bar(BAR_SREADY + b), (it >> 1) & 1u, abort_flag, W_SREADY);
-                PROF(1);
-                TRACE(10, it);
                 if (!dead) dead = !mbar_wait_hot(bar(BAR_INFO + (it & (INFO_RING - 1))), (it / INFO_RING) & 1u, abort_flag, W_INFO);
-                PROF(2);
                 if (!dead) {
                     tc_fence_after();
                     tmem_ld32(lane_addr + TM_S + 64 * b + 32 * ch, sv);
@@ -676,8 +622,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) att
                         valid |= vb << (8 * g);
                     }
                     tmem_wait_ld();
-                    PROF(3);
-                    TRACE(11, it);
                     tc_fence_before();
                     __syncwarp();
                     if (lane == 0) mbar_arrive_remote(barp(BAR_SFREEP + b));   // the score buffer may be overwritten
@@ -696,8 +640,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) att
                         mx_loc = fmaxf(mx_loc, fmaf(gm, c_g[g], off_g[g]));
                         if (p.out_max_logits != nullptr) x_max = fmaxf(x_max, gm * c_g[g]);   // without log2(s): the scaled logit itself
                     }
-                    PROF(4);
-                    TRACE(16, it);
                 }
                 // Some row of the group of 128 threads has outgrown its running maximum (or a wait gave up): rare after the
                 // first tiles of a request, so only then the four partial row maxima are exchanged.
@@ -727,13 +669,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) att
                         tmem_wait_st();
                     }
                 }
-                PROF(6);
                 if (it >= 2) {   // the P.V that read this P' buffer two tiles ago has completed
                     dead = !mbar_wait_hot(bar(BAR_PVDONE + b), ((it - 2) >> 1) & 1u, abort_flag, W_PVDONE);
                     if (dead) continue;
                 }
-                PROF(7);
-                TRACE(13, it);
                 const float m_off = ((m_run == -INFINITY) ? 0.f : m_run) - (float)P_SHIFT;
                 uint32_t pw[8];
 #pragma unroll
@@ -757,23 +696,16 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) att
                     unpack_f32x2(l2, l0, l1);
                     l_run = fmaf(l0 + l1, inv_g[g], l_run);
                 }
-                PROF(8);
-                TRACE(15, it);
                 // P' of tokens [64*thalf + 32*ch, +32) of head hrow: two 16-byte pieces of the row
                 uint8_t* pb = sm + PB_OFF + b * CHUNK;
                 *reinterpret_cast<uint4*>(pb + swz(hrow, 4 * thalf + 2 * ch)) = make_uint4(pw[0], pw[1], pw[2], pw[3]);
                 *reinterpret_cast<uint4*>(pb + swz(hrow, 4 * thalf + 2 * ch + 1)) = make_uint4(pw[4], pw[5], pw[6], pw[7]);
                 fence_proxy_async();
-                PROF(9);
-                TRACE(17, it);
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive_remote(barp(BAR_PREADYP + b));
-                PROF(10);
-                TRACE(14, it);
             }
             if (stop) break;
-            TRACE(3, it);
             prev_valid = true; prev_no_split = w.no_split; prev_req = req; prev_split = w.split_idx;
             prev_last = it - 1; prev_m = m_run; prev_l = l_run; prev_x = x_max;
         }
@@ -807,9 +739,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) att
 #pragma unroll 1
         while (cur.have) {
             const uint32_t t_it = item / N_GROUPS, gw = item % N_GROUPS, ks = t_it % NK, slot = item % NR;
-            TRACE(60, t_it);
             ok = mbar_wait_hot(bar(BAR_RAWFULL + slot), (item / NR) & 1u, abort_flag, W_RAWFULL);
-            TRACE(61, t_it);
             if (!ok) break;
             const uint32_t vbits = __ballot_sync(0xffffffffu, cur.idx >= 0) & ((1u << RPW) - 1u);
             const uint2 sc8 = sc8_nxt;
@@ -851,7 +781,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) att
             const float s_half = __uint_as_float(max(__reduce_max_sync(0xffffffffu, __float_as_uint(wm)), MIN_SCALE_BITS));
             // the maximum needed the last shared-memory load of every lane (they return in order): the rows have left the slot
             if (lane == 0) mbar_arrive(bar(BAR_RAWEMPTY + slot));
-            TRACE(62, t_it);
             const float inv_half = __uint_as_float(0x7f000000u - __float_as_uint(s_half));
             const __nv_bfloat162 rope_f = __float2bfloat162_rn(inv_half);
             // V32: exponent shift of the block whose scale this lane loaded (row lane / 4, block lane % 4): 0 for a block at the scale.
@@ -861,7 +790,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) att
             const int bk = lane >> 2;                            // MODEL1: 64-value block of this lane's piece (0-6 in the lanes that store)
             if (t_it >= NK) ok = mbar_wait_hot(bar(BAR_KEMPTY + ks), ((t_it / NK) - 1) & 1u, abort_flag, W_KEMPTY);
             if (STAGE_Q && ok && t_it == NK - 1 && first_work) ok = mbar_wait_hot(bar(BAR_QFREE), 0u, abort_flag, W_QFREE);   // K stage 1 held Q until now
-            TRACE(63, t_it);
             if (!ok) break;
             uint8_t* kp = sm + KS_OFF + ks * KS_BYTES;
 #pragma unroll
@@ -902,14 +830,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) att
                 *reinterpret_cast<float4*>(rec) =
                     make_float4(s_half, (float)((int)(__float_as_uint(s_half) >> 23) - 127), inv_half, __uint_as_float(vbits));
             }
-            TRACE(64, t_it);
             fence_proxy_async();
             __syncwarp();
             if (lane == 0) {
                 mbar_arrive(bar(BAR_KSTORED + ks));
                 mbar_arrive_remote(barp(BAR_KFULLP + ks));
             }
-            TRACE(65, t_it);
             item += N_G_WARPS;
         }
     } else if (warp == MMA_WARP && rank == 0) {
@@ -926,17 +852,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) att
             ++rq;
             for (int j = 0; j < nst && ok; ++j, ++it) {
                 const uint32_t ks = it % NK, b = it & 1u;
-                PROF(0);
                 if (it >= 2) {
                     ok = mbar_wait_hot(bar(BAR_SFREEP + b), ((it - 2) >> 1) & 1u, abort_flag, W_SFREE);
                     if (!ok) break;
                 }
-                PROF(1);
                 ok = mbar_wait_hot(bar(BAR_KFULLP + ks), (it / NK) & 1u, abort_flag, W_KFULL);
                 if (!ok) break;
-                PROF(2);
                 tc_fence_after();
-                TRACE(40, it);
                 const uint32_t kb_lo = desc_lo(base + KS_OFF + ks * KS_BYTES, 16);
                 const uint32_t d = tmem + TM_S + 64 * b;
                 if (elect_one()) {
@@ -960,8 +882,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) att
                     tc_commit_pair(mapa_shared(bar(BAR_KEMPTY + ks), 1));
                 }
                 __syncwarp();
-                PROF(3);
-                TRACE(41, it);
             }
         }
     } else if (warp == MMA_WARP + 1 && rank == 0) {
@@ -974,16 +894,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) att
             const int nst = (w.nblk + 1) >> 1;
             for (int j = 0; j < nst && ok; ++j, ++it) {
                 const uint32_t vs = it % NV, b = it & 1u;
-                PROF(0);
                 ok = mbar_wait_hot(bar(BAR_PREADYP + b), (it >> 1) & 1u, abort_flag, W_PREADY);
                 if (!ok) break;
-                PROF(1);
-                TRACE(50, it);
                 ok = mbar_wait_hot(bar(BAR_VFULLP + vs), (it / NV) & 1u, abort_flag, W_VFULL);
                 if (!ok) break;
-                PROF(2);
                 tc_fence_after();
-                TRACE(51, it);
                 const uint32_t pa_lo = desc_lo(base + PB_OFF + b * CHUNK, 16);
                 const uint32_t vb_lo = desc_lo(base + VS_OFF + vs * VS_BYTES, VSLOT);
                 if (elect_one()) {
@@ -1001,8 +916,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) att
                     tc_commit_pair(mapa_shared(bar(BAR_PVDONE + b), 1));
                 }
                 __syncwarp();
-                PROF(3);
-                TRACE(52, it);
             }
         }
     } else if (warp == FWD_WARP) {
@@ -1022,10 +935,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) att
             const int nst = (w.nblk + 1) >> 1;
             for (int j = 0; j < nst && ok; ++j, ++it) {
                 const uint32_t ks = it % NK, vs = it % NV;
-                TRACE(70, it);
                 ok = mbar_wait_hot(bar(BAR_KSTORED + ks), (it / NK) & 1u, abort_flag, W_KSTORED);
                 if (!ok) break;
-                TRACE(71, it);
                 if (it >= NV) {
                     ok = mbar_wait_hot(bar(BAR_VEMPTY + vs), ((it / NV) - 1) & 1u, abort_flag, W_VEMPTY);
                     if (!ok) break;
@@ -1033,7 +944,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) att
                     ok = mbar_wait_hot(bar(BAR_QFREE), 0u, abort_flag, W_QFREE);
                     if (!ok) break;
                 }
-                TRACE(72, it);
                 if (elect_one()) {
                     mbar_arrive_expect_tx(bar(BAR_VFULL + vs), 4 * CHUNK);
 #pragma unroll
@@ -1047,10 +957,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) att
                     }
                 }
                 __syncwarp();
-                TRACE(73, it);
                 ok = mbar_wait_hot(bar(BAR_VFULL + vs), (it / NV) & 1u, abort_flag, W_VFULL_CTA);
                 if (!ok) break;
-                TRACE(74, it);
                 if (lane == 0) {
                     mbar_arrive_remote(barp(BAR_VFULLP + vs));
                     // the copies out of this CTA's K stage into its own slots and the partner's copies into them are done
@@ -1137,32 +1045,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) att
         tc_fence_after();
         tmem_dealloc_pair(tmem, TMEM_COLS);
     }
-    TRACE(5, 0);
-#ifdef SMLA_PROF
-    if (g_prof_buf != nullptr && (int)blockIdx.x == g_prof_block && lane == 0) {
-        g_prof_buf[warp * 2] = prof_acc;
-        g_prof_buf[warp * 2 + 1] = (unsigned)clock() - prof_start;
-    }
-#endif
 }
 
 }  // namespace
 
-#ifdef SMLA_TRACE
-extern "C" int smla_trace_set(long long* buf, int cap, int block) {
-    cudaMemcpyToSymbol(g_trace_buf, &buf, sizeof(buf));
-    cudaMemcpyToSymbol(g_trace_cap, &cap, sizeof(cap));
-    cudaMemcpyToSymbol(g_trace_block, &block, sizeof(block));
-    return (int)cudaGetLastError();
-}
-#endif
-#ifdef SMLA_PROF
-extern "C" int smla_prof_set(long long* buf, int block) {
-    cudaMemcpyToSymbol(g_prof_buf, &buf, sizeof(buf));
-    cudaMemcpyToSymbol(g_prof_block, &block, sizeof(block));
-    return (int)cudaGetLastError();
-}
-#endif
 
 namespace {
 

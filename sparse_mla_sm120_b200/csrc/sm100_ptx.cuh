@@ -34,16 +34,6 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity, uin
     (void)hint_ns;     // passing the hint as the instruction's time limit made waits on the critical path wake later
     return ok != 0;
 }
-// One non-blocking poll.
-__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-    return ok != 0;
-}
 
 // Warp-wide wait for the phase with the given parity.  Lane 0 polls (32 lanes polling one
 // mbarrier only add shared-memory traffic), the warp reconverges on the result.  The wait gives
@@ -138,26 +128,12 @@ __device__ __forceinline__ void st_global_v8(void* p, const uint32_t (&v)[8]) {
                  : "memory");
 }
 
-__device__ __forceinline__ void st_cluster_v4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
-    asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
-}
-__device__ __forceinline__ void st_cluster_f32(uint32_t addr, float v) {
-    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
-}
-// Arrive on a barrier of another CTA of the cluster; releases this thread's earlier writes to it.
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t remote_bar) {
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(remote_bar) : "memory");
-}
 // Arrive on a barrier given by its shared::cluster address (this CTA's or, through mapa_shared, another
 // CTA's) with the default CTA-scope release.  For signals that only say "my part is ready" about data
 // that stays inside this SM (shared-memory operands of a pair MMA, tensor memory): a cluster-scope
 // release makes every such arrive wait for a memory barrier (about a thousand cycles under load).
 __device__ __forceinline__ void mbar_arrive_remote(uint32_t cluster_bar) {
     asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
-}
-// Arrive on a barrier of another CTA and add `bytes` to its pending transaction count.
-__device__ __forceinline__ void mbar_arrive_expect_tx_cluster(uint32_t remote_bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.release.cluster.shared::cluster.b64 _, [%0], %1;" ::"r"(remote_bar), "r"(bytes) : "memory");
 }
 // Bulk copy from this CTA's shared memory into another CTA's (both 16-byte aligned, size a
 // multiple of 16); the destination CTA's barrier receives the byte count when the data has landed.
@@ -171,54 +147,7 @@ __device__ __forceinline__ void bulk_copy_g2s(uint32_t dst, unsigned long long s
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                  ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
 }
-// One poll with cluster-scope acquire: for barriers that another CTA arrives on after writing here.
-__device__ __forceinline__ bool mbar_try_wait_cluster(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-    return ok != 0;
-}
-// mbar_wait_hot with cluster-scope acquire.
-__device__ __forceinline__ bool mbar_wait_hot_cluster(uint32_t bar, uint32_t parity, volatile int* abort, int code) {
-    uint32_t ok = 0;
-    for (uint32_t i = 0; i < WAIT_POLLS; ++i) {
-        if (mbar_try_wait_cluster(bar, parity)) { ok = 1; break; }
-        if ((i & 255u) == 255u && *abort != 0) break;
-    }
-    if (!ok) atomicCAS(const_cast<int*>(abort), 0, code);
-    return __all_sync(0xffffffffu, ok != 0);
-}
-__device__ __forceinline__ bool mbar_wait_thread_cluster(uint32_t bar, uint32_t parity, volatile int* abort, int code) {
-    for (uint32_t i = 0; i < WAIT_POLLS; ++i) {
-        if (mbar_try_wait_cluster(bar, parity)) return true;
-        if ((i & 255u) == 255u && *abort != 0) return false;
-    }
-    atomicCAS(const_cast<int*>(abort), 0, code);
-    return false;
-}
 
-// Single-thread variant of mbar_wait (same bounds and give-up protocol), for a role that is run
-// by one lane only.
-__device__ __forceinline__ bool mbar_wait_thread(uint32_t bar, uint32_t parity, volatile int* abort, int code) {
-    for (uint32_t i = 0; i < WAIT_POLLS; ++i) {
-        if (mbar_try_wait(bar, parity, WAIT_HINT_NS)) return true;
-        if ((i & 255u) == 255u && *abort != 0) return false;
-    }
-    atomicCAS(const_cast<int*>(abort), 0, code);
-    return false;
-}
-
-// ------------------------------------------------------------------ cp.async (16-byte, L2 only)
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-}
-// Copies src_bytes (0 or 16) bytes and zero-fills the rest of the 16-byte destination.
-__device__ __forceinline__ void cp_async16_zfill(uint32_t dst, const void* src, uint32_t src_bytes) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(src_bytes) : "memory");
-}
 // ------------------------------------------------------------------ TMA (tiled bulk tensor copy)
 // Adds `bytes` to the barrier's pending transaction count and arrives once.
 __device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t bytes) {
@@ -238,17 +167,6 @@ __device__ __forceinline__ void tma_gather4(uint32_t dst, const void* tensor_map
                  ::"r"(dst), "l"(tensor_map), "r"(x), "r"(r0), "r"(r1), "r"(r2), "r"(r3), "r"(bar) : "memory");
 }
 
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
-// Arrives on the mbarrier (without adding to its pending count) once every cp.async issued so
-// far by this thread has landed.
-__device__ __forceinline__ void cp_async_arrive_noinc(uint32_t bar) {
-    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 // Makes generic-proxy writes to shared memory visible to the async proxy (tcgen05.mma operands).
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
@@ -338,12 +256,6 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16
           "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
         : "memory");
 }
-// 32 lanes x 8 columns: thread i of the warp writes 8 consecutive columns of its lane.
-__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8]) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
-                 ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
-                 : "memory");
-}
 
 // Register reallocation between warpgroups (all four warps of a warpgroup execute it together).
 template <int N> __device__ __forceinline__ void setmaxnreg_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
@@ -370,10 +282,6 @@ __device__ __forceinline__ bool named_bar_or(uint32_t id, uint32_t threads, bool
 // Shared-memory matrix descriptor of tcgen05.mma: start address, leading / stride byte offsets
 // (all in 16-byte units), descriptor version 1 (bits 46-47) and the swizzle mode (bits 61-63).
 enum : uint64_t { SWIZZLE_NONE = 0, SWIZZLE_128B = 2, SWIZZLE_64B = 4, SWIZZLE_32B = 6 };
-__device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo_bytes, uint32_t sbo_bytes, uint64_t swizzle) {
-    return (uint64_t)((addr >> 4) & 0x3fffu) | ((uint64_t)((lbo_bytes >> 4) & 0x3fffu) << 16) |
-           ((uint64_t)((sbo_bytes >> 4) & 0x3fffu) << 32) | (1ull << 46) | (swizzle << 61);
-}
 
 // Instruction descriptor: fp32 accumulator, operand formats, majorness, N >> 3, M >> 4.
 constexpr uint32_t FMT_F16 = 0, FMT_BF16 = 1, FMT_E4M3 = 0, FMT_E5M2 = 1;
@@ -405,14 +313,6 @@ __device__ __forceinline__ void mma_mxf8(uint32_t d_tmem, uint64_t a_desc, uint6
         "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %6, 0;\n\t"
         "tcgen05.mma.cta_group::1.kind::mxf8f6f4.block_scale.scale_vec::1X [%0], %1, %2, %3, [%4], [%5], p;\n\t}"
         ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(sfa_tmem), "r"(sfb_tmem), "r"((uint32_t)accumulate) : "memory");
-}
-
-// Same with the A operand read from tensor memory (lane = row, K packed along the columns).
-__device__ __forceinline__ void mma_f8_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, bool accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], [%1], %2, %3, p;\n\t}"
-        ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"((uint32_t)accumulate) : "memory");
 }
 
 // ------------------------------------------------------------------ CTA-pair forms (cta_group::2)
