@@ -650,7 +650,7 @@ def run_extras(device, hbm_peak, bf16_peak, peak_kind):
         exact_ms = _time_cuda(lambda: flash_ops.sparse_mla_decode_fwd(qm, pool1, im, 512 ** -0.5, impl=1), 3, warm=1)
         out["decode_model1"] = {"workload": "64 requests, h=128, topk=2048 over a MODEL1 cache (584 bytes per token, q 512 wide), "
                                             "262144-token pool; CUDA graph replay of the whole step on the tensor-core kernel "
-                                            "(impl=IMPL_TC; the default for this layout is the exact fp32 kernel)",
+                                            "(impl=IMPL_TC; the default for this layout is exact numerics, attn_exact_kernel, timed beside it)",
                                 "exact_fp32_kernel_us_per_step": exact_ms * 1e3, **res}
         # prefill of the C3 shape over the same layout: 4096 query tokens, causal top-k over 8192 rows
         pool_p = m1_pool(128)

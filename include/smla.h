@@ -52,7 +52,8 @@ const char* smla_status_string(int code);
 /* Kernel selection for the attention entry points. */
 enum {
     SMLA_IMPL_AUTO = 0,    /* tcgen05 kernel */
-    SMLA_IMPL_SCALAR = 1,  /* fp32 CUDA-core kernel: slow, exact; a second opinion in tests */
+    SMLA_IMPL_SCALAR = 1,  /* exact numerics: the fp32 CUDA-core kernel (slow; a second opinion in tests), or bf16 operands and fp32
+                              sums on the tensor cores for SMLA_LAYOUT_MODEL1 in 16-byte aligned caches */
     SMLA_IMPL_TC = 2       /* tcgen05/TMEM kernel on a pair of SMs (cta_group::2), FP8 QK^T and PV */
 };
 

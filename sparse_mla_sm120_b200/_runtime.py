@@ -122,7 +122,8 @@ def pick_num_sm_parts_fp32(num_tokens: int, num_heads: int, sms: int) -> int:
 
 
 # attn_exact_kernel (exact numerics over MODEL1, aligned caches): microseconds of a partition's fixed part (q, epilogue),
-# of a 128-token tile, and of what a split adds (scheduler and combine launches, partial records).
+# of a 128-token tile, and of what a split adds (scheduler and combine launches, partial records).  Estimates, not fitted: a tile
+# takes about 11000 cycles (5.6 us) in the kernel; what the rule needs is their proportion.
 _EXACT_US_FIXED, _EXACT_US_TILE, _EXACT_US_SPLIT = 6.0, 4.0, 9.0
 
 
@@ -210,7 +211,9 @@ def pick_split_tile(num_tokens: int, num_heads: int, sms: int, blocks_per_token:
     """(partitions, fixed overhead) for attn_tile_kernel, which runs one CTA per partition.  Requests of equal length are
     cut into as many equal partitions as pay off while all of them run at once.  Where no equal cut exists the rule is the
     general one: a partition that straddles two requests pays its fixed part twice, so that more of them, one per SM,
-    are slower than half as many (16 requests of top-k 2048: 34 us in 148 partitions, 28 us in 74)."""
+    are slower than half as many (ragged requests of top-k 2048, 16 heads: 16 of them 35 us in 148 partitions, 27 us in 74; 24: 35 and
+    30).  That rule leaves 37 and more requests whole: 64 of them take 42.5 us so, 44.3 in 111 partitions and 46.7 in 148; 48: 41.9,
+    41.2, 42.3; only near 37 is a cut better (39.7 whole, 35.2 in 74)."""
     n = max(blocks_per_token, 1)
     if not uniform:
         return pick_num_sm_parts(num_tokens, sms, blocks_per_token), FIXED_OVERHEAD

@@ -25,8 +25,8 @@
 // tokens, since the rows as bf16 leave no room for a second tile.  Shared memory is the resource: 96 MMAs at N = 64 read
 // 6 KB each (49 cycles, measured), the rows are another 128 KB written.  The conversion of the next tile therefore starts
 // as soon as P.V has read a quarter of this one, and its loads (which registers and L1 hold only in part) are sent ahead by
-// an L2 prefetch two tiles away.  32 requests of 128 heads, up to 1024 entries and a second cache of 128: 48 us; the
-// CUDA-core kernel that served this layout before took 2034 us.
+// an L2 prefetch two tiles away.  32 requests of 128 heads, up to 1024 entries and a second cache of 128: 51 us; the
+// CUDA-core kernel that served this layout before took 1924 us.
 // Every wait is bounded; a wait that gives up records a code in status[] and the CTA drains and exits.
 #include "attn_common.cuh"
 #include "sm100_ptx.cuh"
