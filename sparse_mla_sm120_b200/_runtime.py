@@ -224,6 +224,34 @@ def pick_split_tile(num_tokens: int, num_heads: int, sms: int, blocks_per_token:
     return (num_tokens, FIXED_OVERHEAD) if k == 1 else (k * num_tokens, 0)
 
 
+# attn_duo_kernel (65 to 128 heads over one linear array of rows): microseconds of a partition's fixed part, of a 128-token tile (more
+# when many pairs of SMs share the memory), and of what a split adds per piece of a request and per record.  Fitted to 1 to 64
+# requests of top-k 2048, 1024 and 512 in 1 to 16 equal partitions each, rows in HBM (one of 2048: 37.3, 28.2, 22.9, 22.8 and 24.9 us
+# in 1, 2, 4, 8 and 16; 16: 39.3, 31.0, 27.8 in 1, 2, 4; 32: 39.9, 35.1; 64 whole 47.0); the cut that it names is the fastest measured
+# one or within a microsecond of it.
+def _duo_us(num_tokens: int, blocks: int, k: int, max_pairs: int) -> float:
+    pairs = min(k * num_tokens, max_pairs)
+    t = -(-num_tokens // max_pairs) * (12.3 + -(-(blocks // k) // 2) * (1.6 + 0.009 * max(pairs - 8, 0)))
+    return t if k == 1 else t + 3.0 + 0.5 * k + 0.03 * k * num_tokens
+
+
+def pick_split_duo(num_tokens: int, sms: int, blocks_per_token: int, uniform: bool) -> Tuple[int, int]:
+    """(partitions, fixed overhead) where whole requests and equal partitions run on attn_duo_kernel and partitions of the
+    scheduler on the pair kernel.  Ragged requests are left whole where the scheduler and combine launches and the partitions that
+    straddle two requests cost more than the longest request: lists of up to 16 blocks (8 of up to 1024 entries 22.9 us whole, 26.9
+    cut; of up to 2048 33.0 and 29.0), and from a third of the pairs on (24 of up to 2048: 39.0 whole, 46.3 cut; 20: 39.2 and 35.1)."""
+    n = max(blocks_per_token, 1)
+    max_pairs = max(sms // CTAS_PER_PART, 1)
+    whole = (num_tokens, FIXED_OVERHEAD)
+    cuts = [k for k in range(2, n // 2 + 1) if n % k == 0 and k * num_tokens <= max_pairs]
+    if uniform and (cuts or n < 2 * BLOCKS_PER_PARTITION):
+        k = min([1] + cuts, key=lambda c: _duo_us(num_tokens, n, c, max_pairs))
+        return whole if k == 1 else (k * num_tokens, 0)
+    if n <= 16 or 3 * num_tokens >= max_pairs - 2:
+        return whole
+    return pick_num_sm_parts(num_tokens, sms, blocks_per_token), FIXED_OVERHEAD
+
+
 def split_plan(device: int, num_tokens: int, num_heads: int, blocks: int, uniform: int, layout: int, ext: int, aligned: int,
                impl: int) -> Tuple[int, int, int]:
     """(partitions, the scheduler's fixed overhead, equal partitions per request) of a decode step: the one choice that
@@ -239,6 +267,8 @@ def split_plan(device: int, num_tokens: int, num_heads: int, blocks: int, unifor
         return pick_num_sm_parts_fp32(num_tokens, num_heads, sms), FIXED_OVERHEAD, 0
     if not ext and aligned and num_heads <= 64 and impl != _lib.IMPL_SCALAR:
         parts, overhead = pick_split_tile(num_tokens, num_heads, sms, blocks, bool(uniform))
+    elif not ext and aligned and impl != _lib.IMPL_SCALAR:
+        parts, overhead = pick_split_duo(num_tokens, sms, blocks, bool(uniform))
     else:
         parts, overhead = pick_split(num_tokens, sms, blocks, uniform=bool(uniform))
     k = parts // num_tokens

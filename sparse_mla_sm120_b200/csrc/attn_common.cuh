@@ -75,6 +75,31 @@ __device__ __forceinline__ int fetch_entry(const AttnParams& p, const Work& w, i
     return pos < w.extra_len ? __ldg(p.extra_indices + (size_t)w.req * p.extra_topk + pos) : -1;
 }
 
+// The requests of a CTA and their tiles, in the order in which every role walks them.
+struct Tiles {
+    Work w;
+    int req, step, last, j, nst;
+    __device__ __forceinline__ Tiles(int first, int step_, int last_) : req(first - step_), step(step_), last(last_), j(0), nst(0) {}
+    __device__ __forceinline__ bool next_request(const AttnParams& p, const SchedMeta& m) {
+        do {
+            if (req + step > last) return false;
+            req += step;
+        } while (!get_work(p, m, req, w));
+        nst = (w.nblk + 1) >> 1;
+        j = 0;
+        return true;
+    }
+    __device__ __forceinline__ bool next_tile(const AttnParams& p, const SchedMeta& m) {
+        if (++j < nst) return true;
+        return next_request(p, m);
+    }
+    // Row r of the current tile: its index in the cache, -1 where there is no entry.
+    __device__ __forceinline__ int row_index(const AttnParams& p, int r) const {
+        const int pos = (w.blk0 + 2 * j) * BLOCK_N + r, lim = min(w.len, (w.blk0 + w.nblk) * BLOCK_N);
+        return pos < lim ? __ldg(p.indices + (size_t)w.req * p.topk + pos) : -1;
+    }
+};
+
 // Smallest scale of a row, as a biased exponent: smaller ones (a zero-filled row has scales of 0) are taken for it.  The
 // denominator divides weights of up to 2^8 by the scale, and 2^95 times any number of rows is finite; what such a row
 // itself holds stays far below anything that matters (448 * 2^-87), and its weight is that of its logit.
@@ -104,10 +129,11 @@ __device__ __forceinline__ uint32_t pack_e4m3x4(float a, float b, float c, float
 // below 2^-6 is cut to the subnormal grid or to zero (off by at most 2^-7, i.e. 2^-15 of the largest
 // e4m3 value), which is far below the rounding step of the values that dominate a row.
 __device__ __forceinline__ uint32_t shift_down_e4m3x4(uint32_t w, uint32_t sub) {
-    const uint32_t t = ((w & 0x7f7f7f7fu) | 0x80808080u) - sub;   // bit 7 of a byte survives iff its magnitude >= sub
+    const uint32_t n = ~w & 0x80808080u;                           // w + n sets bit 7 of every byte: it survives iff the magnitude is >= sub
+    const uint32_t t = w + n - sub;
     uint32_t keep;                                                 // every byte's bit 7 spread over the byte: 0xff where no underflow
     asm("prmt.b32 %0, %1, %1, 0xba98;" : "=r"(keep) : "r"(t));     // (selector bit 3 = replicate the sign of the chosen byte)
-    return (t & 0x7f7f7f7fu & keep) | (w & 0x80808080u);
+    return (t & keep) ^ n;                                         // gives the sign back (a value that underflowed is a zero of either sign)
 }
 // d * 8 in every byte for a ratio 2^-d (a power of two <= 1).
 __device__ __forceinline__ uint32_t shift_bytes_of_ratio(float ratio) {

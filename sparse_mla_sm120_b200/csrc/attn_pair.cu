@@ -1094,6 +1094,7 @@ bool attn_pair_takes(const AttnParams& p) {
 int launch_attn_pair(const AttnParams& p, cudaStream_t stream) {
     if (p.num_tokens == 0) return 0;
     if (attn_tile_takes(p)) return launch_attn_tile(p, stream);
+    if (attn_duo_takes(p)) return launch_attn_duo(p, stream);
     // Staging of the first request's Q only where the kernel follows the scheduler (see STAGE_Q).
     const bool stage = p.sched != nullptr || p.uniform_k > 1;      // short partitions
     if (p.layout == SMLA_LAYOUT_MODEL1) {

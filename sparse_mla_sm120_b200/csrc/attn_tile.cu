@@ -45,9 +45,8 @@
 //   warps 12-15  scales: the rows' scale words into tensor memory (each warp the 32 lanes it can reach) and shared memory.
 //   warp 16      issues the score MMAs, warp 17 the P.V MMAs (one elected lane each).
 // Every wait is bounded; a wait that gives up records a code in status[] and the CTA drains and exits.
-#include <cuda.h>
-
 #include "attn_common.cuh"
+#include "rows_map.cuh"
 #include "sm100_ptx.cuh"
 
 namespace smla {
@@ -102,7 +101,6 @@ __host__ __device__ constexpr uint32_t idesc_mx(uint32_t a_byte) {
 constexpr uint32_t IDESC_ROPE = instr_desc(FMT_BF16, FMT_BF16, false, false, T_TILE, T_HEADS);
 constexpr uint32_t IDESC_PV = instr_desc(FMT_E4M3, FMT_E4M3, true, true, 128, T_HEADS);
 constexpr uint32_t HI_128 = desc_hi(1024, (uint32_t)SWIZZLE_128B), HI_P = desc_hi(512, (uint32_t)SWIZZLE_64B);
-constexpr int NO_ROW = 0x7fffffff;             // outside the tensor map: arrives as zeros
 
 enum { WT_KFULL = 51, WT_RFULL = 52, WT_KFREE = 53, WT_SREADY = 54, WT_SFREE = 55, WT_SCALES = 56, WT_PREADY = 57, WT_PVDONE = 58, WT_QREADY = 59 };
 
@@ -119,31 +117,6 @@ __device__ __forceinline__ float lanes_max(float v) {
 // exponent of the group of eight tokens (a byte per block, at most NO_SHIFT), and e_g itself (biased; 0: no entry).
 struct TokenScale { uint32_t below, e_g; };
 constexpr uint32_t NO_SHIFT = 0x7fu;
-
-// The requests of a CTA and their tiles, in the order in which every role walks them.
-struct Tiles {
-    Work w;
-    int req, step, last, j, nst;
-    __device__ __forceinline__ Tiles(const SchedMeta& m, int first, int step_, int last_) : req(first - step_), step(step_), last(last_), j(0), nst(0) {}
-    __device__ __forceinline__ bool next_request(const AttnParams& p, const SchedMeta& m) {
-        do {
-            if (req + step > last) return false;
-            req += step;
-        } while (!get_work(p, m, req, w));
-        nst = (w.nblk + 1) >> 1;
-        j = 0;
-        return true;
-    }
-    __device__ __forceinline__ bool next_tile(const AttnParams& p, const SchedMeta& m) {
-        if (++j < nst) return true;
-        return next_request(p, m);
-    }
-    // Row r of the current tile: its index in the cache, -1 where there is no entry.
-    __device__ __forceinline__ int row_index(const AttnParams& p, int r) const {
-        const int pos = (w.blk0 + 2 * j) * BLOCK_N + r, lim = min(w.len, (w.blk0 + w.nblk) * BLOCK_N);
-        return pos < lim ? __ldg(p.indices + (size_t)w.req * p.topk + pos) : -1;
-    }
-};
 
 template <bool MAXL>
 __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParams p, const __grid_constant__ CUtensorMap kv_map) {
@@ -209,7 +182,7 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
         // logits in log2 units are scores times a positive number: the sign of the softmax scale goes into q
         const float c = fabsf(p.sm_scale) * LOG2E;
         const uint32_t scale_sign = __float_as_uint(p.sm_scale) & 0x80000000u;
-        Tiles tiles(meta, first, step, last);
+        Tiles tiles(first, step, last);
         uint32_t it = 0;
         bool dead = false;
         bool prev = false, prev_no_split = false;          // a request's epilogue runs after the next request's Q phase
@@ -546,7 +519,7 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
     } else if (warp < T_SCALE) {
         // =================================================================== rows -> K stages (TMA gather)
         const int quarter = warp - T_PROD;
-        Tiles tiles(meta, first, step, last);
+        Tiles tiles(first, step, last);
         bool have = tiles.next_tile(p, meta), ok = true;
         int idx = have ? tiles.row_index(p, quarter * 32 + lane) : -1;
         for (uint32_t it = 0; have; ++it) {
@@ -590,7 +563,7 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
         // The next tile's scales are asked for when this tile's words have been handed over, and looked at a tile later.
         const int quarter = warp - T_SCALE;
         const uint32_t lane_addr = tmem + ((uint32_t)(quarter * 32) << 16);
-        Tiles tiles(meta, first, step, last);
+        Tiles tiles(first, step, last);
         bool have = tiles.next_tile(p, meta), ok = true;
         int idx[4];
         uint4 sc[4];
@@ -650,7 +623,7 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
     } else if (warp == T_QK) {
         // =================================================================== score MMAs
         const uint32_t q_lo = desc_lo(base + Q_OFF, 16), qr_lo = desc_lo(base + QR_OFF, 16), r_lo = desc_lo(base + R_OFF, 16);
-        Tiles tiles(meta, first, step, last);
+        Tiles tiles(first, step, last);
         uint32_t it = 0, rq = 0;
         bool ok = true;
         while (ok && tiles.next_request(p, meta)) {
@@ -687,7 +660,7 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
         }
     } else if (warp == T_PV) {
         // =================================================================== P.V MMAs
-        Tiles tiles(meta, first, step, last);
+        Tiles tiles(first, step, last);
         const uint32_t p_lo = desc_lo(base + P_OFF, 16);
         uint32_t it = 0;
         bool ok = true;
@@ -728,9 +701,6 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
     if (warp == T_QK) { tc_fence_after(); tmem_dealloc(tmem, 512); }
 }
 
-typedef CUresult (*EncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
-                             const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
 }  // namespace
 
 // Whole requests that each get a pair of SMs to themselves take as long as one request does, and two CTAs walk a long list
@@ -749,24 +719,17 @@ static bool pair_is_faster(const AttnParams& p) {
 
 // One linear array of 656-byte rows (pages without padding between them) and one CTA's worth of heads.
 bool attn_tile_takes(const AttnParams& p) {
-    return !pair_is_faster(p) && p.num_heads <= T_HEADS && p.layout == SMLA_LAYOUT_V32 && p.extra_topk == 0 && p.block_stride == (int64_t)p.page_block_size * ROW_BYTES &&
-           (reinterpret_cast<uintptr_t>(p.kv) & 15u) == 0;
+    return !pair_is_faster(p) && p.num_heads <= T_HEADS && one_linear_array(p);
 }
 
 int launch_attn_tile(const AttnParams& p, cudaStream_t stream) {
     if (p.num_tokens == 0) return 0;
     static std::atomic<bool> attr_set[64];
     static int sm_count[64] = {};
-    static std::atomic<EncodeFn> encode{nullptr};
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64) return set_error(SMLA_E_SHAPE, "attn_tile_kernel: device ordinal %d not supported", dev);
     if (!attr_set[dev]) {
-        cudaDriverEntryPointQueryResult qres;
-        void* fn = nullptr;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &qres) != cudaSuccess || fn == nullptr)
-            return set_error(SMLA_E_DEVICE, "attn_tile_kernel: the driver has no cuTensorMapEncodeTiled");
-        encode = (EncodeFn)fn;
         cudaFuncAttributes fa[2];
         if (cudaFuncGetAttributes(&fa[0], attn_tile_kernel<false>) != cudaSuccess || cudaFuncGetAttributes(&fa[1], attn_tile_kernel<true>) != cudaSuccess ||
             fa[0].numRegs != T_REGS_LAUNCH || fa[1].numRegs != T_REGS_LAUNCH)
@@ -778,13 +741,8 @@ int launch_attn_tile(const AttnParams& p, cudaStream_t stream) {
         cudaDeviceGetAttribute(&sm_count[dev], cudaDevAttrMultiProcessorCount, dev);
         attr_set[dev] = true;
     }
-    // the cache as 32-bit words, 164 per row; boxes of 32 words (128 bytes) of one row
     CUtensorMap map;
-    const cuuint64_t dims[2] = {ROW_BYTES / 4, (cuuint64_t)NO_ROW}, strides[1] = {ROW_BYTES};
-    const cuuint32_t box[2] = {32, 1}, estr[2] = {1, 1};
-    const CUresult r = encode.load()(&map, CU_TENSOR_MAP_DATA_TYPE_INT32, 2, const_cast<uint8_t*>(p.kv), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return set_error(SMLA_E_DEVICE, "attn_tile_kernel: cuTensorMapEncodeTiled failed (%d)", (int)r);
+    if (int e = rows_tensor_map(p.kv, &map)) return e;
     const int parts = p.sched ? p.num_parts : p.uniform_k > 1 ? p.uniform_k * p.num_tokens : (p.num_tokens < sm_count[dev] ? p.num_tokens : sm_count[dev]);
     const dim3 grid(parts);
     auto* kernel = p.out_max_logits != nullptr ? attn_tile_kernel<true> : attn_tile_kernel<false>;

@@ -134,6 +134,8 @@ int launch_attn_scalar(const AttnParams& p, cudaStream_t stream);
 int launch_attn_pair(const AttnParams& p, cudaStream_t stream);
 bool attn_tile_takes(const AttnParams& p);   // 656-byte rows, one cache, pages without padding
 int launch_attn_tile(const AttnParams& p, cudaStream_t stream);
+bool attn_duo_takes(const AttnParams& p);    // the same caches, the calls that attn_tile leaves
+int launch_attn_duo(const AttnParams& p, cudaStream_t stream);
 int launch_attn_exact(const AttnParams& p, cudaStream_t stream);   // MODEL1 layout, caches aligned as for the pair kernel
 bool attn_pair_takes(const AttnParams& p);   // alignment of the caches that the tensor-core kernel's bulk copies need
 int launch_pack_kv(const __nv_bfloat16* kv, uint8_t* packed, int64_t num_rows, cudaStream_t stream);

@@ -35,6 +35,13 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity, uin
     return ok != 0;
 }
 
+// Has the phase with the given parity completed?  Never suspends.
+__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    return ok != 0;
+}
+
 // Warp-wide wait for the phase with the given parity.  Lane 0 polls (32 lanes polling one
 // mbarrier only add shared-memory traffic), the warp reconverges on the result.  The wait gives
 // up after a bounded number of polls (about half a second) or as soon as another thread of the
@@ -69,6 +76,20 @@ __device__ __forceinline__ bool mbar_wait_hot(uint32_t bar, uint32_t parity, vol
         if ((i & 255u) == 255u && *abort != 0) break;
     }
     if (!ok) atomicCAS(const_cast<int*>(abort), 0, code);
+    return __all_sync(0xffffffffu, ok != 0);
+}
+
+// The same in as few instructions as it can have, for a kernel whose roles together are larger than the instruction caches: at
+// most 2^20 polls (of up to 4 us each), then `code` goes to the abort flag (given by its shared-memory address).
+__device__ __forceinline__ bool mbar_wait_lean(uint32_t bar, uint32_t parity, uint32_t abort_addr, int code) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t.reg .u32 n;\n\tmov.u32 n, 0x100000;\n"
+        "POLL:\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t@p bra DONE;\n\t"
+        "add.u32 n, n, -1;\n\tsetp.ne.u32 q, n, 0;\n\t@q bra POLL;\n\t"
+        "st.volatile.shared.u32 [%3], %4;\n"
+        "DONE:\n\tselp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok) : "r"(bar), "r"(parity), "r"(abort_addr), "r"(code) : "memory");
     return __all_sync(0xffffffffu, ok != 0);
 }
 
@@ -354,6 +375,17 @@ __device__ __forceinline__ void mma_pair_f16(uint32_t d_tmem, uint64_t a_desc, u
         "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
         ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"((uint32_t)accumulate) : "memory");
+}
+
+// The block-scaled form over the pair.  Every lane quarter reads the words of B's rows from its own lanes, and as lanes 0-63 hold
+// columns [0, N/2) of D and lanes 64-127 the rest, quarters 0 and 1 want the words of rows [0, N/2) and quarters 2 and 3 those of
+// rows [N/2, N) (row r of its half: lane r % 32, column r / 32), in both CTAs.
+__device__ __forceinline__ void mma_pair_mxf8(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t sfa_tmem, uint32_t sfb_tmem,
+                                              bool accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %6, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::mxf8f6f4.block_scale.scale_vec::1X [%0], %1, %2, %3, [%4], [%5], p;\n\t}"
+        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(sfa_tmem), "r"(sfb_tmem), "r"((uint32_t)accumulate) : "memory");
 }
 
 // Descriptor halves for operands whose address changes while everything else stays fixed:

@@ -1,0 +1,24 @@
+"""pick_split_duo (65 to 128 heads over one linear array of rows): cuts that the library accepts, and the two sides of each line."""
+import pytest
+
+from sparse_mla_sm120_b200._runtime import FIXED_OVERHEAD, pick_split_duo
+
+
+@pytest.mark.parametrize("blocks", [1, 2, 3, 4, 7, 8, 16, 17, 24, 32, 64])
+def test_equal_cuts_divide_the_blocks_and_fit_the_machine(blocks):
+    for tokens in (1, 2, 5, 16, 37, 38, 64, 74, 75, 300):
+        parts, overhead = pick_split_duo(tokens, 148, blocks, True)
+        assert parts >= tokens
+        if overhead == 0:
+            k = parts // tokens
+            assert k > 1 and k * tokens == parts <= 74 and blocks % k == 0 and blocks // k >= 2
+        else:
+            assert overhead == FIXED_OVERHEAD
+
+
+def test_ragged_requests():
+    assert pick_split_duo(8, 148, 16, False) == (8, FIXED_OVERHEAD)          # short lists stay whole
+    assert pick_split_duo(8, 148, 17, False)[0] > 8
+    assert pick_split_duo(23, 148, 32, False)[0] > 23
+    assert pick_split_duo(24, 148, 32, False) == (24, FIXED_OVERHEAD)        # a third of the pairs
+    assert pick_split_duo(1, 148, 32, True) == (8, 0) and pick_split_duo(64, 148, 32, True) == (64, FIXED_OVERHEAD)
