@@ -75,17 +75,31 @@ __device__ __forceinline__ int fetch_entry(const AttnParams& p, const Work& w, i
     return pos < w.extra_len ? __ldg(p.extra_indices + (size_t)w.req * p.extra_topk + pos) : -1;
 }
 
-// The requests of a CTA and their tiles, in the order in which every role walks them.
-struct Tiles {
-    Work w;
+constexpr int TILE_N = 128;   // tokens per tile of the kernels that gather by TMA: two scheduler blocks
+
+// The requests of a CTA and their tiles, in the order in which every role walks them, for calls over one cache.  (Every role has a walker: it
+// holds what they all need and no more, code being what these kernels wait for.)
+struct Walk {
     int req, step, last, j, nst;
-    __device__ __forceinline__ Tiles(int first, int step_, int last_) : req(first - step_), step(step_), last(last_), j(0), nst(0) {}
+    int pos0, lim;         // positions of the current request's share: its first one and the end
+    int next_len;          // of the request after this one, asked for a request ahead
+    __device__ __forceinline__ Walk(const AttnParams& p, int first, int step_, int last_) : req(first - step_), step(step_), last(last_), j(0), nst(0) {
+        next_len = first <= last_ ? length(p, first) : 0;
+    }
+    __device__ __forceinline__ static int length(const AttnParams& p, int r) { return p.topk_length ? __ldg(p.topk_length + r) : p.topk; }
     __device__ __forceinline__ bool next_request(const AttnParams& p, const SchedMeta& m) {
+        int b0, b1;
         do {
             if (req + step > last) return false;
             req += step;
-        } while (!get_work(p, m, req, w));
-        nst = (w.nblk + 1) >> 1;
+            const int len = min(next_len, p.topk), blocks = max((len + BLOCK_N - 1) / BLOCK_N, 1);
+            if (req + step <= last) next_len = length(p, req + step);
+            b0 = req == m.begin_req ? m.begin_block : 0;
+            b1 = min(req == m.end_req ? m.end_block : blocks, blocks);
+            pos0 = b0 * BLOCK_N;
+            lim = min(len, b1 * BLOCK_N);
+        } while (b1 <= b0);
+        nst = (b1 - b0 + 1) >> 1;
         j = 0;
         return true;
     }
@@ -95,8 +109,8 @@ struct Tiles {
     }
     // Row r of the current tile: its index in the cache, -1 where there is no entry.
     __device__ __forceinline__ int row_index(const AttnParams& p, int r) const {
-        const int pos = (w.blk0 + 2 * j) * BLOCK_N + r, lim = min(w.len, (w.blk0 + w.nblk) * BLOCK_N);
-        return pos < lim ? __ldg(p.indices + (size_t)w.req * p.topk + pos) : -1;
+        const int pos = pos0 + j * TILE_N + r;
+        return pos < lim ? __ldg(p.indices + (size_t)req * p.topk + pos) : -1;
     }
 };
 

@@ -55,7 +55,7 @@ constexpr int DUO_THREADS = 32 * 32;
 constexpr int REGS_LAUNCH = 64, REGS_SOFTMAX = 88, REGS_AUX = 80, REGS_COPY = 40, REGS_FIX = 48;
 static_assert((N_SM_WARPS * REGS_SOFTMAX + N_AUX_WARPS * REGS_AUX + 8 * REGS_COPY + N_FIX_WARPS * REGS_FIX) * 32 <= DUO_THREADS * REGS_LAUNCH, "register budgets exceed what the CTA owns");
 
-constexpr int TILE_N = 128, OWN_N = 64;  // tokens per tile: two scheduler blocks, 64 rows of K gathered by each CTA
+constexpr int OWN_N = 64;                // rows of K that each CTA gathers of a tile
 constexpr int P_SHIFT = 5;               // P' is stored as e4m3(P' * 2^P_SHIFT)
 constexpr float RESCALE_TAU = 3.0f;      // lazy-rescale threshold (log2 units); P' <= 2^TAU
 constexpr int NST = 2;                   // K stages, score buffers and P' buffers follow the tile's parity
@@ -77,7 +77,8 @@ constexpr uint32_t GRP_BYTES = TILE_N / 8 * 4;
 constexpr uint32_t IDX_OFF = GRP_OFF + REC_RING * GRP_BYTES;  // the rows that a gathering warp is about to ask for, 32 each
 constexpr uint32_t FIX_OFF = IDX_OFF + 6 * 32 * 4;      // the V pieces that a warp is about to shift
 constexpr uint32_t FIX_LIST = 48;
-constexpr uint32_t XCH_OFF = FIX_OFF + N_FIX_WARPS * FIX_LIST * 4;       // row-maximum exchange [4][64] fp32
+constexpr uint32_t WORD_OFF = FIX_OFF + N_FIX_WARPS * FIX_LIST * 4;    // the rows' scale words on their way to tensor memory: [2][128]
+constexpr uint32_t XCH_OFF = WORD_OFF + 2 * TILE_N * 4;       // row-maximum exchange [4][64] fp32
 constexpr int REQ_RING = 4;                                   // requests that the roles may be apart
 constexpr uint32_t SQ_OFF = XCH_OFF + 4 * 64 * 4;             // exponents of the heads' q scales, [REQ_RING][64] bytes
 constexpr uint32_t SUM_OFF = SQ_OFF + REQ_RING * 64;          // a finished request's sums: [2] x ([4][64] denominators, [4][64] maxima, [64] m)
@@ -105,51 +106,14 @@ constexpr uint32_t IDESC_ROPE = instr_desc(FMT_BF16, FMT_BF16, false, false, 128
 constexpr uint32_t IDESC_PV = instr_desc(FMT_E4M3, FMT_E4M3, false, true, 128, 256);
 constexpr uint32_t HI_128 = desc_hi(1024, (uint32_t)SWIZZLE_128B);
 
-// Named barriers: softmax warps of 32 heads (two), the warps that share the first q.
-enum { NB_SOFTMAX = 1, NB_FIRST_Q = 4 };
+// Named barriers: softmax warps of 32 heads (two), the warps that share the first q, those that hand over the scales.
+enum { NB_SOFTMAX = 1, NB_FIRST_Q = 4, NB_SCALE = 5 };
 
 // give-up codes reported through status[0]
 enum { WD_KFULL = 71, WD_KPEER = 72, WD_VFULL = 73, WD_VREADY = 74, WD_SCALES = 75, WD_SREADY = 76, WD_SFREE = 77, WD_PREADY = 78, WD_PVDONE = 79, WD_QREADY = 80,
        WD_QSCALE = 81, WD_SUMS = 82, WD_OFREE = 83, WD_QFREE = 84, WD_VFREE = 85, WD_SUMFREE = 86, WD_QPART = 87 };
 
 __device__ __forceinline__ uint32_t swz(uint32_t row, uint32_t piece) { return row * 128u + ((piece ^ (row & 7u)) << 4); }
-
-// The requests of a CTA and their tiles, in the order in which every role walks them.  (A walker of its own: every role has one,
-// and code that this kernel does not need is code that the others wait for.)
-struct Walk {
-    int req, step, last, j, nst;
-    int pos0, lim;         // positions of the current request's share: its first one and the end
-    int next_len;          // of the request after this one, asked for a request ahead
-    __device__ __forceinline__ Walk(const AttnParams& p, int first, int step_, int last_) : req(first - step_), step(step_), last(last_), j(0), nst(0) {
-        next_len = first <= last_ ? length(p, first) : 0;
-    }
-    __device__ __forceinline__ static int length(const AttnParams& p, int r) { return p.topk_length ? __ldg(p.topk_length + r) : p.topk; }
-    __device__ __forceinline__ bool next_request(const AttnParams& p, const SchedMeta& m) {
-        int b0, b1;
-        do {
-            if (req + step > last) return false;
-            req += step;
-            const int len = min(next_len, p.topk), blocks = max((len + BLOCK_N - 1) / BLOCK_N, 1);
-            if (req + step <= last) next_len = length(p, req + step);
-            b0 = req == m.begin_req ? m.begin_block : 0;
-            b1 = min(req == m.end_req ? m.end_block : blocks, blocks);
-            pos0 = b0 * BLOCK_N;
-            lim = min(len, b1 * BLOCK_N);
-        } while (b1 <= b0);
-        nst = (b1 - b0 + 1) >> 1;
-        j = 0;
-        return true;
-    }
-    __device__ __forceinline__ bool next_tile(const AttnParams& p, const SchedMeta& m) {
-        if (++j < nst) return true;
-        return next_request(p, m);
-    }
-    // Row r of the current tile: its index in the cache, -1 where there is no entry.
-    __device__ __forceinline__ int row_index(const AttnParams& p, int r) const {
-        const int pos = pos0 + j * TILE_N + r;
-        return pos < lim ? __ldg(p.indices + (size_t)req * p.topk + pos) : -1;
-    }
-};
 
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(DUO_THREADS, 1) attn_duo_kernel(const AttnParams p, const __grid_constant__ CUtensorMap kv_map) {
     extern __shared__ uint8_t smem_raw[];
@@ -418,7 +382,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(DUO_THREADS, 1) attn
         // under the first scores and weights of the next.
         // Scales: a pair MMA with M = 128 leaves the scores of tokens 0-63 in lanes 0-63 and those of tokens 64-127 in lanes 64-127,
         // and every lane quarter takes the tokens' scale words from its own lanes: column c of lane i of quarter q holds the word
-        // of token 64 (q / 2) + 32 c + i.  The next tile's scales are asked for when this tile's words have been handed over.
+        // of token 64 (q / 2) + 32 c + i; a warp makes the words of tokens 32 q + i and passes them on.  The next tile's scales are asked for when this tile's words have been handed over.
         const bool scaler = warp < QUANT_WARP0;
         const int quarter = warp & 3, ch = scaler ? 0 : 1;
         const int grp = quarter & 1, thalf = quarter >> 1, hrow = grp * 32 + lane, head = head0 + hrow;
@@ -470,9 +434,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(DUO_THREADS, 1) attn
         bool ok = true;
         Walk ahead(p, first, step, last);                 // the tile whose rows are named next
         uint32_t sit = 0, primed = 0;                     // number of the next tile to hand over; stages of the read-ahead that are filled
-        int idx[2] = {-1, -1};
-        uint4 sc[2];
-        uint32_t there = 0u;
+        int idx = -1;
+        uint4 sc = make_uint4(0u, 0u, 0u, 0u);
+        bool there = false;
+        uint32_t* words = reinterpret_cast<uint32_t*>(sm + WORD_OFF);
         if (scaler) {
             const uint32_t ones[4] = {0x7f7f7f7fu, 0x7f7f7f7fu, 0x7f7f7f7fu, 0x7f7f7f7fu};
             tmem_st4(lane_addr + TM_SFA, ones);           // the heads' scales stay outside the MMAs
@@ -480,6 +445,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(DUO_THREADS, 1) attn
         Walk tiles(p, first, step, last);
         uint32_t it = 0, rq = 0;                          // first tile and number of the request
         const bool whole = p.uniform_k <= 1;              // requests are not cut
+        bool together = false;                            // the scalers leave because one of them has given up, and all know it
         bool prev = false;
         int prev_req = 0, last_nst = 0;
         while (true) {
@@ -503,16 +469,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(DUO_THREADS, 1) attn
                     filling = primed < 2;
                     if (!filling) {
                         const uint32_t ring = sit & (REC_RING - 1), b = sit & 1u;
-                        uint32_t word[2], mx[2];
-#pragma unroll
-                        for (int k = 0; k < 2; ++k) {
-                            auto bits = [](uint32_t v) { return max(v, MIN_SCALE_BITS) << 1; };         // the exponent is the upper byte
-                            const uint32_t lo = __byte_perm(bits(sc[k].x), bits(sc[k].y), 0x0073), hi = __byte_perm(bits(sc[k].z), bits(sc[k].w), 0x0073);
-                            word[k] = (there >> k) & 1u ? __byte_perm(lo, hi, 0x5410) : 0u;
-                            mx[k] = (there >> k) & 1u ? word[k] : 0x7f7f7f7fu;
-                        }
-                        const uint32_t mine = grp ? word[1] : word[0];
-                        const uint32_t valid = __ballot_sync(0xffffffffu, (there >> grp) & 1u);
+                        auto bits = [](uint32_t v) { return max(v, MIN_SCALE_BITS) << 1; };             // the exponent is the upper byte
+                        const uint32_t lo = __byte_perm(bits(sc.x), bits(sc.y), 0x0073), hi = __byte_perm(bits(sc.z), bits(sc.w), 0x0073);
+                        const uint32_t mine = there ? __byte_perm(lo, hi, 0x5410) : 0u;
+                        words[b * TILE_N + 32 * quarter + lane] = there ? mine : 0x7f7f7f7fu;
+                        const uint32_t valid = __ballot_sync(0xffffffffu, there);
                         uint32_t e_g = max(max(max(mine & 0xffu, (mine >> 8) & 0xffu), max((mine >> 16) & 0xffu, mine >> 24)), MIN_SCALE_BITS >> 23);
                         e_g = max(e_g, __shfl_xor_sync(0xffffffffu, e_g, 4));
                         e_g = max(e_g, __shfl_xor_sync(0xffffffffu, e_g, 2));
@@ -522,7 +483,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(DUO_THREADS, 1) attn
                         d |= d >> 4;
                         d = __byte_perm(d, 0u, 0x4420);
                         if (sit >= 2) ok = mbar_wait_lean(bar(B_SREADY + b), ((sit >> 1) - 1) & 1u, abort_addr, WD_SREADY);   // the scores two tiles ago are done
-                        if (!ok) break;
+                        together = named_bar_or(NB_SCALE, 128, !ok);
+                        if (together) { ok = false; break; }
+                        const uint32_t mx[2] = {words[b * TILE_N + 64 * thalf + lane], words[b * TILE_N + 64 * thalf + 32 + lane]};
                         tc_fence_after();
                         tmem_st2(lane_addr + TM_SFB + 4 * b, mx);
                         *reinterpret_cast<uint16_t*>(sm + REC_OFF + (ring * TILE_N + 32 * quarter + lane) * 2) = (uint16_t)d;
@@ -538,17 +501,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(DUO_THREADS, 1) attn
                         }
                         ++sit;
                     }
-                    there = 0u;
-#pragma unroll
-                    for (int k = 0; k < 2; ++k) {
-                        if (idx[k] >= 0) {
-                            sc[k] = __ldg(reinterpret_cast<const uint4*>(p.kv + (size_t)idx[k] * ROW_BYTES + SCALE_OFF));
-                            there |= 1u << k;
-                        }
-                    }
-                    const bool more = ahead.next_tile(p, meta);
-#pragma unroll
-                    for (int k = 0; k < 2; ++k) idx[k] = more ? ahead.row_index(p, 64 * thalf + 32 * k + lane) : -1;
+                    there = idx >= 0;
+                    if (there) sc = __ldg(reinterpret_cast<const uint4*>(p.kv + (size_t)idx * ROW_BYTES + SCALE_OFF));
+                    idx = ahead.next_tile(p, meta) ? ahead.row_index(p, 32 * quarter + lane) : -1;
                     primed += filling ? 1u : 0u;
                 }
                 if (!ok) break;
@@ -657,6 +612,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(DUO_THREADS, 1) attn
             it += (uint32_t)tiles.nst;
             ++rq;
         }
+        if (scaler && !together) named_bar_or(NB_SCALE, 128, !ok);     // (nobody stays behind at their barrier)
     } else if (warp == QK_WARP) {
         // =================================================================== score MMAs (odd CTA: its K rows have landed)
         Walk tiles(p, first, step, last);

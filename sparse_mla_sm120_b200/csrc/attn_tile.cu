@@ -57,7 +57,7 @@ using namespace ptx;
 using namespace attn;
 
 constexpr int T_HEADS = 64;                    // heads per CTA
-constexpr int T_TILE = 128;                    // tokens per tile: two scheduler blocks
+constexpr int T_TILE = TILE_N;
 constexpr int T_SM_WARPS = 8, T_PROD = 8, T_SCALE = 12, T_QK = 16, T_PV = 17;
 constexpr int T_THREADS = 20 * 32;
 constexpr int T_REGS_LAUNCH = 96, T_REGS_SOFTMAX = 152, T_REGS_REST = 56;
@@ -83,13 +83,15 @@ constexpr uint32_t NM_OFF = SW_OFF + SW_RING * T_TILE * 8; // -m of the 64 heads
 constexpr uint32_t QW_OFF = NM_OFF + T_HEADS * 4;          // the heads' scale words
 constexpr uint32_t XX_OFF = QW_OFF + T_HEADS * 4;          // exchange between the four warps of a head half: [2][4][64] fp32
 constexpr uint32_t KX_OFF = XX_OFF + 2 * 4 * T_HEADS * 4;  // the same for the blocks' shifts: [2 halves][4]
-constexpr uint32_t B_OFF = KX_OFF + 2 * 4 * 4;
+constexpr uint32_t IDX_OFF = KX_OFF + 2 * 4 * 4;           // the rows that a producer is about to ask for: [4][32]
+constexpr uint32_t WORD_OFF = IDX_OFF + 4 * 32 * 4;        // the rows' scale words on their way to tensor memory: [2][128]
+constexpr uint32_t B_OFF = WORD_OFF + 2 * T_TILE * 4;
 constexpr int B_KFULL = 0, B_RFULL = B_KFULL + NSTAGE, B_KFREE = B_RFULL + 1, B_SREADY = B_KFREE + 4 * NSTAGE, B_SFREE = B_SREADY + 2,
               B_SCALES = B_SFREE + 2, B_PREADY = B_SCALES + SW_RING, B_PVDONE = B_PREADY + 1, B_QREADY = B_PVDONE + 1, B_N = B_QREADY + 1;
 constexpr uint32_t MISC_OFF = B_OFF + B_N * 8;
 constexpr uint32_t T_SMEM = MISC_OFF + 16 + 1024;
 static_assert(T_SMEM <= 227 * 1024, "shared memory budget");
-static_assert(R_OFF % 1024 == 0 && Q_OFF % 1024 == 0 && P_OFF % 1024 == 0 && B_OFF % 8 == 0, "alignment");
+static_assert(IDX_OFF % 16 == 0 && R_OFF % 1024 == 0 && Q_OFF % 1024 == 0 && P_OFF % 1024 == 0 && B_OFF % 8 == 0, "alignment");
 
 // tensor memory: dims block b of O^T at 64 b, score buffers, scale words of the rows (4 columns per tile) and of the heads
 constexpr uint32_t TM_O = 0, TM_S = 256, TM_SFA = 384, TM_SFB = 400;
@@ -125,6 +127,7 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
     const uint32_t base = (raw + 1023u) & ~1023u;
     uint8_t* sm = smem_raw + (base - raw);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(sm + MISC_OFF + 4);
+    const uint32_t abort_addr = base + MISC_OFF + 4;
     auto bar = [&](int i) -> uint32_t { return base + B_OFF + 8u * i; };
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int part = blockIdx.x, my_heads = p.num_heads;   // at most T_HEADS
@@ -182,7 +185,7 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
         // logits in log2 units are scores times a positive number: the sign of the softmax scale goes into q
         const float c = fabsf(p.sm_scale) * LOG2E;
         const uint32_t scale_sign = __float_as_uint(p.sm_scale) & 0x80000000u;
-        Tiles tiles(first, step, last);
+        Walk tiles(p, first, step, last);
         uint32_t it = 0;
         bool dead = false;
         bool prev = false, prev_no_split = false;          // a request's epilogue runs after the next request's Q phase
@@ -196,8 +199,8 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
             if (named_bar_or(3, T_SM_WARPS * 32, dead || *abort_flag != 0)) break;
             if (have) {
                 // ---- Q: warp w quantises heads [8 w, +8), a lane 16 of the 512 no-PE dims of each
-                const __nv_bfloat16* q0 = p.q + ((size_t)tiles.w.req * my_heads) * D_QK;
-#pragma unroll
+                const __nv_bfloat16* q0 = p.q + ((size_t)tiles.req * my_heads) * D_QK;
+#pragma unroll 1
                 for (int u = 0; u < 8; u += 4) {
                     uint4 v[8];
 #pragma unroll
@@ -256,7 +259,7 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
             }
             // ---- epilogue of the request before
             auto epilogue = [&]() {
-                if (!dead) dead = !mbar_wait_hot(bar(B_PVDONE), (it - 1) & 1u, abort_flag, WT_PVDONE);
+                if (!dead) dead = !mbar_wait_lean(bar(B_PVDONE), (it - 1) & 1u, abort_addr, WT_PVDONE);
                 tc_fence_after();
                 xx[quarter * T_HEADS + hl] = prev_l;
                 if (MAXL) xx[(4 + quarter) * T_HEADS + hl] = prev_x;
@@ -383,12 +386,12 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
                     }
                     return mx;
                 };
-                if (!dead) dead = !mbar_wait_hot(bar(B_SCALES + (it & (SW_RING - 1))), (it / SW_RING) & 1u, abort_flag, WT_SCALES);
+                if (!dead) dead = !mbar_wait_lean(bar(B_SCALES + (it & (SW_RING - 1))), (it / SW_RING) & 1u, abort_addr, WT_SCALES);
                 if (!dead) {
                     const uint2 t2 = *reinterpret_cast<const uint2*>(sm + SW_OFF + ((it & (SW_RING - 1)) * T_TILE + token) * 8);
                     ts.below = t2.x; ts.e_g = t2.y;
                     off = (float)((int)ts.e_g - 127 + T_P_SHIFT);
-                    dead = !mbar_wait_hot(bar(B_SREADY + b), (it >> 1) & 1u, abort_flag, WT_SREADY);
+                    dead = !mbar_wait_lean(bar(B_SREADY + b), (it >> 1) & 1u, abort_addr, WT_SREADY);
                 }
                 if (!dead) {
                     tc_fence_after();
@@ -418,7 +421,7 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
 #pragma unroll
                         for (int o = 16; o >= 1; o >>= 1) low = __vminu4(low, __shfl_xor_sync(0xffffffffu, low, o));
                         kx[half * 4 + quarter] = low;
-                        if (j > 0) dead = !mbar_wait_hot(bar(B_PVDONE), (it - 1) & 1u, abort_flag, WT_PVDONE);
+                        if (j > 0) dead = !mbar_wait_lean(bar(B_PVDONE), (it - 1) & 1u, abort_addr, WT_PVDONE);
                     }
                     const float m_old = -nm[hl];
                     if (named_bar_or(1 + half, 128, dead || *abort_flag != 0)) { dead = true; break; }
@@ -470,7 +473,7 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
                     fma_f32x2(l2[i / 2], pack_f32x2(p0, p1), is2);
                     z[i] = __float_as_uint(p0); z[i + 1] = __float_as_uint(p1);
                 }
-                if (it > 0 && !dead) dead = !mbar_wait_hot(bar(B_PVDONE), (it - 1) & 1u, abort_flag, WT_PVDONE);   // the weights of the last tile have been read
+                if (it > 0 && !dead) dead = !mbar_wait_lean(bar(B_PVDONE), (it - 1) & 1u, abort_addr, WT_PVDONE);   // the weights of the last tile have been read
                 if (dead) continue;
                 const uint32_t under = ts.below - shift;   // (no borrows: the shifts are the smallest so far)
 #pragma unroll
@@ -514,131 +517,125 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
             }
             prev_m = -nm[hl];
             prev_shift = shift;
-            prev = true; prev_no_split = tiles.w.no_split; prev_req = tiles.w.req; prev_split = tiles.w.split_idx;
+            const bool at_begin = tiles.req == meta.begin_req;
+            prev = true; prev_req = tiles.req;
+            prev_no_split = !p.force_partial && !(at_begin ? meta.first_split : prev_req == meta.end_req ? meta.last_split : 0);
+            prev_split = (p.num_splits ? p.num_splits[prev_req] : 0) + (at_begin ? meta.begin_split : 0);
         }
     } else if (warp < T_SCALE) {
         // =================================================================== rows -> K stages (TMA gather)
+        // The lanes read the rows' numbers ahead and hand them to the lane that issues the copies through shared memory (by shuffles, under
+        // an election for every four rows, the copies took three times the instructions).
         const int quarter = warp - T_PROD;
-        Tiles tiles(first, step, last);
-        bool have = tiles.next_tile(p, meta), ok = true;
-        int idx = have ? tiles.row_index(p, quarter * 32 + lane) : -1;
-        for (uint32_t it = 0; have; ++it) {
-            const uint32_t st = it % NSTAGE;
-            const int row = idx >= 0 ? idx : NO_ROW;
+        int* mine = reinterpret_cast<int*>(sm + IDX_OFF) + 32 * quarter;
+        Walk tiles(p, first, step, last);
+        bool ok = true;
+        int idx = 0;
+        uint32_t it = 0;
+        for (bool have = true, warm = false; have; warm = true) {
+            mine[lane] = idx >= 0 ? idx : NO_ROW;
             have = tiles.next_tile(p, meta);
-            int idx_next = have ? tiles.row_index(p, quarter * 32 + lane) : -1;     // read ahead of its use
-            if (it >= NSTAGE) ok = mbar_wait_hot(bar(B_KFREE + 4 * st + quarter), ((it / NSTAGE) - 1) & 1u, abort_flag, WT_KFREE);
+            idx = have ? tiles.row_index(p, quarter * 32 + lane) : -1;     // read ahead of its use
+            if (!warm) continue;
+            const uint32_t st = it % NSTAGE;
+            if (it >= NSTAGE) ok = mbar_wait_lean(bar(B_KFREE + 4 * st + quarter), ((it / NSTAGE) - 1) & 1u, abort_addr, WT_KFREE);
             if (!ok) break;
-            const uint32_t dst = base + K_OFF + st * K_STAGE + quarter * (32 * 128);
-            if (elect_one()) mbar_arrive_expect_tx(bar(B_KFULL + st), 4 * 32 * 128);
             __syncwarp();
+            if (elect_one()) {
+                uint32_t dst = base + K_OFF + st * K_STAGE + quarter * (32 * 128);
+                const uint32_t full = bar(B_KFULL + st);
+                mbar_arrive_expect_tx(full, 4 * 32 * 128);
+#pragma unroll 1
+                for (int q = 0; q < 32; q += 4, dst += 512) {
+                    const int4 r = *reinterpret_cast<const int4*>(mine + q);
 #pragma unroll
-            for (int q = 0; q < 8; ++q) {
-                const int r0 = __shfl_sync(0xffffffffu, row, 4 * q), r1 = __shfl_sync(0xffffffffu, row, 4 * q + 1);
-                const int r2 = __shfl_sync(0xffffffffu, row, 4 * q + 2), r3 = __shfl_sync(0xffffffffu, row, 4 * q + 3);
-                if (elect_one()) {
-#pragma unroll
-                    for (int b = 0; b < 4; ++b) tma_gather4(dst + b * K_CHUNK + q * 512, &kv_map, 32 * b, r0, r1, r2, r3, bar(B_KFULL + st));
+                    for (int b = 0; b < 4; ++b) tma_gather4(dst + b * K_CHUNK, &kv_map, 32 * b, r.x, r.y, r.z, r.w, full);
                 }
-                __syncwarp();
             }
-            // the RoPE stage is free when the scores of the tile before are done
-            if (it >= 1) ok = mbar_wait_hot(bar(B_SREADY + ((it - 1) & 1u)), ((it - 1) >> 1) & 1u, abort_flag, WT_SREADY);
-            if (!ok) break;
-            if (elect_one()) mbar_arrive_expect_tx(bar(B_RFULL), 32 * 128);
             __syncwarp();
-#pragma unroll
-            for (int q = 0; q < 8; ++q) {
-                const int r0 = __shfl_sync(0xffffffffu, row, 4 * q), r1 = __shfl_sync(0xffffffffu, row, 4 * q + 1);
-                const int r2 = __shfl_sync(0xffffffffu, row, 4 * q + 2), r3 = __shfl_sync(0xffffffffu, row, 4 * q + 3);
-                if (elect_one()) tma_gather4(base + R_OFF + quarter * (32 * 128) + q * 512, &kv_map, ROPE_OFF / 4, r0, r1, r2, r3, bar(B_RFULL));
-                __syncwarp();
+            // the RoPE stage is free when the scores of the tile before are done
+            if (it >= 1) ok = mbar_wait_lean(bar(B_SREADY + ((it - 1) & 1u)), ((it - 1) >> 1) & 1u, abort_addr, WT_SREADY);
+            if (!ok) break;
+            if (elect_one()) {
+                uint32_t dst = base + R_OFF + quarter * (32 * 128);
+                mbar_arrive_expect_tx(bar(B_RFULL), 32 * 128);
+#pragma unroll 1
+                for (int q = 0; q < 32; q += 4, dst += 512) {
+                    const int4 r = *reinterpret_cast<const int4*>(mine + q);
+                    tma_gather4(dst, &kv_map, ROPE_OFF / 4, r.x, r.y, r.z, r.w, bar(B_RFULL));
+                }
             }
-            idx = idx_next;
+            __syncwarp();
+            ++it;
         }
     } else if (warp < T_QK) {
         // =================================================================== scale words
-        // Lane i reads the scales of tokens i, 32 + i, 64 + i, 96 + i: row r's word belongs into column r / 32 of lane r % 32, in
-        // all four lane quarters.
-        // The next tile's scales are asked for when this tile's words have been handed over, and looked at a tile later.
+        // A warp reads the scales of 32 tokens, makes their words and passes them to the others: row r's word belongs into column r / 32 of
+        // lane r % 32, in all four lane quarters, and a warp reaches one of them.  The rows' numbers are read two tiles ahead, their
+        // scales one.
         const int quarter = warp - T_SCALE;
         const uint32_t lane_addr = tmem + ((uint32_t)(quarter * 32) << 16);
-        Tiles tiles(first, step, last);
-        bool have = tiles.next_tile(p, meta), ok = true;
-        int idx[4];
-        uint4 sc[4];
-        auto fetch = [&]() {
-#pragma unroll
-            for (int k = 0; k < 4; ++k) idx[k] = have ? tiles.row_index(p, 32 * k + lane) : -1;
-        };
-        uint32_t there = 0u;                               // bit k: token 32 k + lane has an entry
-        auto load = [&]() {
-            there = 0u;
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                sc[k] = make_uint4(0u, 0u, 0u, 0u);
-                if (idx[k] >= 0) {
-                    sc[k] = __ldg(reinterpret_cast<const uint4*>(p.kv + (size_t)idx[k] * ROW_BYTES + SCALE_OFF));
-                    there |= 1u << k;
+        uint32_t* words = reinterpret_cast<uint32_t*>(sm + WORD_OFF);
+        Walk tiles(p, first, step, last);
+        bool ok = true, have = true, have1 = false, have2 = false;     // is there a tile whose rows, scales, words are next
+        int idx = -1;
+        bool there = false;
+        uint4 sc = make_uint4(0u, 0u, 0u, 0u);
+        for (uint32_t it = 0, primed = 0; ok && (have || have1 || have2); ) {
+            if (primed >= 2 && have2) {
+                auto bits = [](uint32_t v) { return max(v, MIN_SCALE_BITS) << 1; };             // the exponent is the upper byte
+                const uint32_t lo = __byte_perm(bits(sc.x), bits(sc.y), 0x0073), hi = __byte_perm(bits(sc.z), bits(sc.w), 0x0073);
+                const uint32_t mine = there ? __byte_perm(lo, hi, 0x5410) : 0u;
+                words[(it & 1u) * T_TILE + quarter * 32 + lane] = there ? mine : 0x7f7f7f7fu;
+                uint32_t e_g = max(max(mine & 0xffu, (mine >> 8) & 0xffu), max((mine >> 16) & 0xffu, mine >> 24));
+                e_g = max(e_g, __shfl_xor_sync(0xffffffffu, e_g, 4));
+                e_g = max(e_g, __shfl_xor_sync(0xffffffffu, e_g, 2));
+                e_g = max(e_g, __shfl_xor_sync(0xffffffffu, e_g, 1));
+                uint2 ts = make_uint2(NO_SHIFT * 0x01010101u, 0u);
+                if (mine != 0u) {
+                    ts = make_uint2(e_g * 0x01010101u - mine, e_g);
+                    if ((ts.x & 0x80808080u) != 0u) ts.x = __vminu4(ts.x, NO_SHIFT * 0x01010101u);
                 }
-            }
-        };
-        fetch();
-        load();
-        bool cur = have;
-        have = have && tiles.next_tile(p, meta);
-        fetch();
-        for (uint32_t it = 0; cur; ++it) {
-            uint32_t word[4], mx[4];
+                if (it >= 2) ok = mbar_wait_lean(bar(B_SREADY + (it & 1u)), ((it >> 1) - 1) & 1u, abort_addr, WT_SREADY);   // the scores two tiles ago are done
+                if (named_bar_or(4, 128, !ok)) break;
+                uint32_t mx[4];
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                auto bits = [](uint32_t v) { return max(v, MIN_SCALE_BITS) << 1; };         // the exponent is the upper byte
-                const uint32_t lo = __byte_perm(bits(sc[k].x), bits(sc[k].y), 0x0073), hi = __byte_perm(bits(sc[k].z), bits(sc[k].w), 0x0073);
-                word[k] = ((there >> k) & 1u) != 0u ? __byte_perm(lo, hi, 0x5410) : 0u;
-                mx[k] = word[k] != 0u ? word[k] : 0x7f7f7f7fu;
+                for (int k = 0; k < 4; ++k) mx[k] = words[(it & 1u) * T_TILE + 32 * k + lane];
+                tc_fence_after();
+                tmem_st4(lane_addr + TM_SFA + 4 * (it & 1u), mx);
+                *reinterpret_cast<uint2*>(sm + SW_OFF + ((it & (SW_RING - 1)) * T_TILE + quarter * 32 + lane) * 8) = ts;
+                tmem_wait_st();
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar(B_SCALES + (it & (SW_RING - 1))));
+                ++it;
             }
-            const uint32_t mine = quarter == 0 ? word[0] : quarter == 1 ? word[1] : quarter == 2 ? word[2] : word[3];
-            uint32_t e_g = max(max(mine & 0xffu, (mine >> 8) & 0xffu), max((mine >> 16) & 0xffu, mine >> 24));
-#pragma unroll
-            for (int o = 4; o >= 1; o >>= 1) e_g = max(e_g, __shfl_xor_sync(0xffffffffu, e_g, o));
-            uint2 ts = make_uint2(NO_SHIFT * 0x01010101u, 0u);
-            if (mine != 0u) {
-                ts = make_uint2(e_g * 0x01010101u - mine, e_g);
-                if ((ts.x & 0x80808080u) != 0u) ts.x = __vminu4(ts.x, NO_SHIFT * 0x01010101u);
-            }
-            if (it >= 2) ok = mbar_wait_hot(bar(B_SREADY + (it & 1u)), ((it >> 1) - 1) & 1u, abort_flag, WT_SREADY);   // the scores two tiles ago are done
-            if (!ok) break;
-            tc_fence_after();
-            tmem_st4(lane_addr + TM_SFA + 4 * (it & 1u), mx);
-            *reinterpret_cast<uint2*>(sm + SW_OFF + ((it & (SW_RING - 1)) * T_TILE + quarter * 32 + lane) * 8) = ts;
-            tmem_wait_st();
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(bar(B_SCALES + (it & (SW_RING - 1))));
-            load();                                        // of the next tile
-            cur = have;
-            have = have && tiles.next_tile(p, meta);
-            fetch();
+            there = idx >= 0;
+            if (there) sc = __ldg(reinterpret_cast<const uint4*>(p.kv + (size_t)idx * ROW_BYTES + SCALE_OFF));
+            have2 = have1;
+            have1 = have = have && tiles.next_tile(p, meta);
+            idx = have ? tiles.row_index(p, quarter * 32 + lane) : -1;
+            if (primed < 2) ++primed;
         }
     } else if (warp == T_QK) {
         // =================================================================== score MMAs
         const uint32_t q_lo = desc_lo(base + Q_OFF, 16), qr_lo = desc_lo(base + QR_OFF, 16), r_lo = desc_lo(base + R_OFF, 16);
-        Tiles tiles(first, step, last);
+        Walk tiles(p, first, step, last);
         uint32_t it = 0, rq = 0;
         bool ok = true;
         while (ok && tiles.next_request(p, meta)) {
-            ok = mbar_wait_hot(bar(B_QREADY), rq & 1u, abort_flag, WT_QREADY);
+            ok = mbar_wait_lean(bar(B_QREADY), rq & 1u, abort_addr, WT_QREADY);
             ++rq;
             for (int j = 0; j < tiles.nst && ok; ++j, ++it) {
                 const uint32_t st = it % NSTAGE, b = it & 1u;
-                if (it >= 2) ok = mbar_wait_hot(bar(B_SFREE + b), ((it >> 1) - 1) & 1u, abort_flag, WT_SFREE);
-                if (ok) ok = mbar_wait_hot(bar(B_SCALES + (it & (SW_RING - 1))), (it / SW_RING) & 1u, abort_flag, WT_SCALES);
-                if (ok) ok = mbar_wait_hot(bar(B_KFULL + st), (it / NSTAGE) & 1u, abort_flag, WT_KFULL);
+                if (it >= 2) ok = mbar_wait_lean(bar(B_SFREE + b), ((it >> 1) - 1) & 1u, abort_addr, WT_SFREE);
+                if (ok) ok = mbar_wait_lean(bar(B_SCALES + (it & (SW_RING - 1))), (it / SW_RING) & 1u, abort_addr, WT_SCALES);
+                if (ok) ok = mbar_wait_lean(bar(B_KFULL + st), (it / NSTAGE) & 1u, abort_addr, WT_KFULL);
                 if (!ok) break;
                 tc_fence_after();
                 const uint32_t k_lo = desc_lo(base + K_OFF + st * K_STAGE, 16), d = tmem + TM_S + 64 * b;
                 if (elect_one()) {
-#pragma unroll
+#pragma unroll 1
                     for (int bb = 0; bb < 4; ++bb) {
 #pragma unroll
                         for (int k = 0; k < 4; ++k)
@@ -647,7 +644,7 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
                     }
                 }
                 __syncwarp();
-                ok = mbar_wait_hot(bar(B_RFULL), it & 1u, abort_flag, WT_RFULL);
+                ok = mbar_wait_lean(bar(B_RFULL), it & 1u, abort_addr, WT_RFULL);
                 if (!ok) break;
                 if (elect_one()) {
 #pragma unroll
@@ -660,19 +657,19 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
         }
     } else if (warp == T_PV) {
         // =================================================================== P.V MMAs
-        Tiles tiles(first, step, last);
+        Walk tiles(p, first, step, last);
         const uint32_t p_lo = desc_lo(base + P_OFF, 16);
         uint32_t it = 0;
         bool ok = true;
         while (ok && tiles.next_request(p, meta)) {
             for (int j = 0; j < tiles.nst && ok; ++j, ++it) {
                 const uint32_t st = it % NSTAGE;
-                ok = mbar_wait_hot(bar(B_PREADY), it & 1u, abort_flag, WT_PREADY);
+                ok = mbar_wait_lean(bar(B_PREADY), it & 1u, abort_addr, WT_PREADY);
                 if (!ok) break;
                 tc_fence_after();
                 const uint32_t v_lo = desc_lo(base + K_OFF + st * K_STAGE, 16);
                 if (elect_one()) {
-#pragma unroll
+#pragma unroll 1
                     for (int k = 0; k < 4; ++k) {          // 32 tokens: their rows may be overwritten as soon as they have been read
 #pragma unroll
                         for (int b = 0; b < 4; ++b)
