@@ -136,6 +136,7 @@ __global__ void __launch_bounds__(X_THREADS, 1) attn_exact_kernel(const AttnPara
     const uint32_t base = (raw + 1023u) & ~1023u;
     uint8_t* sm = smem_raw + (base - raw);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(sm + XMISC_OFF + 4);
+    const uint32_t abort_addr = base + XMISC_OFF + 4;
     auto bar = [&](int i) -> uint32_t { return base + XB_OFF + 8u * i; };
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int head0 = (int)blockIdx.y * X_HEADS;
@@ -213,7 +214,7 @@ __global__ void __launch_bounds__(X_THREADS, 1) attn_exact_kernel(const AttnPara
             for (int j = 0; j < nst; ++j, ++it) {
                 uint32_t sv[32];
                 bool valid = false;
-                if (!dead) dead = !mbar_wait_hot(bar(XB_SREADY), it & 1u, abort_flag, WX_SREADY);
+                if (!dead) dead = !mbar_wait_lean(bar(XB_SREADY), it & 1u, abort_addr, WX_SREADY);
                 if (!dead) {
                     tc_fence_after();
                     tmem_ld32(lane_addr + XT_S + 32 * half, sv);
@@ -285,7 +286,7 @@ __global__ void __launch_bounds__(X_THREADS, 1) attn_exact_kernel(const AttnPara
             }
             if (stop) break;
             // ---- epilogue
-            if (!dead) dead = !mbar_wait_hot(bar(XB_PVDONE), (it - 1) & 1u, abort_flag, WX_PVDONE);
+            if (!dead) dead = !mbar_wait_lean(bar(XB_PVDONE), (it - 1) & 1u, abort_addr, WX_PVDONE);
             tc_fence_after();
             // sum over the warp's tokens: halve the list at every exchange, lane i ends with head i
 #pragma unroll
@@ -440,7 +441,7 @@ __global__ void __launch_bounds__(X_THREADS, 1) attn_exact_kernel(const AttnPara
             }
 #pragma unroll
             for (int i = 0; i < X_RPW; ++i) {
-                if (it >= 1 && (i & 1) == 0 && ok) ok = mbar_wait_hot(bar(XB_KFREE + (i >> 1)), (it - 1) & 1u, abort_flag, WX_KFREE);
+                if (it >= 1 && (i & 1) == 0 && ok) ok = mbar_wait_lean(bar(XB_KFREE + (i >> 1)), (it - 1) & 1u, abort_addr, WX_KFREE);
                 const uint32_t w0 = __shfl_sync(0xffffffffu, sc8.x, i), w1 = __shfl_sync(0xffffffffu, sc8.y, i);
                 const uint32_t e = (((bk & 4) ? w1 : w0) >> (8 * (bk & 3))) & 0xffu;
                 // the block's scale 2^(e - 127) times the 2^120 of e4m3_as_bf16x2; what does not fit a bf16 power is made up below
@@ -495,10 +496,10 @@ __global__ void __launch_bounds__(X_THREADS, 1) attn_exact_kernel(const AttnPara
             Work w;
             if (!get_work(p, meta, req, w)) continue;
             const int nst = (w.nblk + 1) >> 1;
-            ok = mbar_wait_hot(bar(XB_QREADY), rq & 1u, abort_flag, WX_QREADY);
+            ok = mbar_wait_lean(bar(XB_QREADY), rq & 1u, abort_addr, WX_QREADY);
             ++rq;
             for (int j = 0; j < nst && ok; ++j, ++it) {
-                ok = mbar_wait_hot(bar(XB_KFULL), it & 1u, abort_flag, WX_KFULL);
+                ok = mbar_wait_lean(bar(XB_KFULL), it & 1u, abort_addr, WX_KFULL);
                 if (!ok) break;
                 tc_fence_after();
                 if (elect_one()) {
@@ -512,7 +513,7 @@ __global__ void __launch_bounds__(X_THREADS, 1) attn_exact_kernel(const AttnPara
                     tc_commit(bar(XB_SREADY));
                 }
                 __syncwarp();
-                ok = mbar_wait_hot(bar(XB_PREADY), it & 1u, abort_flag, WX_PREADY);
+                ok = mbar_wait_lean(bar(XB_PREADY), it & 1u, abort_addr, WX_PREADY);
                 if (!ok) break;
                 tc_fence_after();
                 if (elect_one()) {

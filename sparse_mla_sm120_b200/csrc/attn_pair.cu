@@ -240,6 +240,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) att
     const uint32_t base = (raw + 1023u) & ~1023u;
     uint8_t* sm = smem_raw + (base - raw);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(sm + MISC_OFF + 4);
+    const uint32_t abort_addr = base + MISC_OFF + 4;
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(sm + MISC_OFF);
     auto bar = [&](int i) -> uint32_t { return base + BAR_OFF + 8u * i; };
 
@@ -365,7 +366,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) att
             {
                 const int g = lane >> 2, c4 = lane & 3;
                 const bool from_smem = STAGE_Q && q_staged && req == meta.begin_req;
-                if (from_smem && !dead) dead = !mbar_wait_hot(bar(BAR_QSTAGE), 0u, abort_flag, W_QSTAGE);
+                if (from_smem && !dead) dead = !mbar_wait_lean(bar(BAR_QSTAGE), 0u, abort_addr, W_QSTAGE);
                 // row (head0 + r) of the request's Q, wherever it lies
                 const __nv_bfloat16* qrows = from_smem ? reinterpret_cast<const __nv_bfloat16*>(sm + QSTAGE_OFF) - (size_t)head0 * L::QD
                                                        : p.q + (size_t)req * p.num_heads * L::QD;
@@ -488,7 +489,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) att
             // ---- epilogue of the request before ------------------------------------------------
             if (prev_valid) {
                 const uint32_t last = prev_last;
-                if (!dead) dead = !mbar_wait_hot(bar(BAR_PVDONE + (last & 1u)), (last >> 1) & 1u, abort_flag, W_PVDONE);
+                if (!dead) dead = !mbar_wait_lean(bar(BAR_PVDONE + (last & 1u)), (last >> 1) & 1u, abort_addr, W_PVDONE);
                 tc_fence_after();
                 if (named_bar_or(1 + grp, 128, dead || *abort_flag != 0)) { stop = true; break; }   // the partners have read the last tile's row maxima
                 xch[xpart * 64 + hrow] = prev_l;
@@ -606,8 +607,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) att
                 float c_g[4], off_g[4], inv_g[4];          // of the four groups of eight tokens that this thread holds: z = s * c + off, 1/s
                 // the records of this thread's 32 tokens: half tile thalf, gather warps [4 ch, 4 ch + 4)
                 const uint8_t* info = sm + INFO_OFF + (it & (INFO_RING - 1)) * (2 * INFO_HALF) + thalf * INFO_HALF + ch * 64;
-                if (!dead) dead = !mbar_wait_hot(bar(BAR_SREADY + b), (it >> 1) & 1u, abort_flag, W_SREADY);
-                if (!dead) dead = !mbar_wait_hot(bar(BAR_INFO + (it & (INFO_RING - 1))), (it / INFO_RING) & 1u, abort_flag, W_INFO);
+                if (!dead) dead = !mbar_wait_lean(bar(BAR_SREADY + b), (it >> 1) & 1u, abort_addr, W_SREADY);
+                if (!dead) dead = !mbar_wait_lean(bar(BAR_INFO + (it & (INFO_RING - 1))), (it / INFO_RING) & 1u, abort_addr, W_INFO);
                 if (!dead) {
                     tc_fence_after();
                     tmem_ld32(lane_addr + TM_S + 64 * b + 32 * ch, sv);
@@ -650,7 +651,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) att
                     const float mx = fmaxf(fmaxf(xr[0], xr[64]), fmaxf(xr[128], xr[192]));
                     const bool grow = mx > m_run + RESCALE_TAU;   // false while the row has seen no valid entry
                     if (j > 0) {   // the accumulator holds earlier tiles: wait for the last P.V, then scale it
-                        dead = !mbar_wait_hot(bar(BAR_PVDONE + ((it - 1) & 1u)), ((it - 1) >> 1) & 1u, abort_flag, W_PVDONE);
+                        dead = !mbar_wait_lean(bar(BAR_PVDONE + ((it - 1) & 1u)), ((it - 1) >> 1) & 1u, abort_addr, W_PVDONE);
                         if (dead) continue;
                         tc_fence_after();
                     }
@@ -670,7 +671,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) att
                     }
                 }
                 if (it >= 2) {   // the P.V that read this P' buffer two tiles ago has completed
-                    dead = !mbar_wait_hot(bar(BAR_PVDONE + b), ((it - 2) >> 1) & 1u, abort_flag, W_PVDONE);
+                    dead = !mbar_wait_lean(bar(BAR_PVDONE + b), ((it - 2) >> 1) & 1u, abort_addr, W_PVDONE);
                     if (dead) continue;
                 }
                 const float m_off = ((m_run == -INFINITY) ? 0.f : m_run) - (float)P_SHIFT;
@@ -739,7 +740,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) att
 #pragma unroll 1
         while (cur.have) {
             const uint32_t t_it = item / N_GROUPS, gw = item % N_GROUPS, ks = t_it % NK, slot = item % NR;
-            ok = mbar_wait_hot(bar(BAR_RAWFULL + slot), (item / NR) & 1u, abort_flag, W_RAWFULL);
+            ok = mbar_wait_lean(bar(BAR_RAWFULL + slot), (item / NR) & 1u, abort_addr, W_RAWFULL);
             if (!ok) break;
             const uint32_t vbits = __ballot_sync(0xffffffffu, cur.idx >= 0) & ((1u << RPW) - 1u);
             const uint2 sc8 = sc8_nxt;
@@ -788,8 +789,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) att
             const uint32_t my_sub = L::M1 ? ((lane & 8) ? sc8.y : sc8.x) : ((sc > 0.f) ? shift_bytes_of_ratio(sc * inv_half) : 0u);
             const uint32_t e_grp = __float_as_uint(s_half) >> 23;
             const int bk = lane >> 2;                            // MODEL1: 64-value block of this lane's piece (0-6 in the lanes that store)
-            if (t_it >= NK) ok = mbar_wait_hot(bar(BAR_KEMPTY + ks), ((t_it / NK) - 1) & 1u, abort_flag, W_KEMPTY);
-            if (STAGE_Q && ok && t_it == NK - 1 && first_work) ok = mbar_wait_hot(bar(BAR_QFREE), 0u, abort_flag, W_QFREE);   // K stage 1 held Q until now
+            if (t_it >= NK) ok = mbar_wait_lean(bar(BAR_KEMPTY + ks), ((t_it / NK) - 1) & 1u, abort_addr, W_KEMPTY);
+            if (STAGE_Q && ok && t_it == NK - 1 && first_work) ok = mbar_wait_lean(bar(BAR_QFREE), 0u, abort_addr, W_QFREE);   // K stage 1 held Q until now
             if (!ok) break;
             uint8_t* kp = sm + KS_OFF + ks * KS_BYTES;
 #pragma unroll
@@ -847,16 +848,16 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) att
             Work w;
             if (!get_work(p, meta, req, w)) continue;
             const int nst = (w.nblk + 1) >> 1;
-            ok = mbar_wait_hot(bar(BAR_QREADYP), rq & 1u, abort_flag, W_QREADY);
+            ok = mbar_wait_lean(bar(BAR_QREADYP), rq & 1u, abort_addr, W_QREADY);
             if (!ok) break;
             ++rq;
             for (int j = 0; j < nst && ok; ++j, ++it) {
                 const uint32_t ks = it % NK, b = it & 1u;
                 if (it >= 2) {
-                    ok = mbar_wait_hot(bar(BAR_SFREEP + b), ((it - 2) >> 1) & 1u, abort_flag, W_SFREE);
+                    ok = mbar_wait_lean(bar(BAR_SFREEP + b), ((it - 2) >> 1) & 1u, abort_addr, W_SFREE);
                     if (!ok) break;
                 }
-                ok = mbar_wait_hot(bar(BAR_KFULLP + ks), (it / NK) & 1u, abort_flag, W_KFULL);
+                ok = mbar_wait_lean(bar(BAR_KFULLP + ks), (it / NK) & 1u, abort_addr, W_KFULL);
                 if (!ok) break;
                 tc_fence_after();
                 const uint32_t kb_lo = desc_lo(base + KS_OFF + ks * KS_BYTES, 16);
@@ -894,9 +895,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) att
             const int nst = (w.nblk + 1) >> 1;
             for (int j = 0; j < nst && ok; ++j, ++it) {
                 const uint32_t vs = it % NV, b = it & 1u;
-                ok = mbar_wait_hot(bar(BAR_PREADYP + b), (it >> 1) & 1u, abort_flag, W_PREADY);
+                ok = mbar_wait_lean(bar(BAR_PREADYP + b), (it >> 1) & 1u, abort_addr, W_PREADY);
                 if (!ok) break;
-                ok = mbar_wait_hot(bar(BAR_VFULLP + vs), (it / NV) & 1u, abort_flag, W_VFULL);
+                ok = mbar_wait_lean(bar(BAR_VFULLP + vs), (it / NV) & 1u, abort_addr, W_VFULL);
                 if (!ok) break;
                 tc_fence_after();
                 const uint32_t pa_lo = desc_lo(base + PB_OFF + b * CHUNK, 16);
@@ -935,13 +936,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) att
             const int nst = (w.nblk + 1) >> 1;
             for (int j = 0; j < nst && ok; ++j, ++it) {
                 const uint32_t ks = it % NK, vs = it % NV;
-                ok = mbar_wait_hot(bar(BAR_KSTORED + ks), (it / NK) & 1u, abort_flag, W_KSTORED);
+                ok = mbar_wait_lean(bar(BAR_KSTORED + ks), (it / NK) & 1u, abort_addr, W_KSTORED);
                 if (!ok) break;
                 if (it >= NV) {
-                    ok = mbar_wait_hot(bar(BAR_VEMPTY + vs), ((it / NV) - 1) & 1u, abort_flag, W_VEMPTY);
+                    ok = mbar_wait_lean(bar(BAR_VEMPTY + vs), ((it / NV) - 1) & 1u, abort_addr, W_VEMPTY);
                     if (!ok) break;
                 } else if (STAGE_Q && first_work) {    // the V stages of both CTAs held Q until the softmax warps had read it
-                    ok = mbar_wait_hot(bar(BAR_QFREE), 0u, abort_flag, W_QFREE);
+                    ok = mbar_wait_lean(bar(BAR_QFREE), 0u, abort_addr, W_QFREE);
                     if (!ok) break;
                 }
                 if (elect_one()) {
@@ -957,7 +958,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) att
                     }
                 }
                 __syncwarp();
-                ok = mbar_wait_hot(bar(BAR_VFULL + vs), (it / NV) & 1u, abort_flag, W_VFULL_CTA);
+                ok = mbar_wait_lean(bar(BAR_VFULL + vs), (it / NV) & 1u, abort_addr, W_VFULL_CTA);
                 if (!ok) break;
                 if (lane == 0) {
                     mbar_arrive_remote(barp(BAR_VFULLP + vs));
@@ -981,7 +982,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) att
             const int nst = (w.nblk + 1) >> 1;
             for (int j = 0; j < nst && ok; ++j, ++it) {
                 const uint32_t ks = it % NK, ir = it & (INFO_RING - 1);
-                ok = mbar_wait_hot(bar(BAR_KSTORED + ks), (it / NK) & 1u, abort_flag, W_KSTORED);
+                ok = mbar_wait_lean(bar(BAR_KSTORED + ks), (it / NK) & 1u, abort_addr, W_KSTORED);
                 if (!ok) break;
                 if (elect_one()) {
                     mbar_arrive_expect_tx(bar(BAR_INFO + ir), INFO_HALF);
@@ -1018,7 +1019,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) att
                 src = reinterpret_cast<unsigned long long>(pg + (int64_t)in * L::DATA);
             }
             const uint32_t nvalid = __popc(__ballot_sync(0xffffffffu, src != 0ull) & ((1u << RPW) - 1u));
-            if (item >= NR) ok = mbar_wait_hot(bar(BAR_RAWEMPTY + slot), ((item / NR) - 1) & 1u, abort_flag, W_RAWEMPTY);
+            if (item >= NR) ok = mbar_wait_lean(bar(BAR_RAWEMPTY + slot), ((item / NR) - 1) & 1u, abort_addr, W_RAWEMPTY);
             if (!ok) break;
             if (lane == 0) mbar_arrive_expect_tx(bar(BAR_RAWFULL + slot), nvalid * L::DATA);
             __syncwarp();

@@ -79,18 +79,18 @@ __device__ __forceinline__ bool mbar_wait_hot(uint32_t bar, uint32_t parity, vol
     return __all_sync(0xffffffffu, ok != 0);
 }
 
-// The same in as few instructions as it can have, for a kernel whose roles together are larger than the instruction caches: at
-// most 2^20 polls (of up to 4 us each), then `code` goes to the abort flag (given by its shared-memory address).
+// The same in as few instructions as it can have, for a kernel whose roles together are larger than the instruction caches: nearly always
+// the first poll, which the hardware suspends for up to 4 us, is the only one.  The warp decides by votes, so nothing here
+// diverges.  At most 2^20 polls, then `code` goes to the abort flag (given by its shared-memory address).
 __device__ __forceinline__ bool mbar_wait_lean(uint32_t bar, uint32_t parity, uint32_t abort_addr, int code) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p, q;\n\t.reg .u32 n;\n\tmov.u32 n, 0x100000;\n"
-        "POLL:\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t@p bra DONE;\n\t"
-        "add.u32 n, n, -1;\n\tsetp.ne.u32 q, n, 0;\n\t@q bra POLL;\n\t"
-        "st.volatile.shared.u32 [%3], %4;\n"
-        "DONE:\n\tselp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok) : "r"(bar), "r"(parity), "r"(abort_addr), "r"(code) : "memory");
-    return __all_sync(0xffffffffu, ok != 0);
+#pragma unroll 1
+    for (uint32_t left = 1u << 20; ; --left) {
+        if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity, WAIT_HINT_NS))) return true;
+        if (left == 0u) {
+            asm volatile("st.volatile.shared.u32 [%0], %1;" ::"r"(abort_addr), "r"(code) : "memory");
+            return false;
+        }
+    }
 }
 
 // True in one lane of the (converged) warp, the same one every time.  Instructions whose operands live in uniform
