@@ -75,6 +75,7 @@ __global__ void __launch_bounds__(LX_THREADS, 1) mqa_logits_tc_kernel(const Logi
     const uint32_t base = (raw + 1023u) & ~1023u;
     uint8_t* sm = smem_raw + (base - raw);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(sm + LX_MISC_OFF + 4);
+    const uint32_t abort_addr = base + LX_MISC_OFF + 4;
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(sm + LX_MISC_OFF);
     auto bar = [&](int i) -> uint32_t { return base + LX_BAR_OFF + 8u * i; };
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -170,7 +171,7 @@ __global__ void __launch_bounds__(LX_THREADS, 1) mqa_logits_tc_kernel(const Logi
             for (int t = t0; t < t1; ++t, ++it, key += LX_KT) {
                 const uint32_t b = it & 1u;
                 const float sc = key < p.s_k ? __ldg(p.k_scale + key) : 0.f;
-                ok = mbar_wait_hot(bar(LXB_DFULL + b), (it >> 1) & 1u, abort_flag, 12);
+                ok = mbar_wait_lean(bar(LXB_DFULL + b), (it >> 1) & 1u, abort_addr, 12);
                 if (!ok) break;
                 tc_fence_after();
                 uint64_t a01 = 0ull, a23 = 0ull;
@@ -226,7 +227,7 @@ __global__ void __launch_bounds__(LX_THREADS, 1) mqa_logits_tc_kernel(const Logi
             for (int t = t0; t < t1 && ok; ++t, ++it) {
                 const uint32_t st = it % LX_KSTAGE;
                 if (it >= LX_KSTAGE) {
-                    ok = mbar_wait_hot(bar(LXB_KEMPTY + st), ((it / LX_KSTAGE) - 1) & 1u, abort_flag, 14);
+                    ok = mbar_wait_lean(bar(LXB_KEMPTY + st), ((it / LX_KSTAGE) - 1) & 1u, abort_addr, 14);
                     if (!ok) break;
                 }
                 if (elect_one()) {
@@ -246,15 +247,15 @@ __global__ void __launch_bounds__(LX_THREADS, 1) mqa_logits_tc_kernel(const Logi
             int g, t0, t1, j0, j1;
             item_range(w, g, t0, t1, j0, j1);
             if (t1 <= t0) continue;
-            ok = mbar_wait_hot(bar(LXB_QFULL), qn & 1u, abort_flag, 15);
+            ok = mbar_wait_lean(bar(LXB_QFULL), qn & 1u, abort_addr, 15);
             if (!ok) break;
             ++qn;
             for (int t = t0; t < t1; ++t, ++it) {
                 const uint32_t st = it % LX_KSTAGE, b = it & 1u;
-                ok = mbar_wait_hot(bar(LXB_KFULL + st), (it / LX_KSTAGE) & 1u, abort_flag, 16);
+                ok = mbar_wait_lean(bar(LXB_KFULL + st), (it / LX_KSTAGE) & 1u, abort_addr, 16);
                 if (!ok) break;
                 if (it >= 2) {
-                    ok = mbar_wait_hot(bar(LXB_DEMPTY + b), ((it >> 1) - 1) & 1u, abort_flag, 17);
+                    ok = mbar_wait_lean(bar(LXB_DEMPTY + b), ((it >> 1) - 1) & 1u, abort_addr, 17);
                     if (!ok) break;
                 }
                 tc_fence_after();
@@ -338,12 +339,20 @@ int launch_mqa_logits_tc(const uint8_t* q, const uint8_t* k, const float* k_scal
     const int groups = (s_q + LX_QG - 1) / LX_QG;
     const int nsm = sms[dev < 64 ? dev : 0];
     const int tiles = (s_k + LX_KT - 1) / LX_KT;
-    // About eight work items per SM, so that the CTAs finish together: with few query groups the
-    // key tiles are cut into runs (at least 8 tiles long, so that the q load and the pipeline fill
-    // stay a small share).
-    int chunks = groups >= 8 * nsm ? 1 : (8 * nsm + groups - 1) / groups;
-    if (chunks > (tiles + 7) / 8) chunks = (tiles + 7) / 8;
-    if (chunks < 1) chunks = 1;
+    // Query groups enough for eight items per SM: whole, the CTAs then finish together.  Fewer: the key tiles are cut into runs so that all
+    // CTAs get the same number of items in one to eight rounds, by what the longest share costs (an item pays about two tiles for its q
+    // and for filling and draining the pipeline): 16 tokens over 131072 keys in one run of 28 tiles per CTA instead of 512 of eight.
+    int chunks = 1;
+    if (groups < 8 * nsm) {
+        long long best = -1;
+        for (int r = 1; r <= 8; ++r) {
+            int c = r * nsm / groups;
+            if (c > (tiles + 7) / 8) c = (tiles + 7) / 8;
+            if (c < 1) c = 1;
+            const long long cost = (long long)((groups * c + nsm - 1) / nsm) * ((tiles + c - 1) / c + 2);
+            if (best < 0 || cost < best) { best = cost; chunks = c; }
+        }
+    }
     const int chunk_tiles = (tiles + chunks - 1) / chunks;
     const int items = groups * ((tiles + chunk_tiles - 1) / chunk_tiles);
     LogitsParams p{q, k, k_scale, weights, ks, ke, logits, status, s_q, num_heads, s_k, logits_stride, chunk_tiles};

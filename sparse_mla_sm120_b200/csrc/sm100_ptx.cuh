@@ -65,22 +65,9 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
     return ok != 0;
 }
 
-// Variant for waits on the critical path: every lane blocks in mbarrier.try_wait itself (the
-// hardware parks the thread until the phase completes or its own time limit passes), so the warp
-// resumes as soon as the barrier flips instead of after a sleep interval.  Same bounds and
-// give-up protocol as mbar_wait.
-__device__ __forceinline__ bool mbar_wait_hot(uint32_t bar, uint32_t parity, volatile int* abort, int code) {
-    uint32_t ok = 0;
-    for (uint32_t i = 0; i < WAIT_POLLS; ++i) {
-        if (mbar_try_wait(bar, parity, WAIT_HINT_NS)) { ok = 1; break; }
-        if ((i & 255u) == 255u && *abort != 0) break;
-    }
-    if (!ok) atomicCAS(const_cast<int*>(abort), 0, code);
-    return __all_sync(0xffffffffu, ok != 0);
-}
-
-// The same in as few instructions as it can have, for a kernel whose roles together are larger than the instruction caches: nearly always
-// the first poll, which the hardware suspends for up to 4 us, is the only one.  The warp decides by votes, so nothing here
+// The wait of the critical paths, in as few instructions as it can have (the roles of these kernels together are larger than the
+// instruction caches): every lane blocks in mbarrier.try_wait itself, nearly always the first poll, which the hardware
+// suspends until the phase completes or 4 us have passed, is the only one.  The warp decides by votes, so nothing here
 // diverges.  At most 2^20 polls, then `code` goes to the abort flag (given by its shared-memory address).
 __device__ __forceinline__ bool mbar_wait_lean(uint32_t bar, uint32_t parity, uint32_t abort_addr, int code) {
 #pragma unroll 1
