@@ -19,13 +19,22 @@ constexpr int WARPS = 8;
 // skipped unless OutT is float (then the single record is passed through).  Strided
 // (num_splits == null): every token has fixed_ns parts and part g of token t is record
 // g * batch + t, the layout an all-gather of per-GPU [T, H, 512] partials produces.
-// Four consecutive values of a partial record as fp32 (records are fp32, or fp16 where the attention kernel wrote them so).
-__device__ __forceinline__ float4 load4(const float* p) { return __ldcs(reinterpret_cast<const float4*>(p)); }
-__device__ __forceinline__ float4 load4(const __half* p) {
-    const uint2 v = __ldcs(reinterpret_cast<const uint2*>(p));
-    const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&v.x)), b = __half22float2(*reinterpret_cast<const __half2*>(&v.y));
-    return make_float4(a.x, a.y, b.x, b.y);
-}
+// Four consecutive values of a partial record, as they lie there and as fp32 (records are fp32, or fp16 where the attention kernel wrote
+// them so), and how many splits a lane asks for at once.
+template <typename T> struct Rec;
+template <> struct Rec<float> {
+    typedef float4 Raw;
+    static constexpr int AHEAD = 2;
+    static __device__ __forceinline__ float4 value(const float4& v) { return v; }
+};
+template <> struct Rec<__half> {
+    typedef uint2 Raw;
+    static constexpr int AHEAD = 4;
+    static __device__ __forceinline__ float4 value(const uint2& v) {
+        const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&v.x)), b = __half22float2(*reinterpret_cast<const __half2*>(&v.y));
+        return make_float4(a.x, a.y, b.x, b.y);
+    }
+};
 
 template <typename OutT, typename InT = float>
 __global__ void __launch_bounds__(WARPS * 32)
@@ -58,12 +67,27 @@ combine_kernel(const InT* __restrict__ o_accum, const float* __restrict__ lse_ac
     const float* lse_p = lse_accum + (size_t)s0 * num_heads + h;
     const InT* o_p = o_accum + (size_t)s0 * num_heads * D_V + (size_t)h * D_V + lane * 4;
 
-    float mx = NEG_BIG;
-    for (int s = lane; s < ns; s += 32) mx = fmaxf(mx, lse_p[(size_t)s * l_stride]);
+    // The first records are asked for before anything is known of their weights: the merge is a chain of latencies, the LSEs, their sum,
+    // the records, and this takes one of them out (one request cut into eight: 1 us of the step).
+    typedef Rec<InT> R;
+    constexpr int U = R::AHEAD;
+    typename R::Raw v[U][4];
+    auto load = [&](int s) {
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (s + u < ns) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) v[u][i] = __ldcs(reinterpret_cast<const typename R::Raw*>(o_p + (size_t)(s + u) * o_stride + i * 128));
+            }
+    };
+    load(0);
+    const float mine = lane < ns ? lse_p[(size_t)lane * l_stride] : NEG_BIG;      // of split `lane`
+    float mx = mine;
+    for (int s = lane + 32; s < ns; s += 32) mx = fmaxf(mx, lse_p[(size_t)s * l_stride]);
     mx = warp_max(mx);
     if (mx == NEG_BIG) mx = 0.f;
-    float sum = 0.f;
-    for (int s = lane; s < ns; s += 32) sum += exp2f(lse_p[(size_t)s * l_stride] - mx);
+    float sum = lane < ns ? exp2f(mine - mx) : 0.f;
+    for (int s = lane + 32; s < ns; s += 32) sum += exp2f(lse_p[(size_t)s * l_stride] - mx);
     sum = warp_sum(sum);
     float lse = (sum > 0.f) ? (log2f(sum) + mx) : NEG_BIG;
     // Weights are taken against the sink-free LSE; the sink then only scales the result.
@@ -94,30 +118,33 @@ combine_kernel(const InT* __restrict__ o_accum, const float* __restrict__ lse_ac
     float4 acc[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-    int s = 0;
-    for (; s + 1 < ns; s += 2) {
-        float4 a[4], b[4];
+    const float w_mine = exp2f(mine - lse_w) * sink_scale;
+    auto weight = [&](int s) {
+        const float w = __shfl_sync(0xffffffffu, w_mine, s & 31);
+        return s < 32 ? w : exp2f(lse_p[(size_t)s * l_stride] - lse_w) * sink_scale;
+    };
+    for (int s = 0; s < ns; s += U) {
+        if (s > 0) load(s);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            a[i] = load4(o_p + (size_t)s * o_stride + i * 128);
-            b[i] = load4(o_p + (size_t)(s + 1) * o_stride + i * 128);
-        }
-        const float wa = exp2f(lse_p[(size_t)s * l_stride] - lse_w) * sink_scale;
-        const float wb = exp2f(lse_p[(size_t)(s + 1) * l_stride] - lse_w) * sink_scale;
+        for (int u = 0; u < U; u += 2) {
+            if (s + u + 1 < ns) {
+                const float wa = weight(s + u), wb = weight(s + u + 1);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            acc[i].x += wa * a[i].x + wb * b[i].x;
-            acc[i].y += wa * a[i].y + wb * b[i].y;
-            acc[i].z += wa * a[i].z + wb * b[i].z;
-            acc[i].w += wa * a[i].w + wb * b[i].w;
-        }
-    }
-    if (s < ns) {
-        const float wa = exp2f(lse_p[(size_t)s * l_stride] - lse_w) * sink_scale;
+                for (int i = 0; i < 4; ++i) {
+                    const float4 a = R::value(v[u][i]), b = R::value(v[u + 1][i]);
+                    acc[i].x += wa * a.x + wb * b.x;
+                    acc[i].y += wa * a.y + wb * b.y;
+                    acc[i].z += wa * a.z + wb * b.z;
+                    acc[i].w += wa * a.w + wb * b.w;
+                }
+            } else if (s + u < ns) {
+                const float wa = weight(s + u);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const float4 a = load4(o_p + (size_t)s * o_stride + i * 128);
-            acc[i].x += wa * a.x; acc[i].y += wa * a.y; acc[i].z += wa * a.z; acc[i].w += wa * a.w;
+                for (int i = 0; i < 4; ++i) {
+                    const float4 a = R::value(v[u][i]);
+                    acc[i].x += wa * a.x; acc[i].y += wa * a.y; acc[i].z += wa * a.z; acc[i].w += wa * a.w;
+                }
+            }
         }
     }
     if constexpr (F32) {
