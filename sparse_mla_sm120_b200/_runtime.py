@@ -239,7 +239,10 @@ def pick_split_duo(num_tokens: int, sms: int, blocks_per_token: int, uniform: bo
     """(partitions, fixed overhead) where whole requests and equal partitions run on attn_duo_kernel and partitions of the
     scheduler on the pair kernel.  Ragged requests are left whole where the scheduler and combine launches and the partitions that
     straddle two requests cost more than the longest request: lists of up to 16 blocks (8 of up to 1024 entries 22.9 us whole, 26.9
-    cut; of up to 2048 33.0 and 29.0), and from a third of the pairs on (24 of up to 2048: 39.0 whole, 46.3 cut; 20: 39.2 and 35.1)."""
+    cut; of up to 2048 33.0 and 29.0), and from a third of the pairs on (24 of up to 2048: 39.0 whole, 46.3 cut; 20: 39.2 and 35.1).
+    Otherwise they are cut into partitions of eight of the list's blocks (lengths are shorter, and a partition that is nearly all fixed part
+    gains nothing: 8 of up to 2048 in 32 partitions 29.0 us, in 64 34.9; 13 in 52 31.0, in 74 35.2), or into as many as there are
+    pairs of SMs when that is nearly as many (16: 44.1 in 64, 35.3 in 74)."""
     n = max(blocks_per_token, 1)
     max_pairs = max(sms // CTAS_PER_PART, 1)
     whole = (num_tokens, FIXED_OVERHEAD)
@@ -249,6 +252,9 @@ def pick_split_duo(num_tokens: int, sms: int, blocks_per_token: int, uniform: bo
         return whole if k == 1 else (k * num_tokens, 0)
     if n <= 16 or 3 * num_tokens >= max_pairs - 2:
         return whole
+    if not uniform:
+        parts = max(-(-num_tokens * n // 8), 8)
+        return max(num_tokens, parts if 4 * parts <= 3 * max_pairs else max_pairs), FIXED_OVERHEAD
     return pick_num_sm_parts(num_tokens, sms, blocks_per_token), FIXED_OVERHEAD
 
 
