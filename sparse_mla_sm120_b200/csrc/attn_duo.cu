@@ -168,7 +168,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(DUO_THREADS, 1) attn
     tc_fence_after();
     const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(sm + MISC_OFF);
 
-    grid_dep_launch();                                // (the kernel after this one may start its own prologue)
+    // Everything above needs nothing from the kernels before this one, and the one after it may start its own prologue.
+    grid_dep_wait();
+    grid_dep_launch();
     SchedMeta meta;
     int first, step, last;
     if (p.uniform_k > 1) {
@@ -936,7 +938,7 @@ int launch_attn_duo(const AttnParams& p, cudaStream_t stream) {
     if (int e = rows_tensor_map(p.kv, &map)) return e;
     const int max_pairs = sm_count[dev] >= 2 ? sm_count[dev] / 2 : 1;
     const int parts = p.uniform_k > 1 ? p.uniform_k * p.num_tokens : (p.num_tokens < max_pairs ? p.num_tokens : max_pairs);
-    attn_duo_kernel<<<2 * parts, DUO_THREADS, SMEM_ALLOC, stream>>>(p, map);
+    launch_dependent(attn_duo_kernel, dim3(2 * parts), dim3(DUO_THREADS), SMEM_ALLOC, stream, p, map);
     return check_launch("attn_duo_kernel");
 }
 

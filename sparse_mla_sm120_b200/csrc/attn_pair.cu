@@ -1075,10 +1075,7 @@ int launch_pair_instance(const AttnParams& p, cudaStream_t stream) {
     const int max_pairs = sm_count[dev] >= 2 ? sm_count[dev] / 2 : 1;
     const int parts = p.sched ? p.num_parts : p.uniform_k > 1 ? p.uniform_k * p.num_tokens
                                                               : (p.num_tokens < max_pairs ? p.num_tokens : max_pairs);
-    if (p.sched != nullptr)      // the scheduler kernel runs just before: start while it finishes
-        launch_dependent(attn_pair_kernel<LAYOUT, EXTRA, STAGE_Q>, dim3(2 * parts), dim3(PAIR_THREADS), SMEM_ALLOC, stream, p);
-    else
-        attn_pair_kernel<LAYOUT, EXTRA, STAGE_Q><<<2 * parts, PAIR_THREADS, SMEM_ALLOC, stream>>>(p);
+    launch_dependent(attn_pair_kernel<LAYOUT, EXTRA, STAGE_Q>, dim3(2 * parts), dim3(PAIR_THREADS), SMEM_ALLOC, stream, p);
     return check_launch("attn_pair_kernel");
 }
 

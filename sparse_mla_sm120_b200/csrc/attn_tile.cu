@@ -743,8 +743,7 @@ int launch_attn_tile(const AttnParams& p, cudaStream_t stream) {
     const int parts = p.sched ? p.num_parts : p.uniform_k > 1 ? p.uniform_k * p.num_tokens : (p.num_tokens < sm_count[dev] ? p.num_tokens : sm_count[dev]);
     const dim3 grid(parts);
     auto* kernel = p.out_max_logits != nullptr ? attn_tile_kernel<true> : attn_tile_kernel<false>;
-    if (p.sched != nullptr) launch_dependent(kernel, grid, dim3(T_THREADS), T_SMEM, stream, p, map);
-    else kernel<<<grid, T_THREADS, T_SMEM, stream>>>(p, map);
+    launch_dependent(kernel, grid, dim3(T_THREADS), T_SMEM, stream, p, map);
     return check_launch("attn_tile_kernel");
 }
 

@@ -46,6 +46,7 @@ combine_kernel(const InT* __restrict__ o_accum, const float* __restrict__ lse_ac
     constexpr bool F32 = sizeof(OutT) == 4;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t row = (int64_t)blockIdx.x * WARPS + warp;   // (token, head)
+    grid_dep_launch();    // the kernel after this one may start its own prologue
     grid_dep_wait();      // the partials of the attention kernel before this one are complete
     if (row >= (int64_t)batch * num_heads) return;
     const int tok = (int)(row / num_heads), h = (int)(row % num_heads);

@@ -91,6 +91,12 @@ __device__ __forceinline__ float warp_sum(float v) {
 // when that kernel has completed and its writes are visible.  A kernel that calls grid_dep_launch() lets the next
 // one start early.  Both are no-ops in a kernel that was launched the ordinary way.  The reference uses the same
 // mechanism between its scheduler, decode and combine kernels (csrc/kernel/decode/decode_launch.cu:46-49).
+//
+// The rule that makes a chain of such kernels safe: before grid_dep_wait() a kernel touches only its parameters, its
+// shared memory and its tensor memory, and every thread of it passes the wait before it ends.  Then a kernel that has
+// completed says that all before it on the stream have, so that scratch and results of earlier calls may be read and
+// written after the wait.  A kernel early on the SMs cannot hold up what it waits for: it is only launched once all
+// blocks of the kernel before it run or have ended.
 __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
