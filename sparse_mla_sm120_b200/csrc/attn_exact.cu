@@ -577,8 +577,7 @@ int launch_attn_exact(const AttnParams& p, cudaStream_t stream) {
     const int most = sm_count[dev] / halves > 0 ? sm_count[dev] / halves : 1;
     const int parts = p.sched ? p.num_parts : (p.num_tokens < most ? p.num_tokens : most);
     const dim3 grid(parts, halves);
-    if (p.sched != nullptr) launch_dependent(attn_exact_kernel, grid, dim3(X_THREADS), X_SMEM, stream, p);
-    else attn_exact_kernel<<<grid, X_THREADS, X_SMEM, stream>>>(p);
+    launch_dependent(attn_exact_kernel, grid, dim3(X_THREADS), X_SMEM, stream, p);
     return check_launch("attn_exact_kernel");
 }
 

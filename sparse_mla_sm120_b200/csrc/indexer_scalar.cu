@@ -292,6 +292,8 @@ topk_select_kernel(const float* __restrict__ logits, const int32_t* __restrict__
     __shared__ int last_col_s;
     __shared__ int cw[TS_WARPS], cc[TS_WARPS], wsum[TS_WARPS];
 
+    grid_dep_launch();
+    grid_dep_wait();
     const int row = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const float* x = logits + (size_t)row * logits_stride;
     int lo = ks ? max(ks[row], 0) : 0;
@@ -588,6 +590,8 @@ topk_cluster_kernel(const float* __restrict__ logits, const int32_t* __restrict_
     __shared__ uint32_t kmin_s, kmax_s, last_key_s;
     __shared__ int last_col_s;
 
+    grid_dep_launch();
+    grid_dep_wait();
     const int row = blockIdx.x / TC_CTAS, rank = blockIdx.x % TC_CTAS;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int vw = warp / TC_SUB, sub = warp % TC_SUB, vwarp = rank * TC_VW + vw;
@@ -985,11 +989,11 @@ int launch_topk(const float* logits, const int32_t* ks, const int32_t* ke, int32
     }
     const int n = sms[dev < 64 ? dev : 0];
     if (num_rows <= clusters[dev < 64 ? dev : 0])  // a cluster per row, all at once (one row more takes a second wave: 17 -> 26 us)
-        topk_cluster_kernel<<<num_rows * TC_CTAS, TC_THREADS, TC_SMEM, stream>>>(logits, ks, ke, out, num_cols, logits_stride, k, emit);
+        launch_dependent(topk_cluster_kernel, dim3(num_rows * TC_CTAS), dim3(TC_THREADS), TC_SMEM, stream, logits, ks, ke, out, num_cols, logits_stride, k, emit);
     else if (num_rows <= n)                        // every row has an SM to itself
-        topk_select_kernel<1024><<<num_rows, 1024, TS_SMEM, stream>>>(logits, ks, ke, out, num_cols, logits_stride, k, emit);
+        launch_dependent(topk_select_kernel<1024>, dim3(num_rows), dim3(1024), TS_SMEM, stream, logits, ks, ke, out, num_cols, logits_stride, k, emit);
     else
-        topk_select_kernel<512><<<num_rows, 512, TS_SMEM, stream>>>(logits, ks, ke, out, num_cols, logits_stride, k, emit);
+        launch_dependent(topk_select_kernel<512>, dim3(num_rows), dim3(512), TS_SMEM, stream, logits, ks, ke, out, num_cols, logits_stride, k, emit);
     return check_launch("topk_select_kernel");
 }
 

@@ -94,6 +94,8 @@ __global__ void __launch_bounds__(LX_THREADS, 1) mqa_logits_tc_kernel(const Logi
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    grid_dep_wait();
+    grid_dep_launch();
 
     const int num_groups = (p.s_q + LX_QG - 1) / LX_QG;
     // key tiles a group needs: up to the largest ke of its queries (and from the smallest ks)
@@ -357,8 +359,7 @@ int launch_mqa_logits_tc(const uint8_t* q, const uint8_t* k, const float* k_scal
     const int items = groups * ((tiles + chunk_tiles - 1) / chunk_tiles);
     LogitsParams p{q, k, k_scale, weights, ks, ke, logits, status, s_q, num_heads, s_k, logits_stride, chunk_tiles};
     const int grid = items < nsm ? items : nsm;
-    if (num_heads == 64) mqa_logits_tc_kernel<64><<<grid, LX_THREADS, LX_SMEM, stream>>>(p, qmap, kmap);
-    else mqa_logits_tc_kernel<32><<<grid, LX_THREADS, LX_SMEM, stream>>>(p, qmap, kmap);
+    launch_dependent(num_heads == 64 ? mqa_logits_tc_kernel<64> : mqa_logits_tc_kernel<32>, dim3(grid), dim3(LX_THREADS), LX_SMEM, stream, p, qmap, kmap);
     return check_launch("mqa_logits_tc_kernel");
 }
 

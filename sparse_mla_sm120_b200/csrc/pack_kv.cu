@@ -18,6 +18,8 @@ __device__ __forceinline__ float pow2_ceil(float x) {   // smallest power of two
 
 __global__ void __launch_bounds__(256) pack_kv_kernel(const __nv_bfloat16* __restrict__ kv,
                                                       uint8_t* __restrict__ packed, int64_t rows) {
+    grid_dep_launch();
+    grid_dep_wait();
     const int lane = threadIdx.x & 31;
     const int64_t row = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
     if (row >= rows) return;
@@ -64,7 +66,7 @@ __global__ void __launch_bounds__(256) pack_kv_kernel(const __nv_bfloat16* __res
 int launch_pack_kv(const __nv_bfloat16* kv, uint8_t* packed, int64_t num_rows, cudaStream_t stream) {
     if (num_rows == 0) return 0;
     const unsigned grid = (unsigned)((num_rows + 7) / 8);
-    pack_kv_kernel<<<grid, 256, 0, stream>>>(kv, packed, num_rows);
+    launch_dependent(pack_kv_kernel, dim3(grid), dim3(256), 0, stream, kv, packed, num_rows);
     return check_launch("pack_kv_kernel");
 }
 

@@ -23,6 +23,7 @@ struct SchedArgs {
 
 __global__ void __launch_bounds__(32) sched_meta_kernel(const SchedArgs a) {
     grid_dep_launch();   // the attention kernel may start its prologue; it waits for this kernel before it reads the records
+    grid_dep_wait();
     extern __shared__ int sh[];
     int* nblk = sh;                    // [b]   blocks of request i
     int* nsp = sh + a.b;               // [b+1] nsp[i+1] = splits of request i, then their prefix sum
@@ -121,7 +122,7 @@ int launch_sched_meta(int b, int topk, int extra_topk, int num_sm_parts, int fix
             big_smem[dev] = true;
         }
     }
-    sched_meta_kernel<<<1, 32, smem, stream>>>(a);
+    launch_dependent(sched_meta_kernel, dim3(1), dim3(32), smem, stream, a);
     return check_launch("sched_meta_kernel");
 }
 
