@@ -1,4 +1,6 @@
-// Sparse-MLA attention on a pair of SMs (sm_100a): split-KV decode and prefill, tcgen05.mma.cta_group::2.
+// Sparse-MLA attention on a pair of SMs (sm_100a): split-KV decode and prefill, tcgen05.mma.cta_group::2.  Over linear arrays of 656-byte
+// rows attn_tile.cu and attn_duo.cu take what they are faster at (launch_attn_pair); this kernel has the scheduler's partitions of more
+// than 64 heads, many short requests of as many heads, pages with padding between them, MODEL1 pages and a second cache.
 //
 // Work unit.  A cluster of two CTAs owns one scheduler partition (a run of 64-token blocks of
 // consecutive requests, see sched.cu; without a scheduler: a contiguous share of the requests).  Every

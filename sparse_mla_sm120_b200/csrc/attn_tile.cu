@@ -1,12 +1,13 @@
 // Sparse-MLA attention of up to 64 query heads over packed 656-byte rows (sm_100a): split-KV decode and prefill, one CTA per
 // partition (a run of 64-token blocks of consecutive requests, see sched.cu; without a scheduler every parts-th request).
 //
-// Why not the pair kernel: it spends two CTAs on a partition whatever the number of heads, copies every row through registers
-// and splits the work over half as many partitions.  48 requests of top-k 2048 at 16 heads: 45.1 us there, 32.8 us here; 1237
-// ragged prompt tokens of top-k 1024 at 64 heads: 395 us there, 175 us here.  At 128 heads two of these CTAs would gather every
-// row twice: 2400 us against 2238 us for 4096 tokens of top-k 2048, so the pair kernel keeps those.
+// Why not two CTAs as in attn_pair.cu and attn_duo.cu: they spend both on a partition whatever the number of heads and split the work
+// over half as many partitions.  48 requests of top-k 2048 at 16 heads: 45.1 us in attn_pair_kernel, 28.0 us here; 1237 ragged prompt
+// tokens of top-k 1024 at 64 heads: 395 us there, 163 us here.  At 128 heads two of these CTAs would gather every row twice: 2400 us for
+// 4096 tokens of top-k 2048, against 1815 us in attn_duo_kernel.
 //
-// What bounds it (clock64 at 64 heads, 1.9 GHz): a tile of 128 tokens takes 4300 cycles, half of the way of a tile from the load
+// What bounds it (clock64 at 64 heads, 1.9 GHz, before the copies were issued from indices in shared memory and the MMAs from loops, which
+// took 48 requests from 32.8 to 30.7 us and the ragged prompt from 175 to 165): a tile of 128 tokens takes 4300 cycles, half of the way of a tile from the load
 // of its rows (2000 cycles: the gather delivers 35 bytes per cycle and SM) over its scores (2100, with the hand-overs) and its
 // weights (2700) to P.V (1300), because two tiles are all that shared memory holds.  A request costs another 15000 cycles for its
 // q and its epilogue, which the softmax warps do in between.  Tried without gain: sixteen softmax warps (2485 us where
@@ -701,13 +702,15 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
 }  // namespace
 
 // Whole requests that each get a pair of SMs to themselves take as long as one request does, and two CTAs walk a long list
-// faster than one.  us of this kernel / of the pair kernel, 8 to 74 requests that use all of their list:
-//     above 32 heads             512 entries 18.8-20.6 / 18.8-20.9, 768: 22.9-25.1 / 22.9-25.3, 1024: 27.7-31.2 / 27.0-30.6, 2048: 45.5-51.4 / 42.6-47.5
-//       with maximum logits      256: 16.2-16.7 / 16.7-16.8, 512: 20.8-21.3 / 18.8-20.8, 2048: 45.7-55.6 / 42.5-47.6
-//     up to 32 heads             512: 16.8-18.1 / 18.8-20.8, 2048: 40.2-44.9 / 41.4-47.4 (never)
-//       with maximum logits      768: 22.9-24.8 / 22.5-25.0, 1024: 27.0-29.2 / 25.4-29.1, 2048: 44.2-49.0 / 41.4-47.5
-// With more requests than pairs the pair kernel needs another round: 80 requests of 2048 entries 51.4 / 86.6.
-static bool pair_is_faster(const AttnParams& p) {
+// faster than one (attn_duo.cu).  us of this kernel / of attn_duo_kernel, rows in HBM:
+//   with maximum logits, 64 heads   8 requests of 256 entries 12.8 / 10.5, 512: 17.3 / 13.5, 1024: 26.0 / 19.2, 2048: 43.6 / 30.0;
+//                                   74 of 128: 10.7 / 10.4, 512: 18.5 / 15.0, 2048: 47.1 / 33.0
+//                        16 heads   8 of 256 10.3 / 9.9, 1024: 22.6 / 18.5, 2048: 38.5 / 29.3; 74 of 256 11.1 / 11.5, 512: 15.1 / 14.5
+//   without them, 64 heads          74 of 128 10.3 / 10.4, 512: 17.7 / 15.0, 768: 22.3 / 17.9
+// So the line could lie lower.  It lies where two CTAs took these calls already, because shorter lists would lose something: here the
+// weights carry the scale of every block of 128 dims, there a block of V far below its group's scale is shifted into e4m3's subnormals.
+// With more requests than pairs of SMs two CTAs need another round: 80 requests of 2048 entries took 51 here and 87 there.
+static bool duo_is_faster(const AttnParams& p) {
     if (p.sched != nullptr || p.uniform_k > 1 || p.num_tokens > smla_num_sms() / 2) return false;
     const int blocks = (p.topk + BLOCK_N - 1) / BLOCK_N;
     if (p.num_heads > 32) return blocks >= (p.out_max_logits != nullptr ? 8 : 12);
@@ -716,7 +719,7 @@ static bool pair_is_faster(const AttnParams& p) {
 
 // One linear array of 656-byte rows (pages without padding between them) and one CTA's worth of heads.
 bool attn_tile_takes(const AttnParams& p) {
-    return !pair_is_faster(p) && p.num_heads <= T_HEADS && one_linear_array(p);
+    return !duo_is_faster(p) && p.num_heads <= T_HEADS && one_linear_array(p);
 }
 
 int launch_attn_tile(const AttnParams& p, cudaStream_t stream) {

@@ -5,7 +5,7 @@
 // left untouched (the decode kernel wrote their bf16 output directly), optional per-head sink
 // folded into the merged LSE.  The kernel is HBM-bound: it reads splits * 2 KB per (token, head)
 // and writes 1 KB.  One warp owns one (token, head) row, 16 floats per lane per split as four
-// 16-byte loads, two splits in flight per iteration.
+// 16-byte loads, two splits in flight per iteration (four where records are fp16), the first of them before the weights are known.
 #include "common.cuh"
 
 namespace smla {

@@ -96,7 +96,8 @@ __device__ __forceinline__ float warp_sum(float v) {
 // shared memory and its tensor memory, and every thread of it passes the wait before it ends.  Then a kernel that has
 // completed says that all before it on the stream have, so that scratch and results of earlier calls may be read and
 // written after the wait.  A kernel early on the SMs cannot hold up what it waits for: it is only launched once all
-// blocks of the kernel before it run or have ended.
+// blocks of the kernel before it run or have ended.  A decode step behind another one in a graph: one request 16.5 -> 15.2 us,
+// 64 requests 34.6 -> 33.2 (rows in L2); behind a kernel that does not let the next one start early, 17.6 -> 17.3 and 36.1 -> 36.2.
 __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

@@ -35,13 +35,6 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity, uin
     return ok != 0;
 }
 
-// Has the phase with the given parity completed?  Never suspends.
-__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-    return ok != 0;
-}
-
 // Warp-wide wait for the phase with the given parity.  Lane 0 polls (32 lanes polling one
 // mbarrier only add shared-memory traffic), the warp reconverges on the result.  The wait gives
 // up after a bounded number of polls (about half a second) or as soon as another thread of the
