@@ -238,11 +238,12 @@ def _duo_us(num_tokens: int, blocks: int, k: int, max_pairs: int) -> float:
 def pick_split_duo(num_tokens: int, sms: int, blocks_per_token: int, uniform: bool) -> Tuple[int, int]:
     """(partitions, fixed overhead) where whole requests and equal partitions run on attn_duo_kernel and partitions of the
     scheduler on the pair kernel.  Ragged requests are left whole where the scheduler and combine launches and the partitions that
-    straddle two requests cost more than the longest request: lists of up to 16 blocks (8 of up to 1024 entries 22.9 us whole, 26.9
-    cut; of up to 2048 33.0 and 29.0), and from a third of the pairs on (24 of up to 2048: 39.0 whole, 46.3 cut; 20: 39.2 and 35.1).
-    Otherwise they are cut into partitions of eight of the list's blocks (lengths are shorter, and a partition that is nearly all fixed part
-    gains nothing: 8 of up to 2048 in 32 partitions 29.0 us, in 64 34.9; 13 in 52 31.0, in 74 35.2), or into as many as there are
-    pairs of SMs when that is nearly as many (16: 44.1 in 64, 35.3 in 74)."""
+    straddle two requests cost more than the longest request: lists of up to 16 blocks, and from half as many requests on as a
+    list has blocks (us whole / cut, rows in HBM: 16 requests of up to 1024 entries 21.7 / 28.1; 8 of up to 1536 27.1 / 26.8, 13: 27.6 /
+    29.7; 13 of up to 2048 33.6 / 30.7, 16: 33.5 / 34.1, 20: 34.1 / 39.6; 24 of up to 4096 59.4 / 54.6, 30: 60.1 / 60.4).  Otherwise the
+    general rule cuts them into partitions of four blocks, as many as there are pairs of SMs at most; partitions of eight blocks
+    take longer now that launches run under one another (4 requests of up to 2048 25.1 in 32, 27.2 in 16; 13: 30.7 in 74, 34.0 in
+    52; 8: 29.3 and 29.6)."""
     n = max(blocks_per_token, 1)
     max_pairs = max(sms // CTAS_PER_PART, 1)
     whole = (num_tokens, FIXED_OVERHEAD)
@@ -250,11 +251,8 @@ def pick_split_duo(num_tokens: int, sms: int, blocks_per_token: int, uniform: bo
     if uniform and (cuts or n < 2 * BLOCKS_PER_PARTITION):
         k = min([1] + cuts, key=lambda c: _duo_us(num_tokens, n, c, max_pairs))
         return whole if k == 1 else (k * num_tokens, 0)
-    if n <= 16 or 3 * num_tokens >= max_pairs - 2:
+    if n <= 16 or 2 * num_tokens >= n:
         return whole
-    if not uniform:
-        parts = max(-(-num_tokens * n // 8), 8)
-        return max(num_tokens, parts if 4 * parts <= 3 * max_pairs else max_pairs), FIXED_OVERHEAD
     return pick_num_sm_parts(num_tokens, sms, blocks_per_token), FIXED_OVERHEAD
 
 

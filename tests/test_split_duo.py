@@ -19,6 +19,6 @@ def test_equal_cuts_divide_the_blocks_and_fit_the_machine(blocks):
 def test_ragged_requests():
     assert pick_split_duo(8, 148, 16, False) == (8, FIXED_OVERHEAD)          # short lists stay whole
     assert pick_split_duo(8, 148, 17, False)[0] > 8
-    assert pick_split_duo(23, 148, 32, False)[0] > 23
-    assert pick_split_duo(24, 148, 32, False) == (24, FIXED_OVERHEAD)        # a third of the pairs
+    assert pick_split_duo(15, 148, 32, False) == (74, FIXED_OVERHEAD)
+    assert pick_split_duo(16, 148, 32, False) == (16, FIXED_OVERHEAD)        # half as many as a list has blocks
     assert pick_split_duo(1, 148, 32, True) == (8, 0) and pick_split_duo(64, 148, 32, True) == (64, FIXED_OVERHEAD)
