@@ -42,9 +42,6 @@ NSETS = 8   # rotating (q, indices) sets so that consecutive steps gather differ
 SM_SCALE = D_QK ** -0.5
 WORKLOAD = ("V3.2-shape sparse-MLA decode: b=64/GPU, s_q=1, h_q=128, topk=2048, d_qk=576, d_v=512, "
             "KV len U[4096,32768], paged block 64, packed FP8 656 B rows")
-# DRAM bytes of one launch of the attention kernel on this workload's shape, from one ncu capture
-# (dram__bytes_read.sum + dram__bytes_write.sum); the capture's summary is kept with the other profiles.
-NCU_TRAFFIC_BYTES = 90_347_008
 CPU_SAMPLE_REQUESTS = 64   # requests of one step that the CPU legs compute: the whole step (about 0.13 s on 16 host threads)
 
 
@@ -367,9 +364,9 @@ def run_ours(args):
                     "note": "paged KV cache is device-resident state; q and indices come from pinned host memory, output and LSE go "
                             "back, every step; copies and kernel of neighbouring steps overlap on three streams"},
             "gpu_launches": launches_per_step * args.steps,
-            "roofline": {"bound": "hbm", "kernel": "attn_pair_kernel", "achieved": bytes_step / k_secs / 1e9, "peak": hbm_peak,
+            "roofline": {"bound": "hbm", "kernel": "attn_duo_kernel", "achieved": bytes_step / k_secs / 1e9, "peak": hbm_peak,
                          "unit": "GB/s", "frac": bytes_step / k_secs / 1e9 / hbm_peak, "peak_kind": f"of {peak_kind}",
-                         "kernel_us": k_secs * 1e6, "traffic": NCU_TRAFFIC_BYTES,
+                         "kernel_us": k_secs * 1e6, "traffic": None,
                          "frac_of_8TBs_nominal": bytes_step / k_secs / 8e12},
             "cpu_baseline": cpu, "clocks": clocks, "extras": extras,
         }
@@ -544,7 +541,7 @@ def run_extras(device, hbm_peak, bf16_peak, peak_kind):
     cpu_s = _cpu_attention_slice(q, kv, idx, cpu_tokens)
     out["prefill"] = {
         "workload": "s_q=4096, h=128, topk=2048, KV 8192 rows, causal top-k", "ms": ms, "tflops": flops / ms / 1e9,
-        "roofline": {"bound": "tensor", "kernel": "attn_pair_kernel", "achieved": flops / ms / 1e9, "peak": bf16_peak, "unit": "TFLOP/s",
+        "roofline": {"bound": "tensor", "kernel": "attn_duo_kernel", "achieved": flops / ms / 1e9, "peak": bf16_peak, "unit": "TFLOP/s",
                      "frac": flops / ms / 1e9 / bf16_peak, "peak_kind": f"of {peak_kind} (dense BF16; the kernel's MMAs are FP8)",
                      "traffic": None},
         "cpu_baseline": {"value": flops * cpu_tokens / s_q / cpu_s / 1e12, "unit": "TFLOP/s", "cores": os.cpu_count(), "kind": "port",
@@ -561,7 +558,7 @@ def run_extras(device, hbm_peak, bf16_peak, peak_kind):
     out["prefill_causal_padded"] = {
         "workload": "s_q=4096 from the start of a sequence: token i has min(i+1, 2048) entries, the rest of its list is -1",
         "ms": ms_c, "valid_entries": valid, "tflops": fl_c / ms_c / 1e9,
-        "roofline": {"bound": "tensor", "kernel": "attn_pair_kernel", "achieved": fl_c / ms_c / 1e9, "peak": bf16_peak, "unit": "TFLOP/s",
+        "roofline": {"bound": "tensor", "kernel": "attn_duo_kernel", "achieved": fl_c / ms_c / 1e9, "peak": bf16_peak, "unit": "TFLOP/s",
                      "frac": fl_c / ms_c / 1e9 / bf16_peak, "peak_kind": f"of {peak_kind} (dense BF16; flops of valid entries only)",
                      "traffic": None}}
     del q, idx, idx_c, kv
@@ -587,7 +584,7 @@ def run_extras(device, hbm_peak, bf16_peak, peak_kind):
         out["decode_mtp_sq2"] = {
             "workload": "the headline's decode with s_q=2: 64 requests x 2 query tokens, h=128, topk=2048, through flash_mla_with_kvcache",
             "us_per_step": ms2 * 1e3, "num_sm_parts": meta.num_sm_parts,
-            "roofline": {"bound": "hbm", "kernel": "attn_pair_kernel", "achieved": by2 / ms2 / 1e6, "peak": hbm_peak, "unit": "GB/s",
+            "roofline": {"bound": "hbm", "kernel": "attn_duo_kernel", "achieved": by2 / ms2 / 1e6, "peak": hbm_peak, "unit": "GB/s",
                          "frac": by2 / ms2 / 1e6 / hbm_peak, "peak_kind": f"of {peak_kind}", "traffic": None,
                          "note": "whole step (CUDA graph replay), algorithmic bytes count each token's gathered rows"}}
         # ---- small decode batches of the same shape (the split-KV path: scheduler + attention + combine as
