@@ -42,6 +42,9 @@ NSETS = 8   # rotating (q, indices) sets so that consecutive steps gather differ
 SM_SCALE = D_QK ** -0.5
 WORKLOAD = ("V3.2-shape sparse-MLA decode: b=64/GPU, s_q=1, h_q=128, topk=2048, d_qk=576, d_v=512, "
             "KV len U[4096,32768], paged block 64, packed FP8 656 B rows")
+# DRAM bytes of one launch of the attention kernel on this workload's shape (dram__bytes_read.sum + dram__bytes_write.sum of a capture
+# of `--case decode`): the rows, q and the outputs once.
+NCU_TRAFFIC_BYTES = 85_335_040 + 2_774_784
 CPU_SAMPLE_REQUESTS = 64   # requests of one step that the CPU legs compute: the whole step (about 0.13 s on 16 host threads)
 
 
@@ -366,7 +369,7 @@ def run_ours(args):
             "gpu_launches": launches_per_step * args.steps,
             "roofline": {"bound": "hbm", "kernel": "attn_duo_kernel", "achieved": bytes_step / k_secs / 1e9, "peak": hbm_peak,
                          "unit": "GB/s", "frac": bytes_step / k_secs / 1e9 / hbm_peak, "peak_kind": f"of {peak_kind}",
-                         "kernel_us": k_secs * 1e6, "traffic": None,
+                         "kernel_us": k_secs * 1e6, "traffic": NCU_TRAFFIC_BYTES,
                          "frac_of_8TBs_nominal": bytes_step / k_secs / 8e12},
             "cpu_baseline": cpu, "clocks": clocks, "extras": extras,
         }
