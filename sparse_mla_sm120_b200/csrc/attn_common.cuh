@@ -69,10 +69,10 @@ __device__ __forceinline__ int fetch_entry(const AttnParams& p, const Work& w, i
     if (b >= w.blk0 + w.nblk) return -1;
     if (b < w.main_blocks) {
         const int pos = b * BLOCK_N + r;
-        return pos < w.len ? __ldg(p.indices + (size_t)w.req * p.topk + pos) : -1;
+        return pos < w.len ? ld_in(p.indices + (size_t)w.req * p.topk + pos) : -1;
     }
     const int pos = (b - w.main_blocks) * BLOCK_N + r;
-    return pos < w.extra_len ? __ldg(p.extra_indices + (size_t)w.req * p.extra_topk + pos) : -1;
+    return pos < w.extra_len ? ld_in(p.extra_indices + (size_t)w.req * p.extra_topk + pos) : -1;
 }
 
 constexpr int TILE_N = 128;   // tokens per tile of the kernels that gather by TMA: two scheduler blocks
@@ -86,7 +86,7 @@ struct Walk {
     __device__ __forceinline__ Walk(const AttnParams& p, int first, int step_, int last_) : req(first - step_), step(step_), last(last_), j(0), nst(0) {
         next_len = first <= last_ ? length(p, first) : 0;
     }
-    __device__ __forceinline__ static int length(const AttnParams& p, int r) { return p.topk_length ? __ldg(p.topk_length + r) : p.topk; }
+    __device__ __forceinline__ static int length(const AttnParams& p, int r) { return p.topk_length ? ld_in(p.topk_length + r) : p.topk; }
     __device__ __forceinline__ bool next_request(const AttnParams& p, const SchedMeta& m) {
         int b0, b1;
         do {
@@ -110,7 +110,7 @@ struct Walk {
     // Row r of the current tile: its index in the cache, -1 where there is no entry.
     __device__ __forceinline__ int row_index(const AttnParams& p, int r) const {
         const int pos = pos0 + j * TILE_N + r;
-        return pos < lim ? __ldg(p.indices + (size_t)req * p.topk + pos) : -1;
+        return pos < lim ? ld_in(p.indices + (size_t)req * p.topk + pos) : -1;
     }
 };
 

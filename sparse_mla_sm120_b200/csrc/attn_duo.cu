@@ -215,13 +215,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(DUO_THREADS, 1) attn
                 const int h = 4 * warp + k;
                 v[2 * k] = v[2 * k + 1] = make_uint4(0, 0, 0, 0);
                 if (h < live_heads) {
-                    v[2 * k] = __ldg(reinterpret_cast<const uint4*>(q0 + (size_t)h * D_QK + lane * 16));
-                    v[2 * k + 1] = __ldg(reinterpret_cast<const uint4*>(q0 + (size_t)h * D_QK + lane * 16 + 8));
+                    v[2 * k] = ld_in(reinterpret_cast<const uint4*>(q0 + (size_t)h * D_QK + lane * 16));
+                    v[2 * k + 1] = ld_in(reinterpret_cast<const uint4*>(q0 + (size_t)h * D_QK + lane * 16 + 8));
                 }
             }
             const uint32_t hr = 4 * warp + (lane >> 3);
             v[8] = make_uint4(0, 0, 0, 0);
-            if ((int)hr < live_heads) v[8] = __ldg(reinterpret_cast<const uint4*>(q0 + (size_t)hr * D_QK + D_NOPE + (lane & 7) * 8));
+            if ((int)hr < live_heads) v[8] = ld_in(reinterpret_cast<const uint4*>(q0 + (size_t)hr * D_QK + D_NOPE + (lane & 7) * 8));
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
                 uint32_t o[4];
@@ -402,8 +402,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(DUO_THREADS, 1) attn
                     const int h = 16 * quarter + i + k;
                     v[2 * k] = v[2 * k + 1] = make_uint4(0, 0, 0, 0);
                     if (h < live_heads) {
-                        v[2 * k] = __ldg(reinterpret_cast<const uint4*>(q0 + (size_t)h * D_QK + lane * 16));
-                        v[2 * k + 1] = __ldg(reinterpret_cast<const uint4*>(q0 + (size_t)h * D_QK + lane * 16 + 8));
+                        v[2 * k] = ld_in(reinterpret_cast<const uint4*>(q0 + (size_t)h * D_QK + lane * 16));
+                        v[2 * k + 1] = ld_in(reinterpret_cast<const uint4*>(q0 + (size_t)h * D_QK + lane * 16 + 8));
                     }
                 }
 #pragma unroll
@@ -422,7 +422,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(DUO_THREADS, 1) attn
                 for (int k = 0; k < 2; ++k) {
                     const int h = 16 * quarter + i + 4 * k + (lane >> 3);
                     v[k] = make_uint4(0, 0, 0, 0);
-                    if (h < live_heads) v[k] = __ldg(reinterpret_cast<const uint4*>(q0 + (size_t)h * D_QK + D_NOPE + (lane & 7) * 8));
+                    if (h < live_heads) v[k] = ld_in(reinterpret_cast<const uint4*>(q0 + (size_t)h * D_QK + D_NOPE + (lane & 7) * 8));
                 }
 #pragma unroll
                 for (int k = 0; k < 2; ++k) {
@@ -504,7 +504,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(DUO_THREADS, 1) attn
                         ++sit;
                     }
                     there = idx >= 0;
-                    if (there) sc = __ldg(reinterpret_cast<const uint4*>(p.kv + (size_t)idx * ROW_BYTES + SCALE_OFF));
+                    if (there) sc = ld_in(reinterpret_cast<const uint4*>(p.kv + (size_t)idx * ROW_BYTES + SCALE_OFF));
                     idx = ahead.next_tile(p, meta) ? ahead.row_index(p, 32 * quarter + lane) : -1;
                     primed += filling ? 1u : 0u;
                 }

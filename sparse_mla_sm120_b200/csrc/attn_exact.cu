@@ -190,7 +190,7 @@ __global__ void __launch_bounds__(X_THREADS, 1) attn_exact_kernel(const AttnPara
                     for (int k = 0; k < 8; ++k) {
                         const int i = tid + (u + k) * (X_SM_WARPS * 32), h = i >> 6;
                         v[k] = make_uint4(0, 0, 0, 0);
-                        if (head0 + h < p.num_heads) v[k] = __ldg(reinterpret_cast<const uint4*>(q0 + (size_t)h * X_DIM + (i & 63) * 8));
+                        if (head0 + h < p.num_heads) v[k] = ld_in(reinterpret_cast<const uint4*>(q0 + (size_t)h * X_DIM + (i & 63) * 8));
                     }
 #pragma unroll
                     for (int k = 0; k < 8; ++k) {
@@ -360,7 +360,7 @@ __global__ void __launch_bounds__(X_THREADS, 1) attn_exact_kernel(const AttnPara
                 const unsigned pbs = (unsigned)(extra ? p.extra_page_block_size : p.page_block_size);
                 const unsigned blk = (unsigned)idx / pbs, in = (unsigned)idx - blk * pbs;
                 const uint8_t* page = kv + (int64_t)blk * (extra ? p.extra_block_stride : p.block_stride);
-                sc8 = __ldg(reinterpret_cast<const uint2*>(page + (int64_t)pbs * X_DATA + (int64_t)in * 8));
+                sc8 = ld_in(reinterpret_cast<const uint2*>(page + (int64_t)pbs * X_DATA + (int64_t)in * 8));
                 const unsigned long long at = reinterpret_cast<unsigned long long>(page + (int64_t)in * X_DATA);
                 lo = (uint32_t)at; hi = (uint32_t)(at >> 32);
             }

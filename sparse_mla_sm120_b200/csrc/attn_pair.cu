@@ -197,7 +197,7 @@ template <bool EXTRA>
 __device__ __forceinline__ int tile_entry(const AttnParams& p, const Work& w, int j, int rank, int r, int nst, int lim) {
     if (EXTRA) return fetch_entry(p, w, w.blk0 + 2 * j + rank, r);
     const int pos = w.blk0 * BLOCK_N + j * TILE_N + rank * OWN_N + r;
-    return (j < nst && pos < lim) ? __ldg(p.indices + (size_t)w.req * p.topk + pos) : -1;
+    return (j < nst && pos < lim) ? ld_in(p.indices + (size_t)w.req * p.topk + pos) : -1;
 }
 
 // A partition's rows as one sequence of groups of eight (eight groups per tile of a CTA, the tiles of all its requests
@@ -401,8 +401,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) att
 #pragma unroll
                         for (int i = 0; i < 8; ++i) {
                             xa[i] = xb[i] = make_uint4(0, 0, 0, 0);
-                            if (v_a && i < nblk32) xa[i] = __ldg(reinterpret_cast<const uint4*>(gsrc_a + 32 * i));
-                            if (v_b && i < nblk32) xb[i] = __ldg(reinterpret_cast<const uint4*>(gsrc_b + 32 * i));
+                            if (v_a && i < nblk32) xa[i] = ld_in(reinterpret_cast<const uint4*>(gsrc_a + 32 * i));
+                            if (v_b && i < nblk32) xb[i] = ld_in(reinterpret_cast<const uint4*>(gsrc_b + 32 * i));
                         }
                     }
                     auto amax2 = [](uint32_t m, const uint4& a) {      // running |.| maximum of bf16 pairs
@@ -730,7 +730,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) att
             const CacheGeom& c = EXTRA && a.extra ? extra_c : main_c;
             unsigned in;
             const uint8_t* pg = cache_page(c, a.idx, in);
-            return __ldg(reinterpret_cast<const uint2*>(pg + (int64_t)c.pbs * L::DATA + (int64_t)in * 8));
+            return ld_in(reinterpret_cast<const uint2*>(pg + (int64_t)c.pbs * L::DATA + (int64_t)in * 8));
         };
         // Which of the group's rows have an entry is read ahead (the rows themselves are brought in by the copy warps).
         ItemWalk<EXTRA> walk(meta.begin_req);

@@ -209,8 +209,8 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
                         const int h = 8 * warp + u + k;
                         v[2 * k] = v[2 * k + 1] = make_uint4(0, 0, 0, 0);
                         if (h < my_heads) {
-                            v[2 * k] = __ldg(reinterpret_cast<const uint4*>(q0 + (size_t)h * D_QK + lane * 16));
-                            v[2 * k + 1] = __ldg(reinterpret_cast<const uint4*>(q0 + (size_t)h * D_QK + lane * 16 + 8));
+                            v[2 * k] = ld_in(reinterpret_cast<const uint4*>(q0 + (size_t)h * D_QK + lane * 16));
+                            v[2 * k + 1] = ld_in(reinterpret_cast<const uint4*>(q0 + (size_t)h * D_QK + lane * 16 + 8));
                         }
                     }
 #pragma unroll
@@ -235,7 +235,7 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
                 for (int u = 0; u < 2; ++u) {              // RoPE
                     const int h = 8 * warp + 4 * u + (lane >> 3);
                     uint4 v = make_uint4(0, 0, 0, 0);
-                    if (h < my_heads) v = __ldg(reinterpret_cast<const uint4*>(q0 + (size_t)h * D_QK + D_NOPE + (lane & 7) * 8));
+                    if (h < my_heads) v = ld_in(reinterpret_cast<const uint4*>(q0 + (size_t)h * D_QK + D_NOPE + (lane & 7) * 8));
                     const uint32_t flip = scale_sign | (scale_sign >> 16);
                     v.x ^= flip; v.y ^= flip; v.z ^= flip; v.w ^= flip;
                     *reinterpret_cast<uint4*>(sm + QR_OFF + swz128((uint32_t)h, (uint32_t)lane & 7u)) = v;
@@ -612,7 +612,7 @@ __global__ void __launch_bounds__(T_THREADS, 1) attn_tile_kernel(const AttnParam
                 ++it;
             }
             there = idx >= 0;
-            if (there) sc = __ldg(reinterpret_cast<const uint4*>(p.kv + (size_t)idx * ROW_BYTES + SCALE_OFF));
+            if (there) sc = ld_in(reinterpret_cast<const uint4*>(p.kv + (size_t)idx * ROW_BYTES + SCALE_OFF));
             have2 = have1;
             have1 = have = have && tiles.next_tile(p, meta);
             idx = have ? tiles.row_index(p, quarter * 32 + lane) : -1;

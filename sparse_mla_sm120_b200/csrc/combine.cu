@@ -38,16 +38,14 @@ template <> struct Rec<__half> {
 
 template <typename OutT, typename InT = float>
 __global__ void __launch_bounds__(WARPS * 32)
-combine_kernel(const InT* __restrict__ o_accum, const float* __restrict__ lse_accum,
-               OutT* __restrict__ out, float* __restrict__ out_lse,
-               const int32_t* __restrict__ num_splits, const float* __restrict__ attn_sink,
+combine_kernel(const InT* o_accum, const float* lse_accum, OutT* out, float* out_lse, const int32_t* num_splits, const float* attn_sink,
                int batch, int num_heads, int fixed_ns, int64_t part_stride_o, int64_t part_stride_l,
                int out_slices, int64_t out_slice_stride) {
     constexpr bool F32 = sizeof(OutT) == 4;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t row = (int64_t)blockIdx.x * WARPS + warp;   // (token, head)
-    grid_dep_launch();    // the kernel after this one may start its own prologue
     grid_dep_wait();      // the partials of the attention kernel before this one are complete
+    grid_dep_launch();
     if (row >= (int64_t)batch * num_heads) return;
     const int tok = (int)(row / num_heads), h = (int)(row % num_heads);
     int s0, ns;
@@ -78,7 +76,7 @@ combine_kernel(const InT* __restrict__ o_accum, const float* __restrict__ lse_ac
         for (int u = 0; u < U; ++u)
             if (s + u < ns) {
 #pragma unroll
-                for (int i = 0; i < 4; ++i) v[u][i] = __ldcs(reinterpret_cast<const typename R::Raw*>(o_p + (size_t)(s + u) * o_stride + i * 128));
+                for (int i = 0; i < 4; ++i) v[u][i] = ld_in_once(reinterpret_cast<const typename R::Raw*>(o_p + (size_t)(s + u) * o_stride + i * 128));
             }
     };
     load(0);

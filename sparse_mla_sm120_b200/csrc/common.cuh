@@ -92,14 +92,56 @@ __device__ __forceinline__ float warp_sum(float v) {
 // one start early.  Both are no-ops in a kernel that was launched the ordinary way.  The reference uses the same
 // mechanism between its scheduler, decode and combine kernels (csrc/kernel/decode/decode_launch.cu:46-49).
 //
-// The rule that makes a chain of such kernels safe: before grid_dep_wait() a kernel touches only its parameters, its
-// shared memory and its tensor memory, and every thread of it passes the wait before it ends.  Then a kernel that has
-// completed says that all before it on the stream have, so that scratch and results of earlier calls may be read and
-// written after the wait.  A kernel early on the SMs cannot hold up what it waits for: it is only launched once all
-// blocks of the kernel before it run or have ended.  A decode step behind another one in a graph: one request 16.5 -> 15.2 us,
+// The rules that make a chain of such kernels safe:
+//  - Before grid_dep_wait() a kernel touches only its parameters, its shared memory and its tensor memory, and every thread of it
+//    passes the wait before it ends.  Then a kernel that has completed says that all before it on the stream have, so that
+//    scratch and results of earlier calls may be read and written after the wait.
+//  - grid_dep_launch() comes after grid_dep_wait(): a kernel then runs beside the one before it at most, never beside the one
+//    before that.
+//  - Global memory that another kernel may write (every tensor of a call: a kernel of this library can have written it just before) is
+//    read by ld_in(), by plain loads through pointers without __restrict__, or by bulk copies.  __ldg, the other cache-hint
+//    intrinsics and const __restrict__ parameters are out: the non-coherent load is defined for memory that nothing writes while
+//    the kernel lives, and this kernel lives while the one before it writes; nor need the compiler keep such loads behind the wait.
+// A kernel early on the SMs cannot hold up what it waits for: it is only launched once all blocks of the kernel before it run or
+// have ended.  A decode step behind another one in a graph: one request 16.5 -> 15.2 us,
 // 64 requests 34.6 -> 33.2 (rows in L2); behind a kernel that does not let the next one start early, 17.6 -> 17.3 and 36.1 -> 36.2.
 __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// Loads of what a kernel before this one may have written: coherent, and kept behind grid_dep_wait() (both are volatile).
+// ld_in_once() for what is read a single time: first to be evicted.
+__device__ __forceinline__ int ld_in(const int* p) { int v; asm volatile("ld.global.s32 %0, [%1];" : "=r"(v) : "l"(p)); return v; }
+__device__ __forceinline__ float ld_in(const float* p) { float v; asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p)); return v; }
+__device__ __forceinline__ uint2 ld_in(const uint2* p) {
+    uint2 v;
+    asm volatile("ld.global.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ uint4 ld_in(const uint4* p) {
+    uint4 v;
+    asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ float4 ld_in(const float4* p) {
+    float4 v;
+    asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ uint2 ld_in_once(const uint2* p) {
+    uint2 v;
+    asm volatile("ld.global.cs.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ uint4 ld_in_once(const uint4* p) {
+    uint4 v;
+    asm volatile("ld.global.cs.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ float4 ld_in_once(const float4* p) {
+    float4 v;
+    asm volatile("ld.global.cs.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+    return v;
+}
 
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {

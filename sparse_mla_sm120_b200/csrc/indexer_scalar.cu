@@ -64,7 +64,7 @@ __device__ __forceinline__ uint32_t order_key(float f) {   // larger float <=> l
 // Applies fn(column, key) to every column of [lo, hi): 16-byte loads over the aligned middle part,
 // four of them in flight per thread, scalar loads at the ragged ends.
 template <typename F>
-__device__ __forceinline__ void for_each_key(const float* __restrict__ x, int lo, int hi, int tid, int nthreads, F fn) {
+__device__ __forceinline__ void for_each_key(const float* x, int lo, int hi, int tid, int nthreads, F fn) {
     const int a0 = min(hi, (int)(((size_t)lo + 3) & ~(size_t)3));                 // first multiple of 4 >= lo (x is 16-byte aligned)
     const int a1 = max(a0, hi & ~3);
     for (int j = lo + tid; j < a0; j += nthreads) fn(j, order_key(x[j]));
@@ -96,15 +96,14 @@ struct Emit {
     __device__ __forceinline__ int32_t operator()(int row, int col) const {
         if (table == nullptr) return col;
         const int page = col / page_size;
-        return page < table_pages ? __ldg(table + (size_t)row * table_stride + page) * page_size + (col - page * page_size) : -1;
+        return page < table_pages ? ld_in(table + (size_t)row * table_stride + page) * page_size + (col - page * page_size) : -1;
     }
 };
 
 // Multi-pass radix select of one row by the whole CTA: any k, any distribution.  A row of 65536 logits is 256 KB; the rows in
 // flight fit the L2 and only the first of the passes over a row reaches DRAM.
 template <int THREADS>
-__device__ void topk_multipass(const float* __restrict__ logits, const int32_t* __restrict__ ks, const int32_t* __restrict__ ke,
-                               int32_t* __restrict__ out, int num_cols, int64_t logits_stride, int k, int row, const Emit& emit) {
+__device__ void topk_multipass(const float* logits, const int32_t* ks, const int32_t* ke, int32_t* out, int num_cols, int64_t logits_stride, int k, int row, const Emit& emit) {
     constexpr int WARPS = THREADS / 32;
     __shared__ int hist[256];
     __shared__ int sel_bin, sel_need;
@@ -257,13 +256,13 @@ constexpr int TS_KMAX = 4096;              // largest k (the lists hold 8192)
 constexpr int TS_ROUNDS = 8;               // rounds of four blocks per warp between two appends
 constexpr int TS_SMEM = TS_CAND * 8 + TS_BINS * 4 + TS_EQ * 8;
 
-__device__ __forceinline__ float4 load_row4(const float* __restrict__ x, int j, int num_cols, bool vec_ok) {
-    if (vec_ok && j + 3 < num_cols) return *reinterpret_cast<const float4*>(x + j);
+__device__ __forceinline__ float4 load_row4(const float* x, int j, int num_cols, bool vec_ok) {
+    if (vec_ok && j + 3 < num_cols) return ld_in(reinterpret_cast<const float4*>(x + j));
     float4 f;
-    f.x = (j + 0 < num_cols) ? x[j + 0] : -INFINITY;
-    f.y = (j + 1 < num_cols) ? x[j + 1] : -INFINITY;
-    f.z = (j + 2 < num_cols) ? x[j + 2] : -INFINITY;
-    f.w = (j + 3 < num_cols) ? x[j + 3] : -INFINITY;
+    f.x = (j + 0 < num_cols) ? ld_in(x + j + 0) : -INFINITY;
+    f.y = (j + 1 < num_cols) ? ld_in(x + j + 1) : -INFINITY;
+    f.z = (j + 2 < num_cols) ? ld_in(x + j + 2) : -INFINITY;
+    f.w = (j + 3 < num_cols) ? ld_in(x + j + 3) : -INFINITY;
     return f;
 }
 
@@ -275,9 +274,8 @@ __device__ __forceinline__ float key_to_float(uint32_t key) {      // inverse of
 // for the few rows of a decode step (every row then has an SM to itself).
 template <int TS_THREADS>
 __global__ void __launch_bounds__(TS_THREADS, 1024 / TS_THREADS)
-topk_select_kernel(const float* __restrict__ logits, const int32_t* __restrict__ ks,
-                   const int32_t* __restrict__ ke, int32_t* __restrict__ out, int num_cols,
-                   int64_t logits_stride, int k, const Emit emit) {
+topk_select_kernel(const float* logits, const int32_t* ks, const int32_t* ke, int32_t* out, int num_cols, int64_t logits_stride,
+                   int k, const Emit emit) {
     constexpr int TS_WARPS = TS_THREADS / 32;
     constexpr int TS_LIST = TS_CAND / TS_WARPS;        // candidates per warp
     constexpr int TS_BPT = TS_BINS / TS_THREADS;       // histogram bins per thread in the suffix sums
@@ -292,8 +290,8 @@ topk_select_kernel(const float* __restrict__ logits, const int32_t* __restrict__
     __shared__ int last_col_s;
     __shared__ int cw[TS_WARPS], cc[TS_WARPS], wsum[TS_WARPS];
 
-    grid_dep_launch();
     grid_dep_wait();
+    grid_dep_launch();
     const int row = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const float* x = logits + (size_t)row * logits_stride;
     int lo = ks ? max(ks[row], 0) : 0;
@@ -319,7 +317,7 @@ topk_select_kernel(const float* __restrict__ logits, const int32_t* __restrict__
 #pragma unroll
         for (int r = 0; r < TS_SAMPLE / TS_THREADS; ++r) {
             const int i = tid + TS_THREADS * r;
-            h[r] = order_key(x[lo + (i >> 3) * run_stride + (i & 7)]) >> 16;
+            h[r] = order_key(ld_in(x + lo + (i >> 3) * run_stride + (i & 7))) >> 16;
         }
 #pragma unroll
         for (int r = 0; r < TS_SAMPLE / TS_THREADS; ++r)
@@ -575,8 +573,8 @@ __device__ __forceinline__ void cluster_barrier() {
 }
 
 __global__ void __cluster_dims__(TC_CTAS, 1, 1) __launch_bounds__(TC_THREADS, 2)
-topk_cluster_kernel(const float* __restrict__ logits, const int32_t* __restrict__ ks, const int32_t* __restrict__ ke,
-                    int32_t* __restrict__ out, int num_cols, int64_t logits_stride, int k, const Emit emit) {
+topk_cluster_kernel(const float* logits, const int32_t* ks, const int32_t* ke, int32_t* out, int num_cols, int64_t logits_stride,
+                    int k, const Emit emit) {
     extern __shared__ __align__(16) uint8_t ts_smem[];
     int* lists = reinterpret_cast<int*>(ts_smem);                               // [TC_VW][TC_LIST] candidate columns
     uint32_t* keys = reinterpret_cast<uint32_t*>(lists + TC_VW * TC_LIST);      // their keys
@@ -590,8 +588,8 @@ topk_cluster_kernel(const float* __restrict__ logits, const int32_t* __restrict_
     __shared__ uint32_t kmin_s, kmax_s, last_key_s;
     __shared__ int last_col_s;
 
-    grid_dep_launch();
     grid_dep_wait();
+    grid_dep_launch();
     const int row = blockIdx.x / TC_CTAS, rank = blockIdx.x % TC_CTAS;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int vw = warp / TC_SUB, sub = warp % TC_SUB, vwarp = rank * TC_VW + vw;
@@ -619,7 +617,7 @@ topk_cluster_kernel(const float* __restrict__ logits, const int32_t* __restrict_
 #pragma unroll
         for (int r = 0; r < TS_SAMPLE / TC_THREADS; ++r) {
             const int i = tid + TC_THREADS * r;
-            h[r] = order_key(x[lo + (i >> 3) * run_stride + (i & 7)]) >> 16;
+            h[r] = order_key(ld_in(x + lo + (i >> 3) * run_stride + (i & 7))) >> 16;
         }
 #pragma unroll
         for (int r = 0; r < TS_SAMPLE / TC_THREADS; ++r)

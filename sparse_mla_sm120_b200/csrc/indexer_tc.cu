@@ -172,7 +172,7 @@ __global__ void __launch_bounds__(LX_THREADS, 1) mqa_logits_tc_kernel(const Logi
 #pragma unroll 1
             for (int t = t0; t < t1; ++t, ++it, key += LX_KT) {
                 const uint32_t b = it & 1u;
-                const float sc = key < p.s_k ? __ldg(p.k_scale + key) : 0.f;
+                const float sc = key < p.s_k ? ld_in(p.k_scale + key) : 0.f;
                 ok = mbar_wait_lean(bar(LXB_DFULL + b), (it >> 1) & 1u, abort_addr, 12);
                 if (!ok) break;
                 tc_fence_after();

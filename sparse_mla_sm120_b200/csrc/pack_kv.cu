@@ -16,18 +16,17 @@ __device__ __forceinline__ float pow2_ceil(float x) {   // smallest power of two
     return __uint_as_float(b);
 }
 
-__global__ void __launch_bounds__(256) pack_kv_kernel(const __nv_bfloat16* __restrict__ kv,
-                                                      uint8_t* __restrict__ packed, int64_t rows) {
-    grid_dep_launch();
+__global__ void __launch_bounds__(256) pack_kv_kernel(const __nv_bfloat16* kv, uint8_t* packed, int64_t rows) {
     grid_dep_wait();
+    grid_dep_launch();
     const int lane = threadIdx.x & 31;
     const int64_t row = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
     if (row >= rows) return;
     const __nv_bfloat16* src = kv + row * D_QK;
     uint8_t* dst = packed + row * ROW_BYTES;
 
-    const uint4 a = __ldcs(reinterpret_cast<const uint4*>(src + lane * 16));
-    const uint4 b = __ldcs(reinterpret_cast<const uint4*>(src + lane * 16 + 8));
+    const uint4 a = ld_in_once(reinterpret_cast<const uint4*>(src + lane * 16));
+    const uint4 b = ld_in_once(reinterpret_cast<const uint4*>(src + lane * 16 + 8));
     const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
     float v[16];
     float amax = 0.f;
@@ -56,7 +55,7 @@ __global__ void __launch_bounds__(256) pack_kv_kernel(const __nv_bfloat16* __res
     *reinterpret_cast<uint4*>(dst + lane * 16) = make_uint4(o[0], o[1], o[2], o[3]);
     if ((lane & 7) == 0) *reinterpret_cast<float*>(dst + SCALE_OFF + (lane >> 3) * 4) = scale;
     if (lane < 8) {
-        const uint4 r = __ldcs(reinterpret_cast<const uint4*>(src + D_NOPE + lane * 8));
+        const uint4 r = ld_in_once(reinterpret_cast<const uint4*>(src + D_NOPE + lane * 8));
         *reinterpret_cast<uint4*>(dst + ROPE_OFF + lane * 16) = r;
     }
 }

@@ -119,7 +119,7 @@ __device__ __forceinline__ void add_f32x2(uint64_t& acc, uint64_t a) {          
 // 16 bytes of read-only global memory that are used once.
 __device__ __forceinline__ uint4 ld_row16(const void* p) {
     uint4 v;
-    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    asm volatile("ld.global.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
     return v;
 }
 // 256-bit global store (sm_100): one full 32-byte sector per lane; p must be 32-byte aligned.

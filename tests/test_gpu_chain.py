@@ -72,3 +72,38 @@ def test_a_capture_that_joins_two_streams_before_the_call(heads, tokens, topk, p
         torch.cuda.synchronize()
         for got, w in ((first, want[1]), (second, want[0])):
             assert torch.equal(got[0], w[0]) and torch.equal(got[1], w[1])
+
+
+@pytest.mark.parametrize("heads", [16, 128])
+@pytest.mark.parametrize("tokens", [2, 90])
+def test_selection_packing_and_attention_over_the_same_buffers(tokens, heads):
+    """Every input of the attention written by library kernels right in front of it: lengths (two places back), indices by the selection,
+    cache rows by the packing, in buffers that every round overwrites."""
+    from sparse_mla_sm120_b200 import _lib, flash_ops
+    lib, topk, rows, rounds = _lib.load(), 512, 4096, 6
+    g = torch.Generator(device=DEV).manual_seed(tokens + heads)
+    latents = [torch.randn(rows, 576, device=DEV, generator=g).to(torch.bfloat16) for _ in range(rounds)]
+    logits = [torch.randn(tokens, rows, device=DEV, generator=g) for _ in range(rounds)]
+    lens = [torch.randint(1, topk + 1, (tokens,), device=DEV, generator=g, dtype=torch.int32) for _ in range(rounds)]
+    q = (0.5 * torch.randn(tokens, heads, 576, device=DEV, generator=g)).to(torch.bfloat16)
+    cache = torch.zeros(rows // 64, 64, 1, 656, dtype=torch.uint8, device=DEV)
+    idx = torch.zeros(tokens, topk, dtype=torch.int32, device=DEV)
+    length = torch.ones(tokens, dtype=torch.int32, device=DEV)
+
+    def one(i, wait):
+        stream = torch.cuda.current_stream().cuda_stream
+        length.copy_(lens[i])
+        wait()
+        assert lib.smla_topk(logits[i].data_ptr(), None, None, idx.data_ptr(), tokens, rows, rows, topk, stream) == 0
+        wait()
+        assert lib.smla_pack_kv(latents[i].data_ptr(), cache.data_ptr(), rows, stream) == 0
+        wait()
+        got = flash_ops.sparse_mla_decode_fwd(q, cache, idx, 576 ** -0.5, topk_length=length)
+        wait()
+        return [t.clone() for t in got] if wait is torch.cuda.synchronize else got
+    want = [one(i, torch.cuda.synchronize) for i in range(rounds)]
+    for _ in range(6):
+        got = [one(i, lambda: None) for i in range(rounds)]
+        torch.cuda.synchronize()
+        for (o, l), (wo, wl) in zip(got, want):
+            assert torch.equal(o, wo) and torch.equal(l, wl)
