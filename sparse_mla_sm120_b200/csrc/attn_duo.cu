@@ -699,90 +699,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(DUO_THREADS, 1) attn
                 }
             }
         }
-    } else if (warp == QK_WARP) {
-        // =================================================================== score MMAs (odd CTA: its K rows have landed)
-        Walk tiles(p, first, step, last);
-        uint32_t it = 0, rq = 0;
-        bool ok = true;
-        const uint32_t q_lo = desc_lo(base + Q_OFF, 16);
-        for (; ok && tiles.next_tile(p, meta); ++it) {
-            const uint32_t b = it & 1u, ph = (it >> 1) & 1u;
-            if (rank == 0) {
-                if (tiles.j == 0) ok = mbar_wait_lean(bar(B_QREADYP), rq++ & 1u, abort_addr, WD_QREADY);
-                // (the P.V of two tiles ago: with the scores the softmax warps also get the buffer of their weights)
-                if (ok && it >= 2) ok = mbar_wait_lean(bar(B_SFREEP + b), ph ^ 1u, abort_addr, WD_SFREE);
-                if (ok && it >= 2) ok = mbar_wait_lean(bar(B_PVDONE + b), ph ^ 1u, abort_addr, WD_PVDONE);
-                if (ok) ok = mbar_wait_lean(bar(B_SCALEP + b), ph, abort_addr, WD_SCALES);
-                if (ok) ok = mbar_wait_lean(bar(B_KPEERP + b), ph, abort_addr, WD_KPEER);
-            }
-            if (ok) ok = mbar_wait_lean(bar(B_KFULL + b), ph, abort_addr, WD_KFULL);
-            if (!ok) break;
-            if (rank != 0) {
-                if (lane == 0) mbar_arrive_remote(barp(B_KPEERP + b));
-                continue;
-            }
-            tc_fence_after();
-            if (elect_one()) {
-                const uint32_t k_lo = desc_lo(base + KS_OFF + b * KS_BYTES, 16), d = tmem + TM_S + 64 * b;
-#pragma unroll 1
-                for (int kc = 0; kc < 4; ++kc) {
-                    const uint32_t a = q_lo + ((kc * CHUNK) >> 4), k = k_lo + ((kc * CHUNK) >> 4), idesc = idesc_mx(0) | ((uint32_t)kc << 4);
-#pragma unroll
-                    for (int s = 0; s < 4; ++s)
-                        mma_pair_mxf8(d, make_desc(a + 2 * s, HI_128), make_desc(k + 2 * s, HI_128), idesc, tmem + TM_SFA, tmem + TM_SFB + 4 * b, (kc | s) != 0);
-                }
-#pragma unroll
-                for (int s = 0; s < 4; ++s)
-                    mma_pair_f16(d, make_desc(q_lo + ((4 * CHUNK) >> 4) + 2 * s, HI_128), make_desc(k_lo + ((4 * CHUNK) >> 4) + 2 * s, HI_128), IDESC_ROPE, true);
-                tc_commit_pair(bar(B_SREADY + b));
-                tc_commit_pair(mapa_shared(bar(B_SREADY + b), 1));
-                if (tiles.j + 1 == tiles.nst) {
-                    tc_commit_pair(bar(B_QFREE));
-                    tc_commit_pair(mapa_shared(bar(B_QFREE), 1));
-                }
-            }
-            __syncwarp();
-        }
-    } else if (warp == PV_WARP) {
-        if (rank == 0) {
-            // ================================================================ P.V MMAs, half a tile at a time
-            Walk tiles(p, first, step, last);
-            uint32_t it = 0, rq = 0;
-            bool ok = true;
-            const uint32_t pb_lo = desc_lo(base + PB_OFF, 16), vs_lo = desc_lo(base + VS_OFF, V_STEP);
-            for (; ok && tiles.next_tile(p, meta); ++it) {
-                const uint32_t b = it & 1u;
-                if (tiles.j == 0) {
-                    if (rq > 0) ok = mbar_wait_lean(bar(B_OFREEP), (rq - 1) & 1u, abort_addr, WD_OFREE);
-                    ++rq;
-                }
-                if (ok) ok = mbar_wait_lean(bar(B_PREADYP + b), (it >> 1) & 1u, abort_addr, WD_PREADY);
-#pragma unroll 1
-                for (uint32_t h = 0; ok && h < 2; ++h) {
-                    const uint32_t slot = 2 * b + h;
-                    ok = mbar_wait_lean(bar(B_VREADYP + slot), (it >> 1) & 1u, abort_addr, WD_VREADY);
-                    if (!ok) break;
-                    tc_fence_after();
-                    if (elect_one()) {
-                        const uint32_t pa = pb_lo + ((b * CHUNK + h * 64) >> 4), va = vs_lo + ((slot * VS_BYTES) >> 4);
-#pragma unroll
-                        for (int kb = 0; kb < 2; ++kb) {
-#pragma unroll
-                            for (int nb = 0; nb < 2; ++nb)
-                                mma_pair_f8(tmem + TM_O + 128 * nb, make_desc(pa + 2 * kb, HI_128), make_desc(va + ((nb * V_BLOCK + kb * V_STEP) >> 4), HI_128),
-                                            IDESC_PV, ((uint32_t)tiles.j | h | (uint32_t)kb) != 0u);
-                        }
-                        tc_commit_pair(bar(B_VFREE + slot));
-                        tc_commit_pair(mapa_shared(bar(B_VFREE + slot), 1));
-                        if (h == 1) {
-                            tc_commit_pair(bar(B_PVDONE + b));
-                            tc_commit_pair(mapa_shared(bar(B_PVDONE + b), 1));
-                        }
-                    }
-                    __syncwarp();
-                }
-            }
-        }
     } else if (warp >= FIX_WARP0) {
         // =================================================================== V onto the groups' scales
         // Each warp looks after 16 rows x two blocks of 128 dims of every tile, a lane after one of these pieces.  Those that have another
