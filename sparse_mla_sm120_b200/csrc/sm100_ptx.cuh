@@ -60,14 +60,22 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
 
 // The wait of the critical paths, in as few instructions as it can have (the roles of these kernels together are larger than the
 // instruction caches): every lane blocks in mbarrier.try_wait itself, nearly always the first poll, which the hardware
-// suspends until the phase completes or 4 us have passed, is the only one.  The warp decides by votes, so nothing here
-// diverges.  At most 2^20 polls, then `code` goes to the abort flag (given by its shared-memory address).
+// suspends until the phase completes or its own time limit has passed, is the only one.  The warp decides by votes, so nothing here
+// diverges.  Gives up after LEAN_POLLS + 1 polls; `code` then goes to the abort flag (given by its shared-memory address) unless there
+// is one already: the first wait to give up is on record, not one that follows from it.
+// It does not look at the flag while it waits, as mbar_wait does: that costs instructions at every wait (two tokens of 64 requests,
+// attn_duo_kernel: 80.5 us without, 82.6 with a look every 256 polls; 4096 tokens 4 % more) and gains little, for the waits that hang on
+// the stuck one begin within microseconds of it and so end with it, and a warp that has given up waits for nothing more.
+#ifndef SMLA_LEAN_POLLS
+#define SMLA_LEAN_POLLS (1u << 20)
+#endif
+constexpr uint32_t LEAN_POLLS = SMLA_LEAN_POLLS;
 __device__ __forceinline__ bool mbar_wait_lean(uint32_t bar, uint32_t parity, uint32_t abort_addr, int code) {
 #pragma unroll 1
-    for (uint32_t left = 1u << 20; ; --left) {
+    for (uint32_t left = LEAN_POLLS; ; --left) {
         if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity, WAIT_HINT_NS))) return true;
         if (left == 0u) {
-            asm volatile("st.volatile.shared.u32 [%0], %1;" ::"r"(abort_addr), "r"(code) : "memory");
+            asm volatile("{\n\t.reg .b32 t;\n\tatom.shared.cas.b32 t, [%0], 0, %1;\n\t}" ::"r"(abort_addr), "r"(code) : "memory");
             return false;
         }
     }
