@@ -55,9 +55,9 @@ const char* smla_last_error(void) { return g_err; }
 const char* smla_status_string(int code) {
     switch (code) {
         case 0: return "";
-        case 11: return "indexer q_full"; case 12: return "indexer k_full"; case 13: return "indexer k_empty";
-        case 14: return "indexer d_full"; case 15: return "indexer d_empty"; case 16: return "indexer q_empty";
-        case 17: return "indexer tmem";
+        case 11: return "indexer weights"; case 12: return "indexer d_full"; case 13: return "indexer q_empty";
+        case 14: return "indexer k_empty"; case 15: return "indexer q_full"; case 16: return "indexer k_full";
+        case 17: return "indexer d_empty";
         case 21: return "attention k_empty"; case 22: return "attention k_stored"; case 23: return "attention k_full";
         case 24: return "attention half-tile record"; case 25: return "attention v_empty"; case 26: return "attention v_full (one CTA)";
         case 27: return "attention v_full"; case 28: return "attention s_ready"; case 29: return "attention s_free";
@@ -69,6 +69,12 @@ const char* smla_status_string(int code) {
         case 54: return "attention tile s_ready"; case 55: return "attention tile s_free"; case 56: return "attention tile scales";
         case 57: return "attention tile p_ready"; case 58: return "attention tile pv_done"; case 59: return "attention tile q_ready";
         case 44: return "exact attention p_ready"; case 45: return "exact attention pv_done"; case 46: return "exact attention q_ready";
+        case 71: return "attention duo k_full"; case 72: return "attention duo k_peer"; case 73: return "attention duo v_full";
+        case 74: return "attention duo v_ready"; case 75: return "attention duo scales"; case 76: return "attention duo s_ready";
+        case 77: return "attention duo s_free"; case 78: return "attention duo p_ready"; case 79: return "attention duo pv_done";
+        case 80: return "attention duo q_ready"; case 81: return "attention duo q_scale"; case 82: return "attention duo sums";
+        case 83: return "attention duo o_free"; case 84: return "attention duo q_free"; case 85: return "attention duo v_free";
+        case 86: return "attention duo sum_free"; case 87: return "attention duo q_part";
         default: return "unknown";
     }
 }

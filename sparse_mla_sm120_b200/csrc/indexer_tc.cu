@@ -59,6 +59,9 @@ constexpr uint32_t LX_SMEM_NEED = LX_MISC_OFF + 16 + 1024;
 // one CTA per SM (each allocates all 512 TMEM columns): ask for more than half of the SM's shared memory
 constexpr uint32_t LX_SMEM = LX_SMEM_NEED > 118 * 1024 ? LX_SMEM_NEED : 118 * 1024;
 
+// give-up codes reported through status[0]
+enum { WL_WEIGHTS = 11, WL_DFULL = 12, WL_QEMPTY = 13, WL_KEMPTY = 14, WL_QFULL = 15, WL_KFULL = 16, WL_DEMPTY = 17 };
+
 struct LogitsParams {
     const uint8_t* q; const uint8_t* k; const float* k_scale; const float* w;
     const int32_t* ks; const int32_t* ke; float* logits; int32_t* status;
@@ -146,7 +149,7 @@ __global__ void __launch_bounds__(LX_THREADS, 1) mqa_logits_tc_kernel(const Logi
                     if (j < t0 * LX_KT || j >= t1 * LX_KT) row[j] = -INFINITY;
             }
             if (t1 <= t0) continue;
-            ok = mbar_wait(bar(LXB_QFULL), qn & 1u, abort_flag, 11);   // weights of the group are in shared memory
+            ok = mbar_wait(bar(LXB_QFULL), qn & 1u, abort_flag, WL_WEIGHTS);   // weights of the group are in shared memory
             if (!ok) break;
             // The head weights of the warp's query stay in registers for the whole run of tiles, as pairs for the packed FMAs:
             // read from shared memory for every tile they cost 16 wide loads per warp and tile, and the 16 warps together
@@ -173,7 +176,7 @@ __global__ void __launch_bounds__(LX_THREADS, 1) mqa_logits_tc_kernel(const Logi
             for (int t = t0; t < t1; ++t, ++it, key += LX_KT) {
                 const uint32_t b = it & 1u;
                 const float sc = key < p.s_k ? ld_in(p.k_scale + key) : 0.f;
-                ok = mbar_wait_lean(bar(LXB_DFULL + b), (it >> 1) & 1u, abort_addr, 12);
+                ok = mbar_wait_lean(bar(LXB_DFULL + b), (it >> 1) & 1u, abort_addr, WL_DFULL);
                 if (!ok) break;
                 tc_fence_after();
                 uint64_t a01 = 0ull, a23 = 0ull;
@@ -210,7 +213,7 @@ __global__ void __launch_bounds__(LX_THREADS, 1) mqa_logits_tc_kernel(const Logi
             item_range(w, g, t0, t1, j0, j1);
             if (t1 <= t0) continue;
             if (qn > 0) {   // the MMAs of the previous group have finished reading q
-                ok = mbar_wait(bar(LXB_QEMPTY), (qn - 1) & 1u, abort_flag, 13);
+                ok = mbar_wait(bar(LXB_QEMPTY), (qn - 1) & 1u, abort_flag, WL_QEMPTY);
                 if (!ok) break;
             }
             // q group: N rows of 128 B, one tile load (rows past s_q * H arrive as zeros); the head
@@ -229,7 +232,7 @@ __global__ void __launch_bounds__(LX_THREADS, 1) mqa_logits_tc_kernel(const Logi
             for (int t = t0; t < t1 && ok; ++t, ++it) {
                 const uint32_t st = it % LX_KSTAGE;
                 if (it >= LX_KSTAGE) {
-                    ok = mbar_wait_lean(bar(LXB_KEMPTY + st), ((it / LX_KSTAGE) - 1) & 1u, abort_addr, 14);
+                    ok = mbar_wait_lean(bar(LXB_KEMPTY + st), ((it / LX_KSTAGE) - 1) & 1u, abort_addr, WL_KEMPTY);
                     if (!ok) break;
                 }
                 if (elect_one()) {
@@ -249,15 +252,15 @@ __global__ void __launch_bounds__(LX_THREADS, 1) mqa_logits_tc_kernel(const Logi
             int g, t0, t1, j0, j1;
             item_range(w, g, t0, t1, j0, j1);
             if (t1 <= t0) continue;
-            ok = mbar_wait_lean(bar(LXB_QFULL), qn & 1u, abort_addr, 15);
+            ok = mbar_wait_lean(bar(LXB_QFULL), qn & 1u, abort_addr, WL_QFULL);
             if (!ok) break;
             ++qn;
             for (int t = t0; t < t1; ++t, ++it) {
                 const uint32_t st = it % LX_KSTAGE, b = it & 1u;
-                ok = mbar_wait_lean(bar(LXB_KFULL + st), (it / LX_KSTAGE) & 1u, abort_addr, 16);
+                ok = mbar_wait_lean(bar(LXB_KFULL + st), (it / LX_KSTAGE) & 1u, abort_addr, WL_KFULL);
                 if (!ok) break;
                 if (it >= 2) {
-                    ok = mbar_wait_lean(bar(LXB_DEMPTY + b), ((it >> 1) - 1) & 1u, abort_addr, 17);
+                    ok = mbar_wait_lean(bar(LXB_DEMPTY + b), ((it >> 1) - 1) & 1u, abort_addr, WL_DEMPTY);
                     if (!ok) break;
                 }
                 tc_fence_after();
