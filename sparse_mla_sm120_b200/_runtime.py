@@ -237,7 +237,10 @@ def _duo_us(num_tokens: int, blocks: int, k: int, max_pairs: int) -> float:
 
 def pick_split_duo(num_tokens: int, sms: int, blocks_per_token: int, uniform: bool) -> Tuple[int, int]:
     """(partitions, fixed overhead) where whole requests and equal partitions run on attn_duo_kernel and partitions of the
-    scheduler on the pair kernel.  Ragged requests are left whole where the scheduler and combine launches and the partitions that
+    scheduler on the pair kernel.  Equal partitions leave fp16 records, so only calls that pick_split cuts equally are cut so here (lists
+    of 8 blocks and more that have a suitable divisor, up to 37 requests), if into another number of pieces.  Others would
+    be faster too (us whole / cut, rows in HBM: 4 requests of 640 entries 16.3 / 14.2, 10 of 896 19.1 / 17.1, 35 of 1024 23.0 / 22.5), but they are
+    computed without such a rounding: their results are whole requests' or go through fp32 records.  Ragged requests are left whole where the scheduler and combine launches and the partitions that
     straddle two requests cost more than the longest request: lists of up to 16 blocks, and from half as many requests on as a
     list has blocks (us whole / cut, rows in HBM: 16 requests of up to 1024 entries 21.7 / 28.1; 8 of up to 1536 27.1 / 26.8, 13: 27.6 /
     29.7; 13 of up to 2048 33.6 / 30.7, 16: 33.5 / 34.1, 20: 34.1 / 39.6; 24 of up to 4096 59.4 / 54.6, 30: 60.1 / 60.4).  Otherwise the
@@ -247,10 +250,14 @@ def pick_split_duo(num_tokens: int, sms: int, blocks_per_token: int, uniform: bo
     n = max(blocks_per_token, 1)
     max_pairs = max(sms // CTAS_PER_PART, 1)
     whole = (num_tokens, FIXED_OVERHEAD)
-    cuts = [k for k in range(2, n // 2 + 1) if n % k == 0 and k * num_tokens <= max_pairs]
-    if uniform and (cuts or n < 2 * BLOCKS_PER_PARTITION):
-        k = min([1] + cuts, key=lambda c: _duo_us(num_tokens, n, c, max_pairs))
-        return whole if k == 1 else (k * num_tokens, 0)
+    if uniform:
+        parts, overhead = pick_split(num_tokens, sms, blocks_per_token, uniform=True)
+        if parts == num_tokens:
+            return whole
+        if overhead == 0:
+            cuts = [k for k in range(2, n // 2 + 1) if n % k == 0 and k * num_tokens <= max_pairs]
+            k = min([1] + cuts, key=lambda c: _duo_us(num_tokens, n, c, max_pairs))
+            return whole if k == 1 else (k * num_tokens, 0)
     if n <= 16 or 2 * num_tokens >= n:
         return whole
     return pick_num_sm_parts(num_tokens, sms, blocks_per_token), FIXED_OVERHEAD

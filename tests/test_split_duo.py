@@ -22,3 +22,13 @@ def test_ragged_requests():
     assert pick_split_duo(15, 148, 32, False) == (74, FIXED_OVERHEAD)
     assert pick_split_duo(16, 148, 32, False) == (16, FIXED_OVERHEAD)        # half as many as a list has blocks
     assert pick_split_duo(1, 148, 32, True) == (8, 0) and pick_split_duo(64, 148, 32, True) == (64, FIXED_OVERHEAD)
+
+
+def test_fp16_records_only_where_they_have_been():
+    """Equal partitions leave fp16 records.  A call that pick_split leaves whole or gives to the scheduler (fp32 records) does not get
+    them here: lists of 9 and 10 blocks of a few requests, of 14 blocks of up to 10, of 16 blocks of 31 to 35 and all others."""
+    from sparse_mla_sm120_b200._runtime import pick_split
+    for blocks in range(1, 129):
+        for tokens in range(1, 150):
+            if pick_split(tokens, 148, blocks, uniform=True)[1] != 0:
+                assert pick_split_duo(tokens, 148, blocks, True)[1] == FIXED_OVERHEAD, (blocks, tokens)
