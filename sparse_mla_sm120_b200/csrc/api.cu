@@ -55,9 +55,9 @@ const char* smla_last_error(void) { return g_err; }
 const char* smla_status_string(int code) {
     switch (code) {
         case 0: return "";
-        case 11: return "indexer weights"; case 12: return "indexer d_full"; case 13: return "indexer q_empty";
-        case 14: return "indexer k_empty"; case 15: return "indexer q_full"; case 16: return "indexer k_full";
-        case 17: return "indexer d_empty";
+        case 11: return "indexer q_full"; case 12: return "indexer k_full"; case 13: return "indexer k_empty";
+        case 14: return "indexer d_full"; case 15: return "indexer d_empty"; case 16: return "indexer q_empty";
+        case 17: return "indexer weights";
         case 21: return "attention k_empty"; case 22: return "attention k_stored"; case 23: return "attention k_full";
         case 24: return "attention half-tile record"; case 25: return "attention v_empty"; case 26: return "attention v_full (one CTA)";
         case 27: return "attention v_full"; case 28: return "attention s_ready"; case 29: return "attention s_free";

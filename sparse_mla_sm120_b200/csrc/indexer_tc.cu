@@ -60,7 +60,7 @@ constexpr uint32_t LX_SMEM_NEED = LX_MISC_OFF + 16 + 1024;
 constexpr uint32_t LX_SMEM = LX_SMEM_NEED > 118 * 1024 ? LX_SMEM_NEED : 118 * 1024;
 
 // give-up codes reported through status[0]
-enum { WL_WEIGHTS = 11, WL_DFULL = 12, WL_QEMPTY = 13, WL_KEMPTY = 14, WL_QFULL = 15, WL_KFULL = 16, WL_DEMPTY = 17 };
+enum { WL_QFULL = 11, WL_KFULL = 12, WL_KEMPTY = 13, WL_DFULL = 14, WL_DEMPTY = 15, WL_QEMPTY = 16, WL_WEIGHTS = 17 };
 
 struct LogitsParams {
     const uint8_t* q; const uint8_t* k; const float* k_scale; const float* w;
