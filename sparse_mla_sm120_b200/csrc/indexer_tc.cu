@@ -26,6 +26,7 @@
 #include <cuda.h>
 
 #include "common.cuh"
+#include "logits_runs.cuh"
 #include "sm100_ptx.cuh"
 
 namespace smla {
@@ -344,20 +345,7 @@ int launch_mqa_logits_tc(const uint8_t* q, const uint8_t* k, const float* k_scal
     const int groups = (s_q + LX_QG - 1) / LX_QG;
     const int nsm = sms[dev < 64 ? dev : 0];
     const int tiles = (s_k + LX_KT - 1) / LX_KT;
-    // Query groups enough for eight items per SM: whole, the CTAs then finish together.  Fewer: the key tiles are cut into runs so that all
-    // CTAs get the same number of items in one to eight rounds, by what the longest share costs (an item pays about two tiles for its q
-    // and for filling and draining the pipeline): 16 tokens over 131072 keys in one run of 28 tiles per CTA instead of 512 of eight.
-    int chunks = 1;
-    if (groups < 8 * nsm) {
-        long long best = -1;
-        for (int r = 1; r <= 8; ++r) {
-            int c = r * nsm / groups;
-            if (c > (tiles + 7) / 8) c = (tiles + 7) / 8;
-            if (c < 1) c = 1;
-            const long long cost = (long long)((groups * c + nsm - 1) / nsm) * ((tiles + c - 1) / c + 2);
-            if (best < 0 || cost < best) { best = cost; chunks = c; }
-        }
-    }
+    const int chunks = logits_runs(groups, tiles, nsm);
     const int chunk_tiles = (tiles + chunks - 1) / chunks;
     const int items = groups * ((tiles + chunk_tiles - 1) / chunk_tiles);
     LogitsParams p{q, k, k_scale, weights, ks, ke, logits, status, s_q, num_heads, s_k, logits_stride, chunk_tiles};

@@ -282,3 +282,22 @@ def test_device_status_report_and_clear():
     with pytest.raises(_lib.SmlaError, match="indexer k_empty"):
         check_status(dev)
     check_status(dev)       # cleared by the report
+
+
+@pytest.mark.parametrize("h", [32, 64])
+@pytest.mark.parametrize("s_q,s_k", [(40, 40000), (13, 3001)])
+def test_mqa_logits_runs_of_any_length(s_q, s_k, h):
+    """Key tiles cut into runs of 23 tiles of which the last has 14 (40 tokens: ten groups, 313 tiles), and into three of eight; windows
+    that begin and end inside them."""
+    from sparse_mla_sm120_b200 import indexer
+    from sparse_mla_sm120_b200._runtime import check_status
+    q, k, k_scale, w, ks, ke = _indexer_case(17, s_q, h, s_k)
+    ks[1::3] = s_k // 3
+    ke[2::4] = s_k // 2 + 1
+    ke[s_q // 2] = 0
+    ref = orc.mqa_logits_ref(q, k, k_scale, w, ks, ke)
+    got = indexer.fp8_mqa_logits(q.to(DEV), k.to(DEV), k_scale.to(DEV), w.to(DEV), ks.to(DEV), ke.to(DEV)).cpu()
+    check_status(torch.device(DEV))
+    assert torch.equal(torch.isinf(got), torch.isinf(ref)), "range mask differs"
+    fin = ~torch.isinf(ref)
+    assert float((got[fin] - ref[fin]).abs().max()) <= 1e-4 * float(ref[fin].abs().max())
