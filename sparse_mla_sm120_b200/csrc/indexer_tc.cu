@@ -79,9 +79,13 @@ __global__ void __launch_bounds__(LX_THREADS, 1) mqa_logits_tc_kernel(const Logi
     const uint32_t base = (raw + 1023u) & ~1023u;
     uint8_t* sm = smem_raw + (base - raw);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(sm + LX_MISC_OFF + 4);
-    const uint32_t abort_addr = base + LX_MISC_OFF + 4;
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(sm + LX_MISC_OFF);
     auto bar = [&](int i) -> uint32_t { return base + LX_BAR_OFF + 8u * i; };
+    // 64 heads: us for 4096 tokens x 65536 keys 2334, 2373 with mbar_wait_lean; for 1024 608 and 620.  32 heads, whose tiles take half as
+    // long and whose warps come to a wait twice as often: 386 for 4096 x 16384 with mbar_wait_hot, 361 so; 438 and 419 for 1024 x 65536.
+    auto wait = [&](uint32_t b, uint32_t parity, int code) -> bool {
+        return HEADS == 64 ? mbar_wait_hot(b, parity, abort_flag, code) : mbar_wait_lean(b, parity, base + LX_MISC_OFF + 4, code);
+    };
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     constexpr int H = HEADS, N = LX_QG * H;
 
@@ -177,7 +181,7 @@ __global__ void __launch_bounds__(LX_THREADS, 1) mqa_logits_tc_kernel(const Logi
             for (int t = t0; t < t1; ++t, ++it, key += LX_KT) {
                 const uint32_t b = it & 1u;
                 const float sc = key < p.s_k ? ld_in(p.k_scale + key) : 0.f;
-                ok = mbar_wait_lean(bar(LXB_DFULL + b), (it >> 1) & 1u, abort_addr, WL_DFULL);
+                ok = wait(bar(LXB_DFULL + b), (it >> 1) & 1u, WL_DFULL);
                 if (!ok) break;
                 tc_fence_after();
                 uint64_t a01 = 0ull, a23 = 0ull;
@@ -233,7 +237,7 @@ __global__ void __launch_bounds__(LX_THREADS, 1) mqa_logits_tc_kernel(const Logi
             for (int t = t0; t < t1 && ok; ++t, ++it) {
                 const uint32_t st = it % LX_KSTAGE;
                 if (it >= LX_KSTAGE) {
-                    ok = mbar_wait_lean(bar(LXB_KEMPTY + st), ((it / LX_KSTAGE) - 1) & 1u, abort_addr, WL_KEMPTY);
+                    ok = wait(bar(LXB_KEMPTY + st), ((it / LX_KSTAGE) - 1) & 1u, WL_KEMPTY);
                     if (!ok) break;
                 }
                 if (elect_one()) {
@@ -253,15 +257,15 @@ __global__ void __launch_bounds__(LX_THREADS, 1) mqa_logits_tc_kernel(const Logi
             int g, t0, t1, j0, j1;
             item_range(w, g, t0, t1, j0, j1);
             if (t1 <= t0) continue;
-            ok = mbar_wait_lean(bar(LXB_QFULL), qn & 1u, abort_addr, WL_QFULL);
+            ok = wait(bar(LXB_QFULL), qn & 1u, WL_QFULL);
             if (!ok) break;
             ++qn;
             for (int t = t0; t < t1; ++t, ++it) {
                 const uint32_t st = it % LX_KSTAGE, b = it & 1u;
-                ok = mbar_wait_lean(bar(LXB_KFULL + st), (it / LX_KSTAGE) & 1u, abort_addr, WL_KFULL);
+                ok = wait(bar(LXB_KFULL + st), (it / LX_KSTAGE) & 1u, WL_KFULL);
                 if (!ok) break;
                 if (it >= 2) {
-                    ok = mbar_wait_lean(bar(LXB_DEMPTY + b), ((it >> 1) - 1) & 1u, abort_addr, WL_DEMPTY);
+                    ok = wait(bar(LXB_DEMPTY + b), ((it >> 1) - 1) & 1u, WL_DEMPTY);
                     if (!ok) break;
                 }
                 tc_fence_after();

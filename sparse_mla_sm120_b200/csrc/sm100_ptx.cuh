@@ -81,6 +81,18 @@ __device__ __forceinline__ bool mbar_wait_lean(uint32_t bar, uint32_t parity, ui
     }
 }
 
+// The same, but every lane leaves the loop by itself, the warp votes once, and the loop looks at the abort flag: faster in the
+// indexer's logits of 64 heads, whose code is small (the times stand there).
+__device__ __forceinline__ bool mbar_wait_hot(uint32_t bar, uint32_t parity, volatile int* abort, int code) {
+    uint32_t ok = 0;
+    for (uint32_t i = 0; i < WAIT_POLLS; ++i) {
+        if (mbar_try_wait(bar, parity, WAIT_HINT_NS)) { ok = 1; break; }
+        if ((i & 255u) == 255u && *abort != 0) break;
+    }
+    if (!ok) atomicCAS(const_cast<int*>(abort), 0, code);
+    return __all_sync(0xffffffffu, ok != 0);
+}
+
 // True in one lane of the (converged) warp, the same one every time.  Instructions whose operands live in uniform
 // registers (tcgen05.mma and its commit, bulk copies) are issued under this predicate: the compiler then knows that
 // one lane runs them and keeps descriptors and addresses in uniform registers.  Under `lane == 0` it does not, and every
