@@ -75,3 +75,35 @@ def test_entries_without_a_row_leave_no_trace():
     moved = dict(case, indices=torch.cat([case["indices"][:, 192:], case["indices"][:, :192]], dim=1).contiguous())
     out, mx, lse = _prefill(moved, TC)              # whole tiles' halves without an entry lead
     _check_hard(out, lse, ref_out, ref_lse, TC, moved)
+
+
+@pytest.mark.parametrize("heads", [65, 97, 127])
+@pytest.mark.parametrize("k", [2, 8])
+def test_head_halves_of_equal_partitions(heads, k):
+    """A CTA has heads without a query and the second fewer than the first; partitions of whole tiles and of two blocks."""
+    import ctypes
+    from sparse_mla_sm120_b200 import _lib, _runtime
+    t, topk = 3, 1024
+    case = make_case(29, t, heads, topk, 40, invalid_tail=0.1)
+    ref_out, ref_lse = oracle_attn(case)
+    dev = torch.device("cuda:0")
+    q, kv, idx = case["q"].to(dev), case["packed"].to(dev), case["indices"].to(dev)
+    o, l = torch.empty(k * t, heads, 512, dtype=torch.half, device=dev), torch.empty(k * t, heads, device=dev)
+    out, lse = torch.empty(t, heads, 512, dtype=torch.bfloat16, device=dev), torch.empty(t, heads, device=dev)
+    assert _lib.load().smla_decode_uniform(q.data_ptr(), kv.data_ptr(), idx.data_ptr(), o.data_ptr(), l.data_ptr(), out.data_ptr(), lse.data_ptr(), t, heads,
+                                           topk, ctypes.c_float(case["sm_scale"]), 64, 64 * 656, k, None, TC, _runtime.status_pointer(0),
+                                           torch.cuda.current_stream().cuda_stream) == 0
+    torch.cuda.synchronize()
+    _runtime.check_status(dev)
+    _check_hard(out.cpu(), lse.cpu(), ref_out, ref_lse, TC, case)
+
+
+@pytest.mark.parametrize("heads", [65, 97, 127])
+def test_head_halves_of_several_requests_per_pair(heads):
+    """More requests than pairs of SMs, of one to three tiles: the next request's q goes through tensor memory."""
+    case = make_case(37, 170, heads, 320, 24, invalid_tail=0.0)
+    g = torch.Generator().manual_seed(heads)
+    tl = torch.randint(0, 321, (170,), generator=g, dtype=torch.int32)
+    ref_out, ref_lse = oracle_attn(case, topk_length=tl)
+    out, mx, lse = _prefill(case, TC, topk_length=tl)
+    _check_hard(out, lse, ref_out, ref_lse, TC, case, topk_length=tl)

@@ -48,7 +48,7 @@ def test_small_blocks_keep_their_precision(heads, pattern):
     magnitude, held to the emulation's error on the same inputs as test_scale_spread_rows does (there at 128 heads, which
     run on the pair kernel).  steady: small in every row; late: rows of a later tile are the first with a large block, so
     what was accumulated for it has to come down; mixed: small in two rows of three."""
-    case = make_case(17, 80, heads, 640, 32, q_std=2.0, invalid_tail=0.0)     # (fewer whole requests run on the pair kernel)
+    case = make_case(17, 80, heads, 640, 32, q_std=2.0, invalid_tail=0.0)     # (fewer whole requests run on attn_duo_kernel)
     scales = case["packed"].view(-1, 656)[:, 512:528].view(torch.float32)
     if pattern == "steady":
         scales[:, 1] *= 2.0 ** -6
