@@ -42,9 +42,9 @@ NSETS = 8   # rotating (q, indices) sets so that consecutive steps gather differ
 SM_SCALE = D_QK ** -0.5
 WORKLOAD = ("V3.2-shape sparse-MLA decode: b=64/GPU, s_q=1, h_q=128, topk=2048, d_qk=576, d_v=512, "
             "KV len U[4096,32768], paged block 64, packed FP8 656 B rows")
-# DRAM bytes of one launch of the attention kernel on this workload's shape (dram__bytes_read.sum + dram__bytes_write.sum of a capture
-# of `--case decode`).
-NCU_TRAFFIC_BYTES = 85_335_040 + 2_774_784
+# DRAM bytes of one launch of the attention kernel over this workload's pool and input sets (dram__bytes_read.sum + dram__bytes_write.sum,
+# the second of three launches captured; outputs stay in L2).
+NCU_TRAFFIC_BYTES = 108_465_920 + 283_904
 CPU_SAMPLE_REQUESTS = 64   # requests of one step that the CPU legs compute: the whole step (about 0.13 s on 16 host threads)
 
 

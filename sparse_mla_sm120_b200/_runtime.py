@@ -122,8 +122,9 @@ def pick_num_sm_parts_fp32(num_tokens: int, num_heads: int, sms: int) -> int:
 
 
 # attn_exact_kernel (exact numerics over MODEL1, aligned caches): microseconds of a partition's fixed part (q, epilogue),
-# of a 128-token tile, and of what a split adds (scheduler and combine launches, partial records).  Estimates, not fitted: a tile
-# takes about 11000 cycles (5.6 us) in the kernel; what the rule needs is their proportion.
+# of a 128-token tile, and of what a split adds (scheduler and combine launches, partial records).  Estimates, not fitted, from before
+# the launches ran under one another (a split adds less since): a tile takes about 11000 cycles (5.6 us) in the kernel; what the
+# rule needs is their proportion.
 _EXACT_US_FIXED, _EXACT_US_TILE, _EXACT_US_SPLIT = 6.0, 4.0, 9.0
 
 
@@ -199,7 +200,7 @@ def pick_split(num_tokens: int, sms: int, blocks_per_token: Optional[int] = None
 
 # attn_tile_kernel (up to 64 heads over one linear array of rows): microseconds of a partition's fixed part, of a 128-token
 # tile, and of what a split adds: a part that grows with the pieces of a request, and the records that are written and
-# read back.  Fitted to 1 to 64 requests of top-k 512, 1024 and 2048 in up to 16 equal partitions each, 16 and 64 heads (48
+# read back.  Fitted, before the kernel's last 15 %, to 1 to 64 requests of top-k 512, 1024 and 2048 in up to 16 equal partitions each, 16 and 64 heads (48
 # requests of top-k 2048 at 16 heads: 40 us whole, 28.6 us in two partitions each; one: 38.5, 25.3, 18.5, 17.9 and 19.9 us in
 # 1, 2, 4, 8 and 16); the cut that it names is the fastest measured one or within a microsecond of it.
 def _tile_us(num_tokens: int, num_heads: int, blocks: int, k: int) -> float:
@@ -237,12 +238,17 @@ def _duo_us(num_tokens: int, blocks: int, k: int, max_pairs: int) -> float:
 
 def pick_split_duo(num_tokens: int, sms: int, blocks_per_token: int, uniform: bool) -> Tuple[int, int]:
     """(partitions, fixed overhead) where whole requests and equal partitions run on attn_duo_kernel and partitions of the
-    scheduler on the pair kernel.  Equal partitions leave fp16 records, so only calls that pick_split cuts equally are cut so here (lists
-    of 8 blocks and more that have a suitable divisor, up to 37 requests), if into another number of pieces.  Others would
-    be faster too (us whole / cut, rows in HBM: 4 requests of 640 entries 16.3 / 14.2, 10 of 896 19.1 / 17.1, 35 of 1024 23.0 / 22.5), but they are
-    computed without such a rounding: their results are whole requests' or go through fp32 records.  Ragged requests are left whole where the scheduler and combine launches and the partitions that
-    straddle two requests cost more than the longest request: lists of up to 16 blocks, and from half as many requests on as a
-    list has blocks (us whole / cut, rows in HBM: 16 requests of up to 1024 entries 21.7 / 28.1; 8 of up to 1536 27.1 / 26.8, 13: 27.6 /
+    scheduler on the pair kernel.
+
+    Equal partitions leave fp16 records, so only calls that pick_split cuts equally are cut so here (lists of 8 blocks and more that
+    have a suitable divisor, up to 37 requests), if into another number of pieces.  Others would be faster too (us whole / cut,
+    rows in HBM: 4 requests of 640 entries 16.3 / 14.2, 10 of 896 19.1 / 17.1, 35 of 1024 23.0 / 22.5), but their results are whole
+    requests' or go through fp32 records, without such a rounding.
+
+    Ragged requests are left whole where the scheduler and combine launches and the partitions that straddle two requests cost
+    more than the longest request: lists of up to 16 blocks (us before, with the scheduler and the pair kernel / whole, graph of steps:
+    1 request of up to 512 entries 20.6 / 12.9, of up to 1024 22.2 / 15.0, 8: 25.0 / 19.9, 30: 34.0 / 20.2), and from half as
+    many requests on as a list has blocks (us whole / cut, rows in HBM: 16 requests of up to 1024 entries 21.7 / 28.1; 8 of up to 1536 27.1 / 26.8, 13: 27.6 /
     29.7; 13 of up to 2048 33.6 / 30.7, 16: 33.5 / 34.1, 20: 34.1 / 39.6; 24 of up to 4096 59.4 / 54.6, 30: 60.1 / 60.4).  Otherwise the
     general rule cuts them into partitions of four blocks, as many as there are pairs of SMs at most; partitions of eight blocks
     take longer now that launches run under one another (4 requests of up to 2048 25.1 in 32, 27.2 in 16; 13: 30.7 in 74, 34.0 in

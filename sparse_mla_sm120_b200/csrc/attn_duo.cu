@@ -14,12 +14,13 @@
 // tokens (the largest of their 4 x 8), in place and only the 128-byte pieces that have another one.
 // Numerics are those of attn_pair.cu (the same groups, the same weights), with K exact instead of shifted.
 //
-// What bounds it (clock64 in an instrumented copy, 2048 entries, 1.9 GHz): a tile takes 2650 cycles where the rows lie in L2, the pair
-// kernel 4000 (first version; the cuts in instructions named below came after).  Of these the copies alone would need 1750 (TMA gather4 moves a row's 128 bytes in 3 cycles, whatever the order), the
-// MMAs 1150; what it waits for are instructions: 9500 per tile and CTA on 32 warps, issue slots 65 % busy, an instruction of a
-// warp every 8 to 10 cycles.  Hence the manner of the code: loops instead of unrolled copies, one place in the code for what is done
-// at several times, walkers and waits of few instructions (at 104 KB of code the instruction cache hit 64 % and the kernel was
-// slower than the pair kernel, at 70 KB 96 %), and shifts of V spread over eight warps, since LOP3 and PRMT go out every other cycle only.
+// What bounds it is the issue of instructions (ncu, 740 tokens of 2048 entries, rows in L2): 8650 per tile and CTA on 32 warps, request
+// switches included, issue slots 72 % busy, the ALU pipe 61 %, the tensor pipe 38 %.  The copies of a tile alone would need 1750 cycles
+// (TMA gather4 moves a row's 128 bytes in 3 cycles, whatever the order), the MMAs 1150; the first version of the kernel, of 9500
+// instructions, took 2650 (clock64), the pair kernel 4000.  Hence the manner of the code: loops instead of unrolled copies, one place in
+// the code for what is done at several times, walkers and waits of few instructions (at 104 KB of code the instruction cache hit 64 %
+// and the kernel was slower than the pair kernel, now 96 %), and shifts of V spread over eight warps, since LOP3 and PRMT go out every
+// other cycle only.
 // A long run is held at 1640 MHz by the power limit (the pair kernel: 1905 MHz), which takes back some of the gain:
 // 4096 tokens of top-k 2048 2230 -> 1815 us in a row (the first version, of 9500 instructions per tile: 1930, and 1620 alone where the
 // pair kernel takes 2170); 64 requests 49.2 -> 43.4 us, two tokens of 64 requests 96.8 -> 83.8 us.

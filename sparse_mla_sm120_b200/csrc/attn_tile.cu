@@ -6,9 +6,10 @@
 // tokens of top-k 1024 at 64 heads: 395 us there, 163 us here.  At 128 heads two of these CTAs would gather every row twice: 2400 us for
 // 4096 tokens of top-k 2048, against 1815 us in attn_duo_kernel.
 //
-// What bounds it (clock64 at 64 heads, 1.9 GHz, before the copies were issued from indices in shared memory and the MMAs from loops, which
-// took 48 requests from 32.8 to 30.7 us and the ragged prompt from 175 to 165): a tile of 128 tokens takes 4300 cycles, half of the way of a tile from the load
-// of its rows (2000 cycles: the gather delivers 35 bytes per cycle and SM) over its scores (2100, with the hand-overs) and its
+// What bounds it: no unit is near its limit (ncu, 592 tokens of 2048 entries at 64 heads, rows in HBM: issue slots 43 %, ALU pipe 32 %,
+// tensor pipe 22 %, 3.1 TB/s); a tile waits for its own way through the SM.  Its parts (clock64 at 64 heads, 1.9 GHz, before the copies
+// were issued from indices in shared memory and the MMAs from loops, which took 48 requests from 32.8 to 30.7 us and the ragged
+// prompt from 175 to 165): a tile of 128 tokens takes 4300 cycles, half of the way of a tile from the load of its rows (2000 cycles: the gather delivers 35 bytes per cycle and SM) over its scores (2100, with the hand-overs) and its
 // weights (2700) to P.V (1300), because two tiles are all that shared memory holds.  A request costs another 15000 cycles for its
 // q and its epilogue, which the softmax warps do in between.  Tried without gain: sixteen softmax warps (2485 us where
 // eight take 2400), q and epilogue on four warps of their own (169 us for the

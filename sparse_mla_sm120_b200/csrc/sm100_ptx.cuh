@@ -37,7 +37,7 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity, uin
 
 // Warp-wide wait for the phase with the given parity.  Lane 0 polls (32 lanes polling one
 // mbarrier only add shared-memory traffic), the warp reconverges on the result.  The wait gives
-// up after a bounded number of polls (about half a second) or as soon as another thread of the
+// up after a bounded number of polls (2^22 of 4 us, some 17 s) or as soon as another thread of the
 // CTA has given up (*abort != 0); it then returns false and records `code` in *abort so that the
 // kernel can report where it stopped.  Must be called by all 32 lanes.
 constexpr uint32_t WAIT_POLLS = 1u << 22;
@@ -61,8 +61,8 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
 // The wait of the critical paths, in as few instructions as it can have (the roles of these kernels together are larger than the
 // instruction caches): every lane blocks in mbarrier.try_wait itself, nearly always the first poll, which the hardware
 // suspends until the phase completes or its own time limit has passed, is the only one.  The warp decides by votes, so nothing here
-// diverges.  Gives up after LEAN_POLLS + 1 polls; `code` then goes to the abort flag (given by its shared-memory address) unless there
-// is one already: the first wait to give up is on record, not one that follows from it.
+// diverges.  Gives up after LEAN_POLLS + 1 polls (7848 cycles each in every warp, 4.2 s in all); `code` then goes to the abort flag (given
+// by its shared-memory address) unless there is one already: the first wait to give up is on record, not one that follows from it.
 // It does not look at the flag while it waits, as mbar_wait does: that costs instructions at every wait (two tokens of 64 requests,
 // attn_duo_kernel: 80.5 us without, 82.6 with a look every 256 polls; 4096 tokens 4 % more) and gains little, for the waits that hang on
 // the stuck one begin within microseconds of it and so end with it, and a warp that has given up waits for nothing more.
